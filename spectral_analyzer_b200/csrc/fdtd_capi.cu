@@ -186,6 +186,14 @@ struct AcousticFDTDState {
     unsigned wait_us = kWaitUs;
     FusedCache* fcache = nullptr;    // TMA descriptors of the fields (fused step)
 
+    // many steps per launch of a small open room (fdtd_resident.cu)
+    bool res_planned = false;
+    ResPlan res;
+    void* res_x = nullptr;           // exchange buffer between bricks
+    unsigned res_epoch = 0;          // steps taken through it
+    float* res_taps = nullptr;       // the receivers' taps of up to kCheckPeriod steps
+    size_t res_taps_n = 0;
+
     long long launches = 0;          // kernels launched by this handle
 
     bool prof_on = false;
@@ -589,6 +597,31 @@ int flush_record(AcousticFDTDState* st)
     return FDTD_OK;
 }
 
+// After a step: the stability check every 256 steps (acoustic_fdtd.cpp:1284-1287).
+int step_check(AcousticFDTDState* st, bool sync_check)
+{
+    cudaStream_t s = st->stream;
+    if ((st->step_count & (kCheckPeriod - 1)) != 0) return FDTD_OK;
+    int phase = st->stab_phase;
+    st->stab_phase = (phase + 1) % kCheckStride;
+    if (sync_check) CK(cudaMemsetAsync(st->d_status + kStatusCell, 0xFF, sizeof(unsigned), s));
+    CK(launch_check(st->g, st->P(), st->N, phase, st->d_status, st->step_count, s));
+    ++st->launches;
+    if (sync_check) {
+        CK(cudaMemcpyAsync(st->h_status, st->d_status, kStatusWords * sizeof(unsigned),
+                           cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (int rc2 = check_timeout(st)) return rc2;
+        unsigned bad = st->h_status[kStatusCell];
+        if (bad != 0xFFFFFFFFu) {
+            report_unstable_cell(st, bad);
+            CK(cudaMemsetAsync(st->d_status + kStatusLatch, 0xFF, sizeof(unsigned), s));
+            return FDTD_ERR_UNSTABLE;
+        }
+    }
+    return FDTD_OK;
+}
+
 // One time step (acoustic_fdtd.cpp:1272-1290 loop body) plus the engine's
 // point-source deposit before it and receiver record after it.
 // sync_check: stop and return FDTD_ERR_UNSTABLE at a failed check (fdtd_step);
@@ -769,27 +802,112 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
         ++st->trace_len;
     }
 
-    // stability check every 256 steps (acoustic_fdtd.cpp:1284-1287)
-    if ((st->step_count & (kCheckPeriod - 1)) == 0) {
-        int phase = st->stab_phase;
-        st->stab_phase = (phase + 1) % kCheckStride;
-        if (sync_check) CK(cudaMemsetAsync(st->d_status + kStatusCell, 0xFF, sizeof(unsigned), s));
-        CK(launch_check(st->g, st->P(), st->N, phase, st->d_status, st->step_count, s));
-        ++st->launches;
-        if (sync_check) {
-            CK(cudaMemcpyAsync(st->h_status, st->d_status, kStatusWords * sizeof(unsigned),
-                               cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            if (int rc2 = check_timeout(st)) return rc2;
-            unsigned bad = st->h_status[kStatusCell];
-            if (bad != 0xFFFFFFFFu) {
-                report_unstable_cell(st, bad);
-                CK(cudaMemsetAsync(st->d_status + kStatusLatch, 0xFF, sizeof(unsigned), s));
-                return FDTD_ERR_UNSTABLE;
-            }
-        }
+    return step_check(st, sync_check);
+}
+
+// How many of the next `left` steps one launch of the resident kernel takes: an
+// open room that fits the chip, up to the next stability check; 0 = none
+// (another kernel was asked for, per-step profiling, the load-hold hook, a stream
+// being captured, more receivers than the kernel records, or no memory for its
+// buffers).
+int resident_window(AcousticFDTDState* st, int left)
+{
+    if (st->kernel_mode == 1 || st->prof_on || st->hold_plane != kNoPlane || !fused_eligible(st)) return 0;
+    if (!st->res_planned) {
+        int sms = 0, coop = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, st->device);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, st->device);
+        if (coop) st->res = resident_plan(st->g, sms);
+        st->res_planned = true;
     }
-    return FDTD_OK;
+    if (!st->res.ok) return 0;
+    if (st->ps_n > 0 && st->ps.n > 0 && (st->ps.n != 1 || st->ps.divisor != 0)) return 0;
+    const bool record = st->n_rec > 0 && st->trace_len < st->trace_cap;
+    const size_t taps = record ? (size_t)8 * st->n_rec : 0;
+    if (taps > (size_t)resident_max_taps()) return 0;
+    // a captured launch would carry the same step numbers at every replay
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return 0;
+    // a single step gains nothing from staying on chip: loading and storing the
+    // bricks costs about what the march does (64^3: 15.5 against 15.3 us per call)
+    const int m = std::min(left, kCheckPeriod - (st->step_count & (kCheckPeriod - 1)));
+    if (m < 2) return 0;
+    if (!st->res_x) {
+        if (cudaMalloc(&st->res_x, st->res.xbytes) != cudaSuccess) {
+            cudaGetLastError();
+            st->res_x = nullptr;
+            st->res.ok = false;
+            return 0;
+        }
+        if (cudaMemsetAsync(st->res_x, 0, st->res.xbytes, st->stream) != cudaSuccess) return 0;
+    }
+    if (taps * kCheckPeriod > st->res_taps_n) {
+        cudaStreamSynchronize(st->stream);
+        cudaFree(st->res_taps);
+        st->res_taps = nullptr;
+        st->res_taps_n = 0;
+        if (cudaMalloc(&st->res_taps, taps * kCheckPeriod * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        st->res_taps_n = taps * kCheckPeriod;
+    }
+    return m;
+}
+
+// `m` steps (resident_window) in one launch: what m calls of one_step leave.
+int resident_steps(AcousticFDTDState* st, int m, bool sync_check)
+{
+    cudaStream_t s = st->stream;
+    if (int rc = flush_record(st)) return rc;
+    if (st->ext_pending) clear_ext_host(st);   // consumed with no plate
+    if (!st->v[st->cv ^ 1][0])
+        if (int rc = alloc_second_velocity_set(st)) return rc;
+    FusedArgs a{st->g, st->cf, st->tb, st->P(), st->Pn(),
+                {st->V(0), st->V(1), st->V(2)},
+                {st->v[st->cv ^ 1][0], st->v[st->cv ^ 1][1], st->v[st->cv ^ 1][2]},
+                st->d_status};
+    a.wait_us = st->wait_us;
+    const int n0 = st->step_count;
+    const int dep_from = st->ps_done_step == n0 ? 1 : 0;
+    const int dep_to = st->ps.n > 0 ? std::min(m, st->ps_n - n0) : 0;
+    if (dep_to > dep_from) {
+        const long long c = st->ps.idx[0], t = c / st->g.sz;
+        a.dep_sig = st->d_ps_sig;
+        a.dep_step = n0;
+        a.dep_i = (int)(t / st->Ny);
+        a.dep_j = (int)(t % st->Ny);
+        a.dep_k = (int)(c % st->g.sz);
+    }
+    const int rows = st->n_rec > 0 ? std::min(m, st->trace_cap - st->trace_len) : 0;
+    CK(launch_resident(a, st->res, m, st->res_x, st->res_epoch, dep_from, dep_to, st->d_rec_idx,
+                       rows > 0 ? 8 * st->n_rec : 0, rows, st->res_taps, s));
+    ++st->launches;
+    if (rows > 0) {
+        CK(launch_tap_rows(st->res_taps, st->d_rec_w, rows, st->n_rec, st->d_trace + (size_t)st->trace_len * st->n_rec, s));
+        ++st->launches;
+        st->trace_len += rows;
+    }
+    st->res_epoch += (unsigned)m;
+    if (dep_to > 0) st->ps_done_step = n0 + dep_to - 1;
+    st->cur ^= 1;
+    st->cv ^= 1;
+    st->step_count += m;
+    return step_check(st, sync_check);
+}
+
+// n_steps steps, several per launch where the room allows it; the last step's
+// receivers are recorded before it returns.
+int run_steps(AcousticFDTDState* st, int n_steps, bool sync_check)
+{
+    int rc = FDTD_OK;
+    for (int s = 0; s < n_steps && rc == FDTD_OK;) {
+        const int m = resident_window(st, n_steps - s);
+        rc = m > 0 ? resident_steps(st, m, sync_check) : one_step(st, sync_check, true);
+        s += m > 0 ? m : 1;
+    }
+    const int rc_rec = flush_record(st);
+    return rc != FDTD_OK ? rc : rc_rec;
 }
 
 void free_state(AcousticFDTDState* st)
@@ -822,6 +940,8 @@ void free_state(AcousticFDTDState* st)
     cudaFreeHost(st->h_sidx); cudaFreeHost(st->h_sw); cudaFreeHost(st->h_sout); cudaFreeHost(st->h_sout_map);
     for (cudaEvent_t e : st->prof.ev) cudaEventDestroy(e);
     fused_cache_destroy(st->fcache);
+    cudaFree(st->res_x);
+    cudaFree(st->res_taps);
     if (st->own_stream) cudaStreamDestroy(st->own_stream);
     if (d >= 0 && d != st->device) cudaSetDevice(d);
     delete st;
@@ -1213,10 +1333,7 @@ int fdtd_step(AcousticFDTDState* st, int n_steps)
     if (!st) return FDTD_ERR_NULL;
     if (n_steps <= 0) return FDTD_OK;
     if (dev_guard(st)) return FDTD_ERR_CUDA;
-    int rc = FDTD_OK;
-    for (int s = 0; s < n_steps && rc == FDTD_OK; ++s) rc = one_step(st, true, true);
-    const int rc_rec = flush_record(st);
-    return rc != FDTD_OK ? rc : rc_rec;
+    return run_steps(st, n_steps, true);
 }
 
 int fdtd_get_step_count(const AcousticFDTDState* st) { return st ? st->step_count : 0; }
@@ -1488,10 +1605,7 @@ int fdtd_b200_step_async(AcousticFDTDState* st, int n_steps)
     if (!st) return FDTD_ERR_NULL;
     if (n_steps <= 0) return FDTD_OK;
     if (dev_guard(st)) return FDTD_ERR_CUDA;
-    int rc = FDTD_OK;
-    for (int s = 0; s < n_steps && rc == FDTD_OK; ++s) rc = one_step(st, false, true);
-    const int rc_rec = flush_record(st);
-    return rc != FDTD_OK ? rc : rc_rec;
+    return run_steps(st, n_steps, false);
 }
 
 int fdtd_b200_synchronize(AcousticFDTDState* st)

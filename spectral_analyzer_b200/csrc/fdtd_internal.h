@@ -258,6 +258,27 @@ int fused_kernel_launches_per_step();
 cudaError_t fused_maps(FusedCache* c, const Grid& g, const float* p, const float* const* v,
                        CUtensorMap out[4], int shape = 0);
 
+// ---- many steps of a small room in one launch (fdtd_resident.cu) ----
+// How a room is cut into bricks, one per SM: planes, rows and quads (of four
+// cells along k) of a brick, bricks per axis, planes per thread, and the bytes
+// of the exchange buffer between bricks (zeroed by its owner once).
+struct ResPlan {
+    bool ok = false;
+    int L = 0, bi = 0, bj = 0, q = 0;
+    int nbi = 0, nbj = 0, nbk = 0;
+    size_t xbytes = 0;
+};
+ResPlan resident_plan(const Grid& g, int sms);   // ok = false: the room does not fit
+int resident_max_taps();
+// `steps` steps from a.p, a.vin to a.pn, a.vout.  `epoch` grows by `steps` from
+// launch to launch of one exchange buffer.  The source (a.dep_*) adds sample
+// a.dep_step + s before step s for dep_from <= s < dep_to.  After step s <
+// rec_steps the pressure at tap t is written to tap_out[s * n_taps + t].
+cudaError_t launch_resident(const FusedArgs& a, const ResPlan& pl, int steps, void* xbuf, unsigned epoch, int dep_from,
+                            int dep_to, const long long* tap_idx, int n_taps, int rec_steps, float* tap_out,
+                            cudaStream_t s);
+cudaError_t launch_tap_rows(const float* tap, const float* w, int rows, int n_rec, float* out, cudaStream_t s);
+
 // ---- batched step (continuous batching of independent rooms) ----
 // Device-resident descriptor of one batch member.  Parity 0 is the member's
 // state when it joined the batch; a step taken at parity q reads p[q], v[q]
