@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -88,7 +89,24 @@ cudaError_t upload(T** d, const std::vector<T>& h)
     return cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
 }
 
+// n values, the array padded with zeros to `room`
+template <class T>
+cudaError_t upload(T** d, const T* h, size_t n, size_t room)
+{
+    if (*d) cudaFree(*d);
+    *d = nullptr;
+    cudaError_t e = cudaMalloc(d, room * sizeof(T));
+    if (e == cudaSuccess && n > 0) e = cudaMemcpy(*d, h, n * sizeof(T), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && room > n) e = cudaMemset(*d + n, 0, (room - n) * sizeof(T));
+    return e;
+}
+
 // ---------------------------------------------------------------- kernels
+__global__ void k_amr_fill(float* p, size_t n, float value)
+{
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) p[q] = value;
+}
+
 struct PlateDev {
     const float* w;      // current displacement
     const float* wp;     // previous
@@ -97,56 +115,179 @@ struct PlateDev {
     float dt;
 };
 
+// The step's kernels are launched with programmatic stream serialisation: a
+// kernel's blocks start while the one before drains, read what never changes
+// during a window (topology, coefficients) and only then wait for its results.
+// The dependents are released after the wait, so a kernel that has started
+// knows that everything before its predecessor is complete.
+__device__ __forceinline__ void wait_previous()
+{
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+constexpr int kOrigin = INT_MIN;   // stencil offset of an unused slot: it reads cell 0
+
+// Gradient-order-8 stencils.  A grid repeats few of them (a uniform region has
+// one set of cell offsets and one row of weights per axis and position), so a
+// face holds the numbers of its offset row and weight row (16 bits each)
+// instead of eight cells and eight weights: 8 bytes per face to read in place
+// of 64, and the rows come from L1.  Grids with more than 65536 rows of either
+// kind keep the rows themselves, slot by slot ([k][face], coalesced).
+struct Stencils {
+    const unsigned* row = nullptr;    // per face: offset row | weight row << 16 (null: full form)
+    const int4* off = nullptr;        // [rows][2]: cell minus the face's negative cell, or kOrigin
+    const float4* wgt = nullptr;      // [rows][2]
+    const int* cell = nullptr;        // full form: [8][n_faces]
+    const float* coef = nullptr;
+};
+
 // Velocity of every face; plate faces take the plate velocity instead
 // (the reference overwrites them after the update, acoustic_amr.cpp:1050-1072).
+// Order 2: four faces per thread, so that the topology comes in 16-byte loads.
+// Both kernels are bound by L2 (a step of 72^3 cells reads 20 MB) and by the gap
+// between dependent kernels.  Per step, velocity and pressure together, before
+// and now: 72^3 cells in order 8 33.1 -> 10.6 us (rows of cells and weights read
+// by scalar loads 32 bytes apart, face lists by CSR rows), 237k cells on two
+// levels in order 2 12.4 -> 6.5 us.
 template <int ORDER>
-__global__ void k_amr_velocity(int n_faces, const float* __restrict__ p, float* __restrict__ v,
-                               const float* __restrict__ vdamp, const float* __restrict__ inv_d,
-                               const int* __restrict__ fneg, const int* __restrict__ fpos,
-                               const int* __restrict__ s_cells, const float* __restrict__ s_coeff,
-                               const int* __restrict__ bc, const int* __restrict__ bc_flat, PlateDev pl,
-                               float dt_over_rho, const unsigned* __restrict__ status, unsigned step)
+__global__ void __launch_bounds__(256) k_amr_velocity(int n_faces, const float* __restrict__ p, float* __restrict__ v,
+                                                      const float* __restrict__ vdamp, const float* __restrict__ inv_d,
+                                                      const int* __restrict__ fneg, const int* __restrict__ fpos,
+                                                      Stencils st, const int* __restrict__ bc,
+                                                      const int* __restrict__ bc_flat, PlateDev pl, float dt_over_rho,
+                                                      const unsigned* __restrict__ status, unsigned step)
 {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_faces || *status < step) return;
-    const int code = bc ? bc[f] : -1;
-    if (code >= 0) {   // plate face: +v_plate above, -v_plate below
-        const int flat = bc_flat[code >> 1];
-        const float vp = fd(fs(pl.w[flat], pl.wp[flat]), pl.dt);
-        v[f] = (code & 1) ? -vp : vp;
-        return;
-    }
-    float grad;
-    if (ORDER == 8) {
-        grad = 0.0f;
-        const int* sc = s_cells + (size_t)f * kSW2;
-        const float* sw = s_coeff + (size_t)f * kSW2;
+    constexpr int N = ORDER == 2 ? 4 : 1;
+    const int f0 = (blockIdx.x * blockDim.x + threadIdx.x) * N;
+    const bool in = f0 < n_faces;
+    int code[N] = {}, neg[N] = {}, pos[N] = {};
+    float damp[N] = {}, inv[N] = {};
+    int off[8] = {};
+    float w[8] = {};
+    if (in) {
+        if constexpr (ORDER == 2) {   // the arrays are padded to a multiple of four
+            const int4 a = *reinterpret_cast<const int4*>(fneg + f0), b = *reinterpret_cast<const int4*>(fpos + f0);
+            const float4 d = *reinterpret_cast<const float4*>(vdamp + f0), e = *reinterpret_cast<const float4*>(inv_d + f0);
+            int4 c = make_int4(-1, -1, -1, -1);
+            if (bc) c = *reinterpret_cast<const int4*>(bc + f0);
+            neg[0] = a.x; neg[1] = a.y; neg[2] = a.z; neg[3] = a.w;
+            pos[0] = b.x; pos[1] = b.y; pos[2] = b.z; pos[3] = b.w;
+            damp[0] = d.x; damp[1] = d.y; damp[2] = d.z; damp[3] = d.w;
+            inv[0] = e.x; inv[1] = e.y; inv[2] = e.z; inv[3] = e.w;
+            code[0] = c.x; code[1] = c.y; code[2] = c.z; code[3] = c.w;
+        } else {
+            code[0] = bc ? bc[f0] : -1;
+            damp[0] = vdamp[f0];
+            if (st.row) {
+                const unsigned r = st.row[f0];
+                const int nb = fneg[f0];
+                const int4 a = st.off[2 * (r & 0xFFFFu)], b = st.off[2 * (r & 0xFFFFu) + 1];
+                const float4 c = st.wgt[2 * (r >> 16)], d = st.wgt[2 * (r >> 16) + 1];
+                const int o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                const float x[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
 #pragma unroll
-        for (int k = 0; k < kSW2; ++k) grad = fa(grad, fm(sw[k], p[sc[k]]));
-    } else {
-        grad = fm(fs(p[fpos[f]], p[fneg[f]]), inv_d[f]);
+                for (int k = 0; k < 8; ++k) {
+                    off[k] = o[k] == kOrigin ? 0 : nb + o[k];
+                    w[k] = x[k];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    off[k] = st.cell[(size_t)k * n_faces + f0];
+                    w[k] = st.coef[(size_t)k * n_faces + f0];
+                }
+            }
+        }
     }
-    v[f] = fm(fs(v[f], fm(dt_over_rho, grad)), vdamp[f]);
+    wait_previous();
+    if (!in || *status < step) return;
+    auto face = [&](int q) {
+        const int f = f0 + q;
+        if (code[q] >= 0) {   // plate face: +v_plate above, -v_plate below
+            const int flat = bc_flat[code[q] >> 1];
+            const float vp = fd(fs(pl.w[flat], pl.wp[flat]), pl.dt);
+            v[f] = (code[q] & 1) ? -vp : vp;
+            return;
+        }
+        float grad;
+        if (ORDER == 8) {
+            grad = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) grad = fa(grad, fm(w[k], p[off[k]]));
+        } else {
+            grad = fm(fs(p[pos[q]], p[neg[q]]), inv[q]);
+        }
+        v[f] = fm(fs(v[f], fm(dt_over_rho, grad)), damp[q]);
+    };
+    if constexpr (ORDER == 2) {
+        bool plain = f0 + 3 < n_faces;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) plain = plain && code[q] < 0;
+        if (plain) {
+            float4 x = *reinterpret_cast<const float4*>(v + f0);
+            float* const xv = &x.x;
+            float a[4], b[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { a[q] = p[neg[q]]; b[q] = p[pos[q]]; }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) xv[q] = fm(fs(xv[q], fm(dt_over_rho, fm(fs(b[q], a[q]), inv[q]))), damp[q]);
+            *reinterpret_cast<float4*>(v + f0) = x;
+            return;
+        }
+        for (int q = 0; q < 4; ++q)
+            if (f0 + q < n_faces) face(q);
+    } else {
+        face(0);
+    }
 }
 
 // Divergence and pressure of every cell, wall/plate cells zeroed, and the
 // divergence check of this step (non-finite anywhere; |p| > 2e3 on steps
-// whose count is a multiple of 256).
-__global__ void k_amr_pressure(int n_cells, float* __restrict__ p, const float* __restrict__ v,
-                               const float* __restrict__ pdamp, const float* __restrict__ psrc,
-                               const float* __restrict__ inv_den, const int* __restrict__ cstart,
-                               const int* __restrict__ cface, const float* __restrict__ cw,
-                               const unsigned char* __restrict__ zero, float bulk,
-                               unsigned* __restrict__ status, unsigned step, int check_max)
+// whose count is a multiple of 256).  A cell's incident faces lie slot by slot
+// beside those of the other cells of its warp (slice s: entries from
+// slice[s], 32 per slot), so the lists are read coalesced; meta is the number
+// of faces, or -1 for a wall or plate cell.
+__global__ void __launch_bounds__(256) k_amr_pressure(int n_cells, float* __restrict__ p, const float* __restrict__ v,
+                                                      const float* __restrict__ pdamp, const float* __restrict__ psrc,
+                                                      const float* __restrict__ inv_den, const int* __restrict__ meta,
+                                                      const int* __restrict__ slice, const int2* __restrict__ inc,
+                                                      float bulk, unsigned* __restrict__ status, unsigned step,
+                                                      int check_max)
 {
+    constexpr int kAhead = 6;   // slots fetched before the wait: a cell of a uniform region has six faces
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells || *status < step) return;
+    const bool in = c < n_cells;
+    int n = -1;
+    float pd = 0.0f, ps = 0.0f, id = 0.0f;
+    const int2* e = nullptr;
+    int2 x[kAhead];
+    if (in) {
+        n = meta[c];
+        pd = pdamp[c];
+        ps = psrc[c];
+        id = inv_den[c];
+        e = inc + slice[c >> 5] + (c & 31);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k < n) x[k] = e[32 * k];
+    }
+    wait_previous();
+    if (!in || *status < step) return;
     float out = 0.0f;
-    if (!zero[c]) {
+    if (n >= 0) {
+        float y[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) y[k] = k < n ? v[x[k].x] : 0.0f;
         float d = 0.0f;
-        const int k1 = cstart[c + 1];
-        for (int k = cstart[c]; k < k1; ++k) d = fa(d, fm(cw[k], v[cface[k]]));
-        out = fs(fm(p[c], pdamp[c]), fm(fm(fm(bulk, d), inv_den[c]), psrc[c]));
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k < n) d = fa(d, fm(__int_as_float(x[k].y), y[k]));
+        for (int k = kAhead; k < n; ++k) {
+            const int2 z = e[32 * k];
+            d = fa(d, fm(__int_as_float(z.y), v[z.x]));
+        }
+        out = fs(fm(p[c], pd), fm(fm(fm(bulk, d), id), ps));
     }
     p[c] = out;
     if (!isfinite(out) || (check_max && fabsf(out) > 2e3f)) atomicMin(status, step);
@@ -178,8 +319,9 @@ __global__ void k_amr_plate(int n_nodes, const int* __restrict__ node_entry, con
                             PlateCoefs k, const unsigned* __restrict__ status, unsigned step)
 {
     const int flat = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = flat < n_nodes ? node_entry[flat] : -1;
+    wait_previous();
     if (flat >= n_nodes || *status < step) return;
-    const int n = node_entry[flat];
     if (n >= 0) {
         float pa = 0.0f, pb = 0.0f;
         if (a_start[n + 1] > a_start[n]) {
@@ -203,7 +345,66 @@ __global__ void k_amr_plate(int n_nodes, const int* __restrict__ node_entry, con
     pl.ext[flat] = 0.0f;
 }
 
-__global__ void k_amr_add(float* p, int idx, float value) { p[idx] = fa(p[idx], value); }
+// Adds `value` to the pressure of the acoustic cell nearest to (x, y, z): the
+// least squared distance, the lowest index among equals (cells that are not
+// Each block leaves its best; the
+// last one to finish picks among them and reports the cell (-1: none).
+__global__ void __launch_bounds__(256) k_amr_add_nearest(int n_cells, const double* __restrict__ centers,
+                                                         const unsigned char* __restrict__ open, double x, double y, double z, double2* __restrict__ best,
+                                                         unsigned* __restrict__ done, float* __restrict__ p, float value,
+                                                         int* __restrict__ found)
+{
+    __shared__ double s_d[256];
+    __shared__ int s_i[256];
+    __shared__ bool s_last;
+    auto reduce = [&](double d, int i) {
+        s_d[threadIdx.x] = d;
+        s_i[threadIdx.x] = i;
+        __syncthreads();
+        for (int h = 128; h > 0; h >>= 1) {
+            if (threadIdx.x < h) {
+                const double d2 = s_d[threadIdx.x + h];
+                const int i2 = s_i[threadIdx.x + h];
+                if (i2 >= 0 && (s_i[threadIdx.x] < 0 || d2 < s_d[threadIdx.x] ||
+                                (d2 == s_d[threadIdx.x] && i2 < s_i[threadIdx.x]))) {
+                    s_d[threadIdx.x] = d2;
+                    s_i[threadIdx.x] = i2;
+                }
+            }
+            __syncthreads();
+        }
+    };
+    double d = 1e300;
+    int bi = -1;
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < n_cells; c += gridDim.x * 256) {
+        const double dx = __dsub_rn(centers[3 * (size_t)c], x), dy = __dsub_rn(centers[3 * (size_t)c + 1], y),
+                     dz = __dsub_rn(centers[3 * (size_t)c + 2], z);
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        if (d2 < d && open[c]) { d = d2; bi = c; }
+    }
+    reduce(d, bi);
+    if (threadIdx.x == 0) {
+        best[blockIdx.x] = make_double2(s_d[0], (double)s_i[0]);
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    d = 1e300;
+    bi = -1;
+    for (int q = threadIdx.x; q < (int)gridDim.x; q += 256) {   // ascending blocks: a strided cell order, so ties compare indices
+        const double2 b = __ldcg(best + q);
+        const int i = (int)b.y;
+        if (i >= 0 && (bi < 0 || b.x < d || (b.x == d && i < bi))) { d = b.x; bi = i; }
+    }
+    reduce(d, bi);
+    if (threadIdx.x == 0) {
+        if (s_i[0] >= 0) p[s_i[0]] = fa(p[s_i[0]], value);
+        *found = s_i[0];
+        *done = 0u;
+    }
+}
 
 // Samples of the plate (4-tap batch, or one weighted sum), in tap order.
 __global__ void k_amr_plate_taps(const float* __restrict__ w, int n_out, int taps, const int* __restrict__ idx,
@@ -241,6 +442,23 @@ __global__ void k_amr_mics(int n_mics, const float* __restrict__ p, const float*
 
 inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 
+template <class... A>
+cudaError_t launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+constexpr int kNearestBlocks = 148;
+
 }  // namespace
 
 // ================================================================ state
@@ -261,9 +479,17 @@ struct AcousticAMRState {
 
     // device
     float *d_p = nullptr, *d_v = nullptr, *d_vdamp = nullptr, *d_inv_d = nullptr;
-    float *d_pdamp = nullptr, *d_psrc = nullptr, *d_inv_den = nullptr, *d_cw = nullptr, *d_scoef = nullptr;
-    int *d_neg = nullptr, *d_pos = nullptr, *d_cstart = nullptr, *d_cface = nullptr, *d_scell = nullptr;
-    unsigned char* d_zero = nullptr;
+    float *d_pdamp = nullptr, *d_psrc = nullptr, *d_inv_den = nullptr, *d_scoef = nullptr;
+    int *d_neg = nullptr, *d_pos = nullptr, *d_meta = nullptr, *d_slice = nullptr, *d_scell = nullptr;
+    int2* d_inc = nullptr;
+    unsigned* d_srow = nullptr;       // order 8: rows of d_soff / d_swgt per face
+    int* d_soff = nullptr;
+    float* d_swgt = nullptr;
+    double* d_centers = nullptr;
+    unsigned char* d_open = nullptr;  // 1: an acoustic cell (a candidate of the nearest-cell search)
+    double2* d_best = nullptr;        // nearest-cell search: a candidate per block, block counter, result
+    unsigned* d_done = nullptr;
+    int* h_found = nullptr;           // pinned
     unsigned* d_status = nullptr;
     float* d_scratch = nullptr;       // staging of sampler weights and results (2 x scratch_n)
     int* d_iscratch = nullptr;        // staging of sampler indices (scratch_n)
@@ -307,15 +533,16 @@ namespace {
 void free_all(AcousticAMRState* st)
 {
     void* ptrs[] = {st->d_p, st->d_v, st->d_vdamp, st->d_inv_d, st->d_pdamp, st->d_psrc, st->d_inv_den,
-                    st->d_cw, st->d_scoef, st->d_neg, st->d_pos, st->d_cstart, st->d_cface, st->d_scell,
-                    st->d_zero, st->d_status, st->d_scratch, st->d_iscratch, st->d_w[0], st->d_w[1],
-                    st->d_w[2], st->d_ext, st->d_node_entry, st->d_astart, st->d_acell, st->d_bstart,
+                    st->d_scoef, st->d_neg, st->d_pos, st->d_meta, st->d_slice, st->d_scell, st->d_inc, st->d_srow,
+                    st->d_soff, st->d_swgt, st->d_centers, st->d_open, st->d_best, st->d_done, st->d_status,
+                    st->d_scratch, st->d_iscratch, st->d_w[0], st->d_w[1], st->d_w[2], st->d_ext, st->d_node_entry, st->d_astart, st->d_acell, st->d_bstart,
                     st->d_bcell, st->d_cabove, st->d_cbelow, st->d_bc, st->d_bc_flat, st->d_awgt,
                     st->d_bwgt, st->d_mps, st->d_mpc, st->d_mvs, st->d_mvf, st->d_mpw, st->d_mwx,
                     st->d_mwy, st->d_mwz};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     if (st->h_ext) cudaFreeHost(st->h_ext);
+    if (st->h_found) cudaFreeHost(st->h_found);
     for (cudaEvent_t e : st->ev) cudaEventDestroy(e);
     if (st->stream) cudaStreamDestroy(st->stream);
 }
@@ -565,6 +792,56 @@ void build_stencil(AcousticAMRState* st, std::vector<int>& sc, std::vector<float
     g_prog_active.store(0);
 }
 
+// Numbers the distinct rows of cell offsets and of weights (eight each), in
+// order of first appearance; false when either kind has more than 65536.
+bool number_stencils(const std::vector<int>& neg, const std::vector<int>& sc, const std::vector<float>& sw,
+                     std::vector<unsigned>& row, std::vector<int>& off, std::vector<float>& wgt)
+{
+    struct Table {   // open addressing over the rows seen so far
+        std::vector<int> words, slot;
+        size_t n = 0, mask = 0;
+        Table() : slot(1 << 18, -1), mask((1 << 18) - 1) {}
+        int last = -1;
+        int number(const int* r)   // neighbouring faces mostly share a row
+        {
+            if (last < 0 || memcmp(&words[(size_t)last * kSW2], r, kSW2 * sizeof(int)) != 0) last = find(r);
+            return last;
+        }
+        int find(const int* r)
+        {
+            uint64_t h = 1469598103934665603ull;
+            for (int k = 0; k < kSW2; ++k) h = (h ^ (uint32_t)r[k]) * 1099511628211ull;
+            for (size_t q = (h ^ h >> 29) & mask;; q = (q + 1) & mask) {
+                if (slot[q] < 0) {
+                    if (n >= 65536) return -1;
+                    slot[q] = (int)n++;
+                    words.insert(words.end(), r, r + kSW2);
+                    return slot[q];
+                }
+                if (memcmp(&words[(size_t)slot[q] * kSW2], r, kSW2 * sizeof(int)) == 0) return slot[q];
+            }
+        }
+    } to, tw;
+    const size_t nf = neg.size();
+    row.resize(nf);
+    for (size_t f = 0; f < nf; ++f) {
+        int o[kSW2], w[kSW2];
+        memcpy(w, &sw[f * kSW2], sizeof w);
+        for (int k = 0; k < kSW2; ++k)
+            o[k] = (sc[f * kSW2 + k] == 0 && w[k] == 0) ? kOrigin : sc[f * kSW2 + k] - neg[f];
+        const int a = to.number(o), b = tw.number(w);
+        if (a < 0 || b < 0) {
+            row.clear();
+            return false;
+        }
+        row[f] = (unsigned)a | (unsigned)b << 16;
+    }
+    off = to.words;
+    wgt.resize(tw.words.size());
+    memcpy(wgt.data(), tw.words.data(), tw.words.size() * sizeof(int));
+    return true;
+}
+
 void prof_mark(AcousticAMRState* st)
 {
     if (!st->prof) return;
@@ -606,25 +883,25 @@ int launch_steps(AcousticAMRState* st, int n_steps)
         PlateDev pl{};
         if (st->plate) pl = PlateDev{st->cur_w(), st->prev_w(), st->next_w(), st->d_ext, dt};
         prof_mark(st);
-        if (st->order == 8)
-            k_amr_velocity<8><<<blocks(st->n_faces, 256), 256, 0, st->stream>>>(
-                st->n_faces, st->d_p, st->d_v, st->d_vdamp, st->d_inv_d, st->d_neg, st->d_pos, st->d_scell,
-                st->d_scoef, st->plate ? st->d_bc : nullptr, st->d_bc_flat, pl, dt_over_rho, st->d_status, step);
-        else
-            k_amr_velocity<2><<<blocks(st->n_faces, 256), 256, 0, st->stream>>>(
-                st->n_faces, st->d_p, st->d_v, st->d_vdamp, st->d_inv_d, st->d_neg, st->d_pos, nullptr, nullptr,
-                st->plate ? st->d_bc : nullptr, st->d_bc_flat, pl, dt_over_rho, st->d_status, step);
-        AK(cudaGetLastError());
-        k_amr_pressure<<<blocks(st->n_cells, 256), 256, 0, st->stream>>>(
-            st->n_cells, st->d_p, st->d_v, st->d_pdamp, st->d_psrc, st->d_inv_den, st->d_cstart, st->d_cface,
-            st->d_cw, st->d_zero, bulk, st->d_status, step, (step & 0xFFu) == 0 ? 1 : 0);
-        AK(cudaGetLastError());
+        const Stencils sten{st->d_srow, reinterpret_cast<const int4*>(st->d_soff),
+                            reinterpret_cast<const float4*>(st->d_swgt), st->d_scell, st->d_scoef};
+        const int* const bc = st->plate ? st->d_bc : nullptr;
+        AK(launch_after(st->order == 8 ? k_amr_velocity<8> : k_amr_velocity<2>,
+                        blocks(st->n_faces, st->order == 8 ? 256 : 1024), 256, st->stream, st->n_faces,
+                        (const float*)st->d_p, st->d_v, (const float*)st->d_vdamp, (const float*)st->d_inv_d,
+                        (const int*)st->d_neg, (const int*)st->d_pos, sten, bc, (const int*)st->d_bc_flat, pl,
+                        dt_over_rho, (const unsigned*)st->d_status, step));
+        AK(launch_after(k_amr_pressure, blocks(st->n_cells, 256), 256, st->stream, st->n_cells, st->d_p,
+                        (const float*)st->d_v, (const float*)st->d_pdamp, (const float*)st->d_psrc,
+                        (const float*)st->d_inv_den, (const int*)st->d_meta, (const int*)st->d_slice,
+                        (const int2*)st->d_inc, bulk, st->d_status, step, (step & 0xFFu) == 0 ? 1 : 0));
         st->launches += 2;
         if (st->plate) {
-            k_amr_plate<<<blocks(st->p_nodes, 128), 128, 0, st->stream>>>(
-                st->p_nodes, st->d_node_entry, st->d_astart, st->d_awgt, st->d_acell, st->d_bstart, st->d_bwgt,
-                st->d_bcell, st->d_cabove, st->d_cbelow, st->d_p, pl, st->pk, st->d_status, step);
-            AK(cudaGetLastError());
+            AK(launch_after(k_amr_plate, blocks(st->p_nodes, 128), 128, st->stream, st->p_nodes,
+                            (const int*)st->d_node_entry, (const int*)st->d_astart, (const float*)st->d_awgt,
+                            (const int*)st->d_acell, (const int*)st->d_bstart, (const float*)st->d_bwgt,
+                            (const int*)st->d_bcell, (const int*)st->d_cabove, (const int*)st->d_cbelow,
+                            (const float*)st->d_p, pl, st->pk, (const unsigned*)st->d_status, step));
             ++st->launches;
             st->wi = (st->wi + 1) % 3;
         }
@@ -734,8 +1011,9 @@ AcousticAMRState* amr_create(int n_cells, const double* cc, const double* cv, co
             flux[f] = (float)(fa_[f] * fo[f]);
         }
         for (int i : st->acoustic) inv_den[i] = (float)(1.0 / (cv[i] * std::max(ov[i], 1e-12)));
-        std::vector<unsigned char> zero(n_cells);
+        std::vector<unsigned char> zero(n_cells), open(n_cells, 0);
         for (int i = 0; i < n_cells; ++i) zero[i] = (ct[i] == 1 || ct[i] == 2) ? 1 : 0;
+        for (int i : st->acoustic) open[i] = 1;
         // incident faces of each cell, in face order: +flux on the face's negative side, -flux on its positive side
         st->csr_start.assign(n_cells + 1, 0);
         for (int f = 0; f < n_faces; ++f) {
@@ -756,30 +1034,84 @@ AcousticAMRState* amr_create(int n_cells, const double* cc, const double* cv, co
                 st->csr_w[kb] = -flux[f];
             }
         }
-        std::vector<int> scell;
-        std::vector<float> scoef;
+        // the same lists slot by slot per slice of 32 cells (k_amr_pressure)
+        std::vector<int> meta(n_cells), slice((n_cells + 31) / 32);
+        size_t n_inc = 0;
+        for (size_t q = 0; q < slice.size(); ++q) {
+            int deg = 0;
+            for (int c = (int)(32 * q); c < std::min((int)(32 * q) + 32, n_cells); ++c) {
+                meta[c] = zero[c] ? -1 : st->csr_start[c + 1] - st->csr_start[c];
+                deg = std::max(deg, meta[c]);
+            }
+            slice[q] = (int)n_inc;
+            n_inc += 32 * (size_t)deg;
+        }
+        if (n_inc > INT_MAX) throw std::bad_alloc();
+        std::vector<int2> inc(n_inc, make_int2(0, 0));
+        for (int c = 0; c < n_cells; ++c) {
+            int2* const e = inc.data() + slice[c >> 5] + (c & 31);
+            for (int k = 0; k < meta[c]; ++k) {
+                e[32 * k].x = st->csr_face[st->csr_start[c] + k];
+                memcpy(&e[32 * k].y, &st->csr_w[st->csr_start[c] + k], 4);
+            }
+        }
+        std::vector<int> scell, soff;
+        std::vector<float> scoef, swgt;
+        std::vector<unsigned> srow;
         if (gradient_order == 8) {
             g_stage = "stencil.build";
             build_stencil(st, scell, scoef);
+            if (number_stencils(st->face_neg, scell, scoef, srow, soff, swgt)) {
+                scell.clear();
+                scoef.clear();
+            } else {   // slot by slot
+                std::vector<int> tc(scell.size());
+                std::vector<float> tw(scoef.size());
+                for (size_t f = 0; f < (size_t)n_faces; ++f)
+                    for (int k = 0; k < kSW2; ++k) {
+                        tc[(size_t)k * n_faces + f] = scell[f * kSW2 + k];
+                        tw[(size_t)k * n_faces + f] = scoef[f * kSW2 + k];
+                    }
+                scell.swap(tc);
+                scoef.swap(tw);
+            }
         }
         g_stage = "device";
         cudaError_t e = cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking);
-        std::vector<float> ones_f(n_faces, 1.0f), ones_c(n_cells, 1.0f), zc(n_cells, 0.0f), zf(n_faces, 0.0f);
-        if (e == cudaSuccess) e = upload(&st->d_p, zc);
-        if (e == cudaSuccess) e = upload(&st->d_v, zf);
-        if (e == cudaSuccess) e = upload(&st->d_vdamp, ones_f);
-        if (e == cudaSuccess) e = upload(&st->d_inv_d, inv_d);
-        if (e == cudaSuccess) e = upload(&st->d_pdamp, ones_c);
-        if (e == cudaSuccess) e = upload(&st->d_psrc, ones_c);
+        // face arrays padded to a multiple of four faces (k_amr_velocity's wide loads)
+        const size_t nf = (size_t)n_faces, nf4 = (nf + 3) / 4 * 4, nc = (size_t)n_cells;
+        auto filled = [&](float** d, size_t n, float value) {
+            cudaError_t r = cudaMalloc(d, n * sizeof(float));
+            if (r == cudaSuccess) {
+                k_amr_fill<<<148, 256, 0, st->stream>>>(*d, n, value);
+                r = cudaGetLastError();
+            }
+            return r;
+        };
+        if (e == cudaSuccess) e = filled(&st->d_p, nc, 0.0f);
+        if (e == cudaSuccess) e = filled(&st->d_v, nf4, 0.0f);
+        if (e == cudaSuccess) e = filled(&st->d_vdamp, nf4, 1.0f);
+        if (e == cudaSuccess) e = filled(&st->d_pdamp, nc, 1.0f);
+        if (e == cudaSuccess) e = filled(&st->d_psrc, nc, 1.0f);
+        if (e == cudaSuccess) e = upload(&st->d_inv_d, inv_d.data(), nf, nf4);
         if (e == cudaSuccess) e = upload(&st->d_inv_den, inv_den);
-        if (e == cudaSuccess) e = upload(&st->d_neg, st->face_neg);
-        if (e == cudaSuccess) e = upload(&st->d_pos, st->face_pos);
-        if (e == cudaSuccess) e = upload(&st->d_cstart, st->csr_start);
-        if (e == cudaSuccess) e = upload(&st->d_cface, st->csr_face);
-        if (e == cudaSuccess) e = upload(&st->d_cw, st->csr_w);
-        if (e == cudaSuccess) e = upload(&st->d_zero, zero);
-        if (e == cudaSuccess && gradient_order == 8) e = upload(&st->d_scell, scell);
-        if (e == cudaSuccess && gradient_order == 8) e = upload(&st->d_scoef, scoef);
+        if (e == cudaSuccess) e = upload(&st->d_neg, st->face_neg.data(), nf, nf4);
+        if (e == cudaSuccess) e = upload(&st->d_pos, st->face_pos.data(), nf, nf4);
+        if (e == cudaSuccess) e = upload(&st->d_meta, meta);
+        if (e == cudaSuccess) e = upload(&st->d_slice, slice);
+        if (e == cudaSuccess) e = upload(&st->d_inc, inc);
+        if (e == cudaSuccess) e = upload(&st->d_scell, scell);
+        if (e == cudaSuccess) e = upload(&st->d_scoef, scoef);
+        if (e == cudaSuccess) e = upload(&st->d_srow, srow);
+        if (e == cudaSuccess) e = upload(&st->d_soff, soff);
+        if (e == cudaSuccess) e = upload(&st->d_swgt, swgt);
+        if (e == cudaSuccess) e = upload(&st->d_centers, st->centers.data(), st->centers.size(), st->centers.size());
+        if (e == cudaSuccess) e = upload(&st->d_open, open);
+        if (e == cudaSuccess) e = cudaMalloc(&st->d_best, kNearestBlocks * sizeof(double2));
+        if (e == cudaSuccess) e = cudaMalloc(&st->d_done, sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMemset(st->d_done, 0, sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMallocHost(&st->h_found, sizeof(int));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st->stream);
         if (e == cudaSuccess) e = cudaMalloc(&st->d_status, sizeof(unsigned));
         if (e == cudaSuccess) e = cudaMemset(st->d_status, 0xFF, sizeof(unsigned));
         if (e != cudaSuccess) {
@@ -865,24 +1197,14 @@ int amr_inject_pressure_nearest(AcousticAMRState* st, const double* xyz, float v
 {
     if (!st || !xyz) return SK_ERR_NULL_STATE;
     if (!std::isfinite(value)) return SK_ERR_DIVERGED;
-    double best = 1e300;
-    int bi = -1;
-    for (int i : st->acoustic) {
-        const double dx = st->centers[3 * i] - xyz[0], dy = st->centers[3 * i + 1] - xyz[1],
-                     dz = st->centers[3 * i + 2] - xyz[2];
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (d2 < best) {
-            best = d2;
-            bi = i;
-        }
-    }
-    if (bi < 0) return SK_ERR_DIM_MISMATCH;
     if (guard(st)) return AMR_B200_ERR_CUDA;
-    k_amr_add<<<1, 1, 0, st->stream>>>(st->d_p, bi, value);
+    *st->h_found = -1;
+    k_amr_add_nearest<<<kNearestBlocks, 256, 0, st->stream>>>(st->n_cells, st->d_centers, st->d_open, xyz[0], xyz[1], xyz[2],
+                                                              st->d_best, st->d_done, st->d_p, value, st->h_found);
     AK(cudaGetLastError());
     ++st->launches;
     AK(cudaStreamSynchronize(st->stream));
-    return SK_OK;
+    return *st->h_found < 0 ? SK_ERR_DIM_MISMATCH : SK_OK;
 }
 
 int amr_get_pressure(const AcousticAMRState* st, float* out, int n)
@@ -1061,6 +1383,7 @@ int amr_setup_plate(AcousticAMRState* st, int pnx, int pny, float pdx, const flo
     AK(upload(&st->d_bcell, bcell));
     AK(upload(&st->d_cabove, std::vector<int>(cell_above, cell_above + n_act)));
     AK(upload(&st->d_cbelow, std::vector<int>(cell_below, cell_below + n_act)));
+    bc.resize(((size_t)st->n_faces + 3) / 4 * 4, -1);   // padded for k_amr_velocity's wide loads
     AK(upload(&st->d_bc, bc));
     AK(upload(&st->d_bc_flat, st->act_flat));
     if (st->h_ext) cudaFreeHost(st->h_ext);
