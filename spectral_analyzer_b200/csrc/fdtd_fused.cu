@@ -371,19 +371,22 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     float axw3 = ax_at(u0 - 3), axw2 = ax_at(u0 - 2), axw1 = ax_at(u0 - 1), axw0 = ax_at(u0);
     float pxw = px_at(u0 - 3);
 
-    // The interior iterations of a tile whose columns are all cells take a
-    // separately compiled body without the general path (the general path
+    // The interior iterations take a separately compiled body without the
+    // general path (the general path
     // present in the loop costs the interior about 12 % although it never runs
     // there).  Iteration u is interior when plane u-3 and faces u-2 .. u-1 have
     // no x absorption, face u-2 has the 4th-order gradient and the planes u-3,
     // u-2 are own ones.  Rows beyond the room and Vy faces at the j ends are
-    // warp-uniform cases the interior body handles itself.  Both bodies
+    // warp-uniform cases the interior body handles itself; columns beyond the
+    // room (a partial k tile) hold zero pressure and velocity, so their faces
+    // come out zero, their stores end at the row's padding and their cells are
+    // set to zero (with the general body on partial tiles the 160x128x112 room,
+    // one partial tile wide, took 31.0 us per step).  Both bodies
     // evaluate the same expressions (alpha_x = 0, px = 1 there), so the results
     // do not depend on the choice.  The step runs in one wave, so a CTA left on
     // the general body for its whole march would set the kernel's time.
-    const bool clean = kfull;
     int fast_lo = u1 + 1, fast_hi = u1 + 1;
-    if (clean && a.tb.xi_hi > a.tb.xi_lo) {
+    if (a.tb.xi_hi > a.tb.xi_lo) {
         fast_lo = max(max(a.tb.xi_lo + 3, 3 - xg0), i_beg + 3);
         fast_hi = min(min(a.tb.xi_hi + 1, nxg - xg0), u1 + 1);
         if (fast_lo >= fast_hi) fast_lo = fast_hi = u1 + 1;
@@ -654,7 +657,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                     out.y = pupd(cf, pown.y, qx2.y, qx1.y, qx3.y, qx0.y, yp.y, ym.y, ypp.y, ymm.y, zb.y, zb.x, zb.z, za.y, pd.y);
                     out.z = pupd(cf, pown.z, qx2.z, qx1.z, qx3.z, qx0.z, yp.z, ym.z, ypp.z, ymm.z, zb.z, zb.y, zb.w, zb.x, pd.z);
                     out.w = pupd(cf, pown.w, qx2.w, qx1.w, qx3.w, qx0.w, yp.w, ym.w, ypp.w, ymm.w, zb.w, zb.z, zc, zb.y, pd.w);
-                    if (!FAST && !kfull) {
+                    if (!kfull) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                             if (kb + q >= nz) at(out, q) = 0.0f;

@@ -358,13 +358,14 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
     float pxw = px_at(u0 - 3);
     int u_fail = u1 + 1;
 
-    // The x-interior iterations of a tile whose columns are all cells run a
-    // separately compiled body without the general path: iteration u is
+    // The x-interior iterations run a separately compiled body without the
+    // general path (columns beyond the room hold zeros and come out zero, and
+    // their cells are set to zero): iteration u is
     // interior when plane u-3 and faces u-2 .. u-1 have alpha_x = 0 (px = 1),
     // face u-2 has the 4th-order gradient and plane u-3 is an own plane.  Both
     // bodies evaluate the same expressions there.
     int fast_lo = u1 + 1, fast_hi = u1 + 1;
-    if (kfull && a.xi_hi > a.xi_lo) {
+    if (a.xi_hi > a.xi_lo) {
         fast_lo = max(max(a.xi_lo + 3, 3), i_beg + 3);
         fast_hi = min(min(a.xi_hi + 1, nx), u1 + 1);
         if (fast_lo >= fast_hi) fast_lo = fast_hi = u1 + 1;
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                 out.y = pup(cf, pown.y, qx2.y, qx1.y, qx3.y, qx0.y, yp.y, ym.y, ypp.y, ymm.y, zb.y, zb.x, zb.z, za.y, pd.y);
                 out.z = pup(cf, pown.z, qx2.z, qx1.z, qx3.z, qx0.z, yp.z, ym.z, ypp.z, ymm.z, zb.z, zb.y, zb.w, zb.x, pd.z);
                 out.w = pup(cf, pown.w, qx2.w, qx1.w, qx3.w, qx0.w, yp.w, ym.w, ypp.w, ymm.w, zb.w, zb.z, zc, zb.y, pd.w);
-                if (!FAST && !kfull) {
+                if (!kfull) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                         if (kb + q >= nz) at4(out, q) = 0.0f;
