@@ -213,8 +213,11 @@ struct Pipe {
 template <class C>
 __device__ __forceinline__ unsigned smem_base_u32(float** smem_out)
 {
-    extern __shared__ float smem_raw[];
-    float* const smem = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    // an offset from the array, not a pointer made from an integer: the compiler
+    // must see shared memory, or every access becomes a generic one with 64-bit
+    // addresses (512x384x256 room: 313 us per step)
+    extern __shared__ __align__(128) float smem_raw[];
+    float* const smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u) / 4u;
     *smem_out = smem;
     return smem_u32(smem);
 }

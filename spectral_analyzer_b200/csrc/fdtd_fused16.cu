@@ -237,9 +237,10 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
     if (i_beg >= nx) return;
     const int i_end = min(i_beg + seg_len, nx);
 
-    extern __shared__ unsigned char smem_raw16[];
-    unsigned char* const sm = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smem_raw16) + 127) & ~uintptr_t(127));
+    // an offset from the array: a pointer made from an integer would turn every
+    // shared-memory access into a generic one
+    extern __shared__ __align__(128) unsigned char smem_raw16[];
+    unsigned char* const sm = smem_raw16 + ((128u - (smem_u32(smem_raw16) & 127u)) & 127u);
     const unsigned sbase = smem_u32(sm);
     const unsigned bar0 = sbase + C::BAR0;
     float* const vyn = reinterpret_cast<float*>(sm + C::VYN0);
