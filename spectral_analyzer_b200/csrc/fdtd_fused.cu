@@ -87,8 +87,8 @@ struct Cfg {
     static constexpr int VZN0 = VYN0 + r32(VY_BOX);
     static constexpr int AY0 = VZN0 + r32(VZ_BOX);
     static constexpr int AZ0 = AY0 + r32(AY_N);
-    static constexpr int BAR0 = AZ0 + r32(PC);  // RING + VSTAGES mbarriers (8 B each)
-    static constexpr int SMEM_FLOATS = BAR0 + 2 * (RING + VSTAGES);
+    static constexpr int BAR0 = AZ0 + r32(PC);  // RING mbarriers (8 B each)
+    static constexpr int SMEM_FLOATS = BAR0 + 2 * RING;
     static constexpr size_t SMEM_BYTES = sizeof(float) * SMEM_FLOATS + 128;   // + base alignment
     static constexpr unsigned P_BYTES = 4u * P_BOX;
     static constexpr unsigned VX_BYTES = 4u * VX_BOX;
@@ -122,7 +122,9 @@ __device__ __forceinline__ float4 mul4(const float4& v, const float4& fr)
 // staggered gradient: 4th order in the interior of the face range, else 2nd
 __device__ __forceinline__ float grad4(const Coef& cf, float pm, float p0, float p1, float p2, bool fourth)
 {
-    return fourth ? fadd(fmul(cf.c1, fsub(p1, p0)), fmul(cf.c2, fsub(p2, pm))) : fsub(p1, p0);
+    // both orders, then a selection: a branch per face costs more than the products
+    const float d = fsub(p1, p0), w = fadd(fmul(cf.c1, d), fmul(cf.c2, fsub(p2, pm)));
+    return fourth ? w : d;
 }
 
 // V^{n+1/2} = (V^{n-1/2} - vc*grad) * damp
@@ -164,7 +166,8 @@ __device__ __forceinline__ float4 vel4_masked(const Coef& cf, float4 pm, float4 
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const float gr = grad4(cf, at(pm, q), at(p0, q), at(p1, q), at(p2, q), (m4 >> q) & 1);
-        at(r, q) = ((ok >> q) & 1) ? vupd(cf, at(vo, q), gr, at(dmp, q)) : 0.0f;
+        const float v = vupd(cf, at(vo, q), gr, at(dmp, q));
+        at(r, q) = ((ok >> q) & 1) ? v : 0.0f;
     }
     return r;
 }
@@ -192,22 +195,12 @@ __device__ __forceinline__ float pupd(const Coef& cf, float p, float xp, float x
     return fmul(fsub(p, fmul(cf.bulk, dv)), pd);
 }
 
-// Load-pipeline state carried by a CTA from one tile to the next: rotating slot
-// ids and the mbarrier parity to wait for next, per slot.  Between tiles every
-// issued load has been consumed, so pslot[3 .. 3+D] and vslot[0 .. D] are free.
-template <class C>
+// Load-pipeline state carried by a CTA from one tile to the next: the ring slot
+// of the next plane and V stage to be loaded, and the mbarrier parity to wait
+// for next, per ring slot.  Between tiles every issued load has been consumed.
 struct Pipe {
-    int pslot[C::RING];
-    int vslot[C::VSTAGES];
-    unsigned pph, vph;
-    __device__ void init()
-    {
-#pragma unroll
-        for (int q = 0; q < C::RING; ++q) pslot[q] = q;
-#pragma unroll
-        for (int q = 0; q < C::VSTAGES; ++q) vslot[q] = q;
-        pph = vph = 0;
-    }
+    int ps = 0, vs = 0;
+    unsigned ph = 0;
 };
 
 template <class C>
@@ -226,7 +219,7 @@ template <class C>
 __device__ __forceinline__ void init_barriers(unsigned bar0)
 {
     if (threadIdx.x == 0) {
-        for (int q = 0; q < C::RING + C::VSTAGES; ++q) mbar_init(bar0 + 8u * q, 1);
+        for (int q = 0; q < C::RING; ++q) mbar_init(bar0 + 8u * q, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
@@ -245,16 +238,12 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                                            const CUtensorMap* tmX, const CUtensorMap* tmY,
                                            const CUtensorMap* tmZ, int tile, int seg, int seg_len,
                                            int tiles_k, float* smem, unsigned sbase, unsigned bar0,
-                                           Pipe<C>& pp, bool acquire_maps = false)
+                                           Pipe& pp, bool acquire_maps = false)
 {
     float* const vyn = smem + C::VYN0;
     float* const vzn = smem + C::VZN0;
     float* const ay_s = smem + C::AY0;
     float* const az_s = smem + C::AZ0;
-    int* const pslot = pp.pslot;
-    int* const vslot = pp.vslot;
-    unsigned& pph = pp.pph;
-    unsigned& vph = pp.vph;
 
     const Grid g = a.g;
     const int nx = g.nx, ny = g.ny, nz = g.nz, sz = g.sz;
@@ -285,24 +274,21 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     __syncthreads();
 
     // Loads feeding iteration u (issued by thread 0): P plane u, Vx face u-2,
-    // Vy/Vz of plane u-3.  An iteration without V loads still completes its V
-    // stage's phase (expect_tx of 0 bytes is a plain arrive).
+    // Vy/Vz of plane u-3, all on the plane's mbarrier.
     auto issue = [&](int u, int ps, int vsg) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         const unsigned pb = bar0 + 8u * ps;
-        mbar_expect_tx(pb, C::P_BYTES);
-        if (u != a.hold_plane)
-            tma_load3(sbase + 4u * (C::RING0 + ps * C::P_STAGE), tmP, k0 - 4, j0 - 3, u, pb);
         const int f = u - 2, io = u - 3, fg = f + xg0;
         const bool vx = (u >= i_beg && fg >= 0 && fg <= nxg - 2);
         const bool vyz = (io >= i_beg && io < i_end);
-        const unsigned vb = bar0 + 8u * (C::RING + vsg);
+        mbar_expect_tx(pb, C::P_BYTES + (vx ? C::VX_BYTES : 0u) + (vyz ? C::VYZ_BYTES : 0u));
+        if (u != a.hold_plane)
+            tma_load3(sbase + 4u * (C::RING0 + ps * C::P_STAGE), tmP, k0 - 4, j0 - 3, u, pb);
         const unsigned vdst = sbase + 4u * (C::VST0 + vsg * C::V_STAGE);
-        mbar_expect_tx(vb, (vx ? C::VX_BYTES : 0u) + (vyz ? C::VYZ_BYTES : 0u));
-        if (vx) tma_load3(vdst + 4u * C::VX_OFF, tmX, k0, j0, f, vb);
+        if (vx) tma_load3(vdst + 4u * C::VX_OFF, tmX, k0, j0, f, pb);
         if (vyz) {
-            tma_load3(vdst + 4u * C::VY_OFF, tmY, k0, j0 - 2, io, vb);
-            tma_load3(vdst + 4u * C::VZ_OFF, tmZ, k0 - 4, j0, io, vb);
+            tma_load3(vdst + 4u * C::VY_OFF, tmY, k0, j0 - 2, io, pb);
+            tma_load3(vdst + 4u * C::VZ_OFF, tmZ, k0 - 4, j0, io, pb);
         }
     };
 
@@ -313,13 +299,24 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         acquire_tensormap(tmZ);
     }
     const int u0 = i_beg - 3, u1 = i_end + 2;
-    // Slot ids, rotated each iteration.  At iteration u: pslot[0..3] hold planes
-    // u-3 .. u, pslot[4 .. 3+D-1] planes u+1 .. u+D-1 in flight, pslot[3+D] is
-    // free; vslot[0] holds iteration u's V data, vslot[1 .. D-1] the next
-    // iterations' in flight, vslot[D] is free.  pph/vph: parity to wait for, per slot.
-    // The first D iterations' loads go into the free slots left by the previous tile.
+    // Plane v of the march lives in ring slot (ps + v - u0) mod RING, iteration
+    // v's V data in stage (vs + v - u0) mod VSTAGES: at iteration u planes u-3
+    // .. u are in use, u+1 .. u+D-1 in flight, and the slots of u+D (held by
+    // plane u-4 and iteration u-1 before) are free.
+    int ps = pp.ps, vs0 = pp.vs;
+    unsigned ph = pp.ph;
+    auto ring = [&](int q) { return q >= C::RING ? q - C::RING : q; };
+    auto vring = [&](int q) { return q >= C::VSTAGES ? q - C::VSTAGES : q; };
     if (tid == 0)
-        for (int q = 0; q < C::D; ++q) issue(u0 + q, pslot[3 + q], vslot[q]);
+        for (int q = 0; q < C::D; ++q) issue(u0 + q, ring(ps + q), vring(vs0 + q));
+    // stage offsets (floats) of planes u-3 .. u, rotated each iteration
+    int o0 = ps * C::P_STAGE, o1 = 0, o2 = 0, o3 = 0;
+    {
+        int q = ps;
+        q = q == 0 ? C::RING - 1 : q - 1; o1 = q * C::P_STAGE;
+        q = q == 0 ? C::RING - 1 : q - 1; o2 = q * C::P_STAGE;
+        q = q == 0 ? C::RING - 1 : q - 1; o3 = q * C::P_STAGE;
+    }
 
     // ---- per-thread constants of the own row and columns
     const int jr = j0 + w;
@@ -402,7 +399,6 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         // wait for plane u (P) and iteration u's V data; the decision to stop on a
         // timeout is made by the whole CTA (the barrier below is also the one that
         // separates the previous iteration's reads from this iteration's writes)
-        const int ps = pslot[3], vsg = vslot[0];
         // WALLS: this iteration's face fractions and solid flags, loaded before
         // the wait so that their latency overlaps it (they do not depend on it)
         float4 pf_x = make_float4(1.f, 1.f, 1.f, 1.f), pf_y0 = pf_x, pf_y1 = pf_x, pf_z = pf_x;
@@ -431,14 +427,13 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                     pf_s = __ldg(reinterpret_cast<const unsigned*>(a.solid + ib + own));
             }
         }
-        const bool ok = mbar_wait(bar0 + 8u * ps, (pph >> ps) & 1u, a.wait_us) &&
-                        mbar_wait(bar0 + 8u * (C::RING + vsg), (vph >> vsg) & 1u, a.wait_us);
+        const bool ok = mbar_wait(bar0 + 8u * ps, (ph >> ps) & 1u, a.wait_us);
         // the source deposit, on the arriving plane's shared copy before anyone reads it
         if (a.dep_sig && u == a.dep_i && tid == 0 && ok) {
             const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 4);
             const float amp = a.dep_sig[a.dep_step];
             if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC && amp != 0.0f) {
-                float* c = smem + C::RING0 + ps * C::P_STAGE + dj * C::PC + dk;
+                float* c = smem + C::RING0 + o0 + dj * C::PC + dk;
                 *c = fadd(*c, amp);
             }
         }
@@ -447,18 +442,17 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
             u_fail = u;
             return false;
         }
-        pph ^= 1u << ps;
-        vph ^= 1u << vsg;
+        ph ^= 1u << ps;
         // iteration u+D's loads go into the slots iteration u-1 freed (their last
         // reads came before the barrier above), so thread 0 issues them before
         // its own work of this iteration rather than after it
-        if (tid == 0 && u + C::D <= u1) issue(u + C::D, pslot[C::RING - 1], vslot[C::VSTAGES - 1]);
+        if (tid == 0 && u + C::D <= u1) issue(u + C::D, ring(ps + C::D), vring(vs0 + C::D));
         float ax_next = 0.0f, px_next = 1.0f;
         if constexpr (!FAST) {
             ax_next = ax_at(u + 1);
             px_next = px_at(u - 2);
         }
-        const float* vs = smem + C::VST0 + vsg * C::V_STAGE;
+        const float* vs = smem + C::VST0 + vs0 * C::V_STAGE;
 
         // ---- new Vx on face f = u-2 of the own columns (planes f-1 .. f+2) ----
         if (FAST || u >= i_beg) {
@@ -466,10 +460,10 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
             float4 vnew = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 vdiv = vnew;   // WALLS: the value the divergence sees
             if (FAST ? row_ok : (fg >= 0 && fg <= nxg - 2 && row_ok)) {
-                const float4 pm = lds4(smem + C::RING0 + pslot[0] * C::P_STAGE + cP);
-                const float4 p0 = lds4(smem + C::RING0 + pslot[1] * C::P_STAGE + cP);
-                const float4 p1 = lds4(smem + C::RING0 + pslot[2] * C::P_STAGE + cP);
-                const float4 p2 = lds4(smem + C::RING0 + pslot[3] * C::P_STAGE + cP);
+                const float4 pm = lds4(smem + C::RING0 + o3 + cP);
+                const float4 p0 = lds4(smem + C::RING0 + o2 + cP);
+                const float4 p1 = lds4(smem + C::RING0 + o1 + cP);
+                const float4 p2 = lds4(smem + C::RING0 + o0 + cP);
                 const float4 vo = lds4(vs + C::VX_OFF + 4 * tid);
                 if constexpr (FAST) {
                     vnew = vel4(cf, pm, p0, p1, p2, vo, dxi);
@@ -515,7 +509,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
             if (FAST || i >= i_beg) {
                 const float axi = FAST ? 0.0f : axw3;    // alpha_x[i]
                 const bool xint = FAST || (axi == 0.0f);
-                const float* pst = smem + C::RING0 + pslot[0] * C::P_STAGE;
+                const float* pst = smem + C::RING0 + o3;
                 const float* vys = vs + C::VY_OFF;
                 const float* vzs = vs + C::VZ_OFF;
                 const long long ib = i * PL;
@@ -688,17 +682,10 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
             axw3 = axw2; axw2 = axw1; axw1 = axw0; axw0 = ax_next;
             pxw = px_next;
         }
-        // rotate: after it pslot[q] holds plane u+1-3+q and vslot[q] iteration u+1+q.
-        {
-            const int pfree = pslot[0];
-#pragma unroll
-            for (int q = 0; q + 1 < C::RING; ++q) pslot[q] = pslot[q + 1];
-            pslot[C::RING - 1] = pfree;
-            const int vfree = vslot[0];
-#pragma unroll
-            for (int q = 0; q + 1 < C::VSTAGES; ++q) vslot[q] = vslot[q + 1];
-            vslot[C::VSTAGES - 1] = vfree;
-        }
+        ps = ring(ps + 1);
+        vs0 = vring(vs0 + 1);
+        o3 = o2; o2 = o1; o1 = o0;
+        o0 = ps * C::P_STAGE;
         return true;
     };
 
@@ -717,6 +704,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         ++u;
     }
 
+    pp.ps = ps;
+    pp.vs = vs0;
+    pp.ph = ph;
     // A normal march waits for every load it issued, so none is in flight here.
     // After a timed-out wait at iteration u_fail, the copies issued for
     // iterations u_fail .. u_fail+D-1 may still be landing: wait for them
@@ -724,9 +714,8 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     if (u_fail <= u1) {
         if (tid == 0) {
             for (int q = 0; q < C::D && u_fail + q <= u1; ++q) {
-                const int ps = pslot[3 + q], vsg = vslot[q];
-                mbar_wait(bar0 + 8u * ps, (pph >> ps) & 1u, a.wait_us);
-                mbar_wait(bar0 + 8u * (C::RING + vsg), (vph >> vsg) & 1u, a.wait_us);
+                const int sl = ring(ps + q);
+                mbar_wait(bar0 + 8u * sl, (ph >> sl) & 1u, a.wait_us);
             }
         }
         __syncthreads();
@@ -754,8 +743,7 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
     const unsigned sbase = smem_base_u32<C>(&smem);
     const unsigned bar0 = sbase + 4u * C::BAR0;
     init_barriers<C>(bar0);
-    Pipe<C> pp;
-    pp.init();
+    Pipe pp;
     fused_tile<C, PEER, WALLS>(a, &tmP, &tmX, &tmY, &tmZ, blockIdx.x, blockIdx.y, seg_len, tiles_k, smem,
                                sbase, bar0, pp);
 }
@@ -779,8 +767,7 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
     const unsigned sbase = smem_base_u32<C>(&smem);
     const unsigned bar0 = sbase + 4u * C::BAR0;
     init_barriers<C>(bar0);
-    Pipe<C> pp;
-    pp.init();
+    Pipe pp;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
