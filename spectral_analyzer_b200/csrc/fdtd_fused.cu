@@ -273,7 +273,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     }
     __syncthreads();
 
-    // Loads feeding iteration u (issued by thread 0): P plane u, Vx face u-2,
+    // Loads feeding iteration u (issued by one thread): P plane u, Vx face u-2,
     // Vy/Vz of plane u-3, all on the plane's mbarrier.
     auto issue = [&](int u, int ps, int vsg) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -292,7 +292,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         }
     };
 
-    if (acquire_maps && tid == 0) {
+    if (acquire_maps && tid == C::NT / 2) {
         acquire_tensormap(tmP);
         acquire_tensormap(tmX);
         acquire_tensormap(tmY);
@@ -307,7 +307,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     unsigned ph = pp.ph;
     auto ring = [&](int q) { return q >= C::RING ? q - C::RING : q; };
     auto vring = [&](int q) { return q >= C::VSTAGES ? q - C::VSTAGES : q; };
-    if (tid == 0)
+    // the issuing thread is in a warp without a second Vy row or halo Vz faces
+    const bool issuer = tid == C::NT / 2;
+    if (issuer)
         for (int q = 0; q < C::D; ++q) issue(u0 + q, ring(ps + q), vring(vs0 + q));
     // stage offsets (floats) of planes u-3 .. u, rotated each iteration
     int o0 = ps * C::P_STAGE, o1 = 0, o2 = 0, o3 = 0;
@@ -392,6 +394,33 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         if (fast_lo >= fast_hi) fast_lo = fast_hi = u1 + 1;
     }
 
+    // What the interior body needs of this thread's items, worked out once: the
+    // existence and gradient order of its Vy faces (jmid: every Vy face of the
+    // tile exists and is of 4th order), its halo Vz face (offsets of P in a P
+    // stage and of the velocity in a V stage, order, damping), the iteration
+    // whose plane receives the source sample in this CTA, and the places of its
+    // results in memory, advanced plane by plane.
+    const bool jmid = j0 - 2 > 0 && j0 + C::TJ < ny - 2;
+    const int jfa = j0 - 2 + w, jfb = j0 - 2 + C::TJ + w;
+    const bool ya_ok = jfa >= 0 && jfa <= ny - 2, yb_ok = jfb >= 0 && jfb <= ny - 2;
+    const bool ya_4 = jfa > 0 && jfa < ny - 2, yb_4 = jfb > 0 && jfb < ny - 2;
+    const int hl = tid - (C::NT - 32 * C::HW);
+    const int h_j = hl / 3, h_c = hl - 3 * h_j < 2 ? 2 + hl - 3 * h_j : C::TK + 4, h_k = k0 - 4 + h_c;
+    const bool h_mine = hl >= 0 && hl < 3 * C::TJ, h_ok = h_mine && j0 + h_j < ny && h_k >= 0 && h_k <= nz - 2;
+    const bool h_4 = h_k > 0 && h_k < nz - 2;
+    float h_d = 1.0f;
+    if (h_ok) h_d = face_damp(fmaxf(ay_s[h_j + 2], az_s[h_c]), fmaxf(ay_s[h_j + 2], az_s[h_c + 1]), cf.dt);
+    const int h_p = (h_j + 3) * C::PC + h_c, h_v = h_j * C::PC + h_c;
+    int dep_u = kNoPlane, dep_at = 0;
+    if (a.dep_sig && tid == 0) {
+        const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 4);
+        if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC) {
+            dep_u = a.dep_i;
+            dep_at = dj * C::PC + dk;
+        }
+    }
+    float *gX = nullptr, *gYa = nullptr, *gYb = nullptr, *gZ = nullptr, *gP = nullptr;
+
     // One iteration of the march; FAST = the interior body.  False when a load
     // wait ran out (u_fail is then set).
     auto iteration = [&](const int u, auto fast_tag) -> bool {
@@ -416,24 +445,17 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                         pf_y1 = ldg4(a.fr[1] + ib + (long long)jf1 * sz + kb);
                 }
                 if (a.fr[2] && st_ok) pf_z = ldg4(a.fr[2] + ib + own);
-                const int hl = tid - (C::NT - 32 * C::HW);
-                if (a.fr[2] && hl >= 0 && hl < 3 * C::TJ) {
-                    const int jl = hl / 3, which = hl - 3 * jl;
-                    const int kf = k0 - 4 + (which < 2 ? 2 + which : C::TK + 4);
-                    if (j0 + jl < ny && kf >= 0 && kf <= nz - 2)
-                        pf_h = __ldg(a.fr[2] + ib + (long long)(j0 + jl) * sz + kf);
-                }
+                if (a.fr[2] && h_ok) pf_h = __ldg(a.fr[2] + ib + (long long)(j0 + h_j) * sz + h_k);
                 if (a.solid && row_ok && kb < sz)
                     pf_s = __ldg(reinterpret_cast<const unsigned*>(a.solid + ib + own));
             }
         }
         const bool ok = mbar_wait(bar0 + 8u * ps, (ph >> ps) & 1u, a.wait_us);
         // the source deposit, on the arriving plane's shared copy before anyone reads it
-        if (a.dep_sig && u == a.dep_i && tid == 0 && ok) {
-            const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 4);
+        if (u == dep_u && ok) {
             const float amp = a.dep_sig[a.dep_step];
-            if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC && amp != 0.0f) {
-                float* c = smem + C::RING0 + o0 + dj * C::PC + dk;
+            if (amp != 0.0f) {
+                float* c = smem + C::RING0 + o0 + dep_at;
                 *c = fadd(*c, amp);
             }
         }
@@ -444,9 +466,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         }
         ph ^= 1u << ps;
         // iteration u+D's loads go into the slots iteration u-1 freed (their last
-        // reads came before the barrier above), so thread 0 issues them before
-        // its own work of this iteration rather than after it
-        if (tid == 0 && u + C::D <= u1) issue(u + C::D, ring(ps + C::D), vring(vs0 + C::D));
+        // reads came before the barrier above), so the issuing thread issues them
+        // before its own work of this iteration rather than after it
+        if (issuer && u + C::D <= u1) issue(u + C::D, ring(ps + C::D), vring(vs0 + C::D));
         float ax_next = 0.0f, px_next = 1.0f;
         if constexpr (!FAST) {
             ax_next = ax_at(u + 1);
@@ -459,7 +481,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
             const int f = u - 2, fg = f + xg0;
             float4 vnew = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 vdiv = vnew;   // WALLS: the value the divergence sees
-            if (FAST ? row_ok : (fg >= 0 && fg <= nxg - 2 && row_ok)) {
+            if (FAST || (fg >= 0 && fg <= nxg - 2 && row_ok)) {   // rows beyond the room hold zeros
                 const float4 pm = lds4(smem + C::RING0 + o3 + cP);
                 const float4 p0 = lds4(smem + C::RING0 + o2 + cP);
                 const float4 p1 = lds4(smem + C::RING0 + o1 + cP);
@@ -493,7 +515,8 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                     }
                 }
                 if (f >= i_beg && f < i_end && st_ok) {
-                    stg4(a.vout[0] + f * PL + own, vnew);
+                    if constexpr (FAST) stg4(gX, vnew);
+                    else stg4(a.vout[0] + f * PL + own, vnew);
 #pragma unroll
                     for (int sd = 0; sd < 2; ++sd)   // the neighbours' ghost faces
                         if (PEER && a.pr.vx[sd] && f >= a.pr.v_lo[sd] && f < a.pr.v_hi[sd])
@@ -515,53 +538,74 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                 const long long ib = i * PL;
 
                 // Vy rows: row w, and row TJ+w for the first VYR-TJ warps
-#pragma unroll
-                for (int m = 0; m < NY_IT; ++m) {
-                    const int r = m == 0 ? w : C::TJ + w;
-                    if (r < C::VYR) {
-                        const int jf = j0 - 2 + r;
-                        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (jf >= 0 && jf <= ny - 2) {
-                            const float* pc = pst + 4 * lane + 4;
-                            const float4 pm = lds4(pc + r * C::PC), p0 = lds4(pc + (r + 1) * C::PC);
-                            const float4 p1 = lds4(pc + (r + 2) * C::PC), p2 = lds4(pc + (r + 3) * C::PC);
-                            const float4 vo = lds4(vys + r * C::TK + 4 * lane);
-                            if constexpr (FAST) {
-                                // the row's gradient order is uniform over its threads
-                                if (jf > 0 && jf < ny - 2) v = vel4(cf, pm, p0, p1, p2, vo, dyi[m]);
-                                else v = vel4_2nd(cf, p0, p1, vo, dyi[m]);
-                            } else {
-                                const bool fourth = (jf > 0 && jf < ny - 2);
-                                if (fourth && xint && kfull) {
-                                    v = vel4(cf, pm, p0, p1, p2, vo, dyi[m]);
-                                } else {
-                                    float4 aL, aR;
-                                    int oky = 0;
-#pragma unroll
-                                    for (int q = 0; q < 4; ++q) {
-                                        const float azk = az_s[4 * lane + 4 + q];
-                                        at(aL, q) = fmaxf(fmaxf(axi, ay_s[r]), azk);
-                                        at(aR, q) = fmaxf(fmaxf(axi, ay_s[r + 1]), azk);
-                                        oky |= (kb + q < nz) ? (1 << q) : 0;
-                                    }
-                                    v = vel4_general(cf, pm, p0, p1, p2, vo, aL, aR, fourth ? 15 : 0, oky);
-                                }
-                            }
-                            float4 fry = make_float4(1.f, 1.f, 1.f, 1.f);
-                            if constexpr (WALLS) {
-                                if (a.fr[1] && kb < sz) {
-                                    fry = m == 0 ? pf_y0 : pf_y1;
-                                    v = close4(v, fry);
-                                }
-                            }
-                            if (r >= 2 && r < C::TJ + 2 && kb < sz)
-                                stg4(a.vout[1] + ib + (long long)jf * sz + kb, v);
-                            if constexpr (WALLS) {
-                                if (a.fr[1] && a.frac_div && kb < sz) v = mul4(v, fry);
-                            }
+                if constexpr (FAST) {
+                    const float* pc = pst + 4 * lane + 4;
+                    auto row = [&](int r, const float4& dmp, bool ex, bool f4, float4 fry, float* dst) {
+                        const float4 pm = lds4(pc + r * C::PC), p0 = lds4(pc + (r + 1) * C::PC);
+                        const float4 p1 = lds4(pc + (r + 2) * C::PC), p2 = lds4(pc + (r + 3) * C::PC);
+                        const float4 vo = lds4(vys + r * C::TK + 4 * lane);
+                        float4 v;
+                        if (jmid) v = vel4(cf, pm, p0, p1, p2, vo, dmp);
+                        else v = vel4_masked(cf, pm, p0, p1, p2, vo, dmp, f4 ? 15 : 0, ex ? 15 : 0);
+                        if constexpr (WALLS) {
+                            if (a.fr[1] && kb < sz && ex) v = close4(v, fry);
+                        }
+                        if (dst) stg4(dst, v);
+                        if constexpr (WALLS) {
+                            if (a.fr[1] && a.frac_div && kb < sz && ex) v = mul4(v, fry);
                         }
                         sts4(vyn + r * C::TK + 4 * lane, v);
+                    };
+                    // own rows are r = 2 .. TJ+1 of the tile's Vy rows
+                    row(w, dyi[0], ya_ok, ya_4, pf_y0, w >= 2 && ya_ok && kb < sz ? gYa : nullptr);
+                    if (C::TJ + w < C::VYR)
+                        row(C::TJ + w, dyi[1], yb_ok, yb_4, pf_y1, w < 2 && yb_ok && kb < sz ? gYb : nullptr);
+                } else {
+#pragma unroll
+                    for (int m = 0; m < NY_IT; ++m) {
+                        const int r = m == 0 ? w : C::TJ + w;
+                        if (r < C::VYR) {
+                            const int jf = j0 - 2 + r;
+                            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (jf >= 0 && jf <= ny - 2) {
+                                const float* pc = pst + 4 * lane + 4;
+                                const float4 pm = lds4(pc + r * C::PC), p0 = lds4(pc + (r + 1) * C::PC);
+                                const float4 p1 = lds4(pc + (r + 2) * C::PC), p2 = lds4(pc + (r + 3) * C::PC);
+                                const float4 vo = lds4(vys + r * C::TK + 4 * lane);
+                                {
+                                    const bool fourth = (jf > 0 && jf < ny - 2);
+                                    if (fourth && xint && kfull) {
+                                        v = vel4(cf, pm, p0, p1, p2, vo, dyi[m]);
+                                    } else {
+                                        float4 aL, aR;
+                                        int oky = 0;
+#pragma unroll
+                                        for (int q = 0; q < 4; ++q) {
+                                            const float azk = az_s[4 * lane + 4 + q];
+                                            at(aL, q) = fmaxf(fmaxf(axi, ay_s[r]), azk);
+                                            at(aR, q) = fmaxf(fmaxf(axi, ay_s[r + 1]), azk);
+                                            oky |= (kb + q < nz) ? (1 << q) : 0;
+                                        }
+                                        v = vel4_general(cf, pm, p0, p1, p2, vo, aL, aR, fourth ? 15 : 0, oky);
+                                    }
+                                }
+                                float4 fry = make_float4(1.f, 1.f, 1.f, 1.f);
+                                if constexpr (WALLS) {
+                                    if (a.fr[1] && kb < sz) {
+                                        fry = m == 0 ? pf_y0 : pf_y1;
+                                        v = close4(v, fry);
+                                    }
+                                }
+                                if (r >= 2 && r < C::TJ + 2 && kb < sz)
+                                    stg4(a.vout[1] + ib + (long long)jf * sz + kb, v);
+                                if constexpr (WALLS) {
+                                    if (a.fr[1] && a.frac_div && kb < sz) v = mul4(v, fry);
+                                }
+                            }
+                            sts4(vyn + r * C::TK + 4 * lane, v);
+                        }
                     }
+
                 }
 
                 // Vz: own faces kb .. kb+3 of row jr
@@ -569,7 +613,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                 {
                     const float* prow = pst + (w + 3) * C::PC;
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (row_ok) {
+                    if (FAST || row_ok) {
                         const int c = 4 * lane + 4;            // col of kb
                         pown = lds4(prow + c);
                         const float4 pb4 = lds4(prow + c + 4);
@@ -598,7 +642,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                                 v = close4(v, frz);
                             }
                         }
-                        if (st_ok) stg4(a.vout[2] + ib + own, v);
+                        if (st_ok) stg4(FAST ? gZ : a.vout[2] + ib + own, v);
                         if constexpr (WALLS) {
                             if (a.fr[2] && a.frac_div && st_ok) v = mul4(v, frz);
                         }
@@ -607,20 +651,17 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                 }
                 // halo Vz faces k0-2, k0-1, k0+TK of every row: 3*TJ faces, one per
                 // thread of the last HW warps
-                const int hl = tid - (C::NT - 32 * C::HW);
-                if (hl >= 0 && hl < 3 * C::TJ) {
-                    const int jl = hl / 3, which = hl - 3 * jl;
-                    const int ch = which < 2 ? 2 + which : C::TK + 4;
-                    const int kf = k0 - 4 + ch;
-                    const float* prow = pst + (jl + 3) * C::PC;
+                if (h_mine) {
+                    const float* pr = pst + h_p;
                     float vh = 0.0f;
-                    if (j0 + jl < ny && kf >= 0 && kf <= nz - 2) {
-                        const bool fourth = (kf > 0 && kf < nz - 2);
-                        const float ay = ay_s[jl + 2];
-                        const float gr = grad4(cf, prow[ch - 1], prow[ch], prow[ch + 1], prow[ch + 2], fourth);
-                        const float dmp = face_damp(fmaxf(fmaxf(axi, ay), az_s[ch]),
-                                                    fmaxf(fmaxf(axi, ay), az_s[ch + 1]), cf.dt);
-                        vh = vupd(cf, vzs[jl * C::PC + ch], gr, dmp);
+                    if (h_ok) {
+                        const float gr = grad4(cf, pr[-1], pr[0], pr[1], pr[2], h_4);
+                        float dmp = h_d;
+                        if constexpr (!FAST) {
+                            const float mxy = fmaxf(axi, ay_s[h_j + 2]);
+                            dmp = face_damp(fmaxf(mxy, az_s[h_c]), fmaxf(mxy, az_s[h_c + 1]), cf.dt);
+                        }
+                        vh = vupd(cf, vzs[h_v], gr, dmp);
                         if constexpr (WALLS) {
                             if (a.fr[2]) {
                                 const float fz = pf_h;
@@ -629,12 +670,12 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                             }
                         }
                     }
-                    vzn[jl * C::PC + ch] = vh;
+                    vzn[h_v] = vh;
                 }
                 __syncthreads();
 
                 // P^{n+1} of the own cells
-                if (row_ok) {
+                if (FAST || row_ok) {
                     const float* yr = vyn + 4 * lane;
                     const float4 ymm = lds4(yr + w * C::TK), ym = lds4(yr + (w + 1) * C::TK);
                     const float4 yp = lds4(yr + (w + 2) * C::TK), ypp = lds4(yr + (w + 3) * C::TK);
@@ -667,8 +708,8 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                                 if ((sol >> (8 * q)) & 0xFFu) at(out, q) = 0.0f;
                         }
                     }
-                    if (kb < sz) {
-                        stg4(a.pn + ib + own, out);
+                    if (FAST ? st_ok : kb < sz) {
+                        stg4(FAST ? gP : a.pn + ib + own, out);
 #pragma unroll
                         for (int sd = 0; sd < 2; ++sd)   // the neighbours' ghost planes
                             if (PEER && a.pr.pn[sd] && i >= a.pr.p_lo[sd] && i < a.pr.p_hi[sd])
@@ -686,12 +727,21 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         vs0 = vring(vs0 + 1);
         o3 = o2; o2 = o1; o1 = o0;
         o0 = ps * C::P_STAGE;
+        if constexpr (FAST) {
+            gX += PL; gYa += PL; gYb += PL; gZ += PL; gP += PL;
+        }
         return true;
     };
 
     for (int u = u0; u <= u1;) {
         if (u == fast_lo) {
             bool ran = true;
+            const long long ib = (long long)(u - 3) * PL;
+            gX = a.vout[0] + ib + PL + own;
+            gYa = a.vout[1] + ib + (long long)jfa * sz + kb;
+            gYb = a.vout[1] + ib + (long long)jfb * sz + kb;
+            gZ = a.vout[2] + ib + own;
+            gP = a.pn + ib + own;
             for (; u < fast_hi; ++u)
                 if (!iteration(u, std::true_type{})) { ran = false; break; }
             if (!ran) break;
