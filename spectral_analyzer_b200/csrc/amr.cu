@@ -30,6 +30,7 @@
  * (:680-895, :1318-1410, :1412-1532, :1647-1760), then uploaded once.
  */
 #include "acoustic_amr_b200.h"
+#include "launch.h"
 
 #include <cuda_runtime.h>
 
@@ -115,16 +116,8 @@ struct PlateDev {
     float dt;
 };
 
-// The step's kernels are launched with programmatic stream serialisation: a
-// kernel's blocks start while the one before drains, read what never changes
-// during a window (topology, coefficients) and only then wait for its results.
-// The dependents are released after the wait, so a kernel that has started
-// knows that everything before its predecessor is complete.
-__device__ __forceinline__ void wait_previous()
-{
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
+// The step's kernels overlap (launch.h): before waiting for the one before they
+// fetch what never changes during a window, the topology and the coefficients.
 
 constexpr int kOrigin = INT_MIN;   // stencil offset of an unused slot: it reads cell 0
 
@@ -201,6 +194,7 @@ __global__ void __launch_bounds__(256) k_amr_velocity(int n_faces, const float* 
         }
     }
     wait_previous();
+    release_next();
     if (!in || *status < step) return;
     auto face = [&](int q) {
         const int f = f0 + q;
@@ -273,6 +267,7 @@ __global__ void __launch_bounds__(256) k_amr_pressure(int n_cells, float* __rest
             if (k < n) x[k] = e[32 * k];
     }
     wait_previous();
+    release_next();
     if (!in || *status < step) return;
     float out = 0.0f;
     if (n >= 0) {
@@ -321,6 +316,7 @@ __global__ void k_amr_plate(int n_nodes, const int* __restrict__ node_entry, con
     const int flat = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = flat < n_nodes ? node_entry[flat] : -1;
     wait_previous();
+    release_next();
     if (flat >= n_nodes || *status < step) return;
     if (n >= 0) {
         float pa = 0.0f, pb = 0.0f;
@@ -441,21 +437,6 @@ __global__ void k_amr_mics(int n_mics, const float* __restrict__ p, const float*
 }
 
 inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
-
-template <class... A>
-cudaError_t launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, A... args)
-{
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, args...);
-}
 
 constexpr int kNearestBlocks = 148;
 
@@ -887,17 +868,17 @@ int launch_steps(AcousticAMRState* st, int n_steps)
                             reinterpret_cast<const float4*>(st->d_swgt), st->d_scell, st->d_scoef};
         const int* const bc = st->plate ? st->d_bc : nullptr;
         AK(launch_after(st->order == 8 ? k_amr_velocity<8> : k_amr_velocity<2>,
-                        blocks(st->n_faces, st->order == 8 ? 256 : 1024), 256, st->stream, st->n_faces,
+                        blocks(st->n_faces, st->order == 8 ? 256 : 1024), 256, 0, st->stream, st->n_faces,
                         (const float*)st->d_p, st->d_v, (const float*)st->d_vdamp, (const float*)st->d_inv_d,
                         (const int*)st->d_neg, (const int*)st->d_pos, sten, bc, (const int*)st->d_bc_flat, pl,
                         dt_over_rho, (const unsigned*)st->d_status, step));
-        AK(launch_after(k_amr_pressure, blocks(st->n_cells, 256), 256, st->stream, st->n_cells, st->d_p,
+        AK(launch_after(k_amr_pressure, blocks(st->n_cells, 256), 256, 0, st->stream, st->n_cells, st->d_p,
                         (const float*)st->d_v, (const float*)st->d_pdamp, (const float*)st->d_psrc,
                         (const float*)st->d_inv_den, (const int*)st->d_meta, (const int*)st->d_slice,
                         (const int2*)st->d_inc, bulk, st->d_status, step, (step & 0xFFu) == 0 ? 1 : 0));
         st->launches += 2;
         if (st->plate) {
-            AK(launch_after(k_amr_plate, blocks(st->p_nodes, 128), 128, st->stream, st->p_nodes,
+            AK(launch_after(k_amr_plate, blocks(st->p_nodes, 128), 128, 0, st->stream, st->p_nodes,
                             (const int*)st->d_node_entry, (const int*)st->d_astart, (const float*)st->d_awgt,
                             (const int*)st->d_acell, (const int*)st->d_bstart, (const float*)st->d_bwgt,
                             (const int*)st->d_bcell, (const int*)st->d_cabove, (const int*)st->d_cbelow,

@@ -40,6 +40,7 @@
  */
 #include "fdtd_internal.h"
 #include "fdtd_tma.h"
+#include "launch.h"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -232,13 +233,15 @@ __device__ __forceinline__ void init_barriers(unsigned bar0)
 // walled-scene rules of the two-pass kernels to the general body: a face whose
 // open fraction is 0 is closed (its new velocity is 0), the divergence sees
 // each face's velocity times its fraction (when fractions were set), and
-// solid cells keep P = 0, in both the interior and the general body.
-template <class C, bool PEER = true, bool WALLS = false>
+// solid cells keep P = 0, in both the interior and the general body.  start()
+// runs before the first load (it waits for what the loads read) and says what
+// to do once the first loads are on their way.
+template <class C, bool PEER = true, bool WALLS = false, class Start>
 __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap* tmP,
                                            const CUtensorMap* tmX, const CUtensorMap* tmY,
                                            const CUtensorMap* tmZ, int tile, int seg, int seg_len,
                                            int tiles_k, float* smem, unsigned sbase, unsigned bar0,
-                                           Pipe& pp, bool acquire_maps = false)
+                                           Pipe& pp, Start start)
 {
     float* const vyn = smem + C::VYN0;
     float* const vzn = smem + C::VZN0;
@@ -292,12 +295,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         }
     };
 
-    if (acquire_maps && tid == C::NT / 2) {
-        acquire_tensormap(tmP);
-        acquire_tensormap(tmX);
-        acquire_tensormap(tmY);
-        acquire_tensormap(tmZ);
-    }
+    auto started = start();
     const int u0 = i_beg - 3, u1 = i_end + 2;
     // Plane v of the march lives in ring slot (ps + v - u0) mod RING, iteration
     // v's V data in stage (vs + v - u0) mod VSTAGES: at iteration u planes u-3
@@ -311,6 +309,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     const bool issuer = tid == C::NT / 2;
     if (issuer)
         for (int q = 0; q < C::D; ++q) issue(u0 + q, ring(ps + q), vring(vs0 + q));
+    started();
     // stage offsets (floats) of planes u-3 .. u, rotated each iteration
     int o0 = ps * C::P_STAGE, o1 = 0, o2 = 0, o3 = 0;
     {
@@ -783,11 +782,6 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
                                                       const __grid_constant__ CUtensorMap tmZ,
                                                       int seg_len, int tiles_k)
 {
-    if (a.n_rec > 0) {   // the previous step's receivers, from this step's input P
-        const int nblk = gridDim.x * gridDim.y, b = blockIdx.x + gridDim.x * blockIdx.y;
-        for (int r = b + nblk * (int)threadIdx.x; r < a.n_rec; r += nblk * C::NT)
-            a.rec_out[r] = sample8(a.p, a.rec_idx + 8 * r, a.rec_w + 8 * r);
-    }
     if ((int)blockIdx.y * seg_len >= (a.xs.nxg > 0 ? a.xs.n_own : a.g.nx)) return;
     float* smem;
     const unsigned sbase = smem_base_u32<C>(&smem);
@@ -795,9 +789,15 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
     init_barriers<C>(bar0);
     Pipe pp;
     fused_tile<C, PEER, WALLS>(a, &tmP, &tmX, &tmY, &tmZ, blockIdx.x, blockIdx.y, seg_len, tiles_k, smem,
-                               sbase, bar0, pp);
+                               sbase, bar0, pp, [&] {
+        return [&] {
+            // the previous step's receivers, from this step's input P
+            const int nblk = gridDim.x * gridDim.y, b = blockIdx.x + gridDim.x * blockIdx.y;
+            for (int r = b + nblk * (int)threadIdx.x; r < a.n_rec; r += nblk * C::NT)
+                a.rec_out[r] = sample8(a.p, a.rec_idx + 8 * r, a.rec_w + 8 * r);
+        };
+    });
 }
-
 
 // Batched step: a persistent kernel whose CTAs pull (member, tile, segment)
 // work items from a device counter until the list is exhausted; members at
@@ -811,13 +811,15 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
                                                           unsigned* __restrict__ status)
 {
     __shared__ int s_item;
-    const int total_items = hdr->total_items;
-    int* const counter = &hdr->counter;
     float* smem;
     const unsigned sbase = smem_base_u32<C>(&smem);
     const unsigned bar0 = sbase + 4u * C::BAR0;
     init_barriers<C>(bar0);
     Pipe pp;
+    wait_previous();
+    release_next();
+    const int total_items = hdr->total_items;
+    int* const counter = &hdr->counter;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
@@ -843,8 +845,11 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
         a.pr = XPeers{};
         const int local = item - m->items_begin;
         if (!fused_tile<C, false>(a, &m->maps[par][0], &m->maps[par][1], &m->maps[par][2], &m->maps[par][3],
-                           local % m->tiles, local / m->tiles, m->seg_len, m->tiles_k, smem, sbase,
-                           bar0, pp, true))
+                           local % m->tiles, local / m->tiles, m->seg_len, m->tiles_k, smem, sbase, bar0, pp, [&] {
+            if (threadIdx.x == C::NT / 2)   // the thread that issues the loads
+                for (int q = 0; q < 4; ++q) acquire_tensormap(&m->maps[par][q]);
+            return [] {};
+        }))
             break;
     }
 }
@@ -855,22 +860,49 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
 // record after step n, deposit before step n+1).  One block per member.  A
 // member whose check fails stops at that step without the next deposit, the
 // state a single room is left in when its step returns UNSTABLE; the batch
-// steps it no further until its set is rebuilt.
-__global__ void k_batch_epilogue(BatchMember* __restrict__ mem, const BatchHeader* __restrict__ hdr)
+// steps it no further until its set is rebuilt.  The first block also returns
+// the work-item counter to zero for the next step.
+__global__ void __launch_bounds__(128) k_batch_epilogue(BatchMember* __restrict__ mem, BatchHeader* __restrict__ hdr)
 {
     const int r = blockIdx.x;
-    if (r >= hdr->n_members) return;
+    const bool in = r < hdr->n_members;
     BatchMember* m = mem + r;
-    const int s = m->step;
-    if (s >= m->limit || m->unstable != 0xFFFFFFFFu) return;
+    // a member's description does not change between steps: fetch it, and the
+    // taps of this thread's receiver, while the step's last tiles finish
+    float *p0 = nullptr, *p1 = nullptr, *trace = nullptr, w[8];
+    long long idx[8];
+    int n_rec = 0, step0 = 0, limit = 0, trace0 = 0, trace_cap = 0;
+    if (in) {
+        p0 = m->p[0];
+        p1 = m->p[1];
+        trace = m->trace;
+        n_rec = m->n_rec;
+        step0 = m->step0;
+        limit = m->limit;
+        trace0 = m->trace0;
+        trace_cap = m->trace_cap;
+        if ((int)threadIdx.x < n_rec)
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                idx[t] = m->rec_idx[8 * threadIdx.x + t];
+                w[t] = m->rec_w[8 * threadIdx.x + t];
+            }
+    }
+    wait_previous();
+    release_next();
+    if (r == 0 && threadIdx.x == 0) hdr->counter = 0;
+    if (!in) return;
+    const int s = *(volatile int*)&m->step;
+    if (s >= limit || *(volatile unsigned*)&m->unstable != 0xFFFFFFFFu) return;
     const int s1 = s + 1;
-    float* P = m->p[(s1 - m->step0) & 1];
-    const int slot = m->trace0 + (s - m->step0);
-    if (slot < m->trace_cap)
-        for (int q = threadIdx.x; q < m->n_rec; q += blockDim.x)
-            m->trace[(size_t)slot * m->n_rec + q] = sample8(P, m->rec_idx + 8 * q, m->rec_w + 8 * q);
+    float* P = ((s1 - step0) & 1) ? p1 : p0;
+    const int slot = trace0 + (s - step0);
+    if (slot < trace_cap)
+        for (int q = threadIdx.x; q < n_rec; q += blockDim.x)
+            trace[(size_t)slot * n_rec + q] =
+                q < (int)blockDim.x ? sample8(P, idx, w) : sample8(P, m->rec_idx + 8 * q, m->rec_w + 8 * q);
     if ((s1 & (kCheckPeriod - 1)) == 0) {
-        const int n_chk = s1 / kCheckPeriod - m->step0 / kCheckPeriod;
+        const int n_chk = s1 / kCheckPeriod - step0 / kCheckPeriod;
         const long long phase = (m->phase0 + n_chk - 1) % kCheckStride;
         const Grid g = m->g;
         for (long long q = phase + (long long)kCheckStride * threadIdx.x; q < m->n_cells;
@@ -884,7 +916,7 @@ __global__ void k_batch_epilogue(BatchMember* __restrict__ mem, const BatchHeade
     __syncthreads();   // receivers have read P and the check's flags are set
     if (threadIdx.x == 0) {
         const bool stopped = *(volatile unsigned*)&m->unstable != 0xFFFFFFFFu;
-        if (!stopped && s1 < m->limit && s1 < m->ps_n) deposit_apply(m->ps, m->ps_sig[s1], P);
+        if (!stopped && s1 < limit && s1 < m->ps_n) deposit_apply(m->ps, m->ps_sig[s1], P);
         m->step = s1;
     }
 }
@@ -1033,6 +1065,8 @@ static cudaError_t launch_step_of(const FusedArgs& a, FusedCache* cache, cudaStr
     const bool peer = a.pr.pn[0] || a.pr.pn[1] || a.pr.vx[0] || a.pr.vx[1];
     const bool walls = a.fr[0] || a.fr[1] || a.fr[2] || a.solid;
     if (walls && (peer || a.xs.nxg > 0)) return cudaErrorInvalidValue;   // walled scenes are whole rooms
+    // Plain launches: overlapping a step's start with the one before (launch.h)
+    // was slower (512x384x256 room 266.6 -> 281 us, 160x128x112 24.7 -> 25.4).
     if (walls)
         k_fused_step<C, false, true><<<grid, C::NT, C::SMEM_BYTES, s>>>(a, maps[0], maps[1], maps[2], maps[3],
                                                                         seg_len, tiles_k);
@@ -1103,18 +1137,15 @@ cudaError_t launch_fused_batch_step(BatchMember* members, BatchHeader* hdr, cons
                                     unsigned* status, int grid_ctas, int epi_blocks, cudaStream_t s,
                                     int shape)
 {
-    cudaError_t e = cudaMemsetAsync(&hdr->counter, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     if (shape == 1)
-        k_fused_batch<NarrowCfg><<<grid_ctas, NarrowCfg::NT, NarrowCfg::SMEM_BYTES, s>>>(members, hdr, item_member,
-                                                                                       status);
+        e = launch_after(k_fused_batch<NarrowCfg>, dim3(grid_ctas), dim3(NarrowCfg::NT), NarrowCfg::SMEM_BYTES, s, members,
+                         hdr, item_member, status);
     else
-        k_fused_batch<FusedCfg><<<grid_ctas, FusedCfg::NT, FusedCfg::SMEM_BYTES, s>>>(members, hdr, item_member,
-                                                                                     status);
-    e = cudaGetLastError();
+        e = launch_after(k_fused_batch<FusedCfg>, dim3(grid_ctas), dim3(FusedCfg::NT), FusedCfg::SMEM_BYTES, s, members,
+                         hdr, item_member, status);
     if (e != cudaSuccess) return e;
-    k_batch_epilogue<<<epi_blocks, 128, 0, s>>>(members, hdr);
-    return cudaGetLastError();
+    return launch_after(k_batch_epilogue, dim3(epi_blocks), dim3(128), 0, s, members, hdr);
 }
 
 }  // namespace fdtd

@@ -315,7 +315,7 @@ cudaError_t fused_batch_slots(int shape, int* slots);
 struct BatchHeader {
     int n_members;
     int total_items;
-    int counter;                 // work-item counter, reset before each step
+    int counter;                 // work-item counter, zero between steps
 };
 // One batched step: every member below its limit advances one step (fused
 // velocity+pressure over item_member's work items, then the epilogue:
