@@ -226,7 +226,7 @@ __device__ __forceinline__ void init_barriers(unsigned bar0)
     __syncthreads();
 }
 
-// One tile (TJ x TK columns, planes [seg*seg_len, ...)) of the fused step.
+// One tile (TJ x TK columns, own planes [first, first + len)) of the fused step.
 // Returns false when a load wait ran out (the CTA must stop; status is set).
 // PEER = false compiles out the neighbour ghost-plane stores (single rooms and
 // batches), which the slab step of a split room needs.  WALLS = true adds the
@@ -239,7 +239,7 @@ __device__ __forceinline__ void init_barriers(unsigned bar0)
 template <class C, bool PEER = true, bool WALLS = false, class Start>
 __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap* tmP,
                                            const CUtensorMap* tmX, const CUtensorMap* tmY,
-                                           const CUtensorMap* tmZ, int tile, int seg, int seg_len,
+                                           const CUtensorMap* tmZ, int tile, int first, int len,
                                            int tiles_k, float* smem, unsigned sbase, unsigned bar0,
                                            Pipe& pp, Start start)
 {
@@ -260,9 +260,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
     const bool slab = a.xs.nxg > 0;
     const int nxg = slab ? a.xs.nxg : nx, xg0 = slab ? a.xs.xg0 : 0;
     const int own_lo = slab ? a.xs.i_lo : 0, own_hi = slab ? a.xs.i_lo + a.xs.n_own : nx;
-    const int i_beg = own_lo + seg * seg_len;
+    const int i_beg = own_lo + first;
     if (i_beg >= own_hi) return true;
-    const int i_end = min(i_beg + seg_len, own_hi);
+    const int i_end = min(i_beg + len, own_hi);
     const Coef cf = a.cf;
 
     __syncthreads();   // the previous tile's readers of the tables are done
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
     const unsigned bar0 = sbase + 4u * C::BAR0;
     init_barriers<C>(bar0);
     Pipe pp;
-    fused_tile<C, PEER, WALLS>(a, &tmP, &tmX, &tmY, &tmZ, blockIdx.x, blockIdx.y, seg_len, tiles_k, smem,
+    fused_tile<C, PEER, WALLS>(a, &tmP, &tmX, &tmY, &tmZ, blockIdx.x, blockIdx.y * seg_len, seg_len, tiles_k, smem,
                                sbase, bar0, pp, [&] {
         return [&] {
             // the previous step's receivers, from this step's input P
@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
 template <class C>
 __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restrict__ mem,
                                                           BatchHeader* __restrict__ hdr,
-                                                          const int* __restrict__ item_member,
+                                                          const int4* __restrict__ items,
                                                           unsigned* __restrict__ status)
 {
     __shared__ int s_item;
@@ -826,7 +826,8 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
         const int item = s_item;
         __syncthreads();
         if (item >= total_items) break;
-        const BatchMember* m = mem + item_member[item];
+        const int4 it = items[item];   // member, tile, first plane, planes
+        const BatchMember* m = mem + it.x;
         const int step = m->step;
         if (step >= m->limit || m->unstable != 0xFFFFFFFFu) continue;   // done, or stopped unstable
         const int par = (step - m->step0) & 1;
@@ -843,9 +844,8 @@ __global__ void __launch_bounds__(C::NT, 2) k_fused_batch(BatchMember* __restric
         a.status = status;
         a.xs = XSpan{0, 0, 0, 0};
         a.pr = XPeers{};
-        const int local = item - m->items_begin;
         if (!fused_tile<C, false>(a, &m->maps[par][0], &m->maps[par][1], &m->maps[par][2], &m->maps[par][3],
-                           local % m->tiles, local / m->tiles, m->seg_len, m->tiles_k, smem, sbase, bar0, pp, [&] {
+                           it.y, it.z, it.w, m->tiles_k, smem, sbase, bar0, pp, [&] {
             if (threadIdx.x == C::NT / 2)   // the thread that issues the loads
                 for (int q = 0; q < 4; ++q) acquire_tensormap(&m->maps[par][q]);
             return [] {};
@@ -1133,17 +1133,17 @@ cudaError_t fused_batch_slots(int shape, int* slots)
     return shape == 1 ? batch_slots_of<NarrowCfg>(slots) : batch_slots_of<FusedCfg>(slots);
 }
 
-cudaError_t launch_fused_batch_step(BatchMember* members, BatchHeader* hdr, const int* item_member,
+cudaError_t launch_fused_batch_step(BatchMember* members, BatchHeader* hdr, const int4* items,
                                     unsigned* status, int grid_ctas, int epi_blocks, cudaStream_t s,
                                     int shape)
 {
     cudaError_t e;
     if (shape == 1)
         e = launch_after(k_fused_batch<NarrowCfg>, dim3(grid_ctas), dim3(NarrowCfg::NT), NarrowCfg::SMEM_BYTES, s, members,
-                         hdr, item_member, status);
+                         hdr, items, status);
     else
         e = launch_after(k_fused_batch<FusedCfg>, dim3(grid_ctas), dim3(FusedCfg::NT), FusedCfg::SMEM_BYTES, s, members,
-                         hdr, item_member, status);
+                         hdr, items, status);
     if (e != cudaSuccess) return e;
     return launch_after(k_batch_epilogue, dim3(epi_blocks), dim3(128), 0, s, members, hdr);
 }

@@ -292,7 +292,7 @@ struct alignas(64) BatchMember {
     float* v[2][3];
     int step;                    // device step counter (advanced by the epilogue)
     int step0, limit;            // step count on joining; stop at this step count
-    int items_begin, tiles, tiles_k, seg_len;
+    int tiles_k;
     // point source
     Deposit ps;
     const float* ps_sig;
@@ -318,10 +318,11 @@ struct BatchHeader {
     int counter;                 // work-item counter, zero between steps
 };
 // One batched step: every member below its limit advances one step (fused
-// velocity+pressure over item_member's work items, then the epilogue:
+// velocity+pressure over the work items {member, tile, first plane, planes},
+// then the epilogue:
 // receivers, step counter, 256-step check, next source sample).  epi_blocks
 // is the member capacity (blocks beyond n_members exit at once).
-cudaError_t launch_fused_batch_step(BatchMember* members, BatchHeader* hdr, const int* item_member,
+cudaError_t launch_fused_batch_step(BatchMember* members, BatchHeader* hdr, const int4* items,
                                     unsigned* status, int grid_ctas, int epi_blocks, cudaStream_t s, int shape = 0);
 
 }  // namespace fdtd
