@@ -3,8 +3,9 @@
  * 16-bit storage modes: BF16, FP16 (scaled), and their compensated forms
  * (value + 16-bit residual).
  *
- * The march is the FP32 step kernel's (fdtd_fused.cu): a CTA owns an 8 x 128
- * (j, k) tile, marches along i over a segment of planes, and one thread issues
+ * The march is the FP32 step kernel's (fdtd_fused.cu): a CTA owns an 8 x 128 or
+ * 16 x 64 (j, k) tile (the one that leaves less of the last k tile idle),
+ * marches along i over a segment of planes, and one thread issues
  * the TMA boxes of each plane (P with a 3-row / 8-column halo, Vx, Vy with its
  * halo rows, Vz with its halo columns) into a shared-memory ring D planes
  * ahead, completed by mbarriers with bounded waits.  The boxes carry the
@@ -41,11 +42,13 @@ namespace prec {
 
 namespace {
 
-template <int M, int D_>
+// TJ rows x TK = 4*LW columns per CTA, LW threads per row, four k per thread.
+template <int M, int D_, int TJ_, int LW_>
 struct H16 {
     static constexpr bool COMP = Traits<M>::comp;
     static constexpr int NB = COMP ? 2 : 1;     // stored arrays per field
-    static constexpr int TJ = 8, TK = 128, NT = 256, D = D_;   // one warp per row, 4 k per lane
+    static constexpr int TJ = TJ_, LW = LW_, TK = 4 * LW, NT = TJ * LW, D = D_;
+    static constexpr int HW = (3 * TJ + 31) / 32;   // warps computing the halo Vz faces
     static constexpr int PR = TJ + 6;           // P rows j0-3 .. j0+TJ+2
     static constexpr int PC = TK + 16;          // P / Vz cols k0-8 .. k0+TK+7 (elements)
     static constexpr int VYR = TJ + 3;          // Vy rows j0-2 .. j0+TJ
@@ -69,7 +72,7 @@ struct H16 {
     static constexpr int AY0 = VZN0 + r128(4 * TJ * ZC);            // float [TJ+4]
     static constexpr int AZ0 = AY0 + r128(4 * (TJ + 4));            // float [ZC]
     static constexpr int BAR0 = AZ0 + r128(4 * ZC);
-    static constexpr size_t SMEM_BYTES = BAR0 + 8 * (RING + VSTAGES) + 128;
+    static constexpr size_t SMEM_BYTES = BAR0 + 8 * RING + 128;
     static constexpr unsigned P_BYTES = NB * P_B, VX_BYTES = NB * VX_B, VYZ_BYTES = NB * (VY_B + VZ_B);
     static_assert((PC * 2) % 16 == 0 && (TK * 2) % 16 == 0, "TMA box rows are 16-byte multiples");
     static_assert(PC <= 256 && PR <= 256, "TMA box extent");
@@ -170,8 +173,9 @@ __device__ __forceinline__ float& at4(float4& v, int q) { return reinterpret_cas
 
 __device__ __forceinline__ float grad(const PCoef<float>& cf, float pm, float p0, float p1, float p2, bool fourth)
 {
-    return fourth ? __fadd_rn(__fmul_rn(cf.c1, __fsub_rn(p1, p0)), __fmul_rn(cf.c2, __fsub_rn(p2, pm)))
-                  : __fsub_rn(p1, p0);
+    // both orders, then a selection: a branch per face costs more than the products
+    const float d = __fsub_rn(p1, p0), w = __fadd_rn(__fmul_rn(cf.c1, d), __fmul_rn(cf.c2, __fsub_rn(p2, pm)));
+    return fourth ? w : d;
 }
 
 __device__ __forceinline__ float vup(const PCoef<float>& cf, float vo, float gr, float dmp)
@@ -192,7 +196,8 @@ __device__ __forceinline__ float4 vel4m(const PCoef<float>& cf, float4 pm, float
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const float gr = grad(cf, at4(pm, q), at4(p0, q), at4(p1, q), at4(p2, q), (m4 >> q) & 1);
-        at4(r, q) = ((ok >> q) & 1) ? vup(cf, at4(vo, q), gr, at4(dmp, q)) : 0.0f;
+        const float v = vup(cf, at4(vo, q), gr, at4(dmp, q));
+        at4(r, q) = ((ok >> q) & 1) ? v : 0.0f;
     }
     return r;
 }
@@ -211,11 +216,11 @@ struct Maps16 {
     CUtensorMap m[8];   // P, Vx, Vy, Vz: value map, then residual map
 };
 
-template <int M>
-__global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constant__ Maps16 mp, int seg_len,
-                                                  int tiles_k)
+template <int M, int TJ, int LW>
+__global__ void __launch_bounds__(TJ * LW) k_fused16(F16Args a, const __grid_constant__ Maps16 mp, int seg_len,
+                                                     int tiles_k)
 {
-    using C = H16<M, depth16<M>()>;
+    using C = H16<M, depth16<M>(), TJ, LW>;
     using K = Code<M>;
     const Grid g = a.g;
     const int nx = g.nx, ny = g.ny, nz = g.nz, sz = g.sz;
@@ -248,12 +253,12 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
     float* const ay_s = reinterpret_cast<float*>(sm + C::AY0);
     float* const az_s = reinterpret_cast<float*>(sm + C::AZ0);
 
-    const int lane = tid % 32, w = tid / 32;
+    const int lane = tid % C::LW, w = tid / C::LW;   // float4 column in the row, row in the tile
     const int tile = blockIdx.x, tk = tile % tiles_k, tj = tile / tiles_k;
     const int j0 = tj * C::TJ, k0 = tk * C::TK;
 
     if (tid == 0) {
-        for (int q = 0; q < C::RING + C::VSTAGES; ++q) mbar_init(bar0 + 8u * q, 1);
+        for (int q = 0; q < C::RING; ++q) mbar_init(bar0 + 8u * q, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     for (int e = tid; e < C::TJ + 4; e += C::NT) {
@@ -266,44 +271,44 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
     }
     __syncthreads();
 
-    int pslot[C::RING], vslot[C::VSTAGES];
-#pragma unroll
-    for (int q = 0; q < C::RING; ++q) pslot[q] = q;
-#pragma unroll
-    for (int q = 0; q < C::VSTAGES; ++q) vslot[q] = q;
-    unsigned pph = 0, vph = 0;
-
-    // loads feeding iteration u: P plane u, Vx face u-2, Vy / Vz of plane u-3
+    // loads feeding iteration u: P plane u, Vx face u-2, Vy / Vz of plane u-3, all
+    // on the plane's mbarrier
     auto issue = [&](int u, int ps, int vsg) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         const unsigned pb = bar0 + 8u * ps;
-        mbar_expect_tx(pb, C::P_BYTES);
-        const unsigned pdst = sbase + C::RING0 + ps * C::P_STAGE;
-        tma_load3(pdst, &mp.m[0], k0 - 8, j0 - 3, u, pb);
-        if constexpr (C::COMP) tma_load3(pdst + C::P_LO, &mp.m[1], k0 - 8, j0 - 3, u, pb);
         const int f = u - 2, io = u - 3;
         const bool vx = (u >= i_beg && f >= 0 && f <= nx - 2);
         const bool vyz = (io >= i_beg && io < i_end);
-        const unsigned vb = bar0 + 8u * (C::RING + vsg);
+        mbar_expect_tx(pb, C::P_BYTES + (vx ? C::VX_BYTES : 0u) + (vyz ? C::VYZ_BYTES : 0u));
+        const unsigned pdst = sbase + C::RING0 + ps * C::P_STAGE;
+        tma_load3(pdst, &mp.m[0], k0 - 8, j0 - 3, u, pb);
+        if constexpr (C::COMP) tma_load3(pdst + C::P_LO, &mp.m[1], k0 - 8, j0 - 3, u, pb);
         const unsigned vdst = sbase + C::VST0 + vsg * C::V_STAGE;
-        mbar_expect_tx(vb, (vx ? C::VX_BYTES : 0u) + (vyz ? C::VYZ_BYTES : 0u));
         if (vx) {
-            tma_load3(vdst + C::VX_OFF, &mp.m[2], k0, j0, f, vb);
-            if constexpr (C::COMP) tma_load3(vdst + C::VX_OFF + C::VX_LO, &mp.m[3], k0, j0, f, vb);
+            tma_load3(vdst + C::VX_OFF, &mp.m[2], k0, j0, f, pb);
+            if constexpr (C::COMP) tma_load3(vdst + C::VX_OFF + C::VX_LO, &mp.m[3], k0, j0, f, pb);
         }
         if (vyz) {
-            tma_load3(vdst + C::VY_OFF, &mp.m[4], k0, j0 - 2, io, vb);
-            tma_load3(vdst + C::VZ_OFF, &mp.m[6], k0 - 8, j0, io, vb);
+            tma_load3(vdst + C::VY_OFF, &mp.m[4], k0, j0 - 2, io, pb);
+            tma_load3(vdst + C::VZ_OFF, &mp.m[6], k0 - 8, j0, io, pb);
             if constexpr (C::COMP) {
-                tma_load3(vdst + C::VY_OFF + C::VY_LO, &mp.m[5], k0, j0 - 2, io, vb);
-                tma_load3(vdst + C::VZ_OFF + C::VZ_LO, &mp.m[7], k0 - 8, j0, io, vb);
+                tma_load3(vdst + C::VY_OFF + C::VY_LO, &mp.m[5], k0, j0 - 2, io, pb);
+                tma_load3(vdst + C::VZ_OFF + C::VZ_LO, &mp.m[7], k0 - 8, j0, io, pb);
             }
         }
     };
 
     const int u0 = i_beg - 3, u1 = i_end + 2;
-    if (tid == 0)
-        for (int q = 0; q < C::D; ++q) issue(u0 + q, pslot[3 + q], vslot[q]);
+    // Plane v of the march lives in ring slot (v - u0) mod RING, iteration v's V
+    // data in stage (v - u0) mod VSTAGES.  The issuing thread is in a warp
+    // without a second Vy row or halo Vz faces.
+    int ps = 0, vs0 = 0, o0 = 0, o3 = (C::RING - 3) * C::P_STAGE;   // slots; stage offsets of planes u and u-3
+    unsigned ph = 0;
+    auto ring = [&](int q) { return q >= C::RING ? q - C::RING : q; };
+    auto vring = [&](int q) { return q >= C::VSTAGES ? q - C::VSTAGES : q; };
+    const bool issuer = tid == C::NT / 2;
+    if (issuer)
+        for (int q = 0; q < C::D; ++q) issue(u0 + q, ring(q), vring(q));
 
     // per-thread constants of the own row and columns
     const int jr = j0 + w;
@@ -372,31 +377,49 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
         if (fast_lo >= fast_hi) fast_lo = fast_hi = u1 + 1;
     }
 
+    // What the interior body needs of this thread's items, worked out once: the
+    // existence and gradient order of its Vy faces (jmid: every Vy face of the
+    // tile exists and is of 4th order), its halo Vz face, the iteration whose
+    // plane receives the source sample in this CTA, and the in-plane places of
+    // its results.
+    const bool jmid = j0 - 2 > 0 && j0 + C::TJ < ny - 2;
+    const int hl = tid - (C::NT - 32 * C::HW);
+    const int h_j = hl / 3, h_c = hl - 3 * h_j < 2 ? 2 + hl - 3 * h_j : C::TK + 4;   // float col: k = k0-4+h_c
+    const int h_k = k0 - 4 + h_c;
+    const bool h_mine = hl >= 0 && hl < 3 * C::TJ, h_ok = h_mine && j0 + h_j < ny && h_k >= 0 && h_k <= nz - 2;
+    const bool h_4 = h_k > 0 && h_k < nz - 2;
+    float h_d = 1.0f;
+    if (h_ok) h_d = damp(fmaxf(ay_s[h_j + 2], az_s[h_c]), fmaxf(ay_s[h_j + 2], az_s[h_c + 1]), cf.dt);
+    const int h_p = (h_j + 3) * C::PC + h_c + 4, h_v = h_j * C::PC + h_c + 4;        // element cols: k = k0-8+col
+    int dep_u = -1, dep_at = 0;
+    if (a.dep_amp != 0.0f && tid == 0) {
+        const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 8);
+        if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC) {
+            dep_u = a.dep_i;
+            dep_at = dj * C::PC + dk;
+        }
+    }
+    long long ib = 0;   // plane u-3 of the march, advanced by the interior body
+
     auto iteration = [&](const int u, auto fast_tag) -> bool {
         constexpr bool FAST = decltype(fast_tag)::value;
-        const int ps = pslot[3], vsg = vslot[0];
-        const bool ok = mbar_wait(bar0 + 8u * ps, (pph >> ps) & 1u, a.wait_us) &&
-                        mbar_wait(bar0 + 8u * (C::RING + vsg), (vph >> vsg) & 1u, a.wait_us);
-        unsigned char* const pbox = sm + C::RING0 + ps * C::P_STAGE;
-        if (a.dep_amp != 0.0f && u == a.dep_i && tid == 0 && ok) {
-            const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 8);
-            if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC)
-                K::add1(pbox, dj * C::PC + dk, C::P_LO, a.dep_amp, a.sp);
-        }
+        const bool ok = mbar_wait(bar0 + 8u * ps, (ph >> ps) & 1u, a.wait_us);
+        unsigned char* const pbox = sm + C::RING0 + o0;
+        if (u == dep_u && ok) K::add1(pbox, dep_at, C::P_LO, a.dep_amp, a.sp);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicMin(a.status + kStatusTimeout, blockIdx.x + gridDim.x * blockIdx.y);
             u_fail = u;
             return false;
         }
-        pph ^= 1u << ps;
-        vph ^= 1u << vsg;
-        if (tid == 0 && u + C::D <= u1) issue(u + C::D, pslot[C::RING - 1], vslot[C::VSTAGES - 1]);
+        ph ^= 1u << ps;
+        if (issuer && u + C::D <= u1) issue(u + C::D, ring(ps + C::D), vring(vs0 + C::D));
         float ax_next = 0.0f, px_next = 1.0f;
         if constexpr (!FAST) {
             ax_next = ax_at(u + 1);
             px_next = px_at(u - 2);
         }
-        const unsigned char* const vs = sm + C::VST0 + vsg * C::V_STAGE;
+        const unsigned char* const vs = sm + C::VST0 + vs0 * C::V_STAGE;
+        if constexpr (!FAST) ib = (long long)(u - 3) * PL;
 
         pq0 = pq1; pq1 = pq2; pq2 = pq3;
         pq3 = K::ld4(pbox, cP, C::P_LO, a.sp);
@@ -405,7 +428,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
         if (FAST || u >= i_beg) {
             const int f = u - 2;
             float4 vnew = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (FAST ? row_ok : (f >= 0 && f <= nx - 2 && row_ok)) {
+            if (FAST || (f >= 0 && f <= nx - 2 && row_ok)) {   // rows beyond the room hold zeros
                 const float4 vo = K::ld4(vs + C::VX_OFF, w * C::TK + 4 * lane, C::VX_LO, a.sv);
                 float4 v;
                 if constexpr (FAST) {
@@ -423,7 +446,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                         v = vel4m(cf, pq0, pq1, pq2, pq3, vo, dm, fourth ? 15 : 0, okk);
                     }
                 }
-                vnew = K::st4(v, a.sv, a.vout_hi[0], a.vout_lo[0], f * PL + own,
+                vnew = K::st4(v, a.sv, a.vout_hi[0], a.vout_lo[0], ib + PL + own,
                               f >= i_beg && f < i_end && st_ok);
             }
             qx0 = qx1; qx1 = qx2; qx2 = qx3; qx3 = vnew;
@@ -434,10 +457,9 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
         if (FAST || i >= i_beg) {
             const float axi = FAST ? 0.0f : axw3;
             const bool xint = FAST || (axi == 0.0f);
-            const unsigned char* const pst = sm + C::RING0 + pslot[0] * C::P_STAGE;
+            const unsigned char* const pst = sm + C::RING0 + o3;
             const unsigned char* const vys = vs + C::VY_OFF;
             const unsigned char* const vzs = vs + C::VZ_OFF;
-            const long long ib = (long long)i * PL;
             const float4 pown = pq0;   // own row of plane i
 
 #pragma unroll
@@ -446,7 +468,8 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                 if (r < C::VYR) {
                     const int jf = j0 - 2 + r;
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (jf >= 0 && jf <= ny - 2) {
+                    const bool ex = jf >= 0 && jf <= ny - 2;
+                    if (FAST || ex) {
                         const int c = 4 * lane + 8;
                         const float4 pm = K::ld4(pst, r * C::PC + c, C::P_LO, a.sp);
                         const float4 p0 = K::ld4(pst, (r + 1) * C::PC + c, C::P_LO, a.sp);
@@ -457,8 +480,8 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                         const bool fourth = (jf > 0 && jf < ny - 2);
                         float4 vv;
                         if constexpr (FAST) {
-                            // the row's gradient order is uniform over its threads
-                            vv = vel4m(cf, pm, p0, p1, p2, vo, dyi[m], fourth ? 15 : 0, 15);
+                            if (jmid) vv = vel4m(cf, pm, p0, p1, p2, vo, dyi[m], 15, 15);
+                            else vv = vel4m(cf, pm, p0, p1, p2, vo, dyi[m], fourth ? 15 : 0, ex ? 15 : 0);
                         } else if (fourth && xint && kfull) {
                             vv = vel4m(cf, pm, p0, p1, p2, vo, dyi[m], 15, 15);
                         } else {
@@ -472,7 +495,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                             vv = vel4m(cf, pm, p0, p1, p2, vo, dm, fourth ? 15 : 0, okk);
                         }
                         v = K::st4(vv, a.sv, a.vout_hi[1], a.vout_lo[1], ib + (long long)jf * sz + kb,
-                                   r >= 2 && r < C::TJ + 2 && kb < sz);
+                                   r >= 2 && r < C::TJ + 2 && ex && kb < sz);
                     }
                     *reinterpret_cast<float4*>(vyn + r * C::TK + 4 * lane) = v;
                 }
@@ -481,7 +504,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
             // Vz: own faces kb .. kb+3 of row jr
             {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (row_ok) {
+                if (FAST || row_ok) {
                     const int c = (w + 3) * C::PC + 4 * lane + 8;
                     const float4 pb4 = K::ld4(pst, c + 4, C::P_LO, a.sp);
                     const float pl = K::ld1(pst, c - 1, C::P_LO, a.sp);
@@ -505,30 +528,25 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                 }
                 *reinterpret_cast<float4*>(vzn + w * C::ZC + 4 * lane + 4) = v;
             }
-            // halo Vz faces k0-2, k0-1, k0+TK of every row (the last warp)
-            const int hl = tid - (C::NT - 32);
-            if (hl >= 0 && hl < 3 * C::TJ) {
-                const int jl = hl / 3, which = hl - 3 * jl;
-                const int ch = which < 2 ? 2 + which : C::TK + 4;    // float col: k = k0-4+ch
-                const int ce = ch + 4;                               // element col: k = k0-8+ce
-                const int kf = k0 - 4 + ch;
+            // halo Vz faces k0-2, k0-1, k0+TK of every row (the last HW warps)
+            if (h_mine) {
                 float vh = 0.0f;
-                if (j0 + jl < ny && kf >= 0 && kf <= nz - 2) {
-                    const bool fourth = (kf > 0 && kf < nz - 2);
-                    const float ay = ay_s[jl + 2];
-                    const int rb = (jl + 3) * C::PC;
-                    const float gr = grad(cf, K::ld1(pst, rb + ce - 1, C::P_LO, a.sp), K::ld1(pst, rb + ce, C::P_LO, a.sp),
-                                          K::ld1(pst, rb + ce + 1, C::P_LO, a.sp),
-                                          K::ld1(pst, rb + ce + 2, C::P_LO, a.sp), fourth);
-                    const float dmp = damp(fmaxf(fmaxf(axi, ay), az_s[ch]), fmaxf(fmaxf(axi, ay), az_s[ch + 1]), cf.dt);
-                    vh = K::round_trip(vup(cf, K::ld1(vzs, jl * C::PC + ce, C::VZ_LO, a.sv), gr, dmp), a.sv);
+                if (h_ok) {
+                    const float gr = grad(cf, K::ld1(pst, h_p - 1, C::P_LO, a.sp), K::ld1(pst, h_p, C::P_LO, a.sp),
+                                          K::ld1(pst, h_p + 1, C::P_LO, a.sp), K::ld1(pst, h_p + 2, C::P_LO, a.sp), h_4);
+                    float dmp = h_d;
+                    if constexpr (!FAST) {
+                        const float mxy = fmaxf(axi, ay_s[h_j + 2]);
+                        dmp = damp(fmaxf(mxy, az_s[h_c]), fmaxf(mxy, az_s[h_c + 1]), cf.dt);
+                    }
+                    vh = K::round_trip(vup(cf, K::ld1(vzs, h_v, C::VZ_LO, a.sv), gr, dmp), a.sv);
                 }
-                vzn[jl * C::ZC + ch] = vh;
+                vzn[h_j * C::ZC + h_c] = vh;
             }
             __syncthreads();
 
             // P^{n+1} of the own cells
-            if (row_ok) {
+            if (FAST || row_ok) {
                 const float* yr = vyn + 4 * lane;
                 const float4 ymm = *reinterpret_cast<const float4*>(yr + w * C::TK);
                 const float4 ym = *reinterpret_cast<const float4*>(yr + (w + 1) * C::TK);
@@ -554,7 +572,7 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
                     for (int q = 0; q < 4; ++q)
                         if (kb + q >= nz) at4(out, q) = 0.0f;
                 }
-                K::st4(out, a.sp, a.pn_hi, a.pn_lo, ib + own, kb < sz);
+                K::st4(out, a.sp, a.pn_hi, a.pn_lo, ib + own, st_ok);
             }
         }
 
@@ -562,22 +580,18 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
             axw3 = axw2; axw2 = axw1; axw1 = axw0; axw0 = ax_next;
             pxw = px_next;
         }
-        {
-            const int pfree = pslot[0];
-#pragma unroll
-            for (int q = 0; q + 1 < C::RING; ++q) pslot[q] = pslot[q + 1];
-            pslot[C::RING - 1] = pfree;
-            const int vfree = vslot[0];
-#pragma unroll
-            for (int q = 0; q + 1 < C::VSTAGES; ++q) vslot[q] = vslot[q + 1];
-            vslot[C::VSTAGES - 1] = vfree;
-        }
+        ps = ring(ps + 1);
+        vs0 = vring(vs0 + 1);
+        o0 = ps * C::P_STAGE;
+        o3 = o3 + C::P_STAGE == C::RING * C::P_STAGE ? 0 : o3 + C::P_STAGE;
+        if constexpr (FAST) ib += PL;
         return true;
     };
 
     for (int u = u0; u <= u1;) {
         if (u == fast_lo) {
             bool ran = true;
+            ib = (long long)(u - 3) * PL;
             for (; u < fast_hi; ++u)
                 if (!iteration(u, std::true_type{})) { ran = false; break; }
             if (!ran) break;
@@ -595,9 +609,8 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
     if (u_fail <= u1) {
         if (tid == 0) {
             for (int q = 0; q < C::D && u_fail + q <= u1; ++q) {
-                const int ps = pslot[3 + q], vsg = vslot[q];
-                mbar_wait(bar0 + 8u * ps, (pph >> ps) & 1u, a.wait_us);
-                mbar_wait(bar0 + 8u * (C::RING + vsg), (vph >> vsg) & 1u, a.wait_us);
+                const int sl = ring(ps + q);
+                mbar_wait(bar0 + 8u * sl, (ph >> sl) & 1u, a.wait_us);
             }
         }
         __syncthreads();
@@ -605,29 +618,30 @@ __global__ void __launch_bounds__(256) k_fused16(F16Args a, const __grid_constan
 }
 
 constexpr int kMaxDev16 = 64;
-int g_slots16[6][kMaxDev16];
+int g_slots16[2][6][kMaxDev16];
 int g_sms16[kMaxDev16];
 std::mutex g_cfg16_mu;
 
-template <int M>
+template <int M, int TJ, int LW>
 cudaError_t launch_of(const F16Args& a, F16Cache* cache, const void* const bases[8], cudaStream_t s)
 {
-    using C = H16<M, depth16<M>()>;
+    using C = H16<M, depth16<M>(), TJ, LW>;
+    constexpr int shape = LW == 16;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDev16) return cudaErrorInvalidDevice;
     {
         std::lock_guard<std::mutex> lk(g_cfg16_mu);
-        if (!g_slots16[M][dev]) {
-            e = cudaFuncSetAttribute(k_fused16<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
+        if (!g_slots16[shape][M][dev]) {
+            e = cudaFuncSetAttribute(k_fused16<M, TJ, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
             if (e != cudaSuccess) return e;
             e = cudaDeviceGetAttribute(&g_sms16[dev], cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return e;
             int slots = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slots, k_fused16<M>, C::NT, C::SMEM_BYTES);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slots, k_fused16<M, TJ, LW>, C::NT, C::SMEM_BYTES);
             if (e != cudaSuccess) return e;
-            g_slots16[M][dev] = slots > 0 ? slots : 1;
+            g_slots16[shape][M][dev] = slots > 0 ? slots : 1;
         }
     }
     Maps16 mp;
@@ -642,7 +656,7 @@ cudaError_t launch_of(const F16Args& a, F16Cache* cache, const void* const bases
     const int tiles_j = (g.ny + C::TJ - 1) / C::TJ;
     const int tiles_k = (g.nz + C::TK - 1) / C::TK;
     const long long tiles = (long long)tiles_j * tiles_k;
-    const long long slots = (long long)g_slots16[M][dev] * g_sms16[dev];
+    const long long slots = (long long)g_slots16[shape][M][dev] * g_sms16[dev];
     long long segs = slots / tiles;
     if (segs < 1) segs = 1;
     if (segs > g.nx) segs = g.nx;
@@ -650,7 +664,7 @@ cudaError_t launch_of(const F16Args& a, F16Cache* cache, const void* const bases
     segs = (g.nx + seg_len - 1) / seg_len;
     if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
     dim3 grid((unsigned)tiles, (unsigned)segs, 1);
-    k_fused16<M><<<grid, C::NT, C::SMEM_BYTES, s>>>(a, mp, seg_len, tiles_k);
+    k_fused16<M, TJ, LW><<<grid, C::NT, C::SMEM_BYTES, s>>>(a, mp, seg_len, tiles_k);
     return cudaGetLastError();
 }
 
@@ -689,24 +703,22 @@ bool f16_supported(int mode, const Grid& g)
            g.nz >= 1 && g.sz % 8 == 0;
 }
 
-size_t f16_smem_bytes(int mode)
+// 16 x 64 tiles when they leave less of the last k tile idle than 8 x 128 tiles
+// (Nz = 160: 192 columns instead of 256), else 8 x 128, as in the FP32 march.
+template <int M>
+cudaError_t launch_shape(const F16Args& a, F16Cache* cache, const void* const bases[8], cudaStream_t s)
 {
-    switch (mode) {
-        case kBF16: return H16<kBF16, depth16<kBF16>()>::SMEM_BYTES;
-        case kFP16: return H16<kFP16, depth16<kFP16>()>::SMEM_BYTES;
-        case kBF16C: return H16<kBF16C, depth16<kBF16C>()>::SMEM_BYTES;
-        case kFP16C: return H16<kFP16C, depth16<kFP16C>()>::SMEM_BYTES;
-        default: return 0;
-    }
+    const int w128 = (a.g.nz + 127) / 128 * 128, w64 = (a.g.nz + 63) / 64 * 64;
+    return w64 < w128 ? launch_of<M, 16, 16>(a, cache, bases, s) : launch_of<M, 8, 32>(a, cache, bases, s);
 }
 
 cudaError_t launch_fused16(int mode, const F16Args& a, F16Cache* cache, const void* const bases[8], cudaStream_t s)
 {
     switch (mode) {
-        case kBF16: return launch_of<kBF16>(a, cache, bases, s);
-        case kFP16: return launch_of<kFP16>(a, cache, bases, s);
-        case kBF16C: return launch_of<kBF16C>(a, cache, bases, s);
-        case kFP16C: return launch_of<kFP16C>(a, cache, bases, s);
+        case kBF16: return launch_shape<kBF16>(a, cache, bases, s);
+        case kFP16: return launch_shape<kFP16>(a, cache, bases, s);
+        case kBF16C: return launch_shape<kBF16C>(a, cache, bases, s);
+        case kFP16C: return launch_shape<kFP16C>(a, cache, bases, s);
         default: return cudaErrorInvalidValue;
     }
 }

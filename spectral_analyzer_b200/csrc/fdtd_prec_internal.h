@@ -178,7 +178,6 @@ F16Cache* f16_cache_create();
 void f16_cache_destroy(F16Cache* c);
 cudaError_t f16_map(F16Cache* c, const void* base, const Grid& g, int bx, int by, CUtensorMap* out);
 bool f16_supported(int mode, const Grid& g);
-size_t f16_smem_bytes(int mode);
 // bases: P^n value, P^n residual, then V^{n-1/2} value / residual of Vx, Vy, Vz
 // (residuals null for the plain 16-bit modes)
 cudaError_t launch_fused16(int mode, const F16Args& a, F16Cache* cache, const void* const bases[8],
