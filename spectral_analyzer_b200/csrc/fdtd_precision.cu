@@ -237,6 +237,17 @@ __global__ void k_src_rec(Field p, long long src, const double* sig, int step, i
     }
 }
 
+// A stored field decoded into the reference's compact layout (T: float holds every
+// mode's values but FP64's).
+template <int M, class T>
+__global__ void __launch_bounds__(256) k_flat(Grid g, Field f, T* __restrict__ out)
+{
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
+    if (k >= g.nz || j >= g.ny) return;
+    const long long row = (long long)i * g.ny + j;
+    out[row * g.nz + k] = (T)ld<M>(f, row * g.sz + k);
+}
+
 }  // namespace prec
 }  // namespace fdtd
 
@@ -276,6 +287,7 @@ struct FdtdB200Prec {
     double* d_rw = nullptr;
     double* d_trace = nullptr;
     int cap = 0, n_rec_steps = 0;
+    void* d_flat = nullptr;     // compact pressure for get_pressure
     double* d_audit = nullptr;  // [cap_audit][2]
     std::vector<int> audit_steps;
     int cap_audit = 0;
@@ -703,42 +715,40 @@ int fdtd_b200_prec_get_pressure(FdtdB200Prec* p, double* out, int out_len)
     if (out_len != p->N) return FDTD_ERR_DIM;
     PCK(cudaStreamSynchronize(p->stream));
     if (check_status(p) != FDTD_OK) return FDTD_ERR_CUDA;
+    // Decoded and made compact on the device (5.7M cells in BF16: 10.5 ms with the
+    // padded field copied and decoded on the host).  Every mode but FP64 decodes
+    // to float: those cross as floats, into the upper half of `out`, and are
+    // widened in place, block by block from the front.
     const Field& f = p->f[p->cur];
-    const size_t eb = elem_bytes(p->mode);
-    std::vector<unsigned char> hi((size_t)p->g.cells * eb), lo;
-    PCK(cudaMemcpy(hi.data(), f.hi, hi.size(), cudaMemcpyDeviceToHost));
-    if (compensated(p->mode)) {
-        lo.resize(hi.size());
-        PCK(cudaMemcpy(lo.data(), f.lo, lo.size(), cudaMemcpyDeviceToHost));
+    const bool dbl = p->mode == kFP64;
+    const size_t n = (size_t)p->N, vb = dbl ? 8 : 4;
+    if (!p->d_flat) {
+        PCK(cudaMalloc(&p->d_flat, n * vb));
+        p->allocs.push_back(p->d_flat);
     }
-    auto h2f = [&](const unsigned char* b) -> float {
-        uint16_t u;
-        memcpy(&u, b, 2);
-        if (p->mode == kBF16 || p->mode == kBF16C) {
-            uint32_t w = (uint32_t)u << 16;
-            float x;
-            memcpy(&x, &w, 4);
-            return x;
+    const dim3 block(32, 8, 1), grid((p->g.nz + 31) / 32, (p->g.ny + 7) / 8, p->g.nx);
+    switch (p->mode) {
+        case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
+        case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, (double*)p->d_flat); break;
+        case kBF16: k_flat<kBF16><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
+        case kFP16: k_flat<kFP16><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
+        case kBF16C: k_flat<kBF16C><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
+        default: k_flat<kFP16C><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat);
+    }
+    PCK(cudaGetLastError());
+    unsigned char* const bytes = reinterpret_cast<unsigned char*>(out);
+    unsigned char* const at = bytes + (dbl ? 0 : 4 * n);
+    PCK(cudaMemcpyAsync(at, p->d_flat, n * vb, cudaMemcpyDeviceToHost, p->stream));
+    PCK(cudaStreamSynchronize(p->stream));
+    if (!dbl) {
+        constexpr size_t B = 2048;
+        float x[B];
+        for (size_t q = 0; q < n; q += B) {   // value q ends at byte 8q+8, float q starts at 4n+4q >= 8q+4
+            const size_t m = std::min(B, n - q);
+            memcpy(x, at + 4 * q, 4 * m);
+            for (size_t t = 0; t < m; ++t) out[q + t] = (double)x[t];
         }
-        __half_raw r;
-        r.x = u;
-        return __half2float(__half(r));
-    };
-    const Grid& g = p->g;
-    for (int i = 0; i < g.nx; ++i)
-        for (int j = 0; j < g.ny; ++j)
-            for (int k = 0; k < g.nz; ++k) {
-                const size_t id = ((size_t)i * g.ny + j) * g.sz + k;
-                double v;
-                if (p->mode == kFP64) memcpy(&v, &hi[id * 8], 8);
-                else if (p->mode == kFP32) { float x; memcpy(&x, &hi[id * 4], 4); v = x; }
-                else {
-                    float x = h2f(&hi[id * 2]);
-                    if (!lo.empty()) x = x + h2f(&lo[id * 2]) * f.inv_lo_scale;
-                    v = (double)(x * f.inv_scale);
-                }
-                out[k + g.nz * (j + (size_t)g.ny * i)] = v;
-            }
+    }
     return FDTD_OK;
 }
 
