@@ -136,13 +136,7 @@ struct AcousticFDTDState {
     int* d_nb13 = nullptr;
     long long* d_above = nullptr;
     long long* d_below = nullptr;
-    long long* d_vzb = nullptr;
-    long long* d_vza = nullptr;
     uint8_t* d_plate_code = nullptr;   // per plate node: bit 0 Vz face below, bit 1 above (PlateFaces)
-    // four-cell groups whose divergence reads a plate face (padded index of the
-    // group's first cell): recomputed after a walled single-pass step
-    long long* d_pfix = nullptr;
-    int n_pfix = 0;
     std::vector<int> h_act;
     float* d_w[3] = {nullptr, nullptr, nullptr};
     int wi_cur = 0, wi_prev = 1, wi_tmp = 2;
@@ -623,8 +617,9 @@ int step_check(AcousticFDTDState* st, bool sync_check)
     return FDTD_OK;
 }
 
-// One time step (acoustic_fdtd.cpp:1272-1290 loop body) plus the engine's
-// point-source deposit before it and receiver record after it.
+// One time step of a scene without a plate (acoustic_fdtd.cpp:1272-1290 loop
+// body) plus the engine's point-source deposit before it and receiver record
+// after it.
 // sync_check: stop and return FDTD_ERR_UNSTABLE at a failed check (fdtd_step);
 // otherwise failures are latched on the device (fdtd_b200_step_async).
 // defer_record: a fused step leaves its receiver record pending, to be taken
@@ -657,15 +652,9 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
 {
     cudaStream_t s = st->stream;
     const bool fused = use_fused(st);
-    if (!fused) {
+    if (!fused)
         if (int rc0 = flush_record(st)) return rc0;
-        // A plate scene on the two-pass kernels waits for its plate guard every
-        // step anyway: take the substep's schedule (all of the step issued, the
-        // guard read with the status words at its end, graph replay where it
-        // applies), which leaves the same state and return codes.
-        if (st->n_act > 0 && sync_check && !st->prof_on) return substep_plate(st, 0, nullptr);
-    }
-    // point source: deposit s[n] before step n (applies before the plate reads P)
+    // point source: deposit s[n] before step n
     bool fuse_deposit = false;
     if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0 && st->ps_done_step != st->step_count) {
         fuse_deposit = fused && st->ps.n == 1 && st->ps.divisor == 0;
@@ -676,45 +665,7 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
         st->ps_done_step = st->step_count;
     }
 
-    // plate step (acoustic_fdtd.cpp:984-1053)
-    if (st->n_act > 0) {
-        if (st->ext_pending) {
-            CK(cudaMemcpyAsync(st->d_ext, st->h_ext, (size_t)st->N_plate * sizeof(float),
-                               cudaMemcpyHostToDevice, s));
-            st->dev_ext_nonzero = true;
-        }
-        CK(cudaMemsetAsync(st->d_status + kStatusPlate, 0xFF, sizeof(unsigned), s));
-        CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below,
-                             st->d_w[st->wi_cur], st->d_w[st->wi_prev], st->d_w[st->wi_tmp],
-                             st->d_ext, st->P(), st->pc, st->d_status, s));
-        ++st->launches;
-        CK(cudaMemcpyAsync(st->h_status + kStatusPlate, st->d_status + kStatusPlate,
-                           sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        unsigned bad = st->h_status[kStatusPlate];
-        if (bad != 0xFFFFFFFFu) {
-            int pidx = st->h_act[bad];
-            float wn = NAN;
-            cudaMemcpy(&wn, st->d_w[st->wi_tmp] + pidx, sizeof(float), cudaMemcpyDeviceToHost);
-            fprintf(stderr,
-                    "[fdtd_plate] UNSTABLE step=%d plate_node=%d (%d,%d) w_new=%.3g m (limit 0.02 m)\n",
-                    st->step_count, pidx, pidx / st->Ny, pidx % st->Ny, (double)wn);
-            fflush(stderr);
-            return FDTD_ERR_UNSTABLE;   // no rotation; pending forces stay (as the reference)
-        }
-        // consume the forces (acoustic_fdtd.cpp:1045-1046) and rotate w
-        if (st->dev_ext_nonzero) {
-            CK(cudaMemsetAsync(st->d_ext, 0, (size_t)st->N_plate * sizeof(float), s));
-            st->dev_ext_nonzero = false;
-        }
-        if (st->ext_pending) clear_ext_host(st);
-        int t = st->wi_prev;
-        st->wi_prev = st->wi_cur;
-        st->wi_cur = st->wi_tmp;
-        st->wi_tmp = t;
-    } else if (st->ext_pending) {
-        clear_ext_host(st);   // consumed with no plate
-    }
+    if (st->ext_pending) clear_ext_host(st);   // consumed with no plate
 
     // velocity + pressure
     cudaEvent_t e1;
@@ -756,30 +707,10 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
         CK(launch_fused_step(a, st->fcache, s));
         ++st->launches;
         st->cv ^= 1;
-        if (walled && st->n_act > 0) {
-            // the plate sets its faces' velocity after the update (as on the
-            // two-pass path); the cells whose divergence reads those faces are
-            // then updated again from P^n and the new velocities
-            CK(launch_plate_inject(st->n_act, st->d_act, st->d_vzb, st->d_vza, st->d_w[st->wi_cur],
-                                   st->d_w[st->wi_prev], st->cf.inv_dt, st->V(2), s));
-            const bool hf = st->has_frac;
-            CK(launch_pressure_groups(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2),
-                                      hf ? st->d_frac[0] : nullptr, hf ? st->d_frac[1] : nullptr,
-                                      hf ? st->d_frac[2] : nullptr, st->d_solid, st->d_pfix, st->n_pfix, s));
-            st->launches += 2;
-        }
         if ((rc = prof_end(st, e1, fused_kernel_launches_per_step()))) return rc;
     } else {
-        PlateFaces pf;   // the plate's face velocities, set inside the velocity pass
-        if (st->n_act > 0) {
-            pf.code = st->d_plate_code;
-            pf.w = st->d_w[st->wi_cur];
-            pf.wp = st->d_w[st->wi_prev];
-            pf.inv_dt = st->cf.inv_dt;
-            pf.iz = st->plate_iz;
-        }
         CK(launch_velocity_general(st->g, st->cf, st->tb, st->P(), st->V(0), st->V(1), st->V(2),
-                                   st->d_frac[0], st->d_frac[1], st->d_frac[2], s, nullptr, &pf));
+                                   st->d_frac[0], st->d_frac[1], st->d_frac[2], s));
         st->launches += 2;
         const bool hf = st->has_frac;
         CK(launch_pressure_general(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1),
@@ -897,15 +828,165 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check)
     return step_check(st, sync_check);
 }
 
+// Reports the plate node of a failed plate update (status read), whose new
+// displacement is in the buffer to be written next.
+int report_plate(AcousticFDTDState* st)
+{
+    const int pidx = st->h_act[st->h_status[kStatusPlate]];
+    float wn = NAN;
+    cudaMemcpy(&wn, st->d_w[st->wi_tmp] + pidx, sizeof(float), cudaMemcpyDeviceToHost);
+    fprintf(stderr, "[fdtd_plate] UNSTABLE step=%d plate_node=%d (%d,%d) w_new=%.3g m (limit 0.02 m)\n",
+            st->step_count, pidx, pidx / st->Ny, pidx % st->Ny, (double)wn);
+    fflush(stderr);
+    return FDTD_ERR_UNSTABLE;   // no rotation; pending forces stay (as the reference)
+}
+
+// Up to n_steps steps of a plate scene (acoustic_fdtd.cpp:1272-1290), queued
+// without waiting for the plate guard after each: a failed plate update records
+// its step, everything queued behind it does nothing, and the host, which reads
+// the status once, takes its bookkeeping back to that step.  The fields stay as
+// a step that fails leaves them, because a step writes the other P buffer, the
+// third displacement buffer and (the single pass) the other velocity set, or
+// (the two passes) is gated.  Forces act in the first step and stay pending if
+// that one fails.  Returns the steps taken in *done.
+int plate_steps(AcousticFDTDState* st, int n_steps, bool sync_check, int* done)
+{
+    cudaStream_t s = st->stream;
+    *done = 0;
+    if (int rc = flush_record(st)) return rc;
+    const bool fused = use_fused(st);
+    int m = std::min(n_steps, kCheckPeriod - (st->step_count & (kCheckPeriod - 1)));
+    if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0) m = 1;   // a deposit is not gated
+    if (m == 1 && !fused && sync_check && !st->prof_on) {   // a cached graph
+        const int rc = substep_plate(st, 0, nullptr);
+        *done = rc == FDTD_OK;
+        return rc;
+    }
+    if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0 && st->ps_done_step != st->step_count) {
+        CK(launch_deposit(st->ps, st->d_ps_sig, st->step_count, 0.0f, st->P(), s));
+        ++st->launches;
+        st->ps_done_step = st->step_count;
+    }
+    if (fused) {
+        if (!st->v[st->cv ^ 1][0])
+            if (int rc = alloc_second_velocity_set(st)) return rc;
+        if (!st->fcache) st->fcache = fused_cache_create();
+    }
+    const int n0 = st->step_count, trace0 = st->trace_len, cur0 = st->cur, cv0 = st->cv;
+    const int w0[3] = {st->wi_cur, st->wi_prev, st->wi_tmp};
+    if (st->ext_pending) {
+        CK(cudaMemcpyAsync(st->d_ext, st->h_ext, (size_t)st->N_plate * sizeof(float), cudaMemcpyHostToDevice, s));
+        st->dev_ext_nonzero = true;
+    }
+    CK(cudaMemsetAsync(st->d_status + kStatusPlate, 0xFF, 2 * sizeof(unsigned), s));   // node and step
+    const bool hf = st->has_frac;
+    const float* const fdiv[3] = {hf ? st->d_frac[0] : nullptr, hf ? st->d_frac[1] : nullptr, hf ? st->d_frac[2] : nullptr};
+    for (int q = 0; q < m; ++q) {
+        const unsigned step = (unsigned)st->step_count;
+        cudaEvent_t e1;
+        if (!fused) {
+            CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below, st->d_w[st->wi_cur],
+                                 st->d_w[st->wi_prev], st->d_w[st->wi_tmp], st->d_ext, st->P(), st->pc, st->d_status,
+                                 step, s));
+            PlateFaces pf;   // the plate's face velocities, set inside the velocity pass
+            pf.code = st->d_plate_code;
+            pf.w = st->d_w[st->wi_tmp];
+            pf.wp = st->d_w[st->wi_cur];
+            pf.inv_dt = st->cf.inv_dt;
+            pf.iz = st->plate_iz;
+            if (int rc = prof_begin(st, &e1)) return rc;
+            CK(launch_velocity_general(st->g, st->cf, st->tb, st->P(), st->V(0), st->V(1), st->V(2), st->d_frac[0],
+                                       st->d_frac[1], st->d_frac[2], s, st->d_status, &pf));
+            CK(launch_pressure_general(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2), fdiv[0],
+                                       fdiv[1], fdiv[2], st->d_solid, s, st->d_status));
+            if (int rc = prof_end(st, e1, 2)) return rc;
+            st->launches += 3;
+        } else {
+            FusedArgs a{st->g, st->cf, st->tb, st->P(), st->Pn(),
+                        {st->V(0), st->V(1), st->V(2)},
+                        {st->v[st->cv ^ 1][0], st->v[st->cv ^ 1][1], st->v[st->cv ^ 1][2]},
+                        st->d_status};
+            a.hold_plane = st->hold_plane;
+            a.wait_us = st->wait_us;
+            for (int c2 = 0; c2 < 3; ++c2) a.fr[c2] = st->d_frac[c2];
+            a.frac_div = hf;
+            a.solid = st->d_solid;
+            if (q > 0) a.gate = st->d_status;
+            if (int rc = prof_begin(st, &e1)) return rc;
+            CK(launch_fused_step(a, st->fcache, s));
+            st->cv ^= 1;
+            PlateStep ps;
+            ps.n_act = st->n_act;
+            ps.iz = st->plate_iz;
+            ps.act = st->d_act;
+            ps.nb13 = st->d_nb13;
+            ps.code = st->d_plate_code;
+            ps.above = st->d_above;
+            ps.below = st->d_below;
+            ps.w = st->d_w[st->wi_cur];
+            ps.wp = st->d_w[st->wi_prev];
+            ps.wt = st->d_w[st->wi_tmp];
+            ps.ext = st->d_ext;
+            ps.pc = st->pc;
+            ps.inv_dt = st->cf.inv_dt;
+            ps.status = st->d_status;
+            ps.step = step;
+            CK(launch_plate_columns(st->g, st->cf, st->tb, ps, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2), fdiv[0],
+                                    fdiv[1], fdiv[2], st->d_solid, s));
+            if (int rc = prof_end(st, e1, 2)) return rc;
+            st->launches += 2;
+        }
+        if (q == 0 && st->dev_ext_nonzero) {   // the forces are consumed (the host keeps them until the guard is read)
+            CK(cudaMemsetAsync(st->d_ext, 0, (size_t)st->N_plate * sizeof(float), s));
+            st->dev_ext_nonzero = false;
+        }
+        const int t = st->wi_prev;
+        st->wi_prev = st->wi_cur;
+        st->wi_cur = st->wi_tmp;
+        st->wi_tmp = t;
+        st->cur ^= 1;
+        ++st->step_count;
+        if (st->n_rec > 0 && st->trace_len < st->trace_cap) {
+            CK(launch_wsum(st->P(), st->d_rec_idx, st->d_rec_w, st->n_rec, 8, 0,
+                           st->d_trace + (size_t)st->trace_len * st->n_rec, s));
+            ++st->launches;
+            ++st->trace_len;
+        }
+    }
+    CK(cudaMemcpyAsync(st->h_status, st->d_status, kStatusWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    const bool bad = st->h_status[kStatusPlate] != 0xFFFFFFFFu;
+    const int k = bad ? (int)st->h_status[kStatusPlateStep] - n0 : m;   // steps taken
+    if (k > 0 && st->ext_pending) clear_ext_host(st);
+    *done = k;
+    if (!bad) return step_check(st, sync_check);
+    st->step_count = n0 + k;
+    st->trace_len = std::min(st->trace_len, trace0 + k);
+    st->cur = cur0 ^ (k & 1);
+    if (fused) st->cv = cv0 ^ (k & 1);
+    // a step moves (current, previous, next) to (next, current, previous)
+    const int r = k % 3;
+    st->wi_cur = w0[(3 - r) % 3];
+    st->wi_prev = w0[(4 - r) % 3];
+    st->wi_tmp = w0[(5 - r) % 3];
+    return report_plate(st);
+}
+
 // n_steps steps, several per launch where the room allows it; the last step's
 // receivers are recorded before it returns.
 int run_steps(AcousticFDTDState* st, int n_steps, bool sync_check)
 {
     int rc = FDTD_OK;
     for (int s = 0; s < n_steps && rc == FDTD_OK;) {
-        const int m = resident_window(st, n_steps - s);
-        rc = m > 0 ? resident_steps(st, m, sync_check) : one_step(st, sync_check, true);
-        s += m > 0 ? m : 1;
+        int m = 1;
+        if (st->n_act > 0) {
+            rc = plate_steps(st, n_steps - s, sync_check, &m);
+        } else {
+            m = resident_window(st, n_steps - s);
+            rc = m > 0 ? resident_steps(st, m, sync_check) : one_step(st, sync_check, true);
+            m = std::max(m, 1);
+        }
+        s += m;
     }
     const int rc_rec = flush_record(st);
     return rc != FDTD_OK ? rc : rc_rec;
@@ -930,7 +1011,7 @@ void free_state(AcousticFDTDState* st)
     cudaFree(st->d_solid);
     for (int c = 0; c < 3; ++c) { cudaFree(st->d_frac[c]); cudaFree(st->d_w[c]); }
     cudaFree(st->d_act); cudaFree(st->d_nb13); cudaFree(st->d_above); cudaFree(st->d_below);
-    cudaFree(st->d_vzb); cudaFree(st->d_vza); cudaFree(st->d_pfix); cudaFree(st->d_plate_code); cudaFree(st->d_ext); cudaFree(st->d_slice);
+    cudaFree(st->d_plate_code); cudaFree(st->d_ext); cudaFree(st->d_slice);
     cudaFreeHost(st->h_ext);
     cudaFreeHost(st->h_ext_pack);
     cudaFree(st->d_ext_pack);
@@ -1116,36 +1197,15 @@ AcousticFDTDState* create_impl(int Nx, int Ny, int Nz, float dx, float c, float 
             CKN(cudaMalloc(&st->d_nb13, na * 13 * sizeof(int)));
             CKN(cudaMalloc(&st->d_above, na * sizeof(long long)));
             CKN(cudaMalloc(&st->d_below, na * sizeof(long long)));
-            CKN(cudaMalloc(&st->d_vzb, na * sizeof(long long)));
-            CKN(cudaMalloc(&st->d_vza, na * sizeof(long long)));
             CKN(cudaMemcpy(st->d_act, st->h_act.data(), na * sizeof(int), cudaMemcpyHostToDevice));
             CKN(cudaMemcpy(st->d_nb13, nb13.data(), na * 13 * sizeof(int), cudaMemcpyHostToDevice));
             CKN(cudaMemcpy(st->d_above, above.data(), na * sizeof(long long), cudaMemcpyHostToDevice));
             CKN(cudaMemcpy(st->d_below, below.data(), na * sizeof(long long), cudaMemcpyHostToDevice));
-            CKN(cudaMemcpy(st->d_vzb, vzb.data(), na * sizeof(long long), cudaMemcpyHostToDevice));
-            CKN(cudaMemcpy(st->d_vza, vza.data(), na * sizeof(long long), cudaMemcpyHostToDevice));
             std::vector<uint8_t> code((size_t)st->N_plate, 0);
             for (size_t q = 0; q < na; ++q)
                 code[st->h_act[q]] = (uint8_t)((vzb[q] >= 0 ? 1 : 0) | (vza[q] >= 0 ? 2 : 0));
             CKN(cudaMalloc(&st->d_plate_code, code.size()));
             CKN(cudaMemcpy(st->d_plate_code, code.data(), code.size(), cudaMemcpyHostToDevice));
-            // cells whose pressure update reads plate face kf: k = kf-1 .. kf+2
-            std::vector<long long> fix;
-            for (const auto* lst : {&vzb, &vza})
-                for (long long q : *lst) {
-                    if (q < 0) continue;
-                    const int kf = (int)(q % st->g.sz);
-                    const long long row = q - kf;
-                    for (int k = kf - 1; k <= kf + 2; ++k)
-                        if (k >= 0 && k < Nz) fix.push_back(row + (k & ~3));
-                }
-            std::sort(fix.begin(), fix.end());
-            fix.erase(std::unique(fix.begin(), fix.end()), fix.end());
-            st->n_pfix = (int)fix.size();
-            if (st->n_pfix > 0) {
-                CKN(cudaMalloc(&st->d_pfix, fix.size() * sizeof(long long)));
-                CKN(cudaMemcpy(st->d_pfix, fix.data(), fix.size() * sizeof(long long), cudaMemcpyHostToDevice));
-            }
         }
     }
 
@@ -2239,9 +2299,9 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
             CK(cudaMemcpyAsync(st->d_ext_pack, st->h_ext_pack, (size_t)n_pack * sizeof(int2), cudaMemcpyHostToDevice, s));
             CK(launch_ext_scatter(st->d_ext, st->d_ext_pack, n_pack, s));
         }
-        CK(cudaMemsetAsync(st->d_status + kStatusPlate, 0xFF, sizeof(unsigned), s));
+        CK(cudaMemsetAsync(st->d_status + kStatusPlate, 0xFF, 2 * sizeof(unsigned), s));   // node and step
         CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below, st->d_w[wc0], st->d_w[wp0],
-                             st->d_w[wt0], st->d_ext, P, st->pc, st->d_status, s));
+                             st->d_w[wt0], st->d_ext, P, st->pc, st->d_status, 0u, s));
         if (ext_left) CK(launch_zero_gated(st->d_ext, st->N_plate, gate, s));
         PlateFaces pf;   // plate face velocities and the consumed forces' zeroing, in the velocity pass
         pf.code = st->d_plate_code;
@@ -2346,13 +2406,7 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
         st->wi_tmp = wt0;
         st->trace_len = trace0;
         if (checked) st->stab_phase = phase0;
-        const int pidx = st->h_act[bad];
-        float wn = NAN;
-        cudaMemcpy(&wn, st->d_w[st->wi_tmp] + pidx, sizeof(float), cudaMemcpyDeviceToHost);
-        fprintf(stderr, "[fdtd_plate] UNSTABLE step=%d plate_node=%d (%d,%d) w_new=%.3g m (limit 0.02 m)\n",
-                st->step_count, pidx, pidx / st->Ny, pidx % st->Ny, (double)wn);
-        fflush(stderr);
-        return FDTD_ERR_UNSTABLE;   // pending forces stay, as after fdtd_step
+        return report_plate(st);   // pending forces stay, as after fdtd_step
     }
     st->dev_ext_nonzero = false;    // consumed by the gated zeroing
     if (ext_was_pending) clear_ext_host(st);

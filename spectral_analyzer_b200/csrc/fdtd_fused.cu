@@ -782,7 +782,11 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
                                                       const __grid_constant__ CUtensorMap tmZ,
                                                       int seg_len, int tiles_k)
 {
+    if constexpr (WALLS) release_next();   // the plate's kernel may line up (it waits for this one's results)
     if ((int)blockIdx.y * seg_len >= (a.xs.nxg > 0 ? a.xs.n_own : a.g.nx)) return;
+    if constexpr (WALLS) {
+        if (a.gate && a.gate[kStatusPlateStep] != 0xFFFFFFFFu) return;
+    }
     float* smem;
     const unsigned sbase = smem_base_u32<C>(&smem);
     const unsigned bar0 = sbase + 4u * C::BAR0;

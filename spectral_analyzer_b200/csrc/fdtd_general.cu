@@ -10,6 +10,7 @@
  * 20 B/cell (+ fractions and solid mask when present).
  */
 #include "fdtd_internal.h"
+#include "launch.h"
 
 #include <math.h>
 
@@ -146,13 +147,15 @@ __global__ void __launch_bounds__(256) k_velocity_general(
 }
 
 // The pressure update of cells k0 .. k0+3 of row (i, j), id = their padded index.
+// Vz faces kp-1 (code bit 0) and kp (bit 1) have the velocity vp in place of the
+// stored one (the plate's faces; code 0: none).
 __device__ __forceinline__ void pressure_cells4(const Grid& g, const Coef& cf, const Tables& tb,
                                                 const float* __restrict__ p, float* __restrict__ pn,
                                                 const float* __restrict__ vx, const float* __restrict__ vy,
                                                 const float* __restrict__ vz, const float* __restrict__ fx,
                                                 const float* __restrict__ fy, const float* __restrict__ fz,
                                                 const uint8_t* __restrict__ solid, int i, int j, int k0,
-                                                long long id)
+                                                long long id, unsigned code = 0, int kp = 0, float vp = 0.0f)
 {
     const long long P = g.plane, S = g.sz;
     // face values times their fractions, four cells at a time (zero when absent)
@@ -179,14 +182,22 @@ __device__ __forceinline__ void pressure_cells4(const Grid& g, const Coef& cf, c
     face4(vy, fy, id + S, j < g.ny - 2, ypp);
     face4(vy, fy, id - 2 * S, j > 1, ymm);
     // Vz (times fraction) at k0-2 .. k0+4: e[t] = FZ[k0 - 2 + t]
-    auto fzv = [&](long long q) { return fz ? fmul(vz[q], fz[q]) : vz[q]; };
+    auto fzv = [&](long long q, int k) {
+        float v = vz[q];
+        if ((k == kp - 1 && (code & 1u)) || (k == kp && (code & 2u))) v = vp;
+        return fz ? fmul(v, fz[q]) : v;
+    };
     float e[7], c4[4], pc[4], out[4];
     face4(vz, fz, id, true, c4);
-    e[0] = k0 >= 2 ? fzv(id - 2) : 0.0f;
-    e[1] = k0 >= 1 ? fzv(id - 1) : 0.0f;
+    e[0] = k0 >= 2 ? fzv(id - 2, k0 - 2) : 0.0f;
+    e[1] = k0 >= 1 ? fzv(id - 1, k0 - 1) : 0.0f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) e[q + 2] = c4[q];
-    e[6] = k0 + 4 < g.nz ? fzv(id + 4) : 0.0f;
+    for (int q = 0; q < 4; ++q) {
+        e[q + 2] = c4[q];
+        if ((k0 + q == kp - 1 && (code & 1u)) || (k0 + q == kp && (code & 2u)))
+            e[q + 2] = fz ? fmul(vp, fz[id + q]) : vp;
+    }
+    e[6] = k0 + 4 < g.nz ? fzv(id + 4, k0 + 4) : 0.0f;
     unpack(ld4(p, id), pc);
     uint32_t sol = 0;
     if (solid) sol = *reinterpret_cast<const uint32_t*>(solid + id);
@@ -223,67 +234,92 @@ __global__ void __launch_bounds__(256) k_pressure_general(
     pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, id);
 }
 
-// The same update on a list of four-cell groups (padded index of each group's
-// first cell): after the single-pass walled step, the cells whose divergence
-// reads a plate face, recomputed once the plate has set those faces.
-__global__ void __launch_bounds__(256) k_pressure_groups(
-    Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ pn,
-    const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz,
-    const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz,
-    const uint8_t* __restrict__ solid, const long long* __restrict__ groups, int n_groups)
+// New displacement of active node q (acoustic_fdtd.cpp:984-1053).
+__device__ __forceinline__ float plate_node(int q, int pidx, const int* __restrict__ nb13, float pa, float pb,
+                                            const float* __restrict__ w, const float* __restrict__ wp, float fb,
+                                            const PlateCoef& pc)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_groups) return;
-    const long long id = groups[t];
-    const int i = (int)(id / g.plane);
-    const long long r = id - (long long)i * g.plane;
-    const int j = (int)(r / g.sz), k0 = (int)(r - (long long)j * g.sz);
-    pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, id);
-}
-
-// Kirchhoff plate step (acoustic_fdtd.cpp:984-1053), one thread per active node.
-// A node whose new displacement is non-finite or above 0.02 m records its
-// ordinal in status[kStatusPlate] (the host reports the lowest one).
-__global__ void k_plate_step(int n_act, const int* __restrict__ act, const int* __restrict__ nb13,
-                             const long long* __restrict__ above,
-                             const long long* __restrict__ below, const float* __restrict__ w,
-                             const float* __restrict__ wp, float* __restrict__ wt,
-                             const float* __restrict__ ext, const float* __restrict__ p,
-                             PlateCoef pc, unsigned* __restrict__ status)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_act) return;
     const float W13[13] = {20.f, -8.f, -8.f, -8.f, -8.f, 2.f, 2.f, 2.f, 2.f, 1.f, 1.f, 1.f, 1.f};
-    const int pidx = act[q];
     const int* nb = nb13 + 13 * q;
     float bh = 0.0f, bhp = 0.0f;
     for (int t = 0; t < 13; ++t) bh = fadd(bh, fmul(W13[t], w[nb[t]]));
-    const float pa = above[q] >= 0 ? p[above[q]] : 0.0f;
-    const float pb = below[q] >= 0 ? p[below[q]] : 0.0f;
-    const float fb = ext[pidx];
     for (int t = 0; t < 13; ++t) bhp = fadd(bhp, fmul(W13[t], wp[nb[t]]));
     const float vel = fsub(w[pidx], wp[pidx]);
     float wn = fadd(w[pidx], fmul(pc.vd, vel));
     wn = fadd(wn, fmul(pc.a, fadd(fsub(pb, pa), fb)));
     wn = fsub(wn, fmul(pc.bh, bh));
-    wn = fsub(wn, fmul(pc.bk, fsub(bh, bhp)));
-    if (!isfinite(wn) || fabsf(wn) > 0.02f) atomicMin(status + kStatusPlate, (unsigned)q);
-    wt[pidx] = wn;
+    return fsub(wn, fmul(pc.bk, fsub(bh, bhp)));
 }
+__device__ __forceinline__ bool plate_bad(float wn) { return !isfinite(wn) || fabsf(wn) > 0.02f; }
 
-// Plate velocity imposed on the Vz faces beside each active node (acoustic_fdtd.cpp:1158-1163).
-__global__ void k_plate_inject(int n_act, const int* __restrict__ act,
-                               const long long* __restrict__ vzb, const long long* __restrict__ vza,
-                               const float* __restrict__ w, const float* __restrict__ wp,
-                               float inv_dt, float* __restrict__ vz, const unsigned* __restrict__ gate)
+// Kirchhoff plate step, one thread per active node.  A node whose new
+// displacement is non-finite or above 0.02 m records its ordinal in
+// status[kStatusPlate] (the host reports the lowest one) and the step; later
+// steps queued behind it then do nothing.
+__global__ void k_plate_step(int n_act, const int* __restrict__ act, const int* __restrict__ nb13,
+                             const long long* __restrict__ above,
+                             const long long* __restrict__ below, const float* __restrict__ w,
+                             const float* __restrict__ wp, float* __restrict__ wt,
+                             const float* __restrict__ ext, const float* __restrict__ p,
+                             PlateCoef pc, unsigned* __restrict__ status, unsigned step)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_act) return;
-    if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
+    if (*(volatile unsigned*)(status + kStatusPlateStep) < step) return;   // an earlier step of the window failed
     const int pidx = act[q];
-    const float v = fmul(fsub(w[pidx], wp[pidx]), inv_dt);
-    if (vzb[q] >= 0) vz[vzb[q]] = v;
-    if (vza[q] >= 0) vz[vza[q]] = v;
+    const float wn = plate_node(q, pidx, nb13, above[q] >= 0 ? p[above[q]] : 0.0f, below[q] >= 0 ? p[below[q]] : 0.0f,
+                                w, wp, ext[pidx], pc);
+    if (plate_bad(wn)) {
+        atomicMin(status + kStatusPlate, (unsigned)q);
+        atomicMin(status + kStatusPlateStep, step);
+    }
+    wt[pidx] = wn;
+}
+
+// The plate's part of a single-pass step, two threads per active node.  Both
+// compute the node's new displacement; the first stores it with the velocity it
+// imposes on the Vz faces beside the plate (acoustic_fdtd.cpp:1158-1163).  The
+// cells whose divergence reads those faces, iz-2 .. iz+2 of the node's own
+// column and so at most two four-cell groups, are then updated again from P^n
+// and the new velocities, a group per thread.  The displacement needs nothing
+// of the march and is computed while it drains.  256x200x128 body scene: 5.5
+// us behind the march where separate plate, face and group kernels and the
+// wait for the guard between them took 47.
+__global__ void __launch_bounds__(128) k_plate_columns(Grid g, Coef cf, Tables tb, PlateStep ps,
+                                                       const float* __restrict__ p, float* __restrict__ pn,
+                                                       const float* __restrict__ vx, const float* __restrict__ vy,
+                                                       float* vz, const float* __restrict__ fx,
+                                                       const float* __restrict__ fy, const float* __restrict__ fz,
+                                                       const uint8_t* __restrict__ solid)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t >> 1;
+    const bool in = q < ps.n_act && *(volatile unsigned*)(ps.status + kStatusPlateStep) >= ps.step;
+    int pidx = 0;
+    float wn = 0.0f, v = 0.0f;
+    if (in) {
+        pidx = ps.act[q];
+        wn = plate_node(q, pidx, ps.nb13, ps.above[q] >= 0 ? p[ps.above[q]] : 0.0f,
+                        ps.below[q] >= 0 ? p[ps.below[q]] : 0.0f, ps.w, ps.wp, ps.ext[pidx], ps.pc);
+        v = fmul(fsub(wn, ps.w[pidx]), ps.inv_dt);
+    }
+    wait_previous();
+    if (!in) return;
+    const int i = pidx / g.ny, j = pidx - i * g.ny;
+    const long long row = ((long long)i * g.ny + j) * g.sz;
+    const unsigned code = ps.code[pidx];
+    if ((t & 1) == 0) {
+        if (plate_bad(wn)) {
+            atomicMin(ps.status + kStatusPlate, (unsigned)q);
+            atomicMin(ps.status + kStatusPlateStep, ps.step);
+        }
+        ps.wt[pidx] = wn;
+        if (code & 1u) vz[row + ps.iz - 1] = v;
+        if (code & 2u) vz[row + ps.iz] = v;
+    }
+    if (code == 0) return;
+    const int lo = max(ps.iz - ((code & 1u) ? 2 : 1), 0) & ~3, hi = min(ps.iz + ((code & 2u) ? 2 : 1), g.nz - 1) & ~3;
+    const int k0 = lo + 4 * (t & 1);
+    if (k0 <= hi) pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, row + k0, code, ps.iz, v);
 }
 
 // One deposit of the open-cell rule (acoustic_fdtd.cpp:840-872).  The amplitude
@@ -395,32 +431,21 @@ cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables&
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,
                               const long long* below, const float* w, const float* wp, float* wt,
                               const float* ext, const float* p, const PlateCoef& pc,
-                              unsigned* status, cudaStream_t s)
+                              unsigned* status, unsigned step, cudaStream_t s)
 {
     if (n_act <= 0) return cudaSuccess;
     k_plate_step<<<(n_act + 127) / 128, 128, 0, s>>>(n_act, act, nb13, above, below, w, wp, wt,
-                                                     ext, p, pc, status);
+                                                     ext, p, pc, status, step);
     return cudaGetLastError();
 }
 
-cudaError_t launch_pressure_groups(const Grid& g, const Coef& cf, const Tables& tb, const float* p, float* pn,
-                                   const float* vx, const float* vy, const float* vz, const float* fx,
-                                   const float* fy, const float* fz, const uint8_t* solid,
-                                   const long long* groups, int n_groups, cudaStream_t s)
+cudaError_t launch_plate_columns(const Grid& g, const Coef& cf, const Tables& tb, const PlateStep& ps, const float* p,
+                                 float* pn, const float* vx, const float* vy, float* vz, const float* fx,
+                                 const float* fy, const float* fz, const uint8_t* solid, cudaStream_t s)
 {
-    if (n_groups <= 0) return cudaSuccess;
-    k_pressure_groups<<<(n_groups + 255) / 256, 256, 0, s>>>(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid,
-                                                             groups, n_groups);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_plate_inject(int n_act, const int* act, const long long* vzb,
-                                const long long* vza, const float* w, const float* wp,
-                                float inv_dt, float* vz, cudaStream_t s, const unsigned* gate)
-{
-    if (n_act <= 0) return cudaSuccess;
-    k_plate_inject<<<(n_act + 127) / 128, 128, 0, s>>>(n_act, act, vzb, vza, w, wp, inv_dt, vz, gate);
-    return cudaGetLastError();
+    if (ps.n_act <= 0) return cudaSuccess;
+    return launch_after(k_plate_columns, dim3((2 * ps.n_act + 127) / 128), dim3(128), 0, s, g, cf, tb, ps, p, pn, vx, vy,
+                        vz, fx, fy, fz, solid);
 }
 
 cudaError_t launch_deposit(const Deposit& d, const float* signal, int step, float amp, float* p,

@@ -106,9 +106,17 @@ struct Deposit {
 };
 
 // Status words (unsigned, 0xFFFFFFFF = none), reset with a 0xFF memset:
-// first unstable cell of a check, first unstable plate node, first failing
-// step latched by async stepping, and a fused-step CTA whose load wait ran out.
-enum StatusSlot { kStatusCell = 0, kStatusPlate = 1, kStatusLatch = 2, kStatusTimeout = 3, kStatusWords = 4 };
+// first unstable cell of a check, first unstable plate node and the step it
+// failed at, first failing step latched by async stepping, and a fused-step CTA
+// whose load wait ran out.
+enum StatusSlot {
+    kStatusCell = 0,
+    kStatusPlate = 1,
+    kStatusPlateStep = 2,
+    kStatusLatch = 3,
+    kStatusTimeout = 4,
+    kStatusWords = 5
+};
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
@@ -148,11 +156,6 @@ cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables&
                                     const float* fx, const float* fy, const float* fz,
                                     cudaStream_t s, const unsigned* gate = nullptr,
                                     const PlateFaces* pf = nullptr);
-// pressure update of listed four-cell groups (plate-face neighbours after a walled single-pass step)
-cudaError_t launch_pressure_groups(const Grid& g, const Coef& cf, const Tables& tb, const float* p, float* pn,
-                                   const float* vx, const float* vy, const float* vz, const float* fx,
-                                   const float* fy, const float* fz, const uint8_t* solid,
-                                   const long long* groups, int n_groups, cudaStream_t s);
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
@@ -161,14 +164,32 @@ cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables&
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,
                               const long long* below, const float* w, const float* wp, float* wt,
                               const float* ext, const float* p, const PlateCoef& pc,
-                              unsigned* status, cudaStream_t s);
+                              unsigned* status, unsigned step, cudaStream_t s);
+// The plate's part of a single-pass step: what the plate update and its coupling
+// read and write (P^n, P^{n+1} and V^{n+1/2} as the march left them).
+struct PlateStep {
+    int n_act = 0, iz = -1;
+    const int* act = nullptr;         // active nodes, j + Ny * i
+    const int* nb13 = nullptr;
+    const uint8_t* code = nullptr;    // per node: bit 0 Vz face below, bit 1 above
+    const long long* above = nullptr;
+    const long long* below = nullptr;
+    const float* w = nullptr;         // displacement, previous, next
+    const float* wp = nullptr;
+    float* wt = nullptr;
+    const float* ext = nullptr;
+    PlateCoef pc{};
+    float inv_dt = 0.0f;
+    unsigned* status = nullptr;
+    unsigned step = 0;
+};
+// Launched directly behind the march, whose end it overlaps (launch.h).
+cudaError_t launch_plate_columns(const Grid& g, const Coef& cf, const Tables& tb, const PlateStep& ps, const float* p,
+                                 float* pn, const float* vx, const float* vy, float* vz, const float* fx,
+                                 const float* fy, const float* fz, const uint8_t* solid, cudaStream_t s);
 // plate forces as (node, value) pairs scattered into the zeroed device buffer
 // (the velocity pass returns them to zero: PlateFaces)
 cudaError_t launch_ext_scatter(float* ext, const int2* pack, int m, cudaStream_t s);
-cudaError_t launch_plate_inject(int n_act, const int* act, const long long* vzb,
-                                const long long* vza, const float* w, const float* wp,
-                                float inv_dt, float* vz, cudaStream_t s,
-                                const unsigned* gate = nullptr);
 cudaError_t launch_deposit(const Deposit& d, const float* signal, int step, float amp, float* p,
                            cudaStream_t s);
 cudaError_t launch_wsum(const float* f, const long long* idx, const float* w, int n_out, int taps,
@@ -247,6 +268,8 @@ struct FusedArgs {
     const float* fr[3] = {nullptr, nullptr, nullptr};
     bool frac_div = false;
     const uint8_t* solid = nullptr;
+    // plate scenes: the step does nothing when an earlier step's plate update failed
+    const unsigned* gate = nullptr;
 };
 struct FusedCache;         // host-side TMA descriptors of a handle's fields
 FusedCache* fused_cache_create();
