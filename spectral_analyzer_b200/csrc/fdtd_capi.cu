@@ -81,7 +81,7 @@ struct SubstepKey {
     cudaStream_t stream;
     const float *p, *pn, *v0, *v1, *v2, *w_cur, *w_prev, *w_tmp, *frac[3], *ext, *h_ext;
     const int2 *pack, *h_pack;
-    const uint8_t* solid;
+    const uint8_t *solid, *walls;
     const long long *sidx;
     const float *sw;
     float *sout, *h_sout;
@@ -126,6 +126,7 @@ struct AcousticFDTDState {
     std::vector<uint8_t> plate_active;
     bool any_solid = false;
     uint8_t* d_solid = nullptr;
+    uint8_t* d_walls = nullptr;          // WallCode per four-cell group, from fractions and mask
     std::vector<float> frac[3];          // reference layouts, built on first need
     float* d_frac[3] = {nullptr, nullptr, nullptr};
     bool has_frac = false;
@@ -316,6 +317,8 @@ int upload_fracs(AcousticFDTDState* st)
     if ((rc = copy_block(st, st->d_frac[0], st->frac[0].data(), st->Nx - 1, st->Ny, st->Nz, true))) return rc;
     if ((rc = copy_block(st, st->d_frac[1], st->frac[1].data(), st->Nx, st->Ny - 1, st->Nz, true))) return rc;
     if ((rc = copy_block(st, st->d_frac[2], st->frac[2].data(), st->Nx, st->Ny, st->Nz - 1, true))) return rc;
+    if (!st->d_walls) CK(cudaMalloc(&st->d_walls, (size_t)st->g.cells / 4));
+    CK(launch_wall_codes(st->g, st->d_frac[0], st->d_frac[1], st->d_frac[2], st->d_solid, st->d_walls, st->stream));
     return FDTD_OK;
 }
 
@@ -508,11 +511,11 @@ bool fused_walled_ok(const AcousticFDTDState* st)
 }
 
 // Walled scenes take the single pass automatically from this many cells on:
-// below it the fields stay in L2 and the two-pass kernels are faster (step
-// kernels per step, two-pass / single pass: 170x140x74 40 / 67 us,
-// 160x128x128 50 / 60; above it 256x200x128 120 / 106, 400x300x256 511 / 430,
-// 512x384x256 827 / 558).
-constexpr long long kWalledFusedCells = 1LL << 22;
+// below it the fields stay in L2 and the two-pass kernels' extra bytes cost less
+// than the march's pipeline fill (fdtd_step per step on plate scenes, two-pass /
+// single pass: 130x110x60 24.9 / 26.9 us, 170x140x74 35.6 / 42.3, 160x128x128
+// 43.2 / 38.9, 200x160x100 56.8 / 53.5, 256x200x128 114 / 74, 300x240x160 187 / 134).
+constexpr long long kWalledFusedCells = 5LL << 19;
 
 bool use_fused(const AcousticFDTDState* st)
 {
@@ -688,6 +691,7 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
             for (int c2 = 0; c2 < 3; ++c2) a.fr[c2] = st->d_frac[c2];
             a.frac_div = st->has_frac;
             a.solid = st->d_solid;
+            a.walls = st->d_walls;
         }
         if (fuse_deposit) {
             const long long c = st->ps.idx[0], t = c / st->g.sz;
@@ -710,13 +714,13 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
         if ((rc = prof_end(st, e1, fused_kernel_launches_per_step()))) return rc;
     } else {
         CK(launch_velocity_general(st->g, st->cf, st->tb, st->P(), st->V(0), st->V(1), st->V(2),
-                                   st->d_frac[0], st->d_frac[1], st->d_frac[2], s));
+                                   st->d_frac[0], st->d_frac[1], st->d_frac[2], st->d_walls, s));
         st->launches += 2;
         const bool hf = st->has_frac;
         CK(launch_pressure_general(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1),
                                    st->V(2), hf ? st->d_frac[0] : nullptr,
                                    hf ? st->d_frac[1] : nullptr, hf ? st->d_frac[2] : nullptr,
-                                   st->d_solid, s));
+                                   st->d_solid, st->d_walls, s));
         if ((rc = prof_end(st, e1, 2))) return rc;
     }
     st->cur ^= 1;
@@ -884,21 +888,21 @@ int plate_steps(AcousticFDTDState* st, int n_steps, bool sync_check, int* done)
     for (int q = 0; q < m; ++q) {
         const unsigned step = (unsigned)st->step_count;
         cudaEvent_t e1;
+        CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below, st->d_w[st->wi_cur],
+                             st->d_w[st->wi_prev], st->d_w[st->wi_tmp], st->d_ext, st->P(), st->pc, st->d_status,
+                             step, s));
+        PlateFaces pf;   // the plate's face velocities, set as the step updates those faces
+        pf.code = st->d_plate_code;
+        pf.w = st->d_w[st->wi_tmp];
+        pf.wp = st->d_w[st->wi_cur];
+        pf.inv_dt = st->cf.inv_dt;
+        pf.iz = st->plate_iz;
         if (!fused) {
-            CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below, st->d_w[st->wi_cur],
-                                 st->d_w[st->wi_prev], st->d_w[st->wi_tmp], st->d_ext, st->P(), st->pc, st->d_status,
-                                 step, s));
-            PlateFaces pf;   // the plate's face velocities, set inside the velocity pass
-            pf.code = st->d_plate_code;
-            pf.w = st->d_w[st->wi_tmp];
-            pf.wp = st->d_w[st->wi_cur];
-            pf.inv_dt = st->cf.inv_dt;
-            pf.iz = st->plate_iz;
             if (int rc = prof_begin(st, &e1)) return rc;
             CK(launch_velocity_general(st->g, st->cf, st->tb, st->P(), st->V(0), st->V(1), st->V(2), st->d_frac[0],
-                                       st->d_frac[1], st->d_frac[2], s, st->d_status, &pf));
+                                       st->d_frac[1], st->d_frac[2], st->d_walls, s, st->d_status, &pf));
             CK(launch_pressure_general(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2), fdiv[0],
-                                       fdiv[1], fdiv[2], st->d_solid, s, st->d_status));
+                                       fdiv[1], fdiv[2], st->d_solid, st->d_walls, s, st->d_status));
             if (int rc = prof_end(st, e1, 2)) return rc;
             st->launches += 3;
         } else {
@@ -911,29 +915,13 @@ int plate_steps(AcousticFDTDState* st, int n_steps, bool sync_check, int* done)
             for (int c2 = 0; c2 < 3; ++c2) a.fr[c2] = st->d_frac[c2];
             a.frac_div = hf;
             a.solid = st->d_solid;
-            if (q > 0) a.gate = st->d_status;
+            a.walls = st->d_walls;
+            a.plate = pf;
+            a.gate = st->d_status;
             if (int rc = prof_begin(st, &e1)) return rc;
             CK(launch_fused_step(a, st->fcache, s));
             st->cv ^= 1;
-            PlateStep ps;
-            ps.n_act = st->n_act;
-            ps.iz = st->plate_iz;
-            ps.act = st->d_act;
-            ps.nb13 = st->d_nb13;
-            ps.code = st->d_plate_code;
-            ps.above = st->d_above;
-            ps.below = st->d_below;
-            ps.w = st->d_w[st->wi_cur];
-            ps.wp = st->d_w[st->wi_prev];
-            ps.wt = st->d_w[st->wi_tmp];
-            ps.ext = st->d_ext;
-            ps.pc = st->pc;
-            ps.inv_dt = st->cf.inv_dt;
-            ps.status = st->d_status;
-            ps.step = step;
-            CK(launch_plate_columns(st->g, st->cf, st->tb, ps, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2), fdiv[0],
-                                    fdiv[1], fdiv[2], st->d_solid, s));
-            if (int rc = prof_end(st, e1, 2)) return rc;
+            if (int rc = prof_end(st, e1, fused_kernel_launches_per_step())) return rc;
             st->launches += 2;
         }
         if (q == 0 && st->dev_ext_nonzero) {   // the forces are consumed (the host keeps them until the guard is read)
@@ -1009,6 +997,7 @@ void free_state(AcousticFDTDState* st)
     }
     cudaFree(st->d_tab);
     cudaFree(st->d_solid);
+    cudaFree(st->d_walls);
     for (int c = 0; c < 3; ++c) { cudaFree(st->d_frac[c]); cudaFree(st->d_w[c]); }
     cudaFree(st->d_act); cudaFree(st->d_nb13); cudaFree(st->d_above); cudaFree(st->d_below);
     cudaFree(st->d_plate_code); cudaFree(st->d_ext); cudaFree(st->d_slice);
@@ -2315,10 +2304,10 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
             pf.m = n_pack;
         }
         CK(launch_velocity_general(st->g, st->cf, st->tb, P, st->V(0), st->V(1), st->V(2), st->d_frac[0],
-                                   st->d_frac[1], st->d_frac[2], s, gate, &pf));
+                                   st->d_frac[1], st->d_frac[2], st->d_walls, s, gate, &pf));
         CK(launch_pressure_general(st->g, st->cf, st->tb, P, Pn, st->V(0), st->V(1), st->V(2),
                                    hf ? st->d_frac[0] : nullptr, hf ? st->d_frac[1] : nullptr,
-                                   hf ? st->d_frac[2] : nullptr, st->d_solid, s, gate));
+                                   hf ? st->d_frac[2] : nullptr, st->d_solid, st->d_walls, s, gate));
         if (record)
             CK(launch_wsum(Pn, st->d_rec_idx, st->d_rec_w, st->n_rec, 8, 0,
                            st->d_trace + (size_t)trace0 * st->n_rec, s));
@@ -2345,7 +2334,7 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
         k.p = P; k.pn = Pn; k.v0 = st->V(0); k.v1 = st->V(1); k.v2 = st->V(2);
         k.w_cur = st->d_w[wc0]; k.w_prev = st->d_w[wp0]; k.w_tmp = st->d_w[wt0];
         for (int c2 = 0; c2 < 3; ++c2) k.frac[c2] = st->d_frac[c2];
-        k.ext = st->d_ext; k.h_ext = st->h_ext; k.solid = st->d_solid;
+        k.ext = st->d_ext; k.h_ext = st->h_ext; k.solid = st->d_solid; k.walls = st->d_walls;
         k.pack = st->d_ext_pack; k.h_pack = st->h_ext_pack; k.n_pack = n_pack;
         k.sidx = st->d_sidx; k.sw = st->d_sw; k.sout = st->d_sout; k.h_sout = st->h_sout;
         k.status = st->d_status; k.h_status = st->h_status;

@@ -419,6 +419,35 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         }
     }
     float *gX = nullptr, *gYa = nullptr, *gYb = nullptr, *gZ = nullptr, *gP = nullptr;
+    // WALLS: the wall codes of the groups whose fractions iteration u reads (Vx
+    // face u-2 and plane u-3), the plate node (at plane 0) whose faces lie in this
+    // thread's quad (-1: none), and whether its halo face is a plate's
+    unsigned wc_x = 0u, wc_a = 0u, wc_b = 0u, wc_z = 0u;
+    const uint8_t* wr = nullptr;      // a.walls at plane u-2, advanced with u
+    const int pl4 = (int)(PL >> 2), own4 = own >> 2, ya4 = ((jfa * sz + kb) >> 2) - pl4, yb4 = ((jfb * sz + kb) >> 2) - pl4;
+    const bool wx_on = st_ok, wa_on = ya_ok && kb < sz, wb_on = yb_ok && kb < sz && C::TJ + w < C::VYR;
+    auto wall_codes = [&](int u) {    // wr at plane u-2
+        const bool in = u - 3 >= i_beg && u - 3 < i_end;
+        wc_x = wx_on && (unsigned)(u - 2) < (unsigned)nx ? __ldg(wr + own4) : 0u;
+        wc_a = wa_on && in ? __ldg(wr + ya4) : 0u;
+        wc_b = wb_on && in ? __ldg(wr + yb4) : 0u;
+        wr += pl4;
+    };
+    int pl_node = -1;
+    bool pl_halo = false;
+    if constexpr (WALLS) {
+        const int iz = a.plate.iz;
+        if (a.plate.code && row_ok && kb <= iz && iz - 1 <= kb + 3) pl_node = jr;
+        pl_halo = a.plate.code && h_ok && (h_k == iz - 1 || h_k == iz);
+        wr = a.walls + (long long)(u0 - 3) * pl4;
+        wall_codes(u0 - 1);
+        wc_z = wc_x;
+        wall_codes(u0);
+    }
+    // a plate face takes the plate's velocity after the update
+    auto plate_face = [&](float v, int k, unsigned c, float vp) {
+        return ((k == a.plate.iz - 1 && (c & 1u)) || (k == a.plate.iz && (c & 2u))) ? vp : v;
+    };
 
     // One iteration of the march; FAST = the interior body.  False when a load
     // wait ran out (u_fail is then set).
@@ -427,27 +456,40 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         // wait for plane u (P) and iteration u's V data; the decision to stop on a
         // timeout is made by the whole CTA (the barrier below is also the one that
         // separates the previous iteration's reads from this iteration's writes)
-        // WALLS: this iteration's face fractions and solid flags, loaded before
-        // the wait so that their latency overlaps it (they do not depend on it)
+        // WALLS: this iteration's face fractions and solid flags, where the groups'
+        // wall codes (read an iteration ahead) call for them, loaded before the
+        // wait so that their latency overlaps it; and the plate's face velocity
         float4 pf_x = make_float4(1.f, 1.f, 1.f, 1.f), pf_y0 = pf_x, pf_y1 = pf_x, pf_z = pf_x;
-        float pf_h = 1.0f;
-        unsigned pf_s = 0u;
+        float pf_h = 1.0f, pl_w = 0.0f, pl_wp = 0.0f, pl_hw = 0.0f, pl_hwp = 0.0f;
+        unsigned pf_s = 0u, pl_c = 0u, pl_hc = 0u;
+        const unsigned cx = wc_x, ca = wc_a, cb = wc_b, cz = wc_z;
         if constexpr (WALLS) {
-            const int f = u - 2, i = u - 3;
-            if (a.fr[0] && st_ok && u >= i_beg && f >= 0 && f <= nx - 2) pf_x = ldg4(a.fr[0] + f * PL + own);
-            if (i >= i_beg) {
+            const int i = u - 3;
+            if ((cx & kWallX) | (ca & kWallY) | (cb & kWallY) | (cz & (kWallZ | kWallSolid))) {
                 const long long ib = (long long)i * PL;
-                if (a.fr[1] && kb < sz) {
-                    const int jf0 = j0 - 2 + w, jf1 = j0 - 2 + C::TJ + w;
-                    if (jf0 >= 0 && jf0 <= ny - 2) pf_y0 = ldg4(a.fr[1] + ib + (long long)jf0 * sz + kb);
-                    if (C::TJ + w < C::VYR && jf1 >= 0 && jf1 <= ny - 2)
-                        pf_y1 = ldg4(a.fr[1] + ib + (long long)jf1 * sz + kb);
-                }
-                if (a.fr[2] && st_ok) pf_z = ldg4(a.fr[2] + ib + own);
-                if (a.fr[2] && h_ok) pf_h = __ldg(a.fr[2] + ib + (long long)(j0 + h_j) * sz + h_k);
-                if (a.solid && row_ok && kb < sz)
-                    pf_s = __ldg(reinterpret_cast<const unsigned*>(a.solid + ib + own));
+                if (cx & kWallX) pf_x = ldg4(a.fr[0] + ib + PL + own);
+                if (ca & kWallY) pf_y0 = ldg4(a.fr[1] + ib + (long long)jfa * sz + kb);
+                if (cb & kWallY) pf_y1 = ldg4(a.fr[1] + ib + (long long)jfb * sz + kb);
+                if (cz & kWallZ) pf_z = ldg4(a.fr[2] + ib + own);
+                if (cz & kWallSolid) pf_s = __ldg(reinterpret_cast<const unsigned*>(a.solid + ib + own));
             }
+            if (i >= i_beg && i < i_end) {
+                if (a.fr[2] && h_ok) pf_h = __ldg(a.fr[2] + (long long)i * PL + (j0 + h_j) * sz + h_k);
+                if (pl_node >= 0) {
+                    const int node = pl_node + ny * i;
+                    pl_c = __ldg(a.plate.code + node);
+                    pl_w = __ldg(a.plate.w + node);
+                    pl_wp = __ldg(a.plate.wp + node);
+                }
+                if (pl_halo) {
+                    const int node = j0 + h_j + ny * i;
+                    pl_hc = __ldg(a.plate.code + node);
+                    pl_hw = __ldg(a.plate.w + node);
+                    pl_hwp = __ldg(a.plate.wp + node);
+                }
+            }
+            wc_z = wc_x;
+            wall_codes(u + 1);
         }
         const bool ok = mbar_wait(bar0 + 8u * ps, (ph >> ps) & 1u, a.wait_us);
         // the source deposit, on the arriving plane's shared copy before anyone reads it
@@ -507,10 +549,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                 }
                 if constexpr (WALLS) {
                     vdiv = vnew;
-                    if (a.fr[0] && st_ok) {
-                        const float4 fr = pf_x;
-                        vnew = close4(vnew, fr);
-                        vdiv = a.frac_div ? mul4(vnew, fr) : vnew;
+                    if (cx & kWallX) {
+                        vnew = close4(vnew, pf_x);
+                        vdiv = a.frac_div ? mul4(vnew, pf_x) : vnew;
                     }
                 }
                 if (f >= i_beg && f < i_end && st_ok) {
@@ -539,7 +580,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                 // Vy rows: row w, and row TJ+w for the first VYR-TJ warps
                 if constexpr (FAST) {
                     const float* pc = pst + 4 * lane + 4;
-                    auto row = [&](int r, const float4& dmp, bool ex, bool f4, float4 fry, float* dst) {
+                    auto row = [&](int r, const float4& dmp, bool ex, bool f4, float4 fry, unsigned c, float* dst) {
                         const float4 pm = lds4(pc + r * C::PC), p0 = lds4(pc + (r + 1) * C::PC);
                         const float4 p1 = lds4(pc + (r + 2) * C::PC), p2 = lds4(pc + (r + 3) * C::PC);
                         const float4 vo = lds4(vys + r * C::TK + 4 * lane);
@@ -547,18 +588,18 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                         if (jmid) v = vel4(cf, pm, p0, p1, p2, vo, dmp);
                         else v = vel4_masked(cf, pm, p0, p1, p2, vo, dmp, f4 ? 15 : 0, ex ? 15 : 0);
                         if constexpr (WALLS) {
-                            if (a.fr[1] && kb < sz && ex) v = close4(v, fry);
+                            if (c & kWallY) v = close4(v, fry);
                         }
                         if (dst) stg4(dst, v);
                         if constexpr (WALLS) {
-                            if (a.fr[1] && a.frac_div && kb < sz && ex) v = mul4(v, fry);
+                            if ((c & kWallY) && a.frac_div) v = mul4(v, fry);
                         }
                         sts4(vyn + r * C::TK + 4 * lane, v);
                     };
                     // own rows are r = 2 .. TJ+1 of the tile's Vy rows
-                    row(w, dyi[0], ya_ok, ya_4, pf_y0, w >= 2 && ya_ok && kb < sz ? gYa : nullptr);
+                    row(w, dyi[0], ya_ok, ya_4, pf_y0, ca, w >= 2 && ya_ok && kb < sz ? gYa : nullptr);
                     if (C::TJ + w < C::VYR)
-                        row(C::TJ + w, dyi[1], yb_ok, yb_4, pf_y1, w < 2 && yb_ok && kb < sz ? gYb : nullptr);
+                        row(C::TJ + w, dyi[1], yb_ok, yb_4, pf_y1, cb, w < 2 && yb_ok && kb < sz ? gYb : nullptr);
                 } else {
 #pragma unroll
                     for (int m = 0; m < NY_IT; ++m) {
@@ -590,7 +631,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                                 }
                                 float4 fry = make_float4(1.f, 1.f, 1.f, 1.f);
                                 if constexpr (WALLS) {
-                                    if (a.fr[1] && kb < sz) {
+                                    if ((m == 0 ? ca : cb) & kWallY) {
                                         fry = m == 0 ? pf_y0 : pf_y1;
                                         v = close4(v, fry);
                                     }
@@ -598,7 +639,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                                 if (r >= 2 && r < C::TJ + 2 && kb < sz)
                                     stg4(a.vout[1] + ib + (long long)jf * sz + kb, v);
                                 if constexpr (WALLS) {
-                                    if (a.fr[1] && a.frac_div && kb < sz) v = mul4(v, fry);
+                                    if (((m == 0 ? ca : cb) & kWallY) && a.frac_div) v = mul4(v, fry);
                                 }
                             }
                             sts4(vyn + r * C::TK + 4 * lane, v);
@@ -636,14 +677,19 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                         }
                         float4 frz = make_float4(1.f, 1.f, 1.f, 1.f);
                         if constexpr (WALLS) {
-                            if (a.fr[2] && st_ok) {
+                            if (cz & kWallZ) {
                                 frz = pf_z;
                                 v = close4(v, frz);
+                            }
+                            if (pl_c) {
+                                const float vp = fmul(fsub(pl_w, pl_wp), a.plate.inv_dt);
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) at(v, q) = plate_face(at(v, q), kb + q, pl_c, vp);
                             }
                         }
                         if (st_ok) stg4(FAST ? gZ : a.vout[2] + ib + own, v);
                         if constexpr (WALLS) {
-                            if (a.fr[2] && a.frac_div && st_ok) v = mul4(v, frz);
+                            if ((cz & kWallZ) && a.frac_div) v = mul4(v, frz);
                         }
                     }
                     sts4(vzn + w * C::PC + 4 * lane + 4, v);
@@ -665,6 +711,7 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                             if (a.fr[2]) {
                                 const float fz = pf_h;
                                 if (fz == 0.0f) vh = 0.0f;
+                                if (pl_hc) vh = plate_face(vh, h_k, pl_hc, fmul(fsub(pl_hw, pl_hwp), a.plate.inv_dt));
                                 if (a.frac_div) vh = fmul(vh, fz);
                             }
                         }
@@ -700,11 +747,10 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                             if (kb + q >= nz) at(out, q) = 0.0f;
                     }
                     if constexpr (WALLS) {
-                        if (a.solid && kb < sz) {   // solid cells keep P = 0
-                            const unsigned sol = pf_s;
+                        if (cz & kWallSolid) {   // solid cells keep P = 0
 #pragma unroll
                             for (int q = 0; q < 4; ++q)
-                                if ((sol >> (8 * q)) & 0xFFu) at(out, q) = 0.0f;
+                                if ((pf_s >> (8 * q)) & 0xFFu) at(out, q) = 0.0f;
                         }
                     }
                     if (FAST ? st_ok : kb < sz) {
@@ -782,10 +828,9 @@ __global__ void __launch_bounds__(C::NT) k_fused_step(FusedArgs a,
                                                       const __grid_constant__ CUtensorMap tmZ,
                                                       int seg_len, int tiles_k)
 {
-    if constexpr (WALLS) release_next();   // the plate's kernel may line up (it waits for this one's results)
     if ((int)blockIdx.y * seg_len >= (a.xs.nxg > 0 ? a.xs.n_own : a.g.nx)) return;
     if constexpr (WALLS) {
-        if (a.gate && a.gate[kStatusPlateStep] != 0xFFFFFFFFu) return;
+        if (a.gate && a.gate[kStatusPlate] != 0xFFFFFFFFu) return;
     }
     float* smem;
     const unsigned sbase = smem_base_u32<C>(&smem);
@@ -1067,7 +1112,7 @@ static cudaError_t launch_step_of(const FusedArgs& a, FusedCache* cache, cudaStr
     segs = (n_own + seg_len - 1) / seg_len;
     dim3 grid((unsigned)tiles, (unsigned)segs, 1);
     const bool peer = a.pr.pn[0] || a.pr.pn[1] || a.pr.vx[0] || a.pr.vx[1];
-    const bool walls = a.fr[0] || a.fr[1] || a.fr[2] || a.solid;
+    const bool walls = a.fr[0] || a.fr[1] || a.fr[2] || a.solid || a.plate.code;
     if (walls && (peer || a.xs.nxg > 0)) return cudaErrorInvalidValue;   // walled scenes are whole rooms
     // Plain launches: overlapping a step's start with the one before (launch.h)
     // was slower (512x384x256 room 266.6 -> 281 us, 160x128x112 24.7 -> 25.4).

@@ -10,7 +10,6 @@
  * 20 B/cell (+ fractions and solid mask when present).
  */
 #include "fdtd_internal.h"
-#include "launch.h"
 
 #include <math.h>
 
@@ -51,13 +50,14 @@ __device__ __forceinline__ void unpack(const float4& x, float (&v)[4]) { v[0] = 
 __global__ void __launch_bounds__(256) k_velocity_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ vx,
     float* __restrict__ vy, float* __restrict__ vz, const float* __restrict__ fx,
-    const float* __restrict__ fy, const float* __restrict__ fz, const unsigned* __restrict__ gate,
-    PlateFaces pf)
+    const float* __restrict__ fy, const float* __restrict__ fz, const uint8_t* __restrict__ walls,
+    const unsigned* __restrict__ gate, PlateFaces pf)
 {
     if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
     if (pf.m > 0 && blockIdx.x == 0 && blockIdx.y == 0)      // the consumed plate forces
         for (int q = threadIdx.x; q < pf.m; q += blockDim.x) pf.ext[pf.pack[q].x] = 0.0f;
     GEN_INDEX
+    const unsigned wall = walls ? walls[id >> 2] : 0u;
     const float ay = __ldg(tb.ay + j), axi = __ldg(tb.ax + i);
     float pc[4], az4[4], ac[4];
     unpack(ld4(p, id), pc);
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
             unpack(ld4(p, id + 2 * g.plane), p2);
         }
         unpack(ld4(vx, id), v);
-        if (fx) unpack(ld4(fx, id), fr);
+        if (wall & kWallX) unpack(ld4(fx, id), fr);
         const float axr = __ldg(tb.ax + i + 1);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
             const float grad = fourth ? fadd(fmul(cf.c1, fsub(pr[q], pc[q])), fmul(cf.c2, fsub(p2[q], pm[q])))
                                       : fsub(pr[q], pc[q]);
             float nv = fmul(fsub(v[q], fmul(cf.vc, grad)), face_damp(ac[q], fmaxf(fmaxf(axr, ay), az4[q]), cf.dt));
-            if (fx && fr[q] == 0.0f) nv = 0.0f;
+            if (fr[q] == 0.0f) nv = 0.0f;
             v[q] = nv;
         }
         st4(vx, id, v);
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
             unpack(ld4(p, id + 2 * g.sz), p2);
         }
         unpack(ld4(vy, id), v);
-        if (fy) unpack(ld4(fy, id), fr);
+        if (wall & kWallY) unpack(ld4(fy, id), fr);
         const float ayr = __ldg(tb.ay + j + 1);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
             const float grad = fourth ? fadd(fmul(cf.c1, fsub(pr[q], pc[q])), fmul(cf.c2, fsub(p2[q], pm[q])))
                                       : fsub(pr[q], pc[q]);
             float nv = fmul(fsub(v[q], fmul(cf.vc, grad)), face_damp(ac[q], fmaxf(fmaxf(axi, ayr), az4[q]), cf.dt));
-            if (fy && fr[q] == 0.0f) nv = 0.0f;
+            if (fr[q] == 0.0f) nv = 0.0f;
             v[q] = nv;
         }
         st4(vy, id, v);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
         e[5] = k0 + 4 < g.nz ? p[id + 4] : 0.0f;
         e[6] = k0 + 5 < g.nz ? p[id + 5] : 0.0f;
         unpack(ld4(vz, id), v);
-        if (fz) unpack(ld4(fz, id), fr);
+        if (wall & kWallZ) unpack(ld4(fz, id), fr);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int k = k0 + q;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) k_velocity_general(
                                    : fsub(e[q + 2], e[q + 1]);
             float nv = fmul(fsub(v[q], fmul(cf.vc, grad)),
                             face_damp(ac[q], fmaxf(fmaxf(axi, ay), __ldg(tb.az + k + 1)), cf.dt));
-            if (fz && fr[q] == 0.0f) nv = 0.0f;
+            if (fr[q] == 0.0f) nv = 0.0f;
             v[q] = nv;
         }
         if (pf.code && k0 <= pf.iz && pf.iz - 1 <= k0 + 3) {   // the plate's faces
@@ -147,15 +147,13 @@ __global__ void __launch_bounds__(256) k_velocity_general(
 }
 
 // The pressure update of cells k0 .. k0+3 of row (i, j), id = their padded index.
-// Vz faces kp-1 (code bit 0) and kp (bit 1) have the velocity vp in place of the
-// stored one (the plate's faces; code 0: none).
 __device__ __forceinline__ void pressure_cells4(const Grid& g, const Coef& cf, const Tables& tb,
                                                 const float* __restrict__ p, float* __restrict__ pn,
                                                 const float* __restrict__ vx, const float* __restrict__ vy,
                                                 const float* __restrict__ vz, const float* __restrict__ fx,
                                                 const float* __restrict__ fy, const float* __restrict__ fz,
                                                 const uint8_t* __restrict__ solid, int i, int j, int k0,
-                                                long long id, unsigned code = 0, int kp = 0, float vp = 0.0f)
+                                                long long id)
 {
     const long long P = g.plane, S = g.sz;
     // face values times their fractions, four cells at a time (zero when absent)
@@ -182,22 +180,14 @@ __device__ __forceinline__ void pressure_cells4(const Grid& g, const Coef& cf, c
     face4(vy, fy, id + S, j < g.ny - 2, ypp);
     face4(vy, fy, id - 2 * S, j > 1, ymm);
     // Vz (times fraction) at k0-2 .. k0+4: e[t] = FZ[k0 - 2 + t]
-    auto fzv = [&](long long q, int k) {
-        float v = vz[q];
-        if ((k == kp - 1 && (code & 1u)) || (k == kp && (code & 2u))) v = vp;
-        return fz ? fmul(v, fz[q]) : v;
-    };
+    auto fzv = [&](long long q) { return fz ? fmul(vz[q], fz[q]) : vz[q]; };
     float e[7], c4[4], pc[4], out[4];
     face4(vz, fz, id, true, c4);
-    e[0] = k0 >= 2 ? fzv(id - 2, k0 - 2) : 0.0f;
-    e[1] = k0 >= 1 ? fzv(id - 1, k0 - 1) : 0.0f;
+    e[0] = k0 >= 2 ? fzv(id - 2) : 0.0f;
+    e[1] = k0 >= 1 ? fzv(id - 1) : 0.0f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        e[q + 2] = c4[q];
-        if ((k0 + q == kp - 1 && (code & 1u)) || (k0 + q == kp && (code & 2u)))
-            e[q + 2] = fz ? fmul(vp, fz[id + q]) : vp;
-    }
-    e[6] = k0 + 4 < g.nz ? fzv(id + 4, k0 + 4) : 0.0f;
+    for (int q = 0; q < 4; ++q) e[q + 2] = c4[q];
+    e[6] = k0 + 4 < g.nz ? fzv(id + 4) : 0.0f;
     unpack(ld4(p, id), pc);
     uint32_t sol = 0;
     if (solid) sol = *reinterpret_cast<const uint32_t*>(solid + id);
@@ -227,11 +217,45 @@ __global__ void __launch_bounds__(256) k_pressure_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ pn,
     const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz,
     const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz,
-    const uint8_t* __restrict__ solid, const unsigned* __restrict__ gate)
+    const uint8_t* __restrict__ solid, const uint8_t* __restrict__ walls, const unsigned* __restrict__ gate)
 {
     GEN_INDEX
     if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
-    pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, id);
+    if (walls && (walls[id >> 2] & kWallNear))
+        pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, id);
+    else   // every fraction it would read is 1
+        pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, nullptr, nullptr, nullptr, nullptr, i, j, k0, id);
+}
+
+// WallCode bytes: the group's own faces and cells, then (after a launch boundary)
+// what its pressure update reads around it.
+__global__ void __launch_bounds__(256) k_wall_own(Grid g, const float* __restrict__ fx, const float* __restrict__ fy,
+                                                  const float* __restrict__ fz, const uint8_t* __restrict__ solid,
+                                                  uint8_t* __restrict__ code)
+{
+    GEN_INDEX
+    unsigned c = 0;
+    for (int q = 0; q < 4; ++q) {
+        const int k = k0 + q;
+        if (k >= g.nz) break;
+        if (fx && i < g.nx - 1 && fx[id + q] != 1.0f) c |= kWallX;
+        if (fy && j < g.ny - 1 && fy[id + q] != 1.0f) c |= kWallY;
+        if (fz && k < g.nz - 1 && fz[id + q] != 1.0f) c |= kWallZ;
+        if (solid && solid[id + q]) c |= kWallSolid;
+    }
+    code[id >> 2] = (uint8_t)c;
+}
+__global__ void __launch_bounds__(256) k_wall_near(Grid g, uint8_t* code)
+{
+    GEN_INDEX
+    unsigned c = code[id >> 2], near = c & (kWallX | kWallY | kWallZ | kWallSolid);
+    for (int d = -2; d <= 1; ++d) {
+        if (i + d >= 0 && i + d < g.nx) near |= code[(id + d * g.plane) >> 2] & kWallX;
+        if (j + d >= 0 && j + d < g.ny) near |= code[(id + (long long)d * g.sz) >> 2] & kWallY;
+    }
+    if (k0 >= 4) near |= code[(id - 4) >> 2] & kWallZ;
+    if (k0 + 4 < g.nz) near |= code[(id + 4) >> 2] & kWallZ;
+    if (near) code[id >> 2] = (uint8_t)(c | kWallNear);   // the bits the neighbours read do not change
 }
 
 // New displacement of active node q (acoustic_fdtd.cpp:984-1053).
@@ -274,52 +298,6 @@ __global__ void k_plate_step(int n_act, const int* __restrict__ act, const int* 
         atomicMin(status + kStatusPlateStep, step);
     }
     wt[pidx] = wn;
-}
-
-// The plate's part of a single-pass step, two threads per active node.  Both
-// compute the node's new displacement; the first stores it with the velocity it
-// imposes on the Vz faces beside the plate (acoustic_fdtd.cpp:1158-1163).  The
-// cells whose divergence reads those faces, iz-2 .. iz+2 of the node's own
-// column and so at most two four-cell groups, are then updated again from P^n
-// and the new velocities, a group per thread.  The displacement needs nothing
-// of the march and is computed while it drains.  256x200x128 body scene: 5.5
-// us behind the march where separate plate, face and group kernels and the
-// wait for the guard between them took 47.
-__global__ void __launch_bounds__(128) k_plate_columns(Grid g, Coef cf, Tables tb, PlateStep ps,
-                                                       const float* __restrict__ p, float* __restrict__ pn,
-                                                       const float* __restrict__ vx, const float* __restrict__ vy,
-                                                       float* vz, const float* __restrict__ fx,
-                                                       const float* __restrict__ fy, const float* __restrict__ fz,
-                                                       const uint8_t* __restrict__ solid)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t >> 1;
-    const bool in = q < ps.n_act && *(volatile unsigned*)(ps.status + kStatusPlateStep) >= ps.step;
-    int pidx = 0;
-    float wn = 0.0f, v = 0.0f;
-    if (in) {
-        pidx = ps.act[q];
-        wn = plate_node(q, pidx, ps.nb13, ps.above[q] >= 0 ? p[ps.above[q]] : 0.0f,
-                        ps.below[q] >= 0 ? p[ps.below[q]] : 0.0f, ps.w, ps.wp, ps.ext[pidx], ps.pc);
-        v = fmul(fsub(wn, ps.w[pidx]), ps.inv_dt);
-    }
-    wait_previous();
-    if (!in) return;
-    const int i = pidx / g.ny, j = pidx - i * g.ny;
-    const long long row = ((long long)i * g.ny + j) * g.sz;
-    const unsigned code = ps.code[pidx];
-    if ((t & 1) == 0) {
-        if (plate_bad(wn)) {
-            atomicMin(ps.status + kStatusPlate, (unsigned)q);
-            atomicMin(ps.status + kStatusPlateStep, ps.step);
-        }
-        ps.wt[pidx] = wn;
-        if (code & 1u) vz[row + ps.iz - 1] = v;
-        if (code & 2u) vz[row + ps.iz] = v;
-    }
-    if (code == 0) return;
-    const int lo = max(ps.iz - ((code & 1u) ? 2 : 1), 0) & ~3, hi = min(ps.iz + ((code & 2u) ? 2 : 1), g.nz - 1) & ~3;
-    const int k0 = lo + 4 * (t & 1);
-    if (k0 <= hi) pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, row + k0, code, ps.iz, v);
 }
 
 // One deposit of the open-cell rule (acoustic_fdtd.cpp:840-872).  The amplitude
@@ -406,12 +384,12 @@ __global__ void k_slice(const float* __restrict__ f, Grid g, int axis, int idx, 
 
 cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* vx, float* vy, float* vz,
-                                    const float* fx, const float* fy, const float* fz,
+                                    const float* fx, const float* fy, const float* fz, const uint8_t* walls,
                                     cudaStream_t s, const unsigned* gate, const PlateFaces* pf)
 {
     dim3 block(256, 1, 1);
     dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
-    k_velocity_general<<<grid, block, 0, s>>>(g, cf, tb, p, vx, vy, vz, fx, fy, fz, gate,
+    k_velocity_general<<<grid, block, 0, s>>>(g, cf, tb, p, vx, vy, vz, fx, fy, fz, walls, gate,
                                               pf ? *pf : PlateFaces());
     return cudaGetLastError();
 }
@@ -419,12 +397,12 @@ cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables&
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
-                                    const float* fz, const uint8_t* solid, cudaStream_t s,
+                                    const float* fz, const uint8_t* solid, const uint8_t* walls, cudaStream_t s,
                                     const unsigned* gate)
 {
     dim3 block(256, 1, 1);
     dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
-    k_pressure_general<<<grid, block, 0, s>>>(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, gate);
+    k_pressure_general<<<grid, block, 0, s>>>(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, walls, gate);
     return cudaGetLastError();
 }
 
@@ -439,13 +417,14 @@ cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const 
     return cudaGetLastError();
 }
 
-cudaError_t launch_plate_columns(const Grid& g, const Coef& cf, const Tables& tb, const PlateStep& ps, const float* p,
-                                 float* pn, const float* vx, const float* vy, float* vz, const float* fx,
-                                 const float* fy, const float* fz, const uint8_t* solid, cudaStream_t s)
+cudaError_t launch_wall_codes(const Grid& g, const float* fx, const float* fy, const float* fz, const uint8_t* solid,
+                              uint8_t* code, cudaStream_t s)
 {
-    if (ps.n_act <= 0) return cudaSuccess;
-    return launch_after(k_plate_columns, dim3((2 * ps.n_act + 127) / 128), dim3(128), 0, s, g, cf, tb, ps, p, pn, vx, vy,
-                        vz, fx, fy, fz, solid);
+    dim3 block(256, 1, 1);
+    dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
+    k_wall_own<<<grid, block, 0, s>>>(g, fx, fy, fz, solid, code);
+    k_wall_near<<<grid, block, 0, s>>>(g, code);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_deposit(const Deposit& d, const float* signal, int step, float amp, float* p,

@@ -150,43 +150,30 @@ __device__ __forceinline__ float sample8(const float* f, const long long* idx, c
     return s;
 }
 
+// Walls by groups of four cells (a byte each, at padded index / 4): bits 0-2, a
+// face of the group (Vx, Vy, Vz) has an open fraction other than 1; bit 3, a
+// cell of it is solid; bit 4, the group's pressure update reads such a face or
+// holds such a cell.  Most groups of a scene are open air (code 0) and their
+// fractions and solid flags are never read: 0.25 instead of 13 bytes a cell.
+enum WallCode { kWallX = 1, kWallY = 2, kWallZ = 4, kWallSolid = 8, kWallNear = 16 };
+
 // ---- launchers (fdtd_general.cu) ----
+cudaError_t launch_wall_codes(const Grid& g, const float* fx, const float* fy, const float* fz, const uint8_t* solid,
+                              uint8_t* code, cudaStream_t s);
 cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* vx, float* vy, float* vz,
-                                    const float* fx, const float* fy, const float* fz,
+                                    const float* fx, const float* fy, const float* fz, const uint8_t* walls,
                                     cudaStream_t s, const unsigned* gate = nullptr,
                                     const PlateFaces* pf = nullptr);
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
-                                    const float* fz, const uint8_t* solid, cudaStream_t s,
+                                    const float* fz, const uint8_t* solid, const uint8_t* walls, cudaStream_t s,
                                     const unsigned* gate = nullptr);
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,
                               const long long* below, const float* w, const float* wp, float* wt,
                               const float* ext, const float* p, const PlateCoef& pc,
                               unsigned* status, unsigned step, cudaStream_t s);
-// The plate's part of a single-pass step: what the plate update and its coupling
-// read and write (P^n, P^{n+1} and V^{n+1/2} as the march left them).
-struct PlateStep {
-    int n_act = 0, iz = -1;
-    const int* act = nullptr;         // active nodes, j + Ny * i
-    const int* nb13 = nullptr;
-    const uint8_t* code = nullptr;    // per node: bit 0 Vz face below, bit 1 above
-    const long long* above = nullptr;
-    const long long* below = nullptr;
-    const float* w = nullptr;         // displacement, previous, next
-    const float* wp = nullptr;
-    float* wt = nullptr;
-    const float* ext = nullptr;
-    PlateCoef pc{};
-    float inv_dt = 0.0f;
-    unsigned* status = nullptr;
-    unsigned step = 0;
-};
-// Launched directly behind the march, whose end it overlaps (launch.h).
-cudaError_t launch_plate_columns(const Grid& g, const Coef& cf, const Tables& tb, const PlateStep& ps, const float* p,
-                                 float* pn, const float* vx, const float* vy, float* vz, const float* fx,
-                                 const float* fy, const float* fz, const uint8_t* solid, cudaStream_t s);
 // plate forces as (node, value) pairs scattered into the zeroed device buffer
 // (the velocity pass returns them to zero: PlateFaces)
 cudaError_t launch_ext_scatter(float* ext, const int2* pack, int m, cudaStream_t s);
@@ -268,7 +255,11 @@ struct FusedArgs {
     const float* fr[3] = {nullptr, nullptr, nullptr};
     bool frac_div = false;
     const uint8_t* solid = nullptr;
-    // plate scenes: the step does nothing when an earlier step's plate update failed
+    const uint8_t* walls = nullptr;   // WallCode bytes (given with fractions or a mask)
+    // Plate scenes: the velocities of the plate's faces (PlateFaces; code null:
+    // none), and the status words: the step does nothing when this or an earlier
+    // step's plate update failed.
+    PlateFaces plate;
     const unsigned* gate = nullptr;
 };
 struct FusedCache;         // host-side TMA descriptors of a handle's fields
