@@ -84,7 +84,7 @@ struct SubstepKey {
     const uint8_t *solid, *walls;
     const long long *sidx;
     const float *sw;
-    float *sout, *h_sout;
+    float *sout;
     unsigned *status, *h_status;
     Grid g;
     Coef cf;
@@ -201,10 +201,8 @@ struct AcousticFDTDState {
     size_t s_cap = 0;
     long long* d_sidx = nullptr;
     float* d_sw = nullptr;
-    float* d_sout = nullptr;
     long long* h_sidx = nullptr;
     float* h_sw = nullptr;
-    float* h_sout = nullptr;
     // sampler results written by the kernel straight into pinned host memory
     // (mapped into the device's address space): no device-to-host copy per call
     float* h_sout_map = nullptr;
@@ -355,20 +353,18 @@ int ensure_scratch(AcousticFDTDState* st, size_t n)
 {
     if (n <= st->s_cap) return FDTD_OK;
     size_t cap = std::max<size_t>(n, 1024);
-    cudaFree(st->d_sidx); cudaFree(st->d_sw); cudaFree(st->d_sout);
-    cudaFreeHost(st->h_sidx); cudaFreeHost(st->h_sw); cudaFreeHost(st->h_sout); cudaFreeHost(st->h_sout_map);
-    st->d_sidx = nullptr; st->d_sw = st->d_sout = nullptr;
-    st->h_sidx = nullptr; st->h_sw = st->h_sout = nullptr;
+    cudaFree(st->d_sidx); cudaFree(st->d_sw);
+    cudaFreeHost(st->h_sidx); cudaFreeHost(st->h_sw); cudaFreeHost(st->h_sout_map);
+    st->d_sidx = nullptr; st->d_sw = nullptr;
+    st->h_sidx = nullptr; st->h_sw = nullptr;
     st->h_sout_map = st->d_sout_map = nullptr;
     st->s_cap = 0;
     st->up_idx.clear();
     st->up_w.clear();
     CK(cudaMalloc(&st->d_sidx, cap * sizeof(long long)));
     CK(cudaMalloc(&st->d_sw, cap * sizeof(float)));
-    CK(cudaMalloc(&st->d_sout, cap * sizeof(float)));
     CK(cudaMallocHost(&st->h_sidx, cap * sizeof(long long)));
     CK(cudaMallocHost(&st->h_sw, cap * sizeof(float)));
-    CK(cudaMallocHost(&st->h_sout, cap * sizeof(float)));
     CK(cudaHostAlloc(&st->h_sout_map, cap * sizeof(float), cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer((void**)&st->d_sout_map, st->h_sout_map, 0));
     st->s_cap = cap;
@@ -513,9 +509,10 @@ bool fused_walled_ok(const AcousticFDTDState* st)
 // Walled scenes take the single pass automatically from this many cells on:
 // below it the fields stay in L2 and the two-pass kernels' extra bytes cost less
 // than the march's pipeline fill (fdtd_step per step on plate scenes, two-pass /
-// single pass: 130x110x60 24.9 / 26.9 us, 170x140x74 35.6 / 42.3, 160x128x128
-// 43.2 / 38.9, 200x160x100 56.8 / 53.5, 256x200x128 114 / 74, 300x240x160 187 / 134).
-constexpr long long kWalledFusedCells = 5LL << 19;
+// single pass: 130x110x60 15.9 / 24.9 us, 170x140x74 24.5 / 40.0, 160x128x128
+// 32.0 / 36.4, 180x150x144 53.1 / 62.6, 256x200x96 (4.9M cells) 72.4 / 72.4,
+// 256x200x128 94 / 73.5, 300x240x160 158 / 132).
+constexpr long long kWalledFusedCells = 19LL << 18;
 
 bool use_fused(const AcousticFDTDState* st)
 {
@@ -1007,8 +1004,8 @@ void free_state(AcousticFDTDState* st)
     cudaFree(st->d_ps_sig);
     cudaFree(st->d_rec_idx); cudaFree(st->d_rec_w); cudaFree(st->d_trace);
     cudaFree(st->d_status); cudaFreeHost(st->h_status);
-    cudaFree(st->d_sidx); cudaFree(st->d_sw); cudaFree(st->d_sout);
-    cudaFreeHost(st->h_sidx); cudaFreeHost(st->h_sw); cudaFreeHost(st->h_sout); cudaFreeHost(st->h_sout_map);
+    cudaFree(st->d_sidx); cudaFree(st->d_sw);
+    cudaFreeHost(st->h_sidx); cudaFreeHost(st->h_sw); cudaFreeHost(st->h_sout_map);
     for (cudaEvent_t e : st->prof.ev) cudaEventDestroy(e);
     fused_cache_destroy(st->fcache);
     cudaFree(st->res_x);
@@ -2281,14 +2278,14 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
     const bool hf = st->has_frac;
     // The substep's device work in stream order: the plate update (its guard
     // gates everything after it), the step as if the plate succeeded (the
-    // plate's new displacement is d_w[wt0], the previous one d_w[wc0]), then
-    // the saddle samples and the status words to the host.
+    // plate's new displacement is d_w[wt0], the previous one d_w[wc0]).  The
+    // first kernel reads the forces from host memory and the last one writes the
+    // saddle samples and the status words there: two copies out, one in, a fill and
+    // a sampling kernel less on the chain that the caller waits for (170x140x74
+    // body, per substep: 73.9 us with them and the kernels one after another, 51.2
+    // now; the step alone 35.5 and 24.8).
     auto issue = [&]() -> int {
-        if (n_pack > 0) {
-            CK(cudaMemcpyAsync(st->d_ext_pack, st->h_ext_pack, (size_t)n_pack * sizeof(int2), cudaMemcpyHostToDevice, s));
-            CK(launch_ext_scatter(st->d_ext, st->d_ext_pack, n_pack, s));
-        }
-        CK(cudaMemsetAsync(st->d_status + kStatusPlate, 0xFF, 2 * sizeof(unsigned), s));   // node and step
+        CK(launch_substep_begin(st->d_ext, st->h_ext_pack, st->d_ext_pack, n_pack, st->d_status, s));
         CK(launch_plate_step(st->n_act, st->d_act, st->d_nb13, st->d_above, st->d_below, st->d_w[wc0], st->d_w[wp0],
                              st->d_w[wt0], st->d_ext, P, st->pc, st->d_status, 0u, s));
         if (ext_left) CK(launch_zero_gated(st->d_ext, st->N_plate, gate, s));
@@ -2305,29 +2302,28 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
         }
         CK(launch_velocity_general(st->g, st->cf, st->tb, P, st->V(0), st->V(1), st->V(2), st->d_frac[0],
                                    st->d_frac[1], st->d_frac[2], st->d_walls, s, gate, &pf));
+        SubstepOut so;
+        so.idx = st->d_sidx; so.sw = st->d_sw; so.w = st->d_w[wt0];
+        so.out = st->d_sout_map; so.n = n_saddle;
+        so.status = st->d_status; so.h_status = st->h_status;
         CK(launch_pressure_general(st->g, st->cf, st->tb, P, Pn, st->V(0), st->V(1), st->V(2),
                                    hf ? st->d_frac[0] : nullptr, hf ? st->d_frac[1] : nullptr,
-                                   hf ? st->d_frac[2] : nullptr, st->d_solid, st->d_walls, s, gate));
+                                   hf ? st->d_frac[2] : nullptr, st->d_solid, st->d_walls, s, gate, &so));
         if (record)
             CK(launch_wsum(Pn, st->d_rec_idx, st->d_rec_w, st->n_rec, 8, 0,
                            st->d_trace + (size_t)trace0 * st->n_rec, s));
         if (checked) {
             CK(cudaMemsetAsync(st->d_status + kStatusCell, 0xFF, sizeof(unsigned), s));
             CK(launch_check(st->g, Pn, st->N, phase0, st->d_status, step1, s, gate));
+            CK(cudaMemcpyAsync(st->h_status, st->d_status, kStatusWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         }
-        if (n_saddle > 0) {
-            CK(launch_wsum(st->d_w[wt0], st->d_sidx, st->d_sw, n_saddle, 4, 0, st->d_sout, s));
-            CK(cudaMemcpyAsync(st->h_sout, st->d_sout, (size_t)n_saddle * sizeof(float), cudaMemcpyDeviceToHost, s));
-        }
-        CK(cudaMemcpyAsync(st->h_status, st->d_status, kStatusWords * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         return FDTD_OK;
     };
-    const long long n_launch = 3 + (n_pack > 0 ? 1 : 0) + (ext_left ? 1 : 0) + (record ? 1 : 0) + (checked ? 1 : 0) +
-                               (n_saddle > 0 ? 1 : 0);
+    const long long n_launch = 4 + (ext_left ? 1 : 0) + (record ? 1 : 0) + (checked ? 1 : 0);
     bool issued = false;
     if (!record && !checked) {
         // The same work recurs every substep with one of a few pointer sets:
-        // replay it as a cached CUDA graph (one launch instead of about ten).
+        // replay it as a cached CUDA graph (51.2 us a substep, 53.2 as four launches).
         SubstepKey k;
         memset(&k, 0, sizeof k);
         k.stream = s;
@@ -2336,7 +2332,7 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
         for (int c2 = 0; c2 < 3; ++c2) k.frac[c2] = st->d_frac[c2];
         k.ext = st->d_ext; k.h_ext = st->h_ext; k.solid = st->d_solid; k.walls = st->d_walls;
         k.pack = st->d_ext_pack; k.h_pack = st->h_ext_pack; k.n_pack = n_pack;
-        k.sidx = st->d_sidx; k.sw = st->d_sw; k.sout = st->d_sout; k.h_sout = st->h_sout;
+        k.sidx = st->d_sidx; k.sw = st->d_sw; k.sout = st->d_sout_map;
         k.status = st->d_status; k.h_status = st->h_status;
         k.g = st->g; k.cf = st->cf; k.tb = st->tb; k.pc = st->pc;
         k.n_act = st->n_act; k.n_plate = st->N_plate; k.n_saddle = n_saddle;
@@ -2408,7 +2404,7 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out)
             return FDTD_ERR_UNSTABLE;
         }
     }
-    if (n_saddle > 0) memcpy(out, st->h_sout, (size_t)n_saddle * sizeof(float));
+    if (n_saddle > 0) memcpy(out, st->h_sout_map, (size_t)n_saddle * sizeof(float));
     return FDTD_OK;
 }
 

@@ -147,18 +147,6 @@ __device__ __forceinline__ float4 vel4(const Coef& cf, const float4& pm, const f
     return r;
 }
 
-// four faces, 2nd-order gradient, given damping (the faces next to a j end)
-__device__ __forceinline__ float4 vel4_2nd(const Coef& cf, const float4& p0, const float4& p1,
-                                          const float4& vo, const float4& dmp)
-{
-    float4 r;
-    r.x = vupd(cf, vo.x, fsub(p1.x, p0.x), dmp.x);
-    r.y = vupd(cf, vo.y, fsub(p1.y, p0.y), dmp.y);
-    r.z = vupd(cf, vo.z, fsub(p1.z, p0.z), dmp.z);
-    r.w = vupd(cf, vo.w, fsub(p1.w, p0.w), dmp.w);
-    return r;
-}
-
 // as vel4, with a per-face gradient order (bit q of m4) and existence (bit q of ok)
 __device__ __forceinline__ float4 vel4_masked(const Coef& cf, float4 pm, float4 p0, float4 p1,
                                              float4 p2, float4 vo, float4 dmp, int m4, int ok)

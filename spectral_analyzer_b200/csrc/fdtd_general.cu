@@ -10,17 +10,15 @@
  * 20 B/cell (+ fractions and solid mask when present).
  */
 #include "fdtd_internal.h"
+#include "launch.h"
 
 #include <math.h>
+
+#include <algorithm>
 
 namespace fdtd {
 
 namespace {
-
-__device__ __forceinline__ float cell_alpha(const Tables& tb, int i, float ay, float az)
-{
-    return fmaxf(fmaxf(__ldg(tb.ax + i), ay), az);
-}
 
 __device__ __forceinline__ float4 ld4(const float* p, long long i) { return *reinterpret_cast<const float4*>(p + i); }
 __device__ __forceinline__ void st4(float* p, long long i, const float (&v)[4])
@@ -29,11 +27,43 @@ __device__ __forceinline__ void st4(float* p, long long i, const float (&v)[4])
 }
 __device__ __forceinline__ void unpack(const float4& x, float (&v)[4]) { v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
 
+// sum_t w[t] * f[id[t]] in tap order; from_zero starts the running sum at 0.0f
+// (the direct samplers, acoustic_fdtd.cpp:1380-1389), otherwise at the first
+// product (the precomputed samplers, :1673-1674).  T = the number of taps, known
+// for the usual 8 and 4 so that their loads do not wait for one another; 0 = any.
+template <int T>
+__device__ __forceinline__ float weighted_sum(const float* __restrict__ f, const long long* __restrict__ id,
+                                              const float* __restrict__ w, int taps, int from_zero)
+{
+    float s = 0.0f;
+    if constexpr (T > 0) {
+        float v[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) v[t] = fmul(w[t], f[id[t]]);
+        s = from_zero ? fadd(0.0f, v[0]) : v[0];
+#pragma unroll
+        for (int t = 1; t < T; ++t) s = fadd(s, v[t]);
+    } else {
+        for (int t = 0; t < taps; ++t) {
+            const float v = fmul(w[t], f[id[t]]);
+            s = (t == 0 && !from_zero) ? v : fadd(s, v);
+        }
+    }
+    return s;
+}
+
 // Threads own four consecutive cells k0 .. k0+3 of a row (k0 a multiple of 4;
 // rows start on 8-float boundaries, so every float4 access is aligned).  The
 // (row, group) pairs of a plane are numbered consecutively over 1-D blocks,
 // so no lane idles when Nz/4 is not a multiple of the warp width (Nz = 74:
 // 19 groups per row), and consecutive lanes read consecutive 16-byte groups.
+//
+// Blocks of 128 threads, six to an SM (80 registers): a small scene is a few
+// waves of blocks, and 256-thread blocks, three to an SM, end in a longer tail.
+// 170x140x74 scene, whole step: 256 threads 31.8 us, 128 threads 24.8 (64 or 96
+// threads 24.9; five or seven 128-thread blocks 26.5 and 25.6); 160x128x128: 42.1
+// and 32.7.
+constexpr int kCellThreads = 128;
 #define GEN_INDEX                                                          \
     const int nq_ = (g.nz + 3) >> 2;                                       \
     const int t_ = blockIdx.x * blockDim.x + threadIdx.x;                  \
@@ -47,90 +77,87 @@ __device__ __forceinline__ void unpack(const float4& x, float (&v)[4]) { v[0] = 
 // then closed faces (fraction == 0) are zeroed (:1152-1154).  A thread handles
 // Vx(i+1/2,j,k), Vy(i,j+1/2,k) and Vz(i,j,k+1/2) of its four cells where they
 // exist; faces that do not exist (and the row padding) keep their stored zero.
-__global__ void __launch_bounds__(256) k_velocity_general(
+__global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ vx,
     float* __restrict__ vy, float* __restrict__ vz, const float* __restrict__ fx,
     const float* __restrict__ fy, const float* __restrict__ fz, const uint8_t* __restrict__ walls,
     const unsigned* __restrict__ gate, PlateFaces pf)
 {
-    if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
-    if (pf.m > 0 && blockIdx.x == 0 && blockIdx.y == 0)      // the consumed plate forces
-        for (int q = threadIdx.x; q < pf.m; q += blockDim.x) pf.ext[pf.pack[q].x] = 0.0f;
+    // With a plate the kernel before this one is the plate update, which writes no
+    // field: the loads start beside it and only the results wait for it.
+    if (!pf.code) wait_previous();
+    release_next();
     GEN_INDEX
+    // Every load first, from addresses kept inside the field (what a 2nd-order
+    // face does not read is loaded and not used): the pass is bound by the latency
+    // of L2, and a thread that loads axis by axis keeps fewer in flight
+    // (170x140x74 scene, whole step: 35.3 us axis by axis, 34.0 us this way).
+    const long long xm = i > 0 ? id - g.plane : id, xp = i < g.nx - 1 ? id + g.plane : id;
+    const long long xq = i < g.nx - 2 ? id + 2 * g.plane : id;
+    const long long ym = j > 0 ? id - g.sz : id, yp = j < g.ny - 1 ? id + g.sz : id, yq = j < g.ny - 2 ? id + 2 * g.sz : id;
     const unsigned wall = walls ? walls[id >> 2] : 0u;
+    const float4 p_c = ld4(p, id), p_xm = ld4(p, xm), p_xp = ld4(p, xp), p_xq = ld4(p, xq);
+    const float4 p_ym = ld4(p, ym), p_yp = ld4(p, yp), p_yq = ld4(p, yq);
+    const float p_zm = k0 > 0 ? p[id - 1] : 0.0f;
+    const float2 p_zp = k0 + 4 < g.nz ? *reinterpret_cast<const float2*>(p + id + 4) : make_float2(0.f, 0.f);
+    const float4 v_x = ld4(vx, id), v_y = ld4(vy, id), v_z = ld4(vz, id);
     const float ay = __ldg(tb.ay + j), axi = __ldg(tb.ax + i);
-    float pc[4], az4[4], ac[4];
-    unpack(ld4(p, id), pc);
+    const float axr = __ldg(tb.ax + min(i + 1, g.nx - 1)), ayr = __ldg(tb.ay + min(j + 1, g.ny - 1));
+    float az[5], ac[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        az4[q] = (k0 + q < g.nz) ? __ldg(tb.az + k0 + q) : 0.0f;
-        ac[q] = fmaxf(fmaxf(axi, ay), az4[q]);
-    }
+    for (int q = 0; q < 5; ++q) az[q] = __ldg(tb.az + min(k0 + q, g.nz - 1));
+    float4 f_x = make_float4(1.f, 1.f, 1.f, 1.f), f_y = f_x, f_z = f_x;
+    if (wall & kWallX) f_x = ld4(fx, id);
+    if (wall & kWallY) f_y = ld4(fy, id);
+    if (wall & kWallZ) f_z = ld4(fz, id);
+    if (pf.code) wait_previous();
+    if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
+    if (pf.m > 0 && i == 0 && blockIdx.x == 0)               // the consumed plate forces
+        for (int q = threadIdx.x; q < pf.m; q += min((int)blockDim.x, g.ny * nq_)) pf.ext[pf.pack[q].x] = 0.0f;
+    float pc[4];
+    unpack(p_c, pc);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ac[q] = fmaxf(fmaxf(axi, ay), az[q]);
+    auto grad = [&](float m, float c, float r, float s, bool fourth) {
+        const float d = fsub(r, c), w = fadd(fmul(cf.c1, d), fmul(cf.c2, fsub(s, m)));
+        return fourth ? w : d;
+    };
+    auto face = [&](float v, float gr, float aL, float aR, float fr) {
+        const float nv = fmul(fsub(v, fmul(cf.vc, gr)), face_damp(aL, aR, cf.dt));
+        return fr == 0.0f ? 0.0f : nv;
+    };
     if (i < g.nx - 1) {
         const bool fourth = i > 0 && i < g.nx - 2;
-        float pr[4], pm[4] = {}, p2[4] = {}, v[4], fr[4] = {1.f, 1.f, 1.f, 1.f};
-        unpack(ld4(p, id + g.plane), pr);
-        if (fourth) {
-            unpack(ld4(p, id - g.plane), pm);
-            unpack(ld4(p, id + 2 * g.plane), p2);
-        }
-        unpack(ld4(vx, id), v);
-        if (wall & kWallX) unpack(ld4(fx, id), fr);
-        const float axr = __ldg(tb.ax + i + 1);
+        float pr[4], pm[4], p2[4], v[4], fr[4];
+        unpack(p_xp, pr); unpack(p_xm, pm); unpack(p_xq, p2); unpack(v_x, v); unpack(f_x, fr);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            if (k0 + q >= g.nz) continue;
-            const float grad = fourth ? fadd(fmul(cf.c1, fsub(pr[q], pc[q])), fmul(cf.c2, fsub(p2[q], pm[q])))
-                                      : fsub(pr[q], pc[q]);
-            float nv = fmul(fsub(v[q], fmul(cf.vc, grad)), face_damp(ac[q], fmaxf(fmaxf(axr, ay), az4[q]), cf.dt));
-            if (fr[q] == 0.0f) nv = 0.0f;
-            v[q] = nv;
+            const float nv = face(v[q], grad(pm[q], pc[q], pr[q], p2[q], fourth), ac[q], fmaxf(fmaxf(axr, ay), az[q]), fr[q]);
+            if (k0 + q < g.nz) v[q] = nv;
         }
         st4(vx, id, v);
     }
     if (j < g.ny - 1) {
         const bool fourth = j > 0 && j < g.ny - 2;
-        float pr[4], pm[4] = {}, p2[4] = {}, v[4], fr[4] = {1.f, 1.f, 1.f, 1.f};
-        unpack(ld4(p, id + g.sz), pr);
-        if (fourth) {
-            unpack(ld4(p, id - g.sz), pm);
-            unpack(ld4(p, id + 2 * g.sz), p2);
-        }
-        unpack(ld4(vy, id), v);
-        if (wall & kWallY) unpack(ld4(fy, id), fr);
-        const float ayr = __ldg(tb.ay + j + 1);
+        float pr[4], pm[4], p2[4], v[4], fr[4];
+        unpack(p_yp, pr); unpack(p_ym, pm); unpack(p_yq, p2); unpack(v_y, v); unpack(f_y, fr);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            if (k0 + q >= g.nz) continue;
-            const float grad = fourth ? fadd(fmul(cf.c1, fsub(pr[q], pc[q])), fmul(cf.c2, fsub(p2[q], pm[q])))
-                                      : fsub(pr[q], pc[q]);
-            float nv = fmul(fsub(v[q], fmul(cf.vc, grad)), face_damp(ac[q], fmaxf(fmaxf(axi, ayr), az4[q]), cf.dt));
-            if (fr[q] == 0.0f) nv = 0.0f;
-            v[q] = nv;
+            const float nv = face(v[q], grad(pm[q], pc[q], pr[q], p2[q], fourth), ac[q], fmaxf(fmaxf(axi, ayr), az[q]), fr[q]);
+            if (k0 + q < g.nz) v[q] = nv;
         }
         st4(vy, id, v);
     }
     {
-        // P at k0-1 .. k0+5: e[t] = P[k0 - 1 + t]
-        float e[7], v[4], fr[4] = {1.f, 1.f, 1.f, 1.f};
-        e[0] = k0 > 0 ? p[id - 1] : 0.0f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) e[q + 1] = pc[q];
-        e[5] = k0 + 4 < g.nz ? p[id + 4] : 0.0f;
-        e[6] = k0 + 5 < g.nz ? p[id + 5] : 0.0f;
-        unpack(ld4(vz, id), v);
-        if (wall & kWallZ) unpack(ld4(fz, id), fr);
+        const float e[7] = {p_zm, pc[0], pc[1], pc[2], pc[3], p_zp.x, p_zp.y};   // P at k0-1 .. k0+5
+        float v[4], fr[4];
+        unpack(v_z, v); unpack(f_z, fr);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int k = k0 + q;
-            if (k >= g.nz - 1) continue;
-            const float grad = (k > 0 && k < g.nz - 2)
-                                   ? fadd(fmul(cf.c1, fsub(e[q + 2], e[q + 1])), fmul(cf.c2, fsub(e[q + 3], e[q])))
-                                   : fsub(e[q + 2], e[q + 1]);
-            float nv = fmul(fsub(v[q], fmul(cf.vc, grad)),
-                            face_damp(ac[q], fmaxf(fmaxf(axi, ay), __ldg(tb.az + k + 1)), cf.dt));
-            if (fr[q] == 0.0f) nv = 0.0f;
-            v[q] = nv;
+            const float nv = face(v[q], grad(e[q], e[q + 1], e[q + 2], e[q + 3], k > 0 && k < g.nz - 2), ac[q],
+                                  fmaxf(fmaxf(axi, ay), az[q + 1]), fr[q]);
+            if (k < g.nz - 1) v[q] = nv;
         }
         if (pf.code && k0 <= pf.iz && pf.iz - 1 <= k0 + 3) {   // the plate's faces
             const int node = j + g.ny * i;
@@ -146,85 +173,86 @@ __global__ void __launch_bounds__(256) k_velocity_general(
     }
 }
 
-// The pressure update of cells k0 .. k0+3 of row (i, j), id = their padded index.
-__device__ __forceinline__ void pressure_cells4(const Grid& g, const Coef& cf, const Tables& tb,
-                                                const float* __restrict__ p, float* __restrict__ pn,
-                                                const float* __restrict__ vx, const float* __restrict__ vy,
-                                                const float* __restrict__ vz, const float* __restrict__ fx,
-                                                const float* __restrict__ fy, const float* __restrict__ fz,
-                                                const uint8_t* __restrict__ solid, int i, int j, int k0,
-                                                long long id)
-{
-    const long long P = g.plane, S = g.sz;
-    // face values times their fractions, four cells at a time (zero when absent)
-    auto face4 = [&](const float* v, const float* f, long long q, bool exists, float (&out)[4]) {
-        if (!exists) {
-            out[0] = out[1] = out[2] = out[3] = 0.0f;
-            return;
-        }
-        unpack(ld4(v, q), out);
-        if (f) {
-            float fr[4];
-            unpack(ld4(f, q), fr);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) out[t] = fmul(out[t], fr[t]);
-        }
-    };
-    float xp[4], xm[4], xpp[4], xmm[4], yp[4], ym[4], ypp[4], ymm[4];
-    face4(vx, fx, id, i < g.nx - 1, xp);
-    face4(vx, fx, id - P, i > 0, xm);
-    face4(vx, fx, id + P, i < g.nx - 2, xpp);
-    face4(vx, fx, id - 2 * P, i > 1, xmm);
-    face4(vy, fy, id, j < g.ny - 1, yp);
-    face4(vy, fy, id - S, j > 0, ym);
-    face4(vy, fy, id + S, j < g.ny - 2, ypp);
-    face4(vy, fy, id - 2 * S, j > 1, ymm);
-    // Vz (times fraction) at k0-2 .. k0+4: e[t] = FZ[k0 - 2 + t]
-    auto fzv = [&](long long q) { return fz ? fmul(vz[q], fz[q]) : vz[q]; };
-    float e[7], c4[4], pc[4], out[4];
-    face4(vz, fz, id, true, c4);
-    e[0] = k0 >= 2 ? fzv(id - 2) : 0.0f;
-    e[1] = k0 >= 1 ? fzv(id - 1) : 0.0f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) e[q + 2] = c4[q];
-    e[6] = k0 + 4 < g.nz ? fzv(id + 4) : 0.0f;
-    unpack(ld4(p, id), pc);
-    uint32_t sol = 0;
-    if (solid) sol = *reinterpret_cast<const uint32_t*>(solid + id);
-    const float pxy = fminf(__ldg(tb.px + i), __ldg(tb.py + j));
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int k = k0 + q;
-        out[q] = 0.0f;
-        if (k >= g.nz || ((sol >> (8 * q)) & 0xFFu)) continue;
-        const float zp = (k < g.nz - 1) ? e[q + 2] : 0.0f;
-        const float zm = (k > 0) ? e[q + 1] : 0.0f;
-        const float zpp = (k < g.nz - 2) ? e[q + 3] : 0.0f;
-        const float zmm = (k > 1) ? e[q] : 0.0f;
-        const float d1 = fadd(fadd(fsub(xp[q], xm[q]), fsub(yp[q], ym[q])), fsub(zp, zm));
-        const float d2 = fadd(fadd(fsub(xpp[q], xmm[q]), fsub(ypp[q], ymm[q])), fsub(zpp, zmm));
-        const float dv = fadd(fmul(cf.c1, d1), fmul(cf.c2, d2));
-        out[q] = fmul(fsub(pc[q], fmul(cf.bulk, dv)), fminf(pxy, __ldg(tb.pz + k)));
-    }
-    st4(pn, id, out);
-}
-
 // Pressure update from the 4th-order divergence (acoustic_fdtd.cpp:894-952,
 // :1176-1234).  Faces outside the grid read as zero; with fractions each face
 // is scaled by its open fraction; solid cells are skipped (they stay zero in
-// both pressure buffers, so the thread writes zero there).
-__global__ void __launch_bounds__(256) k_pressure_general(
+// both pressure buffers, so the thread writes zero there).  Every load first, as
+// in the velocity pass; the fractions of a group near walls come after them.
+__global__ void __launch_bounds__(kCellThreads, 6) k_pressure_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ pn,
     const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz,
     const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz,
-    const uint8_t* __restrict__ solid, const uint8_t* __restrict__ walls, const unsigned* __restrict__ gate)
+    const uint8_t* __restrict__ solid, const uint8_t* __restrict__ walls, const unsigned* __restrict__ gate,
+    SubstepOut so)
 {
+    wait_previous();
+    release_next();
+    if (so.status) {   // what the host waits for, straight into its memory
+        const int n_thr = gridDim.x * gridDim.y * blockDim.x;
+        const int t = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+        for (int r = t; r < so.n; r += n_thr) so.out[r] = weighted_sum<4>(so.w, so.idx + 4LL * r, so.sw + 4LL * r, 4, 0);
+        if (t < kStatusWords) so.h_status[t] = so.status[t];
+    }
     GEN_INDEX
     if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
-    if (walls && (walls[id >> 2] & kWallNear))
-        pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, i, j, k0, id);
-    else   // every fraction it would read is 1
-        pressure_cells4(g, cf, tb, p, pn, vx, vy, vz, nullptr, nullptr, nullptr, nullptr, i, j, k0, id);
+    const long long P = g.plane, S = g.sz;
+    // faces outside the grid: the address stays inside, the value is zero
+    const bool x0 = i < g.nx - 1, y0 = j < g.ny - 1;
+    const bool x1 = i > 0, x2 = i > 1, x3 = i < g.nx - 2, y1 = j > 0, y2 = j > 1, y3 = j < g.ny - 2;
+    const long long ixm = x1 ? id - P : id, ixmm = x2 ? id - 2 * P : id, ixpp = x3 ? id + P : id;
+    const long long iym = y1 ? id - S : id, iymm = y2 ? id - 2 * S : id, iypp = y3 ? id + S : id;
+    const unsigned wall = walls ? walls[id >> 2] : 0u;
+    const float4 q_xp = ld4(vx, id), q_xm = ld4(vx, ixm), q_xpp = ld4(vx, ixpp), q_xmm = ld4(vx, ixmm);
+    const float4 q_yp = ld4(vy, id), q_ym = ld4(vy, iym), q_ypp = ld4(vy, iypp), q_ymm = ld4(vy, iymm);
+    const float4 q_z = ld4(vz, id);
+    const float2 q_zm = k0 >= 2 ? *reinterpret_cast<const float2*>(vz + id - 2) : make_float2(0.f, 0.f);
+    const float q_zp = k0 + 4 < g.nz ? vz[id + 4] : 0.0f;
+    const float4 q_p = ld4(p, id);
+    const float pxy = fminf(__ldg(tb.px + i), __ldg(tb.py + j));
+    float pz[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pz[q] = __ldg(tb.pz + min(k0 + q, g.nz - 1));
+    float xp[4], xm[4], xpp[4], xmm[4], yp[4], ym[4], ypp[4], ymm[4], pc[4], out[4];
+    float e[7] = {q_zm.x, q_zm.y, q_z.x, q_z.y, q_z.z, q_z.w, q_zp};   // Vz at k0-2 .. k0+4
+    unpack(q_xp, xp); unpack(q_xm, xm); unpack(q_xpp, xpp); unpack(q_xmm, xmm);
+    unpack(q_yp, yp); unpack(q_ym, ym); unpack(q_ypp, ypp); unpack(q_ymm, ymm);
+    unpack(q_p, pc);
+    uint32_t sol = 0;
+    if (wall & kWallNear) {   // elsewhere every fraction is 1
+        auto scale = [&](float (&v)[4], const float* f, long long at) {
+            float fr[4];
+            unpack(ld4(f, at), fr);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = fmul(v[q], fr[q]);
+        };
+        if (fx) {
+            scale(xp, fx, id); scale(xm, fx, ixm); scale(xpp, fx, ixpp); scale(xmm, fx, ixmm);
+        }
+        if (fy) {
+            scale(yp, fy, id); scale(ym, fy, iym); scale(ypp, fy, iypp); scale(ymm, fy, iymm);
+        }
+        if (fz) {
+#pragma unroll
+            for (int q = 0; q < 7; ++q)
+                if (k0 + q - 2 >= 0 && k0 + q - 2 < g.nz) e[q] = fmul(e[q], fz[id + q - 2]);
+        }
+        if (solid) sol = *reinterpret_cast<const uint32_t*>(solid + id);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int k = k0 + q;
+        const float a0 = x0 ? xp[q] : 0.0f, b0 = y0 ? yp[q] : 0.0f;
+        const float a1 = x1 ? xm[q] : 0.0f, a2 = x2 ? xmm[q] : 0.0f, a3 = x3 ? xpp[q] : 0.0f;
+        const float b1 = y1 ? ym[q] : 0.0f, b2 = y2 ? ymm[q] : 0.0f, b3 = y3 ? ypp[q] : 0.0f;
+        const float zp = (k < g.nz - 1) ? e[q + 2] : 0.0f;
+        const float zpp = (k < g.nz - 2) ? e[q + 3] : 0.0f;
+        const float d1 = fadd(fadd(fsub(a0, a1), fsub(b0, b1)), fsub(zp, e[q + 1]));
+        const float d2 = fadd(fadd(fsub(a3, a2), fsub(b3, b2)), fsub(zpp, e[q]));
+        const float dv = fadd(fmul(cf.c1, d1), fmul(cf.c2, d2));
+        out[q] = fmul(fsub(pc[q], fmul(cf.bulk, dv)), fminf(pxy, pz[q]));
+        if (k >= g.nz || ((sol >> (8 * q)) & 0xFFu)) out[q] = 0.0f;
+    }
+    st4(pn, id, out);
 }
 
 // WallCode bytes: the group's own faces and cells, then (after a launch boundary)
@@ -287,6 +315,8 @@ __global__ void k_plate_step(int n_act, const int* __restrict__ act, const int* 
                              const float* __restrict__ ext, const float* __restrict__ p,
                              PlateCoef pc, unsigned* __restrict__ status, unsigned step)
 {
+    wait_previous();
+    release_next();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_act) return;
     if (*(volatile unsigned*)(status + kStatusPlateStep) < step) return;   // an earlier step of the window failed
@@ -308,9 +338,7 @@ __global__ void k_deposit(Deposit d, const float* __restrict__ signal, int step,
     deposit_apply(d, signal ? signal[step] : amp, p);
 }
 
-// out[r] = sum_t w[r*taps+t] * f[idx[r*taps+t]] in tap order; from_zero starts
-// the running sum at 0.0f (the direct samplers, acoustic_fdtd.cpp:1380-1389),
-// otherwise at the first product (the precomputed samplers, :1673-1674).
+// out[r] = sum_t w[r*taps+t] * f[idx[r*taps+t]].
 __global__ void k_wsum(const float* __restrict__ f, const long long* __restrict__ idx,
                        const float* __restrict__ w, int n_out, int taps, int from_zero,
                        float* __restrict__ out)
@@ -319,12 +347,8 @@ __global__ void k_wsum(const float* __restrict__ f, const long long* __restrict_
     if (r >= n_out) return;
     const long long* id = idx + (long long)taps * r;
     const float* ww = w + (long long)taps * r;
-    float s;
-    int t0;
-    if (from_zero) { s = 0.0f; t0 = 0; }
-    else { s = fmul(ww[0], f[id[0]]); t0 = 1; }
-    for (int t = t0; t < taps; ++t) s = fadd(s, fmul(ww[t], f[id[t]]));
-    out[r] = s;
+    out[r] = taps == 8 ? weighted_sum<8>(f, id, ww, 8, from_zero)
+           : taps == 4 ? weighted_sum<4>(f, id, ww, 4, from_zero) : weighted_sum<0>(f, id, ww, taps, from_zero);
 }
 
 // Stability check (acoustic_fdtd.cpp:1245-1268): cells phase, phase+1013, ...
@@ -359,12 +383,19 @@ __global__ void k_zero_gated(float* __restrict__ x, int n, const unsigned* __res
     x[q] = 0.0f;
 }
 
-// The pending plate forces, sent as (node, value) pairs: written into the
-// device force buffer (all other entries are zero there).
-__global__ void k_ext_scatter(float* __restrict__ ext, const int2* __restrict__ pack, int m)
+// What a substep starts with: the pending plate forces, (node, value) pairs in
+// host memory, go into the device force buffer (all its other entries are zero),
+// and the plate guard is cleared.
+__global__ void k_substep_begin(float* __restrict__ ext, const int2* __restrict__ h_pack, int2* __restrict__ pack, int m,
+                                unsigned* __restrict__ status)
 {
+    release_next();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < m) ext[pack[q].x] = __int_as_float(pack[q].y);
+    if (q == 0) status[kStatusPlate] = status[kStatusPlateStep] = 0xFFFFFFFFu;
+    if (q >= m) return;
+    const int2 v = h_pack[q];
+    pack[q] = v;
+    ext[v.x] = __int_as_float(v.y);
 }
 
 // One plane of a field across the given axis, rows of the remaining two axes
@@ -387,23 +418,22 @@ cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables&
                                     const float* fx, const float* fy, const float* fz, const uint8_t* walls,
                                     cudaStream_t s, const unsigned* gate, const PlateFaces* pf)
 {
-    dim3 block(256, 1, 1);
-    dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
-    k_velocity_general<<<grid, block, 0, s>>>(g, cf, tb, p, vx, vy, vz, fx, fy, fz, walls, gate,
-                                              pf ? *pf : PlateFaces());
-    return cudaGetLastError();
+    dim3 block(kCellThreads, 1, 1);
+    dim3 grid((g.ny * ((g.nz + 3) / 4) + kCellThreads - 1) / kCellThreads, g.nx, 1);
+    return launch_after(k_velocity_general, grid, block, 0, s, g, cf, tb, p, vx, vy, vz, fx, fy, fz, walls, gate,
+                        pf ? *pf : PlateFaces());
 }
 
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
                                     const float* fz, const uint8_t* solid, const uint8_t* walls, cudaStream_t s,
-                                    const unsigned* gate)
+                                    const unsigned* gate, const SubstepOut* so)
 {
-    dim3 block(256, 1, 1);
-    dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
-    k_pressure_general<<<grid, block, 0, s>>>(g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, walls, gate);
-    return cudaGetLastError();
+    dim3 block(kCellThreads, 1, 1);
+    dim3 grid((g.ny * ((g.nz + 3) / 4) + kCellThreads - 1) / kCellThreads, g.nx, 1);
+    return launch_after(k_pressure_general, grid, block, 0, s, g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, walls,
+                        gate, so ? *so : SubstepOut());
 }
 
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,
@@ -412,9 +442,8 @@ cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const 
                               unsigned* status, unsigned step, cudaStream_t s)
 {
     if (n_act <= 0) return cudaSuccess;
-    k_plate_step<<<(n_act + 127) / 128, 128, 0, s>>>(n_act, act, nb13, above, below, w, wp, wt,
-                                                     ext, p, pc, status, step);
-    return cudaGetLastError();
+    return launch_after(k_plate_step, dim3((n_act + 127) / 128), dim3(128), 0, s, n_act, act, nb13, above, below, w, wp,
+                        wt, ext, p, pc, status, step);
 }
 
 cudaError_t launch_wall_codes(const Grid& g, const float* fx, const float* fy, const float* fz, const uint8_t* solid,
@@ -459,10 +488,9 @@ cudaError_t launch_zero_gated(float* x, int n, const unsigned* gate, cudaStream_
     return cudaGetLastError();
 }
 
-cudaError_t launch_ext_scatter(float* ext, const int2* pack, int m, cudaStream_t s)
+cudaError_t launch_substep_begin(float* ext, const int2* h_pack, int2* pack, int m, unsigned* status, cudaStream_t s)
 {
-    if (m <= 0) return cudaSuccess;
-    k_ext_scatter<<<(m + 255) / 256, 256, 0, s>>>(ext, pack, m);
+    k_substep_begin<<<std::max((m + 127) / 128, 1), 128, 0, s>>>(ext, h_pack, pack, m, status);
     return cudaGetLastError();
 }
 

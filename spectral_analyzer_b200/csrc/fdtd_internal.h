@@ -97,6 +97,18 @@ struct PlateFaces {
     int m = 0;
 };
 
+// What a substep hands back, written by its pressure pass into pinned host
+// memory: 4-tap sums over the plate's new displacement and the status words.
+struct SubstepOut {
+    const long long* idx = nullptr;
+    const float* sw = nullptr;
+    const float* w = nullptr;
+    float* out = nullptr;
+    int n = 0;
+    const unsigned* status = nullptr;
+    unsigned* h_status = nullptr;
+};
+
 // Targets of one pressure deposit (deposit_pressure_open, acoustic_fdtd.cpp:840-872):
 // divisor 0 = add the amplitude to idx[0]; divisor m > 0 = add amp/m to idx[0..n).
 struct Deposit {
@@ -169,14 +181,15 @@ cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables&
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
                                     const float* fz, const uint8_t* solid, const uint8_t* walls, cudaStream_t s,
-                                    const unsigned* gate = nullptr);
+                                    const unsigned* gate = nullptr, const SubstepOut* so = nullptr);
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,
                               const long long* below, const float* w, const float* wp, float* wt,
                               const float* ext, const float* p, const PlateCoef& pc,
                               unsigned* status, unsigned step, cudaStream_t s);
-// plate forces as (node, value) pairs scattered into the zeroed device buffer
-// (the velocity pass returns them to zero: PlateFaces)
-cudaError_t launch_ext_scatter(float* ext, const int2* pack, int m, cudaStream_t s);
+// plate forces as (node, value) pairs, read from pinned host memory, scattered
+// into the zeroed device buffer (the velocity pass returns them to zero:
+// PlateFaces); and the plate guard cleared
+cudaError_t launch_substep_begin(float* ext, const int2* h_pack, int2* pack, int m, unsigned* status, cudaStream_t s);
 cudaError_t launch_deposit(const Deposit& d, const float* signal, int step, float amp, float* p,
                            cudaStream_t s);
 cudaError_t launch_wsum(const float* f, const long long* idx, const float* w, int n_out, int taps,
