@@ -15,17 +15,18 @@
  *
  * Reverse step n, given Lp = dL/dp~^{n+1} and Lv = dL/dv^{n+1/2} (partial,
  * through step n+1's velocity update) and r^n = dL/dy^n:
- *   lam  = Lp + R^T r^n                        (inside k_adj_cells1)
- *   U    = lam (.) q ;  g_c -= q_c^2 lam_c z_c, z = p~^n - bulk D v^{n+1/2}   (k_adj_cells1)
+ *   lam  = Lp + R^T r^n ;  U = lam (.) q ;
+ *          g_c -= q_c^2 lam_c z_c, z = p~^n - bulk D v^{n+1/2}              (k_adj_cells, C1)
  *   mu   = Lv - bulk D^T U ;  W = mu (.) d ;  E_f = mu_f y_f,
  *          y = v^{n-1/2} - vc G p~^n ;  Lv <- W                            (k_adj_faces)
- *   Lp  <- U - vc G^T W ;  g_c -= 1/2 sum_{faces f of c} E_f               (k_adj_cells2)
+ *   Lp  <- U - vc G^T W ;  g_c -= 1/2 sum_{faces f of c} E_f               (k_adj_cells, C2)
  * Gradients accumulate in double.  The forward is recomputed segment by
  * segment from checkpoints (p~^n and v^{n-1/2} every K steps) into K+1
  * device slots, so the reverse sweep reads every state it needs from HBM.
- * Launches per step: forward 3 (velocity, pressure, an epilogue that records
- * the receivers and then adds the next step's source sample), recompute 2
- * (the pressure kernel adds the next sample), reverse 3.
+ * Launches per step: forward and recompute 2 (velocity, which records the
+ * receivers of the step before, and pressure, which adds the next step's source
+ * sample), reverse 2 (faces; the cell updates that end a step and begin the one
+ * before it).
  * Each sweep (forward, forward with checkpoints, backward) is captured once
  * as a CUDA graph and replayed while its length and buffers stay the same:
  * a gradient evaluation is then two graph launches.
@@ -37,6 +38,7 @@
  */
 #include "acoustic_fdtd_b200.h"
 #include "fdtd_internal.h"
+#include "launch.h"
 
 #include <algorithm>
 #include <climits>
@@ -64,58 +66,6 @@ template <class R>
 __device__ __forceinline__ R face_d(R aL, R aR) { return rsub(R(1), rmul(R(0.5), radd(aL, aR))); }
 template <class R>
 __device__ __forceinline__ R cell_q(R a) { return rrcp(radd(R(1), a)); }
-
-// Gradient on face f = cell c's "+" face along an axis of n cells, at stride s.
-template <class R>
-__device__ __forceinline__ R grad_face(const R* p, long long id, long long s, int f, int n, const ACoef<R>& cf)
-{
-    const R pr = p[id + s], pc = p[id];
-    if (f > 0 && f < n - 2)
-        return radd(rmul(cf.c1, rsub(pr, pc)), rmul(cf.c2, rsub(p[id + 2 * s], p[id - s])));
-    return rsub(pr, pc);
-}
-
-// Divergence at cell c (index t along each axis), zero velocity outside faces.
-template <class R>
-__device__ __forceinline__ R div_cell(const Grid& g, const R* vx, const R* vy, const R* vz, long long id,
-                                      int i, int j, int k, const ACoef<R>& cf)
-{
-    const long long P = g.plane, S = g.sz;
-    const R z0 = R(0);
-    const R xp = (i < g.nx - 1) ? vx[id] : z0, xm = (i > 0) ? vx[id - P] : z0;
-    const R xpp = (i < g.nx - 2) ? vx[id + P] : z0, xmm = (i > 1) ? vx[id - 2 * P] : z0;
-    const R yp = (j < g.ny - 1) ? vy[id] : z0, ym = (j > 0) ? vy[id - S] : z0;
-    const R ypp = (j < g.ny - 2) ? vy[id + S] : z0, ymm = (j > 1) ? vy[id - 2 * S] : z0;
-    const R zp = (k < g.nz - 1) ? vz[id] : z0, zm = (k > 0) ? vz[id - 1] : z0;
-    const R zpp = (k < g.nz - 2) ? vz[id + 1] : z0, zmm = (k > 1) ? vz[id - 2] : z0;
-    const R d1 = radd(radd(rsub(xp, xm), rsub(yp, ym)), rsub(zp, zm));
-    const R d2 = radd(radd(rsub(xpp, xmm), rsub(ypp, ymm)), rsub(zpp, zmm));
-    return radd(rmul(cf.c1, d1), rmul(cf.c2, d2));
-}
-
-// Transposed divergence on face f of an axis with n cells, u at stride s.
-template <class R>
-__device__ __forceinline__ R divT_face(const R* u, long long id, long long s, int f, int n, const ACoef<R>& cf)
-{
-    R t = rmul(cf.c1, rsub(u[id], u[id + s]));
-    const R um = (f >= 1) ? u[id - s] : R(0);
-    const R upp = (f <= n - 3) ? u[id + 2 * s] : R(0);
-    return radd(t, rmul(cf.c2, rsub(um, upp)));
-}
-
-// Transposed gradient at cell t of an axis with n cells (faces 0..n-2), w at stride s.
-template <class R>
-__device__ __forceinline__ R gradT_cell(const R* w, long long id, long long s, int t, int n, const ACoef<R>& cf)
-{
-    R acc = R(0);
-    const int nf = n - 1;   // faces 0..n-2
-    auto inner = [&](int f) { return f > 0 && f < n - 2; };
-    if (t - 1 >= 0 && t - 1 < nf) acc = radd(acc, rmul(inner(t - 1) ? cf.c1 : R(1), w[id - s]));
-    if (t < nf) acc = rsub(acc, rmul(inner(t) ? cf.c1 : R(1), w[id]));
-    if (t - 2 >= 0 && inner(t - 2)) acc = radd(acc, rmul(cf.c2, w[id - 2 * s]));
-    if (t + 1 < nf && inner(t + 1)) acc = rsub(acc, rmul(cf.c2, w[id + s]));
-    return acc;
-}
 
 #define ADJ_INDEX                                                        \
     const int k = blockIdx.x * blockDim.x + threadIdx.x;                 \
@@ -149,145 +99,216 @@ __device__ __forceinline__ void st4r(R* p, long long i, const R (&v)[4])
     }
 }
 
-// Threads own four consecutive cells k0 .. k0+3 of a row; every per-cell
-// expression below is the scalar one of the helpers above, in the same order.
-#define ADJ4_INDEX                                                       \
-    const int k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);          \
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;                 \
-    const int i = blockIdx.z;                                            \
-    if (k0 >= g.nz || j >= g.ny) return;                                 \
-    const long long id = ((long long)i * g.ny + j) * g.sz + k0;
-
-// Gradient on the faces of the four cells along x or y (stride s, face index f,
-// n cells on that axis): grad_face for each cell.
 template <class R>
-__device__ __forceinline__ void grad4(const R* p, long long id, long long s, int f, int n, const ACoef<R>& cf,
-                                      const R (&pc)[4], R (&gr)[4])
+__device__ __forceinline__ void ld2r(const R* p, long long i, R& a, R& b)
 {
-    R pr[4], pm[4], p2[4];
-    ld4r(p, id + s, pr);
-    if (f > 0 && f < n - 2) {
-        ld4r(p, id - s, pm);
-        ld4r(p, id + 2 * s, p2);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gr[q] = radd(rmul(cf.c1, rsub(pr[q], pc[q])), rmul(cf.c2, rsub(p2[q], pm[q])));
+    if constexpr (sizeof(R) == 4) {
+        const float2 x = *reinterpret_cast<const float2*>(p + i);
+        a = x.x; b = x.y;
     } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gr[q] = rsub(pr[q], pc[q]);
+        const double2 x = *reinterpret_cast<const double2*>(p + i);
+        a = x.x; b = x.y;
     }
 }
+// the four values at i when they exist, else zero (i stays inside the field)
+template <class R>
+__device__ __forceinline__ void ld4z(const R* p, long long i, bool exists, R (&v)[4])
+{
+    ld4r(p, i, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = exists ? v[q] : R(0);
+}
 
-// P (or any cell field) at k0-1 .. k0+5: e[t] = f[k0 - 1 + t], zero outside the row.
+// Threads own four consecutive cells k0 .. k0+3 of a row; the (row, group) pairs
+// of a plane are numbered over 1-D blocks, so that no lane idles when Nz/4 is not
+// a multiple of the warp.  The passes are bound by the latency of L2 and memory:
+// what a thread reads is loaded at once from addresses kept inside the field,
+// what does not exist is selected away afterwards, and each kernel starts while
+// the one before it drains.
+#define ADJ4_INDEX                                                       \
+    const int nq_ = (g.nz + 3) >> 2;                                     \
+    const int t_ = blockIdx.x * blockDim.x + threadIdx.x;                \
+    if (t_ >= g.ny * nq_) return;                                        \
+    const int j = t_ / nq_;                                              \
+    const int k0 = 4 * (t_ - j * nq_);                                   \
+    const int i = blockIdx.y;                                            \
+    const long long id = ((long long)i * g.ny + j) * g.sz + k0;
+
+// Blocks of 128 threads; the blocks an SM shall hold, given with each kernel, are
+// those of the least time: more warps in flight are worth a few spilled registers
+// (128^3, a reverse step with its recompute: 4 blocks of the cell updates and 5 of
+// the faces 67.5 us, 5 and 7 61.8, 6 and 7 60.5, 7 and 8 60.7; a forward step
+// with 6 and 6 blocks 15.7, 7 and 8 15.2).
+constexpr int kAdjThreads = 128;
+
+// Gradient on the x or y faces of four cells from the values around them: 4th
+// order on interior faces, 2nd order on the first and last.
+template <class R>
+__device__ __forceinline__ R grad1(const ACoef<R>& cf, R pm, R pc, R pr, R p2, bool fourth)
+{
+    const R d = rsub(pr, pc), w = radd(rmul(cf.c1, d), rmul(cf.c2, rsub(p2, pm)));
+    return fourth ? w : d;
+}
+
+// The values of a cell field a face update reads along x (or y): at f-1, f, f+1
+// and f+2 for face f of an axis with n cells and stride st; c = those at f.
+template <class R>
+struct Line {
+    R m[4], r[4], s[4];
+    __device__ __forceinline__ Line(const R* p, long long id, long long st, int f, int n)
+    {
+        ld4r(p, f > 0 ? id - st : id, m);
+        ld4r(p, f < n - 1 ? id + st : id, r);
+        ld4r(p, f < n - 2 ? id + 2 * st : id, s);
+    }
+};
+
+// A cell field at k0-1 .. k0+5, zero outside the row; c = its four own values.
 template <class R>
 __device__ __forceinline__ void zrow(const R* f, long long id, int k0, int nz, const R (&c)[4], R (&e)[7])
 {
     e[0] = k0 > 0 ? f[id - 1] : R(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q) e[q + 1] = c[q];
-    e[5] = k0 + 4 < nz ? f[id + 4] : R(0);
-    e[6] = k0 + 5 < nz ? f[id + 5] : R(0);
+    e[5] = e[6] = R(0);
+    if (k0 + 4 < nz) ld2r(f, id + 4, e[5], e[6]);
+    if (k0 + 5 >= nz) e[6] = R(0);
 }
-
-// z-face gradient of cell k = k0+q from e (zrow of P): grad_face along z.
+// A face field at k0-2 .. k0+4, zero outside the row; c = its four own values.
 template <class R>
-__device__ __forceinline__ R gradz(const R (&e)[7], int q, int k, int nz, const ACoef<R>& cf)
+__device__ __forceinline__ void zfaces(const R* f, long long id, int k0, int nz, const R (&c)[4], R (&e)[7])
 {
-    if (k > 0 && k < nz - 2) return radd(rmul(cf.c1, rsub(e[q + 2], e[q + 1])), rmul(cf.c2, rsub(e[q + 3], e[q])));
-    return rsub(e[q + 2], e[q + 1]);
+    e[0] = e[1] = R(0);
+    if (k0 >= 2) ld2r(f, id - 2, e[0], e[1]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q + 2] = c[q];
+    e[6] = k0 + 4 < nz ? f[id + 4] : R(0);
 }
 
-// Divergence of the four cells (div_cell for each).
+// Divergence of the four cells, zero velocity outside the faces.
 template <class R>
 __device__ __forceinline__ void div4(const Grid& g, const R* vx, const R* vy, const R* vz, long long id, int i,
                                      int j, int k0, const ACoef<R>& cf, R (&dv)[4])
 {
     const long long P = g.plane, S = g.sz;
-    R xp[4] = {}, xm[4] = {}, xpp[4] = {}, xmm[4] = {}, yp[4] = {}, ym[4] = {}, ypp[4] = {}, ymm[4] = {};
-    if (i < g.nx - 1) ld4r(vx, id, xp);
-    if (i > 0) ld4r(vx, id - P, xm);
-    if (i < g.nx - 2) ld4r(vx, id + P, xpp);
-    if (i > 1) ld4r(vx, id - 2 * P, xmm);
-    if (j < g.ny - 1) ld4r(vy, id, yp);
-    if (j > 0) ld4r(vy, id - S, ym);
-    if (j < g.ny - 2) ld4r(vy, id + S, ypp);
-    if (j > 1) ld4r(vy, id - 2 * S, ymm);
-    R zc[4], ez[7];   // ez[t] = Vz[k0 - 2 + t]
+    R xp[4], xm[4], xpp[4], xmm[4], yp[4], ym[4], ypp[4], ymm[4], zc[4], ez[7];
+    ld4z(vx, id, i < g.nx - 1, xp);
+    ld4z(vx, i > 0 ? id - P : id, i > 0, xm);
+    ld4z(vx, i < g.nx - 2 ? id + P : id, i < g.nx - 2, xpp);
+    ld4z(vx, i > 1 ? id - 2 * P : id, i > 1, xmm);
+    ld4z(vy, id, j < g.ny - 1, yp);
+    ld4z(vy, j > 0 ? id - S : id, j > 0, ym);
+    ld4z(vy, j < g.ny - 2 ? id + S : id, j < g.ny - 2, ypp);
+    ld4z(vy, j > 1 ? id - 2 * S : id, j > 1, ymm);
     ld4r(vz, id, zc);
-    ez[0] = k0 >= 2 ? vz[id - 2] : R(0);
-    ez[1] = k0 >= 1 ? vz[id - 1] : R(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ez[q + 2] = zc[q];
-    ez[6] = k0 + 4 < g.nz ? vz[id + 4] : R(0);
+    zfaces(vz, id, k0, g.nz, zc, ez);
     const R z0 = R(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int k = k0 + q;
-        const R zp = (k < g.nz - 1) ? ez[q + 2] : z0, zm = (k > 0) ? ez[q + 1] : z0;
-        const R zpp = (k < g.nz - 2) ? ez[q + 3] : z0, zmm = (k > 1) ? ez[q] : z0;
-        const R d1 = radd(radd(rsub(xp[q], xm[q]), rsub(yp[q], ym[q])), rsub(zp, zm));
-        const R d2 = radd(radd(rsub(xpp[q], xmm[q]), rsub(ypp[q], ymm[q])), rsub(zpp, zmm));
+        const R zp = (k < g.nz - 1) ? ez[q + 2] : z0, zpp = (k < g.nz - 2) ? ez[q + 3] : z0;
+        const R d1 = radd(radd(rsub(xp[q], xm[q]), rsub(yp[q], ym[q])), rsub(zp, ez[q + 1]));
+        const R d2 = radd(radd(rsub(xpp[q], xmm[q]), rsub(ypp[q], ymm[q])), rsub(zpp, ez[q]));
         dv[q] = radd(rmul(cf.c1, d1), rmul(cf.c2, d2));
     }
 }
 
+// The receivers of one step: 8 taps summed w0*p0 + w1*p1 + ... as
+// acoustic_fdtd.cpp:1663-1676, of the pressure before the source sample that the
+// step after it adds to cell src (its value without the sample is *raw).
 template <class R>
-__global__ void __launch_bounds__(256) k_fwd_vel(Grid g, ACoef<R> cf, const R* __restrict__ a,
-                                                 const R* __restrict__ p, const R* vin0, const R* vin1,
-                                                 const R* vin2, R* vout0, R* vout1, R* vout2)
+struct Record {
+    int n = 0;
+    const long long* idx = nullptr;
+    const R* w = nullptr;
+    R* row = nullptr;
+    long long src = -1;
+    const R* raw = nullptr;
+};
+template <class R>
+__device__ __forceinline__ void record_receivers(const Record<R>& rec, const R* p, int first, int stride)
 {
-    ADJ4_INDEX
-    R ac[4], pc[4];
-    ld4r(a, id, ac);
-    ld4r(p, id, pc);
-    if (i < g.nx - 1) {
-        R gr[4], ar[4], v[4];
-        grad4(p, id, g.plane, i, g.nx, cf, pc, gr);
-        ld4r(a, id + g.plane, ar);
-        ld4r(vin0, id, v);
+    for (int r = first; r < rec.n; r += stride) {
+        R v[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (k0 + q < g.nz) v[q] = rmul(rsub(v[q], rmul(cf.vc, gr[q])), face_d(ac[q], ar[q]));
-        st4r(vout0, id, v);
-    }
-    if (j < g.ny - 1) {
-        R gr[4], ar[4], v[4];
-        grad4(p, id, (long long)g.sz, j, g.ny, cf, pc, gr);
-        ld4r(a, id + g.sz, ar);
-        ld4r(vin1, id, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (k0 + q < g.nz) v[q] = rmul(rsub(v[q], rmul(cf.vc, gr[q])), face_d(ac[q], ar[q]));
-        st4r(vout1, id, v);
-    }
-    {
-        R e[7], v[4];
-        zrow(p, id, k0, g.nz, pc, e);
-        const R a4 = k0 + 4 < g.nz ? a[id + 4] : R(0);
-        ld4r(vin2, id, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int k = k0 + q;
-            if (k < g.nz - 1)
-                v[q] = rmul(rsub(v[q], rmul(cf.vc, gradz(e, q, k, g.nz, cf))), face_d(ac[q], q < 3 ? ac[q + 1] : a4));
+        for (int t = 0; t < 8; ++t) {
+            const long long c = rec.idx[8 * r + t];
+            v[t] = rmul(rec.w[8 * r + t], c == rec.src ? *rec.raw : p[c]);
         }
-        st4r(vout2, id, v);
+        R s = v[0];
+#pragma unroll
+        for (int t = 1; t < 8; ++t) s = radd(s, v[t]);
+        rec.row[r] = s;
     }
+}
+template <class R>
+__global__ void k_record(const R* p, Record<R> rec)
+{
+    record_receivers(rec, p, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// Velocity update.  It also records the receivers of the step before (the
+// pressure it reads), which as a kernel of its own was 3.3 us of a 128^3 step
+// (a step of the forward sweep: 18.5 us then, 15.2 now; the bytes its two passes
+// move, 56 a cell, take 17.9 at the measured copy rate: the fields stay in L2).
+template <class R>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? 7 : 3)
+k_fwd_vel(Grid g, ACoef<R> cf, const R* __restrict__ a, const R* __restrict__ p, const R* vin0, const R* vin1,
+          const R* vin2, R* vout0, R* vout1, R* vout2, Record<R> rec)
+{
+    wait_previous();
+    release_next();
+    if (rec.n > 0)
+        record_receivers(rec, p, (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
+                         gridDim.x * gridDim.y * blockDim.x);
+    ADJ4_INDEX
+    const long long P = g.plane, S = g.sz;
+    R ac[4], ax[4], ay[4], pc[4], vx[4], vy[4], vz[4], e[7];
+    ld4r(p, id, pc);
+    const Line<R> lx(p, id, P, i, g.nx), ly(p, id, S, j, g.ny);
+    zrow(p, id, k0, g.nz, pc, e);
+    ld4r(vin0, id, vx);
+    ld4r(vin1, id, vy);
+    ld4r(vin2, id, vz);
+    ld4r(a, id, ac);
+    ld4r(a, i < g.nx - 1 ? id + P : id, ax);
+    ld4r(a, j < g.ny - 1 ? id + S : id, ay);
+    const R az = k0 + 4 < g.nz ? a[id + 4] : R(0);
+    const bool fx = i > 0 && i < g.nx - 2, fy = j > 0 && j < g.ny - 2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int k = k0 + q;
+        const R x = rmul(rsub(vx[q], rmul(cf.vc, grad1(cf, lx.m[q], pc[q], lx.r[q], lx.s[q], fx))), face_d(ac[q], ax[q]));
+        const R y = rmul(rsub(vy[q], rmul(cf.vc, grad1(cf, ly.m[q], pc[q], ly.r[q], ly.s[q], fy))), face_d(ac[q], ay[q]));
+        const R z = rmul(rsub(vz[q], rmul(cf.vc, grad1(cf, e[q], e[q + 1], e[q + 2], e[q + 3], k > 0 && k < g.nz - 2))),
+                         face_d(ac[q], q < 3 ? ac[q + 1] : az));
+        if (k < g.nz) {
+            vx[q] = x;
+            vy[q] = y;
+        }
+        if (k < g.nz - 1) vz[q] = z;
+    }
+    if (i < g.nx - 1) st4r(vout0, id, vx);
+    if (j < g.ny - 1) st4r(vout1, id, vy);
+    st4r(vout2, id, vz);
 }
 
 // dep >= 0: the next step's source sample sig[dep_n] is added to the new
-// pressure of cell dep, as k_deposit would before that step.
+// pressure of cell dep, as k_deposit would before that step; raw (if given)
+// keeps the pressure without it for the receivers.
 template <class R>
-__global__ void __launch_bounds__(256) k_fwd_pres(Grid g, ACoef<R> cf, const R* __restrict__ a,
-                                                  const R* __restrict__ p, const R* __restrict__ vx,
-                                                  const R* __restrict__ vy, const R* __restrict__ vz,
-                                                  R* __restrict__ pn, long long dep, const R* __restrict__ sig,
-                                                  int dep_n)
+__global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? 8 : 3)
+k_fwd_pres(Grid g, ACoef<R> cf, const R* __restrict__ a, const R* __restrict__ p, const R* __restrict__ vx,
+           const R* __restrict__ vy, const R* __restrict__ vz, R* __restrict__ pn, long long dep,
+           const R* __restrict__ sig, int dep_n, R* __restrict__ raw)
 {
+    wait_previous();
+    release_next();
     ADJ4_INDEX
     R dv[4], pc[4], ac[4], out[4];
-    div4(g, vx, vy, vz, id, i, j, k0, cf, dv);
     ld4r(p, id, pc);
     ld4r(a, id, ac);
+    div4(g, vx, vy, vz, id, i, j, k0, cf, dv);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
         out[q] = (k0 + q < g.nz) ? rmul(rsub(pc[q], rmul(cf.bulk, dv[q])), cell_q(ac[q])) : R(0);
@@ -295,7 +316,10 @@ __global__ void __launch_bounds__(256) k_fwd_pres(Grid g, ACoef<R> cf, const R* 
         const R sv = sig[dep_n];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (dep == id + q && sv != R(0)) out[q] = radd(out[q], sv);
+            if (dep == id + q) {
+                if (raw) *raw = out[q];
+                if (sv != R(0)) out[q] = radd(out[q], sv);
+            }
     }
     st4r(pn, id, out);
 }
@@ -308,26 +332,6 @@ __global__ void k_deposit(R* p, long long src, const R* sig, int n)
     if (s != R(0)) p[src] = radd(p[src], s);
 }
 
-// After forward step n: the receivers of P^{n+1} (row; 8 taps summed
-// w0*p0 + w1*p1 + ... as acoustic_fdtd.cpp:1663-1676), then the next step's
-// source sample into P^{n+1} (dep_n >= 0); one block.
-template <class R>
-__global__ void k_fwd_epilogue(R* p, int n_rec, const long long* idx, const R* w, R* row, long long src,
-                               const R* sig, int dep_n)
-{
-    if (row)
-        for (int r = threadIdx.x; r < n_rec; r += blockDim.x) {
-            R s = rmul(w[8 * r], p[idx[8 * r]]);
-            for (int t = 1; t < 8; ++t) s = radd(s, rmul(w[8 * r + t], p[idx[8 * r + t]]));
-            row[r] = s;
-        }
-    __syncthreads();
-    if (threadIdx.x == 0 && dep_n >= 0 && src >= 0) {
-        const R sv = sig[dep_n];
-        if (sv != R(0)) p[src] = radd(p[src], sv);
-    }
-}
-
 __device__ __forceinline__ void ld4d(const double* p, long long i, double (&v)[4]) { ld4r<double>(p, i, v); }
 __device__ __forceinline__ void st4d(double* p, long long i, const double (&v)[4]) { st4r<double>(p, i, v); }
 
@@ -337,229 +341,173 @@ template <class R>
 struct TapSources {
     int n = 0;                       // distinct tap cells (0: none)
     const long long* cell = nullptr;
+    const int* plane = nullptr;      // [nx + 1]: the tap cells of plane i are plane[i] .. plane[i+1]-1
     const int* start = nullptr;      // [n + 1]
     const int* tap = nullptr;        // 8 r + t, ascending within a cell
     const R* w = nullptr;            // tap weights [8 n_rec]
     const R* rrow = nullptr;         // this step's receiver residuals [n_rec]
 };
 
+// lam = Lp + R^T r^n on the tap cells among the four of group id in plane i
 template <class R>
-__global__ void __launch_bounds__(256) k_adj_cells1(Grid g, ACoef<R> cf, const R* __restrict__ a,
-                                                    const R* __restrict__ lam, const R* __restrict__ pt,
-                                                    const R* __restrict__ vx, const R* __restrict__ vy,
-                                                    const R* __restrict__ vz, R* __restrict__ u,
-                                                    double* __restrict__ grad, TapSources<R> ts)
+__device__ __forceinline__ void add_residuals(const TapSources<R>& ts, int i, long long id, R (&l)[4])
 {
-    ADJ4_INDEX
-    R ac[4], l[4], ptc[4], dv[4], uo[4];
-    double gr[4];
-    ld4r(a, id, ac);
-    ld4r(lam, id, l);
-    if (ts.n > 0) {   // lam = Lp + R^T r^n on the tap cells among these four
-        int lo = 0, hi = ts.n;   // first tap cell >= id
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (ts.cell[mid] < id) lo = mid + 1;
-            else hi = mid;
+    const int end = ts.plane[i + 1];
+    for (int c = ts.plane[i]; c < end; ++c) {   // no tap in most planes
+        const long long d = ts.cell[c] - id;
+        if (d < 0 || d > 3) continue;
+        for (int e = ts.start[c]; e < ts.start[c + 1]; ++e) {
+            const int tp = ts.tap[e];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (d == q) l[q] = radd(l[q], rmul(ts.w[tp], ts.rrow[tp >> 3]));
         }
-        for (int c = lo; c < ts.n && ts.cell[c] < id + 4; ++c) {
-            const int q = (int)(ts.cell[c] - id);
-            for (int e = ts.start[c]; e < ts.start[c + 1]; ++e) {
-                const int tp = ts.tap[e];
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq)
-                    if (qq == q) l[qq] = radd(l[qq], rmul(ts.w[tp], ts.rrow[tp >> 3]));
-            }
-        }
-    }
-    ld4r(pt, id, ptc);
-    div4(g, vx, vy, vz, id, i, j, k0, cf, dv);
-    ld4d(grad, id, gr);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uo[q] = R(0);
-        if (k0 + q >= g.nz) continue;
-        const R qq = cell_q(ac[q]);
-        uo[q] = rmul(l[q], qq);
-        const R z = rsub(ptc[q], rmul(cf.bulk, dv[q]));
-        gr[q] -= (double)qq * (double)qq * (double)l[q] * (double)z;
-    }
-    st4r(u, id, uo);
-    st4d(grad, id, gr);
-}
-
-// Transposed divergence on the x or y faces of the four cells (divT_face each).
-template <class R>
-__device__ __forceinline__ void divT4(const R* u, long long id, long long s, int f, int n, const ACoef<R>& cf,
-                                      R (&out)[4])
-{
-    R uc[4], ur[4], um[4] = {}, upp[4] = {};
-    ld4r(u, id, uc);
-    ld4r(u, id + s, ur);
-    if (f >= 1) ld4r(u, id - s, um);
-    if (f <= n - 3) ld4r(u, id + 2 * s, upp);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) out[q] = radd(rmul(cf.c1, rsub(uc[q], ur[q])), rmul(cf.c2, rsub(um[q], upp[q])));
-}
-
-template <class R>
-__global__ void __launch_bounds__(256) k_adj_faces(Grid g, ACoef<R> cf, const R* __restrict__ a,
-                                                   const R* __restrict__ u, const R* __restrict__ pt,
-                                                   const R* __restrict__ vo0, const R* __restrict__ vo1,
-                                                   const R* __restrict__ vo2, R* lv0, R* lv1, R* lv2,
-                                                   R* __restrict__ e0, R* __restrict__ e1, R* __restrict__ e2)
-{
-    ADJ4_INDEX
-    R ac[4], ptc[4];
-    ld4r(a, id, ac);
-    ld4r(pt, id, ptc);
-    // x and y faces
-#pragma unroll
-    for (int ax = 0; ax < 2; ++ax) {
-        const bool exists = ax == 0 ? i < g.nx - 1 : j < g.ny - 1;
-        if (!exists) continue;
-        const long long s = ax == 0 ? g.plane : (long long)g.sz;
-        const int f = ax == 0 ? i : j, n = ax == 0 ? g.nx : g.ny;
-        R* lv = ax == 0 ? lv0 : lv1;
-        R* ef = ax == 0 ? e0 : e1;
-        const R* vo = ax == 0 ? vo0 : vo1;
-        R dt[4], gr[4], ar[4], l[4], v[4], eo[4];
-        divT4(u, id, s, f, n, cf, dt);
-        grad4(pt, id, s, f, n, cf, ptc, gr);
-        ld4r(a, id + s, ar);
-        ld4r(lv, id, l);
-        ld4r(vo, id, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            eo[q] = R(0);
-            if (k0 + q >= g.nz) continue;
-            const R mu = rsub(l[q], rmul(cf.bulk, dt[q]));
-            const R y = rsub(v[q], rmul(cf.vc, gr[q]));
-            l[q] = rmul(mu, face_d(ac[q], ar[q]));
-            eo[q] = rmul(mu, y);
-        }
-        st4r(lv, id, l);
-        st4r(ef, id, eo);
-    }
-    // z faces: U and P at k0-1 .. k0+5, a at k0 .. k0+4
-    {
-        R uc[4], eu[7], ep[7], l[4], v[4], eo[4];
-        ld4r(u, id, uc);
-        zrow(u, id, k0, g.nz, uc, eu);
-        zrow(pt, id, k0, g.nz, ptc, ep);
-        const R a4 = k0 + 4 < g.nz ? a[id + 4] : R(0);
-        ld4r(lv2, id, l);
-        ld4r(vo2, id, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int k = k0 + q;
-            eo[q] = R(0);
-            if (k >= g.nz - 1) continue;
-            // divT_face along z: c1 (u[k] - u[k+1]) + c2 (u[k-1] - u[k+2]), zero outside
-            const R um = k >= 1 ? eu[q] : R(0), upp = k <= g.nz - 3 ? eu[q + 3] : R(0);
-            const R dt = radd(rmul(cf.c1, rsub(eu[q + 1], eu[q + 2])), rmul(cf.c2, rsub(um, upp)));
-            const R mu = rsub(l[q], rmul(cf.bulk, dt));
-            const R y = rsub(v[q], rmul(cf.vc, gradz(ep, q, k, g.nz, cf)));
-            l[q] = rmul(mu, face_d(ac[q], q < 3 ? ac[q + 1] : a4));
-            eo[q] = rmul(mu, y);
-        }
-        st4r(lv2, id, l);
-        st4r(e2, id, eo);
     }
 }
 
-// Transposed gradient of the four cells along x or y (cell index t uniform).
+// Transposed gradient of the four cells along x or y: cell t of an axis with n
+// cells (faces 0 .. n-2).  Terms in the order t-1, t, t-2, t+1.
 template <class R>
 __device__ __forceinline__ void gradT4(const R* w, long long id, long long s, int t, int n, const ACoef<R>& cf,
                                        R (&out)[4])
 {
-    const int nf = n - 1;
     auto inner = [&](int f) { return f > 0 && f < n - 2; };
+    R m[4], c[4], mm[4], r[4];
+    ld4z(w, t > 0 ? id - s : id, t > 0, m);
+    ld4z(w, id, t < n - 1, c);
+    ld4z(w, t > 1 ? id - 2 * s : id, inner(t - 2), mm);
+    ld4z(w, t < n - 1 ? id + s : id, inner(t + 1), r);
+    const R cm = inner(t - 1) ? cf.c1 : R(1), cc = inner(t) ? cf.c1 : R(1);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) out[q] = R(0);
-    R v[4];
-    if (t - 1 >= 0 && t - 1 < nf) {
-        ld4r(w, id - s, v);
-        const R c = inner(t - 1) ? cf.c1 : R(1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) out[q] = radd(out[q], rmul(c, v[q]));
-    }
-    if (t < nf) {
-        ld4r(w, id, v);
-        const R c = inner(t) ? cf.c1 : R(1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) out[q] = rsub(out[q], rmul(c, v[q]));
-    }
-    if (t - 2 >= 0 && inner(t - 2)) {
-        ld4r(w, id - 2 * s, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) out[q] = radd(out[q], rmul(cf.c2, v[q]));
-    }
-    if (t + 1 < nf && inner(t + 1)) {
-        ld4r(w, id + s, v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) out[q] = rsub(out[q], rmul(cf.c2, v[q]));
-    }
+    for (int q = 0; q < 4; ++q)
+        out[q] = rsub(radd(rsub(radd(R(0), rmul(cm, m[q])), rmul(cc, c[q])), rmul(cf.c2, mm[q])), rmul(cf.c2, r[q]));
 }
 
-template <class R>
-__global__ void __launch_bounds__(256) k_adj_cells2(Grid g, ACoef<R> cf, const R* __restrict__ u,
-                                                    const R* __restrict__ w0, const R* __restrict__ w1,
-                                                    const R* __restrict__ w2, const R* __restrict__ e0,
-                                                    const R* __restrict__ e1, const R* __restrict__ e2,
-                                                    R* __restrict__ lp, double* __restrict__ grad)
+// The cell updates of the reverse sweep.  C2: those that end step n (Lp from U, W
+// and the faces' E); C1: those that begin the step before it (U from Lp, z from
+// that step's states).  Both touch only a cell's own Lp, U and gradient, so
+// between two steps of a segment one pass does both: Lp stays in registers and
+// the gradient, 16 of a step's 152 bytes a cell, is read and written once
+// (128^3, a reverse step with its recompute: 73.6 us as three kernels, 60.5 now).
+template <class R, bool C2, bool C1>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? (C1 && C2 ? 6 : 5) : 2)
+k_adj_cells(Grid g, ACoef<R> cf, R* __restrict__ u, const R* __restrict__ w0, const R* __restrict__ w1,
+            const R* __restrict__ w2, const R* __restrict__ e0, const R* __restrict__ e1, const R* __restrict__ e2,
+            R* __restrict__ lp, double* __restrict__ grad, const R* __restrict__ a, const R* __restrict__ pt,
+            const R* __restrict__ vx, const R* __restrict__ vy, const R* __restrict__ vz, TapSources<R> ts)
 {
+    wait_previous();
+    release_next();
     ADJ4_INDEX
     const long long P = g.plane, S = g.sz;
-    R gx[4], gy[4], uc[4], wc[4], ew[7], lo[4];
-    gradT4(w0, id, P, i, g.nx, cf, gx);
-    gradT4(w1, id, S, j, g.ny, cf, gy);
-    ld4r(u, id, uc);
-    // W_z at k0-2 .. k0+4: ew[t] = Wz[k0 - 2 + t]
-    ld4r(w2, id, wc);
-    ew[0] = k0 >= 2 ? w2[id - 2] : R(0);
-    ew[1] = k0 >= 1 ? w2[id - 1] : R(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ew[q + 2] = wc[q];
-    ew[6] = k0 + 4 < g.nz ? w2[id + 4] : R(0);
-    // E: x and y faces of the four cells, and the z faces k0-1 .. k0+3
-    R ex[4] = {}, exm[4] = {}, ey[4] = {}, eym[4] = {}, ezc[4], ez[5];
-    if (i < g.nx - 1) ld4r(e0, id, ex);
-    if (i > 0) ld4r(e0, id - P, exm);
-    if (j < g.ny - 1) ld4r(e1, id, ey);
-    if (j > 0) ld4r(e1, id - S, eym);
-    ld4r(e2, id, ezc);
-    ez[0] = k0 >= 1 ? e2[id - 1] : R(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ez[q + 1] = ezc[q];
     double gr[4];
+    R l[4];
     ld4d(grad, id, gr);
-    const int nzf = g.nz - 1;
-    auto innerz = [&](int f) { return f > 0 && f < g.nz - 2; };
+    if constexpr (C2) {
+        R gx[4], gy[4], uc[4], wc[4], ew[7], ex[4], exm[4], ey[4], eym[4], ez[4];
+        ld4r(u, id, uc);
+        ld4z(e0, id, i < g.nx - 1, ex);
+        ld4z(e0, i > 0 ? id - P : id, i > 0, exm);
+        ld4z(e1, id, j < g.ny - 1, ey);
+        ld4z(e1, j > 0 ? id - S : id, j > 0, eym);
+        ld4r(e2, id, ez);
+        const R ezm = k0 >= 1 ? e2[id - 1] : R(0);
+        ld4r(w2, id, wc);
+        zfaces(w2, id, k0, g.nz, wc, ew);   // W_z at k0-2 .. k0+4
+        gradT4(w0, id, P, i, g.nx, cf, gx);
+        gradT4(w1, id, S, j, g.ny, cf, gy);
+        auto innerz = [&](int f) { return f > 0 && f < g.nz - 2; };
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = k0 + q;
+            const R tm = rmul(innerz(k - 1) ? cf.c1 : R(1), ew[q + 1]);
+            const R tc = rmul(innerz(k) ? cf.c1 : R(1), k < g.nz - 1 ? ew[q + 2] : R(0));
+            const R tmm = rmul(cf.c2, innerz(k - 2) ? ew[q] : R(0)), tr = rmul(cf.c2, innerz(k + 1) ? ew[q + 3] : R(0));
+            const R gz = rsub(radd(rsub(radd(R(0), tm), tc), tmm), tr);
+            l[q] = k < g.nz ? rsub(uc[q], rmul(cf.vc, radd(radd(gx[q], gy[q]), gz))) : R(0);
+            const double e = (double)ex[q] + (double)exm[q] + (double)ey[q] + (double)eym[q] +
+                             (k < g.nz - 1 ? (double)ez[q] : 0.0) + (double)(q ? ez[q - 1] : ezm);
+            if (k < g.nz) gr[q] -= 0.5 * e;
+        }
+        if constexpr (!C1) st4r(lp, id, l);
+    } else {
+        ld4r(lp, id, l);
+    }
+    if constexpr (C1) {
+        R ac[4], ptc[4], dv[4], uo[4];
+        ld4r(a, id, ac);
+        ld4r(pt, id, ptc);
+        if (ts.n > 0) add_residuals(ts, i, id, l);
+        div4(g, vx, vy, vz, id, i, j, k0, cf, dv);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const R qq = cell_q(ac[q]);
+            const R z = rsub(ptc[q], rmul(cf.bulk, dv[q]));
+            uo[q] = k0 + q < g.nz ? rmul(l[q], qq) : R(0);
+            if (k0 + q < g.nz) gr[q] -= (double)qq * (double)qq * (double)l[q] * (double)z;
+        }
+        st4r(u, id, uo);
+    }
+    st4d(grad, id, gr);
+}
+
+// mu = Lv - bulk D^T U, W = mu (.) d and E = mu y on every face of the four cells.
+template <class R>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? 7 : 2)
+k_adj_faces(Grid g, ACoef<R> cf, const R* __restrict__ a, const R* __restrict__ u, const R* __restrict__ pt,
+            const R* __restrict__ vo0, const R* __restrict__ vo1, const R* __restrict__ vo2, R* lv0, R* lv1, R* lv2,
+            R* __restrict__ e0, R* __restrict__ e1, R* __restrict__ e2)
+{
+    wait_previous();
+    release_next();
+    ADJ4_INDEX
+    R ac[4], ptc[4], uc[4];
+    ld4r(a, id, ac);
+    ld4r(pt, id, ptc);
+    ld4r(u, id, uc);
+    // x and y faces
+    auto faces = [&](long long s, int f, int n, const R* vo, R* lv, R* ef) {
+        R ar[4], l[4], v[4], eo[4];
+        const Line<R> lu(u, id, s, f, n), lq(pt, id, s, f, n);
+        ld4r(a, f < n - 1 ? id + s : id, ar);
+        ld4r(lv, id, l);
+        ld4r(vo, id, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const R um = f >= 1 ? lu.m[q] : R(0), us = f <= n - 3 ? lu.s[q] : R(0);
+            const R dt = radd(rmul(cf.c1, rsub(uc[q], lu.r[q])), rmul(cf.c2, rsub(um, us)));
+            const R mu = rsub(l[q], rmul(cf.bulk, dt));
+            const R y = rsub(v[q], rmul(cf.vc, grad1(cf, lq.m[q], ptc[q], lq.r[q], lq.s[q], f > 0 && f < n - 2)));
+            l[q] = k0 + q < g.nz ? rmul(mu, face_d(ac[q], ar[q])) : l[q];
+            eo[q] = k0 + q < g.nz ? rmul(mu, y) : R(0);
+        }
+        if (f < n - 1) {
+            st4r(lv, id, l);
+            st4r(ef, id, eo);
+        }
+    };
+    faces(g.plane, i, g.nx, vo0, lv0, e0);
+    faces(g.sz, j, g.ny, vo1, lv1, e1);
+    // z faces: U and P at k0-1 .. k0+5, a at k0 .. k0+4
+    R eu[7], ep[7], l[4], v[4], eo[4];
+    zrow(u, id, k0, g.nz, uc, eu);
+    zrow(pt, id, k0, g.nz, ptc, ep);
+    const R a4 = k0 + 4 < g.nz ? a[id + 4] : R(0);
+    ld4r(lv2, id, l);
+    ld4r(vo2, id, v);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int k = k0 + q;
-        lo[q] = R(0);
-        if (k >= g.nz) continue;
-        // gradT_cell along z, term order of the scalar helper
-        R gz = R(0);
-        if (k - 1 >= 0 && k - 1 < nzf) gz = radd(gz, rmul(innerz(k - 1) ? cf.c1 : R(1), ew[q + 1]));
-        if (k < nzf) gz = rsub(gz, rmul(innerz(k) ? cf.c1 : R(1), ew[q + 2]));
-        if (k - 2 >= 0 && innerz(k - 2)) gz = radd(gz, rmul(cf.c2, ew[q]));
-        if (k + 1 < nzf && innerz(k + 1)) gz = rsub(gz, rmul(cf.c2, ew[q + 3]));
-        R gt = radd(radd(gx[q], gy[q]), gz);
-        lo[q] = rsub(uc[q], rmul(cf.vc, gt));
-        double e = 0.0;
-        if (i < g.nx - 1) e += (double)ex[q];
-        if (i > 0) e += (double)exm[q];
-        if (j < g.ny - 1) e += (double)ey[q];
-        if (j > 0) e += (double)eym[q];
-        if (k < g.nz - 1) e += (double)ez[q + 1];
-        if (k > 0) e += (double)ez[q];
-        gr[q] -= 0.5 * e;
+        // c1 (u[k] - u[k+1]) + c2 (u[k-1] - u[k+2]), zero outside
+        const R um = k >= 1 ? eu[q] : R(0), upp = k <= g.nz - 3 ? eu[q + 3] : R(0);
+        const R dt = radd(rmul(cf.c1, rsub(eu[q + 1], eu[q + 2])), rmul(cf.c2, rsub(um, upp)));
+        const R mu = rsub(l[q], rmul(cf.bulk, dt));
+        const R y = rsub(v[q], rmul(cf.vc, grad1(cf, ep[q], ep[q + 1], ep[q + 2], ep[q + 3], k > 0 && k < g.nz - 2)));
+        l[q] = k < g.nz - 1 ? rmul(mu, face_d(ac[q], q < 3 ? ac[q + 1] : a4)) : l[q];
+        eo[q] = k < g.nz - 1 ? rmul(mu, y) : R(0);
     }
-    st4r(lp, id, lo);
-    st4d(grad, id, gr);
+    st4r(lv2, id, l);
+    st4r(e2, id, eo);
 }
 
 // a (reference order, float or double) -> padded R array
@@ -594,7 +542,7 @@ struct FdtdB200Adj {
     size_t eb = 4;                 // bytes per value of R
     void* a = nullptr;             // padded R
     // loss-mode state and checkpoints
-    void *P0 = nullptr, *P1 = nullptr, *V0[3] = {}, *V1[3] = {};
+    void *P0 = nullptr, *P1 = nullptr, *V0[3] = {};
     std::vector<void*> ckP, ckV;   // ckV holds 3 per checkpoint
     // segment slots: K+1 P and K+1 x 3 V
     std::vector<void*> sP, sV;
@@ -605,6 +553,7 @@ struct FdtdB200Adj {
     // source/receivers
     long long src = -1;
     void* sig = nullptr;           // R[n_sig]
+    void* raw = nullptr;           // R: the source cell's pressure without the next sample
     int n_sig = 0;
     int n_rec = 0;
     long long* ridx = nullptr;
@@ -614,6 +563,7 @@ struct FdtdB200Adj {
     int n_tap_cells = 0;           // distinct receiver tap cells, sorted (TapSources)
     long long* tap_cell = nullptr;
     int* tap_start = nullptr;
+    int* tap_plane = nullptr;
     int* tap_ord = nullptr;
     int trace_cap = 0;
     int fwd_steps = -1;            // steps of the last checkpointed forward
@@ -651,8 +601,11 @@ void dfree(FdtdB200Adj* h, void*& p)
 size_t field_bytes(const FdtdB200Adj* h) { return (size_t)h->g.cells * h->eb; }
 
 dim3 cell_grid(const Grid& g) { return dim3((g.nz + 31) / 32, (g.ny + 7) / 8, g.nx); }
-dim3 vec_grid(const Grid& g) { return dim3((g.sz / 4 + 31) / 32, (g.ny + 7) / 8, g.nx); }   // four cells per thread
 const dim3 kBlock(32, 8, 1);
+dim3 vec_grid(const Grid& g)   // four cells per thread (ADJ4_INDEX)
+{
+    return dim3((unsigned)(((long long)g.ny * ((g.nz + 3) / 4) + kAdjThreads - 1) / kAdjThreads), g.nx);
+}
 
 template <class R>
 const ACoef<R>& coef(const FdtdB200Adj* h);
@@ -662,31 +615,22 @@ template <>
 const ACoef<double>& coef<double>(const FdtdB200Adj* h) { return h->c64; }
 
 // One forward step from (p, vin) to (pn, vout); p already holds this step's
-// source sample.  With next_deposit the next step's sample is added to pn:
-// by the pressure kernel when no receivers are recorded (a recompute), else
-// by the epilogue after it has recorded the receivers of pn.
+// source sample.  The pressure kernel adds the next step's sample to pn
+// (next_deposit).  rec: the receivers of p, the step before's, to record.
 template <class R>
-void fwd_step(FdtdB200Adj* h, int n, void* p, void* const* vin, void* const* vout, void* pn, bool next_deposit,
-              bool record)
+int fwd_step(FdtdB200Adj* h, int n, void* p, void* const* vin, void* const* vout, void* pn, bool next_deposit,
+             const Record<R>& rec)
 {
     const Grid& g = h->g;
     const ACoef<R>& cf = coef<R>(h);
     const bool dep = next_deposit && h->src >= 0 && n + 1 < h->n_sig;
-    const bool rec = record && h->n_rec > 0 && n < h->trace_cap;
-    k_fwd_vel<R><<<vec_grid(g), kBlock, 0, h->stream>>>(g, cf, (const R*)h->a, (const R*)p, (const R*)vin[0],
-                                                         (const R*)vin[1], (const R*)vin[2], (R*)vout[0],
-                                                         (R*)vout[1], (R*)vout[2]);
-    const bool dep_in_pres = dep && !rec;
-    k_fwd_pres<R><<<vec_grid(g), kBlock, 0, h->stream>>>(g, cf, (const R*)h->a, (const R*)p, (const R*)vout[0],
-                                                          (const R*)vout[1], (const R*)vout[2], (R*)pn,
-                                                          dep_in_pres ? h->src : -1LL, (const R*)h->sig, n + 1);
+    ACK(launch_after(k_fwd_vel<R>, vec_grid(g), dim3(kAdjThreads), 0, h->stream, g, cf, (const R*)h->a, (const R*)p,
+                     (const R*)vin[0], (const R*)vin[1], (const R*)vin[2], (R*)vout[0], (R*)vout[1], (R*)vout[2], rec));
+    ACK(launch_after(k_fwd_pres<R>, vec_grid(g), dim3(kAdjThreads), 0, h->stream, g, cf, (const R*)h->a, (const R*)p,
+                     (const R*)vout[0], (const R*)vout[1], (const R*)vout[2], (R*)pn, dep ? h->src : -1LL,
+                     (const R*)h->sig, n + 1, (R*)h->raw));
     h->launches += 2;
-    if (rec) {
-        k_fwd_epilogue<R><<<1, 128, 0, h->stream>>>((R*)pn, h->n_rec, h->ridx, (const R*)h->rw,
-                                                    (R*)h->traces + (size_t)n * h->n_rec, h->src,
-                                                    (const R*)h->sig, dep ? n + 1 : -1);
-        ++h->launches;
-    }
+    return FDTD_OK;
 }
 
 int ensure_checkpoints(FdtdB200Adj* h, int n_steps)
@@ -716,8 +660,8 @@ int forward_impl(FdtdB200Adj* h, int n_steps, int keep)
     ACK(cudaMemsetAsync(h->P0, 0, fb, h->stream));
     for (int c = 0; c < 3; ++c) ACK(cudaMemsetAsync(h->V0[c], 0, fb, h->stream));
     void* P[2] = {h->P0, h->P1};
-    void* V[2][3] = {{h->V0[0], h->V0[1], h->V0[2]}, {h->V1[0], h->V1[1], h->V1[2]}};
     int cur = 0;
+    Record<R> rec;   // of the step before: recorded as its pressure is read
     if (h->src >= 0 && h->n_sig > 0) {   // step 0's source sample; later ones come with the step before
         k_deposit<R><<<1, 1, 0, h->stream>>>((R*)P[cur], h->src, (const R*)h->sig, 0);
         ++h->launches;
@@ -727,10 +671,22 @@ int forward_impl(FdtdB200Adj* h, int n_steps, int keep)
             const int q = n / h->K;
             ACK(cudaMemcpyAsync(h->ckP[q], P[cur], fb, cudaMemcpyDeviceToDevice, h->stream));
             for (int c = 0; c < 3; ++c)
-                ACK(cudaMemcpyAsync(h->ckV[3 * q + c], V[cur][c], fb, cudaMemcpyDeviceToDevice, h->stream));
+                ACK(cudaMemcpyAsync(h->ckV[3 * q + c], h->V0[c], fb, cudaMemcpyDeviceToDevice, h->stream));
         }
-        fwd_step<R>(h, n, P[cur], V[cur], V[cur ^ 1], P[cur ^ 1], n + 1 < n_steps, true);
+        if (int rc = fwd_step<R>(h, n, P[cur], h->V0, h->V0, P[cur ^ 1], n + 1 < n_steps, rec)) return rc;
         cur ^= 1;
+        if (h->n_rec > 0 && n < h->trace_cap) {
+            rec.n = h->n_rec;
+            rec.idx = h->ridx;
+            rec.w = (const R*)h->rw;
+            rec.row = (R*)h->traces + (size_t)n * h->n_rec;
+            rec.src = n + 1 < n_steps && n + 1 < h->n_sig ? h->src : -1;
+            rec.raw = (const R*)h->raw;
+        }
+    }
+    if (rec.n > 0) {
+        k_record<R><<<(rec.n + 127) / 128, 128, 0, h->stream>>>((const R*)P[cur], rec);
+        ++h->launches;
     }
     ACK(cudaGetLastError());
     return FDTD_OK;
@@ -835,33 +791,38 @@ int backward_impl(FdtdB200Adj* h)
         // recompute: slot t holds p~^{n0+t} (after its deposit; the checkpoint
         // already holds it) and v^{n0+t-1/2}; traces are already recorded
         for (int t = 0; t < len; ++t)
-            fwd_step<R>(h, n0 + t, h->sP[t], &h->sV[3 * t], &h->sV[3 * (t + 1)], h->sP[t + 1], t + 1 < len,
-                        false);
-        for (int t = len - 1; t >= 0; --t) {
-            const int n = n0 + t;
-            void* const* vo = &h->sV[3 * t];       // v^{n-1/2}
-            void* const* vn = &h->sV[3 * (t + 1)]; // v^{n+1/2}
-            TapSources<R> ts;   // R^T r^n, added to Lp inside k_adj_cells1
-            if (h->n_rec > 0) {
+            if (int rc = fwd_step<R>(h, n0 + t, h->sP[t], &h->sV[3 * t], &h->sV[3 * (t + 1)], h->sP[t + 1],
+                                     t + 1 < len, Record<R>()))
+                return rc;
+        // cell updates: c2 those that end step n0 + t + 1, c1 those that begin step n0 + t
+        auto cells = [&](auto kernel, int t) -> int {
+            TapSources<R> ts;   // R^T r^n, added to Lp
+            if (h->n_rec > 0 && t >= 0) {
                 ts.n = h->n_tap_cells;
                 ts.cell = h->tap_cell;
+                ts.plane = h->tap_plane;
                 ts.start = h->tap_start;
                 ts.tap = h->tap_ord;
                 ts.w = (const R*)h->rw;
-                ts.rrow = (const R*)h->resid + (size_t)n * h->n_rec;
+                ts.rrow = (const R*)h->resid + (size_t)(n0 + t) * h->n_rec;
             }
-            k_adj_cells1<R><<<vec_grid(g), kBlock, 0, h->stream>>>(
-                g, cf, (const R*)h->a, (const R*)h->Lp, (const R*)h->sP[t], (const R*)vn[0], (const R*)vn[1],
-                (const R*)vn[2], (R*)h->U, h->grad, ts);
-            k_adj_faces<R><<<vec_grid(g), kBlock, 0, h->stream>>>(
-                g, cf, (const R*)h->a, (const R*)h->U, (const R*)h->sP[t], (const R*)vo[0], (const R*)vo[1],
-                (const R*)vo[2], (R*)h->Lv[0], (R*)h->Lv[1], (R*)h->Lv[2], (R*)h->E[0], (R*)h->E[1],
-                (R*)h->E[2]);
-            k_adj_cells2<R><<<vec_grid(g), kBlock, 0, h->stream>>>(
-                g, cf, (const R*)h->U, (const R*)h->Lv[0], (const R*)h->Lv[1], (const R*)h->Lv[2],
-                (const R*)h->E[0], (const R*)h->E[1], (const R*)h->E[2], (R*)h->Lp, h->grad);
-            h->launches += 3;
+            void* const* vn = &h->sV[3 * (std::max(t, 0) + 1)];   // v^{n+1/2}
+            ACK(launch_after(kernel, vec_grid(g), dim3(kAdjThreads), 0, h->stream, g, cf, (R*)h->U, (const R*)h->Lv[0],
+                             (const R*)h->Lv[1], (const R*)h->Lv[2], (const R*)h->E[0], (const R*)h->E[1],
+                             (const R*)h->E[2], (R*)h->Lp, h->grad, (const R*)h->a, (const R*)h->sP[std::max(t, 0)],
+                             (const R*)vn[0], (const R*)vn[1], (const R*)vn[2], ts));
+            ++h->launches;
+            return FDTD_OK;
+        };
+        for (int t = len - 1; t >= 0; --t) {
+            if (int rc = t == len - 1 ? cells(k_adj_cells<R, false, true>, t) : cells(k_adj_cells<R, true, true>, t)) return rc;
+            void* const* vo = &h->sV[3 * t];       // v^{n-1/2}
+            ACK(launch_after(k_adj_faces<R>, vec_grid(g), dim3(kAdjThreads), 0, h->stream, g, cf, (const R*)h->a,
+                             (const R*)h->U, (const R*)h->sP[t], (const R*)vo[0], (const R*)vo[1], (const R*)vo[2],
+                             (R*)h->Lv[0], (R*)h->Lv[1], (R*)h->Lv[2], (R*)h->E[0], (R*)h->E[1], (R*)h->E[2]));
+            ++h->launches;
         }
+        if (int rc = cells(k_adj_cells<R, true, false>, -1)) return rc;
         ACK(cudaGetLastError());
     }
     return FDTD_OK;
@@ -917,10 +878,10 @@ FdtdB200Adj* fdtd_b200_adj_create(int Nx, int Ny, int Nz, double dx, double c, d
     h->dt = h->dbl ? dt64 : (double)dt32;
     const size_t fb = field_bytes(h);
     int rc = dalloc(h, &h->a, fb);
+    if (!rc) rc = dalloc(h, &h->raw, h->eb);
     if (!rc) rc = dalloc(h, &h->P0, fb);
     if (!rc) rc = dalloc(h, &h->P1, fb);
     for (int q = 0; q < 3 && !rc; ++q) rc = dalloc(h, &h->V0[q], fb);
-    for (int q = 0; q < 3 && !rc; ++q) rc = dalloc(h, &h->V1[q], fb);
     if (!rc && cudaStreamSynchronize(h->stream) != cudaSuccess) rc = FDTD_ERR_CUDA;
     if (rc) {
         fdtd_b200_adj_destroy(h);
@@ -1025,7 +986,10 @@ int fdtd_b200_adj_set_receivers(FdtdB200Adj* h, int n_rec, const int* idx8, cons
         dfree(h, t1);
         dfree(h, t2);
         dfree(h, t3);
+        void* t4 = h->tap_plane;
+        dfree(h, t4);
     }
+    h->tap_plane = nullptr;
     h->tap_cell = nullptr;
     h->tap_start = nullptr;
     h->tap_ord = nullptr;
@@ -1064,10 +1028,16 @@ int fdtd_b200_adj_set_receivers(FdtdB200Adj* h, int n_rec, const int* idx8, cons
         void* tc = nullptr;
         void* tsb = nullptr;
         void* to = nullptr;
+        void* tpl = nullptr;
+        std::vector<int> plane(h->g.nx + 1);
+        for (int i = 0; i <= h->g.nx; ++i)
+            plane[i] = (int)(std::lower_bound(cells.begin(), cells.end(), i * h->g.plane) - cells.begin());
         rc = dalloc(h, &tc, cells.size() * sizeof(long long));
         if (!rc) rc = dalloc(h, &tsb, start.size() * sizeof(int));
         if (!rc) rc = dalloc(h, &to, ord.size() * sizeof(int));
+        if (!rc) rc = dalloc(h, &tpl, plane.size() * sizeof(int));
         if (rc) return rc;
+        h->tap_plane = (int*)tpl;
         h->tap_cell = (long long*)tc;
         h->tap_start = (int*)tsb;
         h->tap_ord = (int*)to;
@@ -1076,6 +1046,7 @@ int fdtd_b200_adj_set_receivers(FdtdB200Adj* h, int n_rec, const int* idx8, cons
                             h->stream));
         ACK(cudaMemcpyAsync(h->tap_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice,
                             h->stream));
+        ACK(cudaMemcpyAsync(h->tap_plane, plane.data(), plane.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         ACK(cudaMemcpyAsync(h->tap_ord, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         ACK(cudaStreamSynchronize(h->stream));
     }
