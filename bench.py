@@ -810,7 +810,7 @@ def walled_arm(args):
                        "cells": cells, "plate_nodes": int(sc.kwargs()["plate_active"].sum())},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": f"{peak_kind} hbm_gbs",
-                         "kernel": "walled single pass (k_fused_step walls + plate faces + k_pressure_groups)",
+                         "kernel": "walled single pass (k_fused_step, walls and plate faces inside)",
                          "algorithmic_bytes_per_update": bpu},
             "kernels": rows, "clocks": clk.summary()}
     print(json.dumps(line), flush=True)

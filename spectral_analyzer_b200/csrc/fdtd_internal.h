@@ -80,12 +80,12 @@ struct PlateCoef {
     float bk;   // beta_K / dt * bh
 };
 
-// Extra jobs of the two-pass velocity pass for a plate scene (code null: none):
-// the plate's face velocities (w - w_prev)/dt on the Vz faces below (code bit 0)
-// and above (bit 1) each active node, which overwrite the updated faces as
-// k_plate_inject does; and, by the first block, the entries of the consumed
-// plate forces back to zero (pack/m, m = 0: none).  Both are skipped when the
-// gate reports a failed plate update.
+// A plate's part in the velocity update of both step kernels (code null: none):
+// the Vz faces below (code bit 0) and above (bit 1) each active node take the
+// plate's velocity (w - w_prev)/dt after their update, as in the reference; and,
+// in the two-pass kernel, the entries of the consumed plate forces go back to zero
+// (pack/m, m = 0: none).  Both are skipped when the gate reports a failed plate
+// update.
 struct PlateFaces {
     const uint8_t* code = nullptr;   // [Nx * Ny], node j + Ny * i
     const float* w = nullptr;
