@@ -522,6 +522,22 @@ bool use_fused(const AcousticFDTDState* st)
     return st->kernel_mode == 2 || (long long)st->N >= kWalledFusedCells;
 }
 
+// An open room's step taken in two passes: sizes between these stay in L2, where
+// the passes' 48 bytes a cell-update cost less than the march's pipeline fill.
+// Not when a kernel was asked for, or profiling or the load-hold hook names the
+// march.  Per step of a run with source and 4 receivers, march / two passes:
+// 112x104x108 21.5 / 13.8 us, 128^3 25.4 / 17.7, 160x128x112 25.9 / 19.0,
+// 160x160x144 40.0 / 28.6, 224x160x128 (4.59M cells) 40.4 / 38.7, 256x200x96 (4.92M)
+// 48.2 / 43.4, 224x192x128 (5.51M) 41.6 / 51.0.  A tick (deposit, step, samples):
+// 64^3 28.4 / 29.7 us, 87x61x109 33.1 / 30.4, 128^3 42.1 / 36.0.
+constexpr long long kOpenTwoPassFrom = 3LL << 17, kOpenTwoPassTo = 9LL << 19;
+
+bool open_two_pass(const AcousticFDTDState* st)
+{
+    return st->kernel_mode == 0 && !st->prof_on && st->hold_plane == kNoPlane && fused_eligible(st) &&
+           (long long)st->N >= kOpenTwoPassFrom && (long long)st->N < kOpenTwoPassTo;
+}
+
 int prof_begin(AcousticFDTDState* st, cudaEvent_t* e1)
 {
     *e1 = nullptr;
@@ -651,13 +667,13 @@ int substep_plate(AcousticFDTDState* st, int n_saddle, float* out);
 int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
 {
     cudaStream_t s = st->stream;
-    const bool fused = use_fused(st);
-    if (!fused)
+    const bool open2 = open_two_pass(st), fused = !open2 && use_fused(st);
+    if (!fused && !open2)
         if (int rc0 = flush_record(st)) return rc0;
     // point source: deposit s[n] before step n
     bool fuse_deposit = false;
     if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0 && st->ps_done_step != st->step_count) {
-        fuse_deposit = fused && st->ps.n == 1 && st->ps.divisor == 0;
+        fuse_deposit = (fused || open2) && st->ps.n == 1 && st->ps.divisor == 0;
         if (!fuse_deposit) {
             CK(launch_deposit(st->ps, st->d_ps_sig, st->step_count, 0.0f, st->P(), s));
             ++st->launches;
@@ -709,6 +725,22 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
         ++st->launches;
         st->cv ^= 1;
         if ((rc = prof_end(st, e1, fused_kernel_launches_per_step()))) return rc;
+    } else if (open2) {
+        StepExtras ex;
+        if (fuse_deposit) {
+            ex.cell = st->ps.idx[0];
+            ex.sig = st->d_ps_sig + st->step_count;
+        }
+        if (st->rec_pending >= 0) {
+            ex.n_rec = st->n_rec;
+            ex.idx = st->d_rec_idx;
+            ex.w = st->d_rec_w;
+            ex.row = st->d_trace + (size_t)st->rec_pending * st->n_rec;
+            st->rec_pending = -1;
+        }
+        CK(launch_open_step(st->g, st->cf, st->tb, st->P(), st->Pn(), st->V(0), st->V(1), st->V(2), ex, s));
+        st->launches += 2;
+        if ((rc = prof_end(st, e1, 2))) return rc;
     } else {
         CK(launch_velocity_general(st->g, st->cf, st->tb, st->P(), st->V(0), st->V(1), st->V(2),
                                    st->d_frac[0], st->d_frac[1], st->d_frac[2], st->d_walls, s));
@@ -725,7 +757,7 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
 
     // receivers
     if (st->n_rec > 0 && st->trace_len < st->trace_cap) {
-        if (fused && defer_record) {
+        if ((fused || open2) && defer_record) {
             st->rec_pending = st->trace_len;
         } else {
             CK(launch_wsum(st->P(), st->d_rec_idx, st->d_rec_w, st->n_rec, 8, 0,

@@ -77,16 +77,22 @@ constexpr int kCellThreads = 128;
 // then closed faces (fraction == 0) are zeroed (:1152-1154).  A thread handles
 // Vx(i+1/2,j,k), Vy(i,j+1/2,k) and Vz(i,j,k+1/2) of its four cells where they
 // exist; faces that do not exist (and the row padding) keep their stored zero.
+// OPEN: a room without walls or plate, with the step's extras (StepExtras).
+template <bool OPEN>
 __global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ vx,
     float* __restrict__ vy, float* __restrict__ vz, const float* __restrict__ fx,
     const float* __restrict__ fy, const float* __restrict__ fz, const uint8_t* __restrict__ walls,
-    const unsigned* __restrict__ gate, PlateFaces pf)
+    const unsigned* __restrict__ gate, PlateFaces pf, StepExtras ex)
 {
     // With a plate the kernel before this one is the plate update, which writes no
     // field: the loads start beside it and only the results wait for it.
-    if (!pf.code) wait_previous();
+    if (OPEN || !pf.code) wait_previous();
     release_next();
+    if constexpr (OPEN)
+        for (int r = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; r < ex.n_rec;
+             r += gridDim.x * gridDim.y * blockDim.x)
+            ex.row[r] = weighted_sum<8>(p, ex.idx + 8LL * r, ex.w + 8LL * r, 8, 0);
     GEN_INDEX
     // Every load first, from addresses kept inside the field (what a 2nd-order
     // face does not read is loaded and not used): the pass is bound by the latency
@@ -95,11 +101,11 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
     const long long xm = i > 0 ? id - g.plane : id, xp = i < g.nx - 1 ? id + g.plane : id;
     const long long xq = i < g.nx - 2 ? id + 2 * g.plane : id;
     const long long ym = j > 0 ? id - g.sz : id, yp = j < g.ny - 1 ? id + g.sz : id, yq = j < g.ny - 2 ? id + 2 * g.sz : id;
-    const unsigned wall = walls ? walls[id >> 2] : 0u;
-    const float4 p_c = ld4(p, id), p_xm = ld4(p, xm), p_xp = ld4(p, xp), p_xq = ld4(p, xq);
-    const float4 p_ym = ld4(p, ym), p_yp = ld4(p, yp), p_yq = ld4(p, yq);
-    const float p_zm = k0 > 0 ? p[id - 1] : 0.0f;
-    const float2 p_zp = k0 + 4 < g.nz ? *reinterpret_cast<const float2*>(p + id + 4) : make_float2(0.f, 0.f);
+    const unsigned wall = !OPEN && walls ? walls[id >> 2] : 0u;
+    float4 p_c = ld4(p, id), p_xm = ld4(p, xm), p_xp = ld4(p, xp), p_xq = ld4(p, xq);
+    float4 p_ym = ld4(p, ym), p_yp = ld4(p, yp), p_yq = ld4(p, yq);
+    float p_zm = k0 > 0 ? p[id - 1] : 0.0f;
+    float2 p_zp = k0 + 4 < g.nz ? *reinterpret_cast<const float2*>(p + id + 4) : make_float2(0.f, 0.f);
     const float4 v_x = ld4(vx, id), v_y = ld4(vy, id), v_z = ld4(vz, id);
     const float ay = __ldg(tb.ay + j), axi = __ldg(tb.ax + i);
     const float axr = __ldg(tb.ax + min(i + 1, g.nx - 1)), ayr = __ldg(tb.ay + min(j + 1, g.ny - 1));
@@ -110,9 +116,30 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
     if (wall & kWallX) f_x = ld4(fx, id);
     if (wall & kWallY) f_y = ld4(fy, id);
     if (wall & kWallZ) f_z = ld4(fz, id);
-    if (pf.code) wait_previous();
-    if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
-    if (pf.m > 0 && i == 0 && blockIdx.x == 0)               // the consumed plate forces
+    if constexpr (OPEN) {
+        // the source cell is within two cells of this group: every value read there
+        // takes the step's sample
+        if (ex.cell >= 0 && ex.cell >= id - 2 * g.plane && ex.cell < id + 2 * g.plane + 4) {
+            const float sv = *ex.sig;
+            if (sv != 0.0f) {
+                auto add = [&](float4& v, long long at) {
+                    const long long d = ex.cell - at;
+                    if (d == 0) v.x = fadd(v.x, sv);
+                    if (d == 1) v.y = fadd(v.y, sv);
+                    if (d == 2) v.z = fadd(v.z, sv);
+                    if (d == 3) v.w = fadd(v.w, sv);
+                };
+                add(p_c, id); add(p_xm, xm); add(p_xp, xp); add(p_xq, xq);
+                add(p_ym, ym); add(p_yp, yp); add(p_yq, yq);
+                if (ex.cell == id - 1) p_zm = fadd(p_zm, sv);
+                if (ex.cell == id + 4) p_zp.x = fadd(p_zp.x, sv);
+                if (ex.cell == id + 5) p_zp.y = fadd(p_zp.y, sv);
+            }
+        }
+    }
+    if (!OPEN && pf.code) wait_previous();
+    if (!OPEN && gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
+    if (!OPEN && pf.m > 0 && i == 0 && blockIdx.x == 0)               // the consumed plate forces
         for (int q = threadIdx.x; q < pf.m; q += min((int)blockDim.x, g.ny * nq_)) pf.ext[pf.pack[q].x] = 0.0f;
     float pc[4];
     unpack(p_c, pc);
@@ -159,7 +186,7 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
                                   fmaxf(fmaxf(axi, ay), az[q + 1]), fr[q]);
             if (k < g.nz - 1) v[q] = nv;
         }
-        if (pf.code && k0 <= pf.iz && pf.iz - 1 <= k0 + 3) {   // the plate's faces
+        if (!OPEN && pf.code && k0 <= pf.iz && pf.iz - 1 <= k0 + 3) {   // the plate's faces
             const int node = j + g.ny * i;
             const unsigned c = pf.code[node];
 #pragma unroll
@@ -178,30 +205,31 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_velocity_general(
 // is scaled by its open fraction; solid cells are skipped (they stay zero in
 // both pressure buffers, so the thread writes zero there).  Every load first, as
 // in the velocity pass; the fractions of a group near walls come after them.
+template <bool OPEN>
 __global__ void __launch_bounds__(kCellThreads, 6) k_pressure_general(
     Grid g, Coef cf, Tables tb, const float* __restrict__ p, float* __restrict__ pn,
     const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz,
     const float* __restrict__ fx, const float* __restrict__ fy, const float* __restrict__ fz,
     const uint8_t* __restrict__ solid, const uint8_t* __restrict__ walls, const unsigned* __restrict__ gate,
-    SubstepOut so)
+    SubstepOut so, StepExtras ex)
 {
     wait_previous();
     release_next();
-    if (so.status) {   // what the host waits for, straight into its memory
+    if (!OPEN && so.status) {   // what the host waits for, straight into its memory
         const int n_thr = gridDim.x * gridDim.y * blockDim.x;
         const int t = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
         for (int r = t; r < so.n; r += n_thr) so.out[r] = weighted_sum<4>(so.w, so.idx + 4LL * r, so.sw + 4LL * r, 4, 0);
         if (t < kStatusWords) so.h_status[t] = so.status[t];
     }
     GEN_INDEX
-    if (gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
+    if (!OPEN && gate && gate[kStatusPlate] != 0xFFFFFFFFu) return;   // this step's plate update failed
     const long long P = g.plane, S = g.sz;
     // faces outside the grid: the address stays inside, the value is zero
     const bool x0 = i < g.nx - 1, y0 = j < g.ny - 1;
     const bool x1 = i > 0, x2 = i > 1, x3 = i < g.nx - 2, y1 = j > 0, y2 = j > 1, y3 = j < g.ny - 2;
     const long long ixm = x1 ? id - P : id, ixmm = x2 ? id - 2 * P : id, ixpp = x3 ? id + P : id;
     const long long iym = y1 ? id - S : id, iymm = y2 ? id - 2 * S : id, iypp = y3 ? id + S : id;
-    const unsigned wall = walls ? walls[id >> 2] : 0u;
+    const unsigned wall = !OPEN && walls ? walls[id >> 2] : 0u;
     const float4 q_xp = ld4(vx, id), q_xm = ld4(vx, ixm), q_xpp = ld4(vx, ixpp), q_xmm = ld4(vx, ixmm);
     const float4 q_yp = ld4(vy, id), q_ym = ld4(vy, iym), q_ypp = ld4(vy, iypp), q_ymm = ld4(vy, iymm);
     const float4 q_z = ld4(vz, id);
@@ -217,6 +245,12 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_pressure_general(
     unpack(q_xp, xp); unpack(q_xm, xm); unpack(q_xpp, xpp); unpack(q_xmm, xmm);
     unpack(q_yp, yp); unpack(q_ym, ym); unpack(q_ypp, ypp); unpack(q_ymm, ymm);
     unpack(q_p, pc);
+    if (OPEN && ex.cell >= id && ex.cell < id + 4) {
+        const float sv = *ex.sig;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (ex.cell == id + q && sv != 0.0f) pc[q] = fadd(pc[q], sv);
+    }
     uint32_t sol = 0;
     if (wall & kWallNear) {   // elsewhere every fraction is 1
         auto scale = [&](float (&v)[4], const float* f, long long at) {
@@ -420,8 +454,8 @@ cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables&
 {
     dim3 block(kCellThreads, 1, 1);
     dim3 grid((g.ny * ((g.nz + 3) / 4) + kCellThreads - 1) / kCellThreads, g.nx, 1);
-    return launch_after(k_velocity_general, grid, block, 0, s, g, cf, tb, p, vx, vy, vz, fx, fy, fz, walls, gate,
-                        pf ? *pf : PlateFaces());
+    return launch_after(k_velocity_general<false>, grid, block, 0, s, g, cf, tb, p, vx, vy, vz, fx, fy, fz, walls, gate,
+                        pf ? *pf : PlateFaces(), StepExtras());
 }
 
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
@@ -432,8 +466,24 @@ cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables&
 {
     dim3 block(kCellThreads, 1, 1);
     dim3 grid((g.ny * ((g.nz + 3) / 4) + kCellThreads - 1) / kCellThreads, g.nx, 1);
-    return launch_after(k_pressure_general, grid, block, 0, s, g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid, walls,
-                        gate, so ? *so : SubstepOut());
+    return launch_after(k_pressure_general<false>, grid, block, 0, s, g, cf, tb, p, pn, vx, vy, vz, fx, fy, fz, solid,
+                        walls, gate, so ? *so : SubstepOut(), StepExtras());
+}
+
+cudaError_t launch_open_step(const Grid& g, const Coef& cf, const Tables& tb, const float* p, float* pn, float* vx,
+                             float* vy, float* vz, const StepExtras& ex, cudaStream_t s)
+{
+    dim3 block(kCellThreads, 1, 1);
+    dim3 grid((g.ny * ((g.nz + 3) / 4) + kCellThreads - 1) / kCellThreads, g.nx, 1);
+    const float* none = nullptr;
+    const uint8_t* no_walls = nullptr;
+    const unsigned* no_gate = nullptr;
+    const cudaError_t e = launch_after(k_velocity_general<true>, grid, block, 0, s, g, cf, tb, p, vx, vy, vz, none, none,
+                                       none, no_walls, no_gate, PlateFaces(), ex);
+    if (e != cudaSuccess) return e;
+    return launch_after(k_pressure_general<true>, grid, block, 0, s, g, cf, tb, p, pn, (const float*)vx,
+                        (const float*)vy, (const float*)vz, none, none, none, no_walls, no_walls, no_gate, SubstepOut(),
+                        ex);
 }
 
 cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const long long* above,

@@ -97,6 +97,19 @@ struct PlateFaces {
     int m = 0;
 };
 
+// What an open room's step carries besides the update (two-pass kernels): the
+// step's sample added to the source cell as it is read (cell < 0: none; the
+// pressure read stays as it is in memory), and the receivers of the step before,
+// recorded from the pressure read (n_rec 0: none).
+struct StepExtras {
+    long long cell = -1;
+    const float* sig = nullptr;   // the step's sample
+    int n_rec = 0;
+    const long long* idx = nullptr;
+    const float* w = nullptr;
+    float* row = nullptr;
+};
+
 // What a substep hands back, written by its pressure pass into pinned host
 // memory: 4-tap sums over the plate's new displacement and the status words.
 struct SubstepOut {
@@ -177,6 +190,9 @@ cudaError_t launch_velocity_general(const Grid& g, const Coef& cf, const Tables&
                                     const float* fx, const float* fy, const float* fz, const uint8_t* walls,
                                     cudaStream_t s, const unsigned* gate = nullptr,
                                     const PlateFaces* pf = nullptr);
+// an open room's step in two passes
+cudaError_t launch_open_step(const Grid& g, const Coef& cf, const Tables& tb, const float* p, float* pn, float* vx,
+                             float* vy, float* vz, const StepExtras& ex, cudaStream_t s);
 cudaError_t launch_pressure_general(const Grid& g, const Coef& cf, const Tables& tb,
                                     const float* p, float* pn, const float* vx, const float* vy,
                                     const float* vz, const float* fx, const float* fy,
