@@ -224,9 +224,11 @@ FDTD_B200_API int fdtd_b200_step_async(AcousticFDTDState* st, int n_steps);
  * by an async step) or FDTD_ERR_CUDA.  Clears the latch. */
 FDTD_B200_API int fdtd_b200_synchronize(AcousticFDTDState* st);
 
-/* Step-kernel selection: 0 automatic (fused single pass for open rooms and
- * for walled scenes of at least 5.0M (19 * 2^18) cells, two-pass for smaller walled
- * scenes), 1 two-pass, 2 fused.  Walled scenes (solid cells, face fractions,
+/* Step-kernel selection: 0 automatic (open rooms: many steps per launch on chip
+ * for small ones, two passes over L2 for the next, the fused single pass for large
+ * ones; walled scenes: the single pass from 5.0M (19 * 2^18) cells on, two-pass
+ * below), 1 two-pass, 2 fused.  All give the same bits; fdtd_b200_get_kernel says
+ * 2 for every open room on automatic.  Walled scenes (solid cells, face fractions,
  * an active plate) run the single pass with the walled rules; both kernels
  * give the same results bit for bit.  FDTD_ERR_ARG for 2 when the row
  * padding does not allow the single pass. */
