@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(TJ * LW) k_fused16(F16Args a, const __grid_con
     float h_d = 1.0f;
     if (h_ok) h_d = damp(fmaxf(ay_s[h_j + 2], az_s[h_c]), fmaxf(ay_s[h_j + 2], az_s[h_c + 1]), cf.dt);
     const int h_p = (h_j + 3) * C::PC + h_c + 4, h_v = h_j * C::PC + h_c + 4;        // element cols: k = k0-8+col
-    int dep_u = -1, dep_at = 0;
+    int dep_u = kNoPlane, dep_at = 0;
     if (a.dep_amp != 0.0f && tid == 0) {
         const int dj = a.dep_j - (j0 - 3), dk = a.dep_k - (k0 - 8);
         if (dj >= 0 && dj < C::PR && dk >= 0 && dk < C::PC) {

@@ -247,8 +247,10 @@ struct XPeers {
 // %globaltimer clock) and, as a backstop, a poll count.
 constexpr unsigned kWaitUs = 2000000u;   // 2 s; a load lands in microseconds
 constexpr int kWaitPolls = 1 << 26;
-// "no plane": plane indices of a march start at -3 (halo planes below i = 0)
+// "no plane": plane indices of a march start at -3 (halo planes below i = 0), so
+// a sentinel that a march compares with its plane must lie below them
 constexpr int kNoPlane = -(1 << 30);
+static_assert(kNoPlane < -3, "a march visits the planes from -3 on");
 
 struct FusedArgs {
     Grid g;

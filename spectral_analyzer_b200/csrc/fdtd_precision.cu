@@ -421,7 +421,7 @@ int fused16_step(FdtdB200Prec* p)
     a.sp = Sc{P.scale, P.inv_scale, P.lo_scale, P.inv_lo_scale};
     a.sv = Sc{vin[0].scale, vin[0].inv_scale, vin[0].lo_scale, vin[0].inv_lo_scale};
     a.dep_amp = 0.0f;
-    a.dep_i = -1000;
+    a.dep_i = kNoPlane;
     if (p->src >= 0 && p->step < p->n_sig) {
         a.dep_amp = (float)p->h_sig[p->step];
         a.dep_i = (int)(p->src / g.plane);
