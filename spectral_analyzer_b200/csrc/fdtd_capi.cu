@@ -514,6 +514,10 @@ bool fused_walled_ok(const AcousticFDTDState* st)
 // 256x200x128 94 / 73.5, 300x240x160 158 / 132).
 constexpr long long kWalledFusedCells = 19LL << 18;
 
+// The two-pass kernels put a plane in each row of blocks, of which a grid has at
+// most 65535; the march's grid has no such limit.  A longer room takes the march.
+constexpr int kTwoPassPlanes = 65535;
+
 bool use_fused(const AcousticFDTDState* st)
 {
     if (st->kernel_mode == 1) return false;
@@ -535,7 +539,7 @@ constexpr long long kOpenTwoPassFrom = 3LL << 17, kOpenTwoPassTo = 9LL << 19;
 bool open_two_pass(const AcousticFDTDState* st)
 {
     return st->kernel_mode == 0 && !st->prof_on && st->hold_plane == kNoPlane && fused_eligible(st) &&
-           (long long)st->N >= kOpenTwoPassFrom && (long long)st->N < kOpenTwoPassTo;
+           (long long)st->N >= kOpenTwoPassFrom && (long long)st->N < kOpenTwoPassTo && st->Nx <= kTwoPassPlanes;
 }
 
 int prof_begin(AcousticFDTDState* st, cudaEvent_t* e1)

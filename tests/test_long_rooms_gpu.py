@@ -1,0 +1,44 @@
+"""Rooms with more planes than a grid has rows of blocks (65535): they step on the
+single pass, whose grid counts tiles and segments, whichever kernel their size
+alone would choose.  Bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal, first_mismatch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    return torch
+
+
+# open: of a size that takes the two passes when it is not this long
+@pytest.mark.parametrize("dims,wall,kernel", [((70000, 4, 4), False, "auto"), ((65536, 3, 5), False, "auto")])
+def test_more_planes_than_rows_of_blocks(cuda, dims, wall, kernel):
+    from oracle import OracleFDTD
+    from spectral_analyzer_b200 import AcousticFDTD
+    nx, ny, nz = dims
+    flat = lambda i, j, k: k + nz * (j + ny * i)
+    ct = np.zeros(nx * ny * nz, np.uint8)
+    if wall:
+        ct[[flat(3, 1, 1), flat(65534, 2, 3), flat(nx - 4, 1, 2)]] = 1
+    kw = dict(Nx=nx, Ny=ny, Nz=nz, dx=0.01, c=343.0, rho_air=1.21, cell_type=ct, plate_iz=-1,
+              plate_active=np.zeros(nx * ny, np.uint8), n_pml=2)
+    f, o = AcousticFDTD(**kw), OracleFDTD(**kw)
+    f.set_kernel(kernel)
+    for s in (f, o):
+        for i in (5, 65533, nx - 6):
+            s.add_pressure(flat(i, 1, 2), 1.0 + i % 3)
+        for _ in range(3):
+            s.step(1)
+    f.step(4)
+    for _ in range(4):
+        o.step(1)
+    for name in ("get_pressure_field", "get_velocity_x", "get_velocity_y", "get_velocity_z"):
+        x, y = np.asarray(getattr(f, name)()).ravel(), np.asarray(getattr(o, name)()).ravel()
+        assert np.abs(y[-ny * nz * 40:]).max() > 0 and bits_equal(x, y), (name, first_mismatch(x, y))
