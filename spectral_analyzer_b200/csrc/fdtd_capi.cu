@@ -523,7 +523,7 @@ bool use_fused(const AcousticFDTDState* st)
     if (st->kernel_mode == 1) return false;
     if (fused_eligible(st)) return true;
     if (!fused_walled_ok(st)) return false;
-    return st->kernel_mode == 2 || (long long)st->N >= kWalledFusedCells;
+    return st->kernel_mode == 2 || (long long)st->N >= kWalledFusedCells || st->Nx > kTwoPassPlanes;
 }
 
 // An open room's step taken in two passes: sizes between these stay in L2, where

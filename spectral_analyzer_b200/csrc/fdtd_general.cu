@@ -290,12 +290,18 @@ __global__ void __launch_bounds__(kCellThreads, 6) k_pressure_general(
 }
 
 // WallCode bytes: the group's own faces and cells, then (after a launch boundary)
-// what its pressure update reads around it.
+// what its pressure update reads around it.  One dimension of blocks over all
+// groups, the rows' padding included (code 0): any extent of a room.
+#define WALL_INDEX                                                         \
+    const long long id = 4 * (blockIdx.x * 256LL + threadIdx.x);           \
+    if (id >= g.cells) return;                                             \
+    const int i = (int)(id / g.plane), r_ = (int)(id - i * g.plane);       \
+    const int j = r_ / g.sz, k0 = r_ - j * g.sz;
 __global__ void __launch_bounds__(256) k_wall_own(Grid g, const float* __restrict__ fx, const float* __restrict__ fy,
                                                   const float* __restrict__ fz, const uint8_t* __restrict__ solid,
                                                   uint8_t* __restrict__ code)
 {
-    GEN_INDEX
+    WALL_INDEX
     unsigned c = 0;
     for (int q = 0; q < 4; ++q) {
         const int k = k0 + q;
@@ -309,7 +315,8 @@ __global__ void __launch_bounds__(256) k_wall_own(Grid g, const float* __restric
 }
 __global__ void __launch_bounds__(256) k_wall_near(Grid g, uint8_t* code)
 {
-    GEN_INDEX
+    WALL_INDEX
+    if (k0 >= g.nz) return;
     unsigned c = code[id >> 2], near = c & (kWallX | kWallY | kWallZ | kWallSolid);
     for (int d = -2; d <= 1; ++d) {
         if (i + d >= 0 && i + d < g.nx) near |= code[(id + d * g.plane) >> 2] & kWallX;
@@ -499,10 +506,9 @@ cudaError_t launch_plate_step(int n_act, const int* act, const int* nb13, const 
 cudaError_t launch_wall_codes(const Grid& g, const float* fx, const float* fy, const float* fz, const uint8_t* solid,
                               uint8_t* code, cudaStream_t s)
 {
-    dim3 block(256, 1, 1);
-    dim3 grid((g.ny * ((g.nz + 3) / 4) + 255) / 256, g.nx, 1);
-    k_wall_own<<<grid, block, 0, s>>>(g, fx, fy, fz, solid, code);
-    k_wall_near<<<grid, block, 0, s>>>(g, code);
+    const unsigned grid = (unsigned)((g.cells / 4 + 255) / 256);
+    k_wall_own<<<grid, 256, 0, s>>>(g, fx, fy, fz, solid, code);
+    k_wall_near<<<grid, 256, 0, s>>>(g, code);
     return cudaGetLastError();
 }
 

@@ -1,6 +1,7 @@
 """Rooms with more planes than a grid has rows of blocks (65535): they step on the
 single pass, whose grid counts tiles and segments, whichever kernel their size
-alone would choose.  Bit for bit against the oracle."""
+alone would choose, and walled ones get their wall codes.  Bit for bit against the
+oracle."""
 import numpy as np
 import pytest
 
@@ -17,8 +18,12 @@ def cuda():
     return torch
 
 
-# open: of a size that takes the two passes when it is not this long
-@pytest.mark.parametrize("dims,wall,kernel", [((70000, 4, 4), False, "auto"), ((65536, 3, 5), False, "auto")])
+# open: of a size that takes the two passes when it is not this long; walled:
+# below and above the number of cells from which the single pass is automatic
+@pytest.mark.parametrize("dims,wall,kernel", [
+    ((70000, 4, 4), False, "auto"), ((65536, 3, 5), False, "auto"), ((66000, 4, 4), True, "fused"),
+    ((66000, 4, 4), True, "auto"), ((70000, 8, 8), True, "auto"),
+])
 def test_more_planes_than_rows_of_blocks(cuda, dims, wall, kernel):
     from oracle import OracleFDTD
     from spectral_analyzer_b200 import AcousticFDTD
