@@ -242,10 +242,9 @@ __global__ void k_src_rec(Field p, long long src, const double* sig, int step, i
 template <int M, class T>
 __global__ void __launch_bounds__(256) k_flat(Grid g, Field f, T* __restrict__ out)
 {
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= g.nz || j >= g.ny) return;
-    const long long row = (long long)i * g.ny + j;
-    out[row * g.nz + k] = (T)ld<M>(f, row * g.sz + k);
+    const long long q = blockIdx.x * 256LL + threadIdx.x, row = q / g.nz;   // one dimension: any extent of a room
+    if (row >= (long long)g.nx * g.ny) return;
+    out[q] = (T)ld<M>(f, row * g.sz + (q - row * g.nz));
 }
 
 }  // namespace prec
@@ -726,7 +725,7 @@ int fdtd_b200_prec_get_pressure(FdtdB200Prec* p, double* out, int out_len)
         PCK(cudaMalloc(&p->d_flat, n * vb));
         p->allocs.push_back(p->d_flat);
     }
-    const dim3 block(32, 8, 1), grid((p->g.nz + 31) / 32, (p->g.ny + 7) / 8, p->g.nx);
+    const unsigned block = 256, grid = (unsigned)((n + block - 1) / block);
     switch (p->mode) {
         case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
         case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, (double*)p->d_flat); break;
