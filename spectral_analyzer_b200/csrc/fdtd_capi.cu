@@ -1228,6 +1228,10 @@ AcousticFDTDState* create_impl(int Nx, int Ny, int Nz, float dx, float c, float 
                 code[st->h_act[q]] = (uint8_t)((vzb[q] >= 0 ? 1 : 0) | (vza[q] >= 0 ? 2 : 0));
             CKN(cudaMalloc(&st->d_plate_code, code.size()));
             CKN(cudaMemcpy(st->d_plate_code, code.data(), code.size(), cudaMemcpyHostToDevice));
+            if (!st->d_walls) {   // a plate of cells that are not solid: no fractions, but the march reads the codes
+                CKN(cudaMalloc(&st->d_walls, (size_t)st->g.cells / 4));
+                CKN(cudaMemset(st->d_walls, 0, (size_t)st->g.cells / 4));
+            }
         }
     }
 

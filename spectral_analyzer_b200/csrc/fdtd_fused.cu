@@ -696,12 +696,9 @@ __device__ __forceinline__ bool fused_tile(const FusedArgs& a, const CUtensorMap
                         }
                         vh = vupd(cf, vzs[h_v], gr, dmp);
                         if constexpr (WALLS) {
-                            if (a.fr[2]) {
-                                const float fz = pf_h;
-                                if (fz == 0.0f) vh = 0.0f;
-                                if (pl_hc) vh = plate_face(vh, h_k, pl_hc, fmul(fsub(pl_hw, pl_hwp), a.plate.inv_dt));
-                                if (a.frac_div) vh = fmul(vh, fz);
-                            }
+                            if (pf_h == 0.0f) vh = 0.0f;   // 1 without fractions
+                            if (pl_hc) vh = plate_face(vh, h_k, pl_hc, fmul(fsub(pl_hw, pl_hwp), a.plate.inv_dt));
+                            if (a.frac_div) vh = fmul(vh, pf_h);
                         }
                     }
                     vzn[h_v] = vh;

@@ -286,7 +286,7 @@ struct FusedArgs {
     const float* fr[3] = {nullptr, nullptr, nullptr};
     bool frac_div = false;
     const uint8_t* solid = nullptr;
-    const uint8_t* walls = nullptr;   // WallCode bytes (given with fractions or a mask)
+    const uint8_t* walls = nullptr;   // WallCode bytes (given with fractions, a mask or a plate)
     // Plate scenes: the velocities of the plate's faces (PlateFaces; code null:
     // none), and the status words: the step does nothing when this or an earlier
     // step's plate update failed.
