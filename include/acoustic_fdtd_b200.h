@@ -227,11 +227,14 @@ FDTD_B200_API int fdtd_b200_synchronize(AcousticFDTDState* st);
 /* Step-kernel selection: 0 automatic (open rooms: many steps per launch on chip
  * for small ones, two passes over L2 for the next, the fused single pass for large
  * ones; walled scenes: the single pass from 5.0M (19 * 2^18) cells on, two-pass
- * below), 1 two-pass, 2 fused.  All give the same bits; fdtd_b200_get_kernel says
- * 2 for every open room on automatic.  Walled scenes (solid cells, face fractions,
- * an active plate) run the single pass with the walled rules; both kernels
- * give the same results bit for bit.  FDTD_ERR_ARG for 2 when the row
- * padding does not allow the single pass. */
+ * below), 1 two-pass, 2 fused (calls of several steps of a small open room on chip,
+ * every other step in the single pass), 3 the march (every step in the single pass,
+ * one launch each).  All give the same bits.  fdtd_b200_get_kernel says 1 for a
+ * walled scene on the two-pass kernels or when these were asked for, 3 when the
+ * march was, else 2: an open room on automatic is 2 whatever its size.  Walled
+ * scenes (solid cells, face fractions, an active plate) run the single pass with
+ * the walled rules.  FDTD_ERR_ARG for 2 and 3 when the row padding does not allow
+ * the single pass. */
 FDTD_B200_API int fdtd_b200_set_kernel(AcousticFDTDState* st, int mode);
 FDTD_B200_API int fdtd_b200_get_kernel(const AcousticFDTDState* st);
 

@@ -523,7 +523,7 @@ bool use_fused(const AcousticFDTDState* st)
     if (st->kernel_mode == 1) return false;
     if (fused_eligible(st)) return true;
     if (!fused_walled_ok(st)) return false;
-    return st->kernel_mode == 2 || (long long)st->N >= kWalledFusedCells || st->Nx > kTwoPassPlanes;
+    return st->kernel_mode >= 2 || (long long)st->N >= kWalledFusedCells || st->Nx > kTwoPassPlanes;
 }
 
 // An open room's step taken in two passes: sizes between these stay in L2, where
@@ -776,12 +776,12 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
 
 // How many of the next `left` steps one launch of the resident kernel takes: an
 // open room that fits the chip, up to the next stability check; 0 = none
-// (another kernel was asked for, per-step profiling, the load-hold hook, a stream
-// being captured, more receivers than the kernel records, or no memory for its
-// buffers).
+// (the two-pass kernels or the march were asked for, per-step profiling, the
+// load-hold hook, a stream being captured, more receivers than the kernel records,
+// or no memory for its buffers).
 int resident_window(AcousticFDTDState* st, int left)
 {
-    if (st->kernel_mode == 1 || st->prof_on || st->hold_plane != kNoPlane || !fused_eligible(st)) return 0;
+    if (st->kernel_mode == 1 || st->kernel_mode == 3 || st->prof_on || st->hold_plane != kNoPlane || !fused_eligible(st)) return 0;
     if (!st->res_planned) {
         int sms = 0, coop = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, st->device);
@@ -1724,8 +1724,8 @@ int fdtd_b200_debug_hold_load(AcousticFDTDState* st, int plane, int wait_us)
 int fdtd_b200_set_kernel(AcousticFDTDState* st, int mode)
 {
     if (!st) return FDTD_ERR_NULL;
-    if (mode < 0 || mode > 2) return FDTD_ERR_ARG;
-    if (mode == 2 && !fused_eligible(st) && !fused_walled_ok(st)) return FDTD_ERR_ARG;
+    if (mode < 0 || mode > 3) return FDTD_ERR_ARG;
+    if (mode >= 2 && !fused_eligible(st) && !fused_walled_ok(st)) return FDTD_ERR_ARG;
     st->kernel_mode = mode;
     return FDTD_OK;
 }
@@ -1733,7 +1733,7 @@ int fdtd_b200_set_kernel(AcousticFDTDState* st, int mode)
 int fdtd_b200_get_kernel(const AcousticFDTDState* st)
 {
     if (!st) return FDTD_ERR_NULL;
-    return use_fused(st) ? 2 : 1;
+    return !use_fused(st) ? 1 : st->kernel_mode == 3 ? 3 : 2;
 }
 
 int fdtd_b200_device_fields(const AcousticFDTDState* st, void** out5)

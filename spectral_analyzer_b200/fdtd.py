@@ -372,12 +372,13 @@ class AcousticFDTD:
         self._check(self._lib.fdtd_b200_debug_hold_load(self._h, int(plane), int(wait_us)), "debug_hold_load")
 
     def set_kernel(self, mode: str):
-        m = {"auto": 0, "two_pass": 1, "fused": 2}[mode]
+        """"auto", "two_pass", "fused" (on chip or single pass) or "march" (single pass, a launch per step)."""
+        m = {"auto": 0, "two_pass": 1, "fused": 2, "march": 3}[mode]
         self._check(self._lib.fdtd_b200_set_kernel(self._h, m), "set_kernel")
 
     @property
     def kernel(self) -> str:
-        return {1: "two_pass", 2: "fused"}[self._lib.fdtd_b200_get_kernel(self._h)]
+        return {1: "two_pass", 2: "fused", 3: "march"}[self._lib.fdtd_b200_get_kernel(self._h)]
 
     @property
     def launch_count(self) -> int:
