@@ -247,6 +247,12 @@ FDTD_B200_API int fdtd_b200_get_kernel(const AcousticFDTDState* st);
  * until fdtd_reset; the CUDA context stays usable.  plane -1 turns it off. */
 FDTD_B200_API int fdtd_b200_debug_hold_load(AcousticFDTDState* st, int plane, int wait_us);
 
+/* Failure-path hook for tests: with on != 0 the cooperative launch that takes many
+ * steps of a small open room is refused by the driver (it asks for more blocks than
+ * a device can hold together, as in a context that owns few SMs); the room then
+ * steps on the other kernels for the rest of the handle's life. */
+FDTD_B200_API int fdtd_b200_debug_refuse_resident(AcousticFDTDState* st, int on);
+
 /* Device pointers of the current fields: out5 = {P (current), P (next), Vx, Vy, Vz}. */
 FDTD_B200_API int fdtd_b200_device_fields(const AcousticFDTDState* st, void** out5);
 

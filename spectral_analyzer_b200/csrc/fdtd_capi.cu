@@ -184,6 +184,7 @@ struct AcousticFDTDState {
 
     // many steps per launch of a small open room (fdtd_resident.cu)
     bool res_planned = false;
+    bool res_refuse = false;         // fdtd_b200_debug_refuse_resident
     ResPlan res;
     void* res_x = nullptr;           // exchange buffer between bricks
     unsigned res_epoch = 0;          // steps taken through it
@@ -796,7 +797,11 @@ int resident_window(AcousticFDTDState* st, int left)
     if (taps > (size_t)resident_max_taps()) return 0;
     // a captured launch would carry the same step numbers at every replay
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return 0;
+    if (cudaStreamIsCapturing(st->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return 0;
     // a single step gains nothing from staying on chip: loading and storing the
     // bricks costs about what the march does (64^3: 15.5 against 15.3 us per call)
     const int m = std::min(left, kCheckPeriod - (st->step_count & (kCheckPeriod - 1)));
@@ -825,8 +830,12 @@ int resident_window(AcousticFDTDState* st, int left)
 }
 
 // `m` steps (resident_window) in one launch: what m calls of one_step leave.
-int resident_steps(AcousticFDTDState* st, int m, bool sync_check)
+// *taken = 0 when the launch is refused (a context that owns fewer SMs than the
+// device, say, where not all bricks can be resident together): nothing has been
+// done, and the room steps on the other kernels from then on.
+int resident_steps(AcousticFDTDState* st, int m, bool sync_check, int* taken)
 {
+    *taken = m;
     cudaStream_t s = st->stream;
     if (int rc = flush_record(st)) return rc;
     if (st->ext_pending) clear_ext_host(st);   // consumed with no plate
@@ -837,6 +846,7 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check)
                 {st->v[st->cv ^ 1][0], st->v[st->cv ^ 1][1], st->v[st->cv ^ 1][2]},
                 st->d_status};
     a.wait_us = st->wait_us;
+    a.refuse = st->res_refuse;
     const int n0 = st->step_count;
     const int dep_from = st->ps_done_step == n0 ? 1 : 0;
     const int dep_to = st->ps.n > 0 ? std::min(m, st->ps_n - n0) : 0;
@@ -849,8 +859,13 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check)
         a.dep_k = (int)(c % st->g.sz);
     }
     const int rows = st->n_rec > 0 ? std::min(m, st->trace_cap - st->trace_len) : 0;
-    CK(launch_resident(a, st->res, m, st->res_x, st->res_epoch, dep_from, dep_to, st->d_rec_idx,
-                       rows > 0 ? 8 * st->n_rec : 0, rows, st->res_taps, s));
+    if (launch_resident(a, st->res, m, st->res_x, st->res_epoch, dep_from, dep_to, st->d_rec_idx,
+                        rows > 0 ? 8 * st->n_rec : 0, rows, st->res_taps, s) != cudaSuccess) {
+        cudaGetLastError();   // an error of an earlier launch comes back from the next one
+        st->res.ok = false;
+        *taken = 0;
+        return FDTD_OK;
+    }
     ++st->launches;
     if (rows > 0) {
         CK(launch_tap_rows(st->res_taps, st->d_rec_w, rows, st->n_rec, st->d_trace + (size_t)st->trace_len * st->n_rec, s));
@@ -1004,8 +1019,11 @@ int run_steps(AcousticFDTDState* st, int n_steps, bool sync_check)
             rc = plate_steps(st, n_steps - s, sync_check, &m);
         } else {
             m = resident_window(st, n_steps - s);
-            rc = m > 0 ? resident_steps(st, m, sync_check) : one_step(st, sync_check, true);
-            m = std::max(m, 1);
+            if (m > 0) rc = resident_steps(st, m, sync_check, &m);
+            if (m == 0) {
+                rc = one_step(st, sync_check, true);
+                m = 1;
+            }
         }
         s += m;
     }
@@ -1718,6 +1736,13 @@ int fdtd_b200_debug_hold_load(AcousticFDTDState* st, int plane, int wait_us)
     if (plane < -1 || plane >= st->Nx || wait_us < 0 || (unsigned)wait_us > kWaitUs) return FDTD_ERR_ARG;
     st->hold_plane = plane < 0 ? kNoPlane : plane;
     st->wait_us = wait_us > 0 ? (unsigned)wait_us : kWaitUs;
+    return FDTD_OK;
+}
+
+int fdtd_b200_debug_refuse_resident(AcousticFDTDState* st, int on)
+{
+    if (!st) return FDTD_ERR_NULL;
+    st->res_refuse = on != 0;
     return FDTD_OK;
 }
 

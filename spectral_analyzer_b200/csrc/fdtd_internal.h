@@ -268,6 +268,9 @@ struct FusedArgs {
     // wait_us microseconds and the kernel takes its timeout exit.
     int hold_plane = kNoPlane;
     unsigned wait_us = kWaitUs;
+    // Failure-path hook (fdtd_b200_debug_refuse_resident): the cooperative launch of
+    // launch_resident asks for more blocks than a device holds, and is refused.
+    bool refuse = false;
     // Fused point-source deposit (an open source cell): every CTA that loads
     // cell (dep_i, dep_j, dep_k) adds dep_sig[dep_step] to its shared-memory
     // copy of it when the plane arrives, so the step sees P^n plus the deposit

@@ -747,7 +747,7 @@ ResMap map_of(int L, int bi, int n_taps)
 }
 
 template <bool KEEP, class B>
-cudaError_t launch_of(ResArgs& a, int n_taps, cudaStream_t s)
+cudaError_t launch_of(ResArgs& a, int n_taps, bool refuse, cudaStream_t s)
 {
     static std::atomic<unsigned long long> ready{0};   // devices whose shared-memory limit is raised
     const void* const fn = (const void*)k_resident<KEEP, B>;
@@ -761,7 +761,7 @@ cudaError_t launch_of(ResArgs& a, int n_taps, cudaStream_t s)
     }
     a.m = map_of<B>(a.L, a.bi, n_taps);
     void* args[] = {&a};
-    const dim3 grid(a.nbi * a.nbj * a.nbk), block(kResThreads);
+    const dim3 grid(refuse ? 1u << 24 : a.nbi * a.nbj * a.nbk), block(kResThreads);
     return cudaLaunchCooperativeKernel(fn, grid, block, args, 4 * (size_t)a.m.total, s);
 }
 
@@ -857,7 +857,7 @@ cudaError_t launch_resident(const FusedArgs& f, const ResPlan& pl, int steps, vo
     cudaError_t e = cudaErrorInvalidValue;
     for_brick(pl.q, pl.bj, [&](auto B) {
         using T = decltype(B);
-        e = pl.L == 1 ? launch_of<true, T>(a, n_taps, s) : launch_of<false, T>(a, n_taps, s);
+        e = pl.L == 1 ? launch_of<true, T>(a, n_taps, f.refuse, s) : launch_of<false, T>(a, n_taps, f.refuse, s);
         return true;
     });
     return e;

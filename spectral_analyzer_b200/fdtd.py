@@ -371,6 +371,11 @@ class AcousticFDTD:
         (0: the normal bound); ``plane=-1`` turns it off."""
         self._check(self._lib.fdtd_b200_debug_hold_load(self._h, int(plane), int(wait_us)), "debug_hold_load")
 
+    def debug_refuse_resident(self, on: bool = True):
+        """Test hook: the launch that takes many steps of a small open room is
+        refused; the room steps on the other kernels from then on."""
+        self._check(self._lib.fdtd_b200_debug_refuse_resident(self._h, int(on)), "debug_refuse_resident")
+
     def set_kernel(self, mode: str):
         """"auto", "two_pass", "fused" (on chip or single pass) or "march" (single pass, a launch per step)."""
         m = {"auto": 0, "two_pass": 1, "fused": 2, "march": 3}[mode]

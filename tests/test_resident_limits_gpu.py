@@ -1,0 +1,58 @@
+"""Small rooms whose many-step launch cannot be had or does not finish: the calls
+step on the other kernels, or report a timeout, and the handle runs on."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal, first_mismatch
+from spectral_analyzer_b200.rooms import seeded_room
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    return torch
+
+
+def solver(room, kernel, capacity):
+    from spectral_analyzer_b200 import AcousticFDTD
+    f = AcousticFDTD(room.nx, room.ny, room.nz, room.dx, room.c, room.rho, cell_type=room.cell_type(), plate_iz=-1,
+                     plate_active=room.plate_active(), n_pml=room.n_pml)
+    f.set_kernel(kernel)
+    f.set_point_source(room.src_flat, room.signal())
+    f.set_receivers(*f.precompute_pressure_samplers(room.receiver_xyz()), capacity)
+    return f
+
+
+def near_room(dims, steps, seed):
+    room = seeded_room(*dims, steps, seed=seed, n_rec=3, n_pml=4, source_kind="gaussian")
+    room.receivers[0] = tuple(c + 2 for c in room.src)
+    return room
+
+
+def same(f, g):
+    tr = f.get_traces(), g.get_traces()
+    assert np.abs(tr[1]).max() > 0 and bits_equal(*tr)
+    for name in ("get_pressure_field", "get_velocity_x", "get_velocity_y", "get_velocity_z"):
+        x, y = getattr(f, name)(), getattr(g, name)()
+        assert bits_equal(x, y), (name, first_mismatch(x, y))
+
+
+@pytest.mark.parametrize("dims", [(40, 36, 44), (96, 80, 72)])   # then the march, and the two passes
+@pytest.mark.parametrize("asynchronous", [False, True])
+def test_refused_launch_steps_on_the_other_kernels(cuda, dims, asynchronous):
+    room = near_room(dims, 40, 7)
+    f, g = solver(room, "auto", 60), solver(room, "two_pass", 60)
+    f.step(9)                                          # one launch and its receivers' rows
+    assert f.launch_count == 2
+    f.debug_refuse_resident()
+    for n in (20, 3, 28):
+        l0 = f.launch_count
+        (f.step_async if asynchronous else f.step)(n)
+        assert f.launch_count - l0 > n
+    assert f.synchronize() == 0
+    g.step(60)
+    same(f, g)
