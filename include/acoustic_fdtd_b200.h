@@ -217,7 +217,10 @@ FDTD_B200_API int fdtd_b200_set_stream(AcousticFDTDState* st, void* stream);
 FDTD_B200_API void* fdtd_b200_get_stream(const AcousticFDTDState* st);
 
 /* Launches n_steps without waiting and without stopping at a failed stability
- * check; the first failure is latched and reported by fdtd_b200_synchronize. */
+ * check; the first failure is latched and reported by fdtd_b200_synchronize.
+ * A handle allocates the device buffers its steps work with on the first call
+ * that needs them: the second velocity set, and for calls of several steps of a
+ * small open room the exchange and tap buffers (at most 21 MB). */
 FDTD_B200_API int fdtd_b200_step_async(AcousticFDTDState* st, int n_steps);
 
 /* Waits for the handle's stream; returns FDTD_OK, FDTD_ERR_UNSTABLE (latched

@@ -188,8 +188,7 @@ struct AcousticFDTDState {
     ResPlan res;
     void* res_x = nullptr;           // exchange buffer between bricks
     unsigned res_epoch = 0;          // steps taken through it
-    float* res_taps = nullptr;       // the receivers' taps of up to kCheckPeriod steps
-    size_t res_taps_n = 0;
+    float* res_taps = nullptr;       // the receivers' taps of up to kCheckPeriod steps (behind it)
 
     long long launches = 0;          // kernels launched by this handle
 
@@ -806,25 +805,17 @@ int resident_window(AcousticFDTDState* st, int left)
     // bricks costs about what the march does (64^3: 15.5 against 15.3 us per call)
     const int m = std::min(left, kCheckPeriod - (st->step_count & (kCheckPeriod - 1)));
     if (m < 2) return 0;
-    if (!st->res_x) {
-        if (cudaMalloc(&st->res_x, st->res.xbytes) != cudaSuccess) {
+    if (!st->res_x) {   // both buffers once, in one allocation (at most 21 MB on 148 SMs), the taps' for the most receivers
+        const size_t xb = (st->res.xbytes + 255) & ~(size_t)255, tb = sizeof(float) * resident_max_taps() * kCheckPeriod;
+        if (cudaMalloc(&st->res_x, xb + tb) != cudaSuccess ||
+            cudaMemsetAsync(st->res_x, 0, st->res.xbytes, st->stream) != cudaSuccess) {
             cudaGetLastError();
+            cudaFree(st->res_x);
             st->res_x = nullptr;
             st->res.ok = false;
             return 0;
         }
-        if (cudaMemsetAsync(st->res_x, 0, st->res.xbytes, st->stream) != cudaSuccess) return 0;
-    }
-    if (taps * kCheckPeriod > st->res_taps_n) {
-        cudaStreamSynchronize(st->stream);
-        cudaFree(st->res_taps);
-        st->res_taps = nullptr;
-        st->res_taps_n = 0;
-        if (cudaMalloc(&st->res_taps, taps * kCheckPeriod * sizeof(float)) != cudaSuccess) {
-            cudaGetLastError();
-            return 0;
-        }
-        st->res_taps_n = taps * kCheckPeriod;
+        st->res_taps = reinterpret_cast<float*>(static_cast<char*>(st->res_x) + xb);
     }
     return m;
 }
@@ -1063,7 +1054,6 @@ void free_state(AcousticFDTDState* st)
     for (cudaEvent_t e : st->prof.ev) cudaEventDestroy(e);
     fused_cache_destroy(st->fcache);
     cudaFree(st->res_x);
-    cudaFree(st->res_taps);
     if (st->own_stream) cudaStreamDestroy(st->own_stream);
     if (d >= 0 && d != st->device) cudaSetDevice(d);
     delete st;

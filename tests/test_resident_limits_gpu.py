@@ -56,3 +56,23 @@ def test_refused_launch_steps_on_the_other_kernels(cuda, dims, asynchronous):
     assert f.synchronize() == 0
     g.step(60)
     same(f, g)
+
+
+def test_async_steps_do_not_wait_when_receivers_grow(cuda):
+    """More receivers than before, then steps queued behind work that is still running."""
+    room = near_room((40, 36, 44), 30, 8)
+    f, g = solver(room, "auto", 60), solver(room, "two_pass", 60)
+    f.step(10)
+    g.step(10)
+    rng = np.random.default_rng(0)
+    xyz = np.concatenate([room.receiver_xyz(), rng.uniform(0, 30, (100, 3)).astype(np.float32)])
+    for h in (f, g):
+        h.set_receivers(*h.precompute_pressure_samplers(xyz), 60)
+    stream = f.torch_stream()
+    with cuda.cuda.stream(stream):
+        cuda.cuda._sleep(1_000_000_000)                # half a second
+    f.step_async(30)
+    assert not stream.query()
+    assert f.synchronize() == 0
+    g.step(30)
+    same(f, g)
