@@ -68,11 +68,12 @@ def test_async_steps_do_not_wait_when_receivers_grow(cuda):
     xyz = np.concatenate([room.receiver_xyz(), rng.uniform(0, 30, (100, 3)).astype(np.float32)])
     for h in (f, g):
         h.set_receivers(*h.precompute_pressure_samplers(xyz), 60)
-    stream = f.torch_stream()
-    with cuda.cuda.stream(stream):
+    done = cuda.cuda.Event()
+    with cuda.cuda.stream(f.torch_stream()):
         cuda.cuda._sleep(1_000_000_000)                # half a second
+        done.record()
     f.step_async(30)
-    assert not stream.query()
+    assert not done.query()
     assert f.synchronize() == 0
     g.step(30)
     same(f, g)
