@@ -250,6 +250,13 @@ FDTD_B200_API int fdtd_b200_get_kernel(const AcousticFDTDState* st);
  * until fdtd_reset; the CUDA context stays usable.  plane -1 turns it off. */
 FDTD_B200_API int fdtd_b200_debug_hold_load(AcousticFDTDState* st, int plane, int wait_us);
 
+/* The same hook for the kernel that takes many steps of a small open room in one
+ * launch: its brick `brick` (0 .. bricks-1, FDTD_ERR_ARG beyond or when the room
+ * does not fit the chip) publishes nothing from the next such launch on, so the
+ * bricks beside it give up after `wait_us` microseconds (0: the normal bound) and
+ * all others with them; reported and cleared as above.  brick -1 turns it off. */
+FDTD_B200_API int fdtd_b200_debug_hold_brick(AcousticFDTDState* st, int brick, int wait_us);
+
 /* Failure-path hook for tests: with on != 0 the cooperative launch that takes many
  * steps of a small open room is refused by the driver (it asks for more blocks than
  * a device can hold together, as in a context that owns few SMs); the room then

@@ -65,6 +65,7 @@ SIGNATURES = {
     "fdtd_b200_synchronize": (i32, [vp]),
     "fdtd_b200_set_kernel": (i32, [vp, i32]),
     "fdtd_b200_debug_hold_load": (i32, [vp, i32, i32]),
+    "fdtd_b200_debug_hold_brick": (i32, [vp, i32, i32]),
     "fdtd_b200_debug_refuse_resident": (i32, [vp, i32]),
     "fdtd_b200_get_kernel": (i32, [vp]),
     "fdtd_b200_device_fields": (i32, [vp, C.POINTER(vp)]),

@@ -185,6 +185,7 @@ struct AcousticFDTDState {
     // many steps per launch of a small open room (fdtd_resident.cu)
     bool res_planned = false;
     bool res_refuse = false;         // fdtd_b200_debug_refuse_resident
+    int hold_brick = -1;             // fdtd_b200_debug_hold_brick
     ResPlan res;
     void* res_x = nullptr;           // exchange buffer between bricks
     unsigned res_epoch = 0;          // steps taken through it
@@ -774,6 +775,19 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
     return step_check(st, sync_check);
 }
 
+// Whether the resident kernel's bricks hold the room (planned once).
+bool resident_ok(AcousticFDTDState* st)
+{
+    if (!st->res_planned) {
+        int sms = 0, coop = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, st->device);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, st->device);
+        if (coop) st->res = resident_plan(st->g, sms);
+        st->res_planned = true;
+    }
+    return st->res.ok;
+}
+
 // How many of the next `left` steps one launch of the resident kernel takes: an
 // open room that fits the chip, up to the next stability check; 0 = none
 // (the two-pass kernels or the march were asked for, per-step profiling, the
@@ -782,14 +796,7 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
 int resident_window(AcousticFDTDState* st, int left)
 {
     if (st->kernel_mode == 1 || st->kernel_mode == 3 || st->prof_on || st->hold_plane != kNoPlane || !fused_eligible(st)) return 0;
-    if (!st->res_planned) {
-        int sms = 0, coop = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, st->device);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, st->device);
-        if (coop) st->res = resident_plan(st->g, sms);
-        st->res_planned = true;
-    }
-    if (!st->res.ok) return 0;
+    if (!resident_ok(st)) return 0;
     if (st->ps_n > 0 && st->ps.n > 0 && (st->ps.n != 1 || st->ps.divisor != 0)) return 0;
     const bool record = st->n_rec > 0 && st->trace_len < st->trace_cap;
     const size_t taps = record ? (size_t)8 * st->n_rec : 0;
@@ -838,6 +845,7 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check, int* taken)
                 st->d_status};
     a.wait_us = st->wait_us;
     a.refuse = st->res_refuse;
+    a.hold_brick = st->hold_brick;
     const int n0 = st->step_count;
     const int dep_from = st->ps_done_step == n0 ? 1 : 0;
     const int dep_to = st->ps.n > 0 ? std::min(m, st->ps_n - n0) : 0;
@@ -1725,6 +1733,16 @@ int fdtd_b200_debug_hold_load(AcousticFDTDState* st, int plane, int wait_us)
     if (!st) return FDTD_ERR_NULL;
     if (plane < -1 || plane >= st->Nx || wait_us < 0 || (unsigned)wait_us > kWaitUs) return FDTD_ERR_ARG;
     st->hold_plane = plane < 0 ? kNoPlane : plane;
+    st->wait_us = wait_us > 0 ? (unsigned)wait_us : kWaitUs;
+    return FDTD_OK;
+}
+
+int fdtd_b200_debug_hold_brick(AcousticFDTDState* st, int brick, int wait_us)
+{
+    if (!st) return FDTD_ERR_NULL;
+    if (brick < -1 || wait_us < 0 || (unsigned)wait_us > kWaitUs) return FDTD_ERR_ARG;
+    if (brick >= 0 && (!resident_ok(st) || brick >= st->res.nbi * st->res.nbj * st->res.nbk)) return FDTD_ERR_ARG;
+    st->hold_brick = brick;
     st->wait_us = wait_us > 0 ? (unsigned)wait_us : kWaitUs;
     return FDTD_OK;
 }

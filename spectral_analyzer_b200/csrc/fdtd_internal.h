@@ -271,6 +271,9 @@ struct FusedArgs {
     // Failure-path hook (fdtd_b200_debug_refuse_resident): the cooperative launch of
     // launch_resident asks for more blocks than a device holds, and is refused.
     bool refuse = false;
+    // Failure-path hook (fdtd_b200_debug_hold_brick): this brick of launch_resident
+    // publishes nothing, so its neighbours' waits run out after wait_us microseconds.
+    int hold_brick = -1;
     // Fused point-source deposit (an open source cell): every CTA that loads
     // cell (dep_i, dep_j, dep_k) adds dep_sig[dep_step] to its shared-memory
     // copy of it when the plane arrives, so the step sees P^n plus the deposit

@@ -117,6 +117,7 @@ struct ResArgs {
     float* vout[3];
     unsigned* status;
     unsigned wait_us;
+    int hold_brick;                    // publishes nothing (-1: none)
     int L, bi;                         // planes per thread, planes of a brick
     int nbi, nbj, nbk;                 // bricks
     ResMap m;
@@ -520,10 +521,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             }
         }
     };
-    // P of the own cells of plane l, published when another step follows;
+    // P of the own cells of plane l, published (post) when another step follows;
     // x0 .. x3 = Vx of faces l-2 .. l+1, mpz = min of the y and z dampings
     auto own_p = [&](int l, auto tests, const float (&x0)[4], const float (&x1)[4], const float (&x2)[4],
-                     const float (&x3)[4], const float (&mpz)[4], uint4* box, unsigned tag, bool more, float amp) {
+                     const float (&x3)[4], const float (&mpz)[4], uint4* box, unsigned tag, bool post, float amp) {
         constexpr bool T = decltype(tests)::value;
         const float* const yl = sm + yc + l * PY;
         const float* const zl = sm + zc + l * PZ;
@@ -565,7 +566,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             for (int t = 0; t < 4; ++t) P[t] = n[t];
         }
         put4(sm + pc + l * PP, n);
-        if (more) {
+        if (post) {
             uint4* const dx = box + 2 * (rx0 + l * BJ * Q);
             uint4* const dy = box + 2 * (ry0 + l * 3 * Q);
             uint4* const dz = box + 2 * (rz0 + l * BJ);
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             post4(pub & 8u, dz + 2 * FZ, n, tag);
         }
     };
-    auto own_ps = [&](auto tests, uint4* box, unsigned tag, bool more, float amp) {
+    auto own_ps = [&](auto tests, uint4* box, unsigned tag, bool post, float amp) {
         float mpz[4], x0[4], x1[4], x2[4], x3[4];
         get4(sm + xc - 2 * PX, x0);
         get4(sm + xc - PX, x1);
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
             get4(sm + xc + PX, x3);
 #pragma unroll
             for (int t = 0; t < 4; ++t) x2[t] = VX[t];
-            own_p(0, tests, x0, x1, x2, x3, mpz, box, tag, more, amp);
+            own_p(0, tests, x0, x1, x2, x3, mpz, box, tag, post, amp);
         } else {
             const float py = pys[lj];
             get4(pzs + 4 * qq, mpz);
@@ -595,7 +596,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
 #pragma unroll 1
             for (int l = 0; l < nl; ++l) {
                 get4(sm + xc + (l + 1) * PX, x3);
-                own_p(l, tests, x0, x1, x2, x3, mpz, box, tag, more, amp);
+                own_p(l, tests, x0, x1, x2, x3, mpz, box, tag, post, amp);
 #pragma unroll
                 for (int t = 0; t < 4; ++t) { x0[t] = x1[t]; x1[t] = x2[t]; x2[t] = x3[t]; }
             }
@@ -659,8 +660,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident(const __grid_consta
         const unsigned tag = a.epoch + (unsigned)s + 1u;
         if (nl > 0) {
             uint4* const box = mine + (s & 1 ? parity : 0);
-            if (fast) own_ps(std::false_type{}, box, tag, more, amp);
-            else own_ps(std::true_type{}, box, tag, more, amp);
+            const bool post = more && b != a.hold_brick;
+            if (fast) own_ps(std::false_type{}, box, tag, post, amp);
+            else own_ps(std::true_type{}, box, tag, post, amp);
         }
         // ---- the neighbours' layers into the halo: all of a thread's records in
         // flight together, polled until each carries this step's number
@@ -844,6 +846,7 @@ cudaError_t launch_resident(const FusedArgs& f, const ResPlan& pl, int steps, vo
     for (int c = 0; c < 3; ++c) { a.vin[c] = f.vin[c]; a.vout[c] = f.vout[c]; }
     a.status = f.status;
     a.wait_us = f.wait_us;
+    a.hold_brick = f.hold_brick;
     a.L = pl.L; a.bi = pl.bi;
     a.nbi = pl.nbi; a.nbj = pl.nbj; a.nbk = pl.nbk;
     a.xbuf = static_cast<uint4*>(xbuf);

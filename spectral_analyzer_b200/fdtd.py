@@ -371,6 +371,12 @@ class AcousticFDTD:
         (0: the normal bound); ``plane=-1`` turns it off."""
         self._check(self._lib.fdtd_b200_debug_hold_load(self._h, int(plane), int(wait_us)), "debug_hold_load")
 
+    def debug_hold_brick(self, brick: int, wait_us: int = 0):
+        """Test hook: brick ``brick`` of a small room's many-step launch publishes
+        nothing, so its neighbours' bounded waits run out after ``wait_us``
+        microseconds (0: the normal bound); ``brick=-1`` turns it off."""
+        self._check(self._lib.fdtd_b200_debug_hold_brick(self._h, int(brick), int(wait_us)), "debug_hold_brick")
+
     def debug_refuse_resident(self, on: bool = True):
         """Test hook: the launch that takes many steps of a small open room is
         refused; the room steps on the other kernels from then on."""
