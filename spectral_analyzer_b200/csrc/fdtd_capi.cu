@@ -588,16 +588,24 @@ void report_unstable_cell(AcousticFDTDState* st, unsigned q)
 
 // The fused step reads one velocity set and writes the other (neighbouring
 // tiles recompute halo faces from the old values, so updates cannot be in
-// place).  Engine-owned fields get the second set on first use.
+// place).  Engine-owned fields get the second set on first use: all three arrays
+// or, when memory runs out, none.
 int alloc_second_velocity_set(AcousticFDTDState* st)
 {
-    const int b = st->cv ^ 1;
-    for (int c2 = 0; c2 < 3; ++c2) {
-        if (st->v[b][c2]) continue;
-        CK(cudaMalloc(&st->v[b][c2], st->field_bytes));
-        CK(cudaMemsetAsync(st->v[b][c2], 0, st->field_bytes, st->stream));
+    float** const v = st->v[st->cv ^ 1];
+    cudaError_t e = cudaSuccess;
+    for (int c2 = 0; c2 < 3 && e == cudaSuccess; ++c2) {
+        e = cudaMalloc(&v[c2], st->field_bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(v[c2], 0, st->field_bytes, st->stream);
     }
-    return FDTD_OK;
+    if (e == cudaSuccess) return FDTD_OK;
+    set_err(e, "second velocity set");
+    for (int c2 = 0; c2 < 3; ++c2) {
+        cudaFree(v[c2]);
+        v[c2] = nullptr;
+    }
+    cudaGetLastError();   // or the next launch would report it
+    return FDTD_ERR_CUDA;
 }
 
 // Records the receivers of the current pressure into the pending trace slot
@@ -828,17 +836,20 @@ int resident_window(AcousticFDTDState* st, int left)
 }
 
 // `m` steps (resident_window) in one launch: what m calls of one_step leave.
-// *taken = 0 when the launch is refused (a context that owns fewer SMs than the
-// device, say, where not all bricks can be resident together): nothing has been
-// done, and the room steps on the other kernels from then on.
+// *taken = 0, with nothing done, when there is no memory for the second velocity
+// set or the launch is refused (a context that owns fewer SMs than the device, say,
+// where not all bricks can be resident together; the room steps on the other
+// kernels from then on).
 int resident_steps(AcousticFDTDState* st, int m, bool sync_check, int* taken)
 {
     *taken = m;
     cudaStream_t s = st->stream;
     if (int rc = flush_record(st)) return rc;
     if (st->ext_pending) clear_ext_host(st);   // consumed with no plate
-    if (!st->v[st->cv ^ 1][0])
-        if (int rc = alloc_second_velocity_set(st)) return rc;
+    if (!st->v[st->cv ^ 1][0] && alloc_second_velocity_set(st) != FDTD_OK) {
+        *taken = 0;   // a room that steps in two passes needs no second set
+        return FDTD_OK;
+    }
     FusedArgs a{st->g, st->cf, st->tb, st->P(), st->Pn(),
                 {st->V(0), st->V(1), st->V(2)},
                 {st->v[st->cv ^ 1][0], st->v[st->cv ^ 1][1], st->v[st->cv ^ 1][2]},
