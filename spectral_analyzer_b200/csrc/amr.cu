@@ -41,6 +41,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -455,17 +456,15 @@ struct AcousticAMRState {
     // host copies used by set-up functions (double inputs, as the reference keeps them)
     std::vector<double> centers, volumes, open_vol, face_area, face_open, face_dist;
     std::vector<int> cell_type, face_neg, face_pos, acoustic;
-    std::vector<int> csr_start, csr_face;
-    std::vector<float> csr_w;
 
     // device
     float *d_p = nullptr, *d_v = nullptr, *d_vdamp = nullptr, *d_inv_d = nullptr;
-    float *d_pdamp = nullptr, *d_psrc = nullptr, *d_inv_den = nullptr, *d_scoef = nullptr;
+    float *d_pdamp = nullptr, *d_psrc = nullptr, *d_inv_den = nullptr;
     int *d_neg = nullptr, *d_pos = nullptr, *d_meta = nullptr, *d_slice = nullptr, *d_scell = nullptr;
     int2* d_inc = nullptr;
     unsigned* d_srow = nullptr;       // order 8: rows of d_soff / d_swgt per face
     int* d_soff = nullptr;
-    float* d_swgt = nullptr;
+    int *d_swgt = nullptr, *d_scoef = nullptr;   // bits of the weights
     double* d_centers = nullptr;
     unsigned char* d_open = nullptr;  // 1: an acoustic cell (a candidate of the nearest-cell search)
     double2* d_best = nullptr;        // nearest-cell search: a candidate per block, block counter, result
@@ -596,8 +595,17 @@ void fornberg_first(const float* x, int n, float xi, float* w)
     for (int k = 0; k < n; ++k) w[k] = c1[k];
 }
 
+// The incident faces of every cell, as k_amr_pressure reads them: {face, signed
+// flux weight} slot by slot per slice of 32 cells.
+struct Incidence {
+    std::vector<int> deg, slice;
+    std::unique_ptr<int2[]> e;
+    int2* of(int c) const { return e.get() + slice[c >> 5] + (c & 31); }   // slots 32 apart
+};
+
 struct Topo {
     const AcousticAMRState* st;
+    const Incidence* inc;
     std::vector<int> nb_pos[3], nb_neg[3];
 };
 
@@ -692,9 +700,12 @@ int walk_cells(const Topo& t, int seed, float face_proj, const float coord[3], c
     while (found < depth) {
         int best = -1;
         float best_dot = 0.5f;
-        for (int k = st->csr_start[cur]; k < st->csr_start[cur + 1]; ++k) {
-            const int fk = st->csr_face[k];
-            const float sg = (st->csr_w[k] > 0.f) ? +1.f : -1.f;
+        const int2* const e = t.inc->of(cur);
+        for (int k = 0; k < t.inc->deg[cur]; ++k) {
+            const int fk = e[32 * k].x;
+            float flux;
+            memcpy(&flux, &e[32 * k].y, 4);
+            const float sg = (flux > 0.f) ? +1.f : -1.f;
             const int a = st->face_neg[fk], b = st->face_pos[fk];
             const float dx = (float)(st->centers[3 * b] - st->centers[3 * a]);
             const float dy = (float)(st->centers[3 * b + 1] - st->centers[3 * a + 1]);
@@ -719,65 +730,12 @@ int walk_cells(const Topo& t, int seed, float face_proj, const float coord[3], c
     return found;
 }
 
-// Per face: with four cells on each side, Fornberg weights over all eight;
-// otherwise the two-cell difference (acoustic_amr.cpp:549-629).  Unused slots
-// keep cell 0 and weight 0.
-void build_stencil(AcousticAMRState* st, std::vector<int>& sc, std::vector<float>& sw)
-{
-    Topo t;
-    t.st = st;
-    build_axis_neighbours(t);
-    const int nf = st->n_faces;
-    sc.assign((size_t)nf * kSW2, 0);
-    sw.assign((size_t)nf * kSW2, 0.0f);
-    g_prog_total.store(nf);
-    g_prog_done.store(0);
-    g_prog_active.store(1);
-    for (int f = 0; f < nf; ++f) {
-        const int cn = st->face_neg[f], cp = st->face_pos[f];
-        const float dxf = (float)(st->centers[3 * cp] - st->centers[3 * cn]);
-        const float dyf = (float)(st->centers[3 * cp + 1] - st->centers[3 * cn + 1]);
-        const float dzf = (float)(st->centers[3 * cp + 2] - st->centers[3 * cn + 2]);
-        const float len = std::sqrt(dxf * dxf + dyf * dyf + dzf * dzf);
-        if (len >= 1e-15f) {
-            const float dir[3] = {dxf / len, dyf / len, dzf / len};
-            const float back[3] = {-dir[0], -dir[1], -dir[2]};
-            const float fp = 0.5f * (proj(st, cn, dir) + proj(st, cp, dir));
-            int nc_[kSW], pc_[kSW];
-            float nx_[kSW], px_[kSW];
-            const int nn = walk_cells(t, cn, fp, dir, back, kSW, nc_, nx_);
-            const int np = walk_cells(t, cp, fp, dir, dir, kSW, pc_, px_);
-            if (nn == kSW && np == kSW) {
-                float xs[kSW2], w[kSW2];
-                for (int k = 0; k < kSW; ++k) {
-                    xs[k] = nx_[kSW - 1 - k];
-                    xs[kSW + k] = px_[k];
-                }
-                fornberg_first(xs, kSW2, 0.0f, w);
-                for (int k = 0; k < kSW; ++k) {
-                    sc[(size_t)f * kSW2 + k] = nc_[k];          // walk order from the face outward
-                    sw[(size_t)f * kSW2 + k] = w[kSW - 1 - k];
-                    sc[(size_t)f * kSW2 + kSW + k] = pc_[k];
-                    sw[(size_t)f * kSW2 + kSW + k] = w[kSW + k];
-                }
-            } else if (nn + np >= 2) {
-                const float inv = st->face_dist[f] > 0.0 ? 1.0f / (float)st->face_dist[f] : 0.0f;
-                sc[(size_t)f * kSW2] = cn;
-                sw[(size_t)f * kSW2] = -inv;
-                sc[(size_t)f * kSW2 + kSW] = cp;
-                sw[(size_t)f * kSW2 + kSW] = inv;
-            }
-        }
-        g_prog_done.store(f + 1);
-    }
-    g_prog_active.store(0);
-}
-
-// Numbers the distinct rows of cell offsets and of weights (eight each), in
-// order of first appearance; false when either kind has more than 65536.
-bool number_stencils(const std::vector<int>& neg, const std::vector<int>& sc, const std::vector<float>& sw,
-                     std::vector<unsigned>& row, std::vector<int>& off, std::vector<float>& wgt)
-{
+// The gradient-order-8 stencils as the faces' rows come in: distinct rows of cell
+// offsets and of weights (eight each) numbered in order of first appearance, or,
+// from the face on where either kind exceeds 65536, all rows slot by slot.  (As a
+// pass over full rows of every face, 64 bytes each, the numbering took 10 of 178 ms
+// of creating a 72^3 grid.)
+struct StencilRows {
     struct Table {   // open addressing over the rows seen so far
         std::vector<int> words, slot;
         size_t n = 0, mask = 0;
@@ -802,25 +760,95 @@ bool number_stencils(const std::vector<int>& neg, const std::vector<int>& sc, co
                 if (memcmp(&words[(size_t)slot[q] * kSW2], r, kSW2 * sizeof(int)) == 0) return slot[q];
             }
         }
-    } to, tw;
-    const size_t nf = neg.size();
-    row.resize(nf);
-    for (size_t f = 0; f < nf; ++f) {
+    } off, wgt;
+    const std::vector<int>& neg;
+    size_t nf;
+    std::vector<unsigned> row;   // offset row | weight row << 16; empty once the full form is taken
+    std::vector<int> cell;       // full form: [slot][face]
+    std::vector<int> coef;       // bits of the weights
+    explicit StencilRows(const std::vector<int>& face_neg) : neg(face_neg), nf(face_neg.size()), row(nf) {}
+
+    void put(size_t f, const int* c, const float* x)
+    {
         int o[kSW2], w[kSW2];
-        memcpy(w, &sw[f * kSW2], sizeof w);
-        for (int k = 0; k < kSW2; ++k)
-            o[k] = (sc[f * kSW2 + k] == 0 && w[k] == 0) ? kOrigin : sc[f * kSW2 + k] - neg[f];
-        const int a = to.number(o), b = tw.number(w);
-        if (a < 0 || b < 0) {
+        memcpy(w, x, sizeof w);
+        for (int k = 0; k < kSW2; ++k) o[k] = (c[k] == 0 && w[k] == 0) ? kOrigin : c[k] - neg[f];
+        if (cell.empty()) {
+            const int a = off.number(o), b = wgt.number(w);
+            if (a >= 0 && b >= 0) {
+                row[f] = (unsigned)a | (unsigned)b << 16;
+                return;
+            }
+            cell.resize(nf * kSW2);
+            coef.resize(nf * kSW2);
+            for (size_t g = 0; g < f; ++g) place(g, &off.words[(row[g] & 0xFFFFu) * kSW2], &wgt.words[(row[g] >> 16) * kSW2]);
             row.clear();
-            return false;
         }
-        row[f] = (unsigned)a | (unsigned)b << 16;
+        place(f, o, w);
     }
-    off = to.words;
-    wgt.resize(tw.words.size());
-    memcpy(wgt.data(), tw.words.data(), tw.words.size() * sizeof(int));
-    return true;
+    void place(size_t f, const int* o, const int* w)
+    {
+        for (int k = 0; k < kSW2; ++k) {
+            cell[k * nf + f] = o[k] == kOrigin ? 0 : neg[f] + o[k];
+            coef[k * nf + f] = w[k];
+        }
+    }
+};
+
+// Per face: with four cells on each side, Fornberg weights over all eight;
+// otherwise the two-cell difference (acoustic_amr.cpp:549-629).  Unused slots
+// keep cell 0 and weight 0.
+void build_stencil(AcousticAMRState* st, const Incidence& inc, StencilRows& rows)
+{
+    Topo t;
+    t.st = st;
+    t.inc = &inc;
+    build_axis_neighbours(t);
+    const int nf = st->n_faces;
+    g_prog_total.store(nf);
+    g_prog_done.store(0);
+    g_prog_active.store(1);
+    for (int f = 0; f < nf; ++f) {
+        const int cn = st->face_neg[f], cp = st->face_pos[f];
+        const float dxf = (float)(st->centers[3 * cp] - st->centers[3 * cn]);
+        const float dyf = (float)(st->centers[3 * cp + 1] - st->centers[3 * cn + 1]);
+        const float dzf = (float)(st->centers[3 * cp + 2] - st->centers[3 * cn + 2]);
+        const float len = std::sqrt(dxf * dxf + dyf * dyf + dzf * dzf);
+        int sc[kSW2] = {};
+        float sw[kSW2] = {};
+        if (len >= 1e-15f) {
+            const float dir[3] = {dxf / len, dyf / len, dzf / len};
+            const float back[3] = {-dir[0], -dir[1], -dir[2]};
+            const float fp = 0.5f * (proj(st, cn, dir) + proj(st, cp, dir));
+            int nc_[kSW], pc_[kSW];
+            float nx_[kSW], px_[kSW];
+            const int nn = walk_cells(t, cn, fp, dir, back, kSW, nc_, nx_);
+            const int np = walk_cells(t, cp, fp, dir, dir, kSW, pc_, px_);
+            if (nn == kSW && np == kSW) {
+                float xs[kSW2], w[kSW2];
+                for (int k = 0; k < kSW; ++k) {
+                    xs[k] = nx_[kSW - 1 - k];
+                    xs[kSW + k] = px_[k];
+                }
+                fornberg_first(xs, kSW2, 0.0f, w);
+                for (int k = 0; k < kSW; ++k) {
+                    sc[k] = nc_[k];          // walk order from the face outward
+                    sw[k] = w[kSW - 1 - k];
+                    sc[kSW + k] = pc_[k];
+                    sw[kSW + k] = w[kSW + k];
+                }
+            } else if (nn + np >= 2) {
+                const float inv = st->face_dist[f] > 0.0 ? 1.0f / (float)st->face_dist[f] : 0.0f;
+                sc[0] = cn;
+                sw[0] = -inv;
+                sc[kSW] = cp;
+                sw[kSW] = inv;
+            }
+        }
+        rows.put(f, sc, sw);
+        g_prog_done.store(f + 1);
+    }
+    g_prog_active.store(0);
 }
 
 void prof_mark(AcousticAMRState* st)
@@ -865,7 +893,8 @@ int launch_steps(AcousticAMRState* st, int n_steps)
         if (st->plate) pl = PlateDev{st->cur_w(), st->prev_w(), st->next_w(), st->d_ext, dt};
         prof_mark(st);
         const Stencils sten{st->d_srow, reinterpret_cast<const int4*>(st->d_soff),
-                            reinterpret_cast<const float4*>(st->d_swgt), st->d_scell, st->d_scoef};
+                            reinterpret_cast<const float4*>(st->d_swgt), st->d_scell,
+                            reinterpret_cast<const float*>(st->d_scoef)};
         const int* const bc = st->plate ? st->d_bc : nullptr;
         AK(launch_after(st->order == 8 ? k_amr_velocity<8> : k_amr_velocity<2>,
                         blocks(st->n_faces, st->order == 8 ? 256 : 1024), 256, 0, st->stream, st->n_faces,
@@ -996,66 +1025,42 @@ AcousticAMRState* amr_create(int n_cells, const double* cc, const double* cv, co
         for (int i = 0; i < n_cells; ++i) zero[i] = (ct[i] == 1 || ct[i] == 2) ? 1 : 0;
         for (int i : st->acoustic) open[i] = 1;
         // incident faces of each cell, in face order: +flux on the face's negative side, -flux on its positive side
-        st->csr_start.assign(n_cells + 1, 0);
+        Incidence inc;
+        inc.deg.assign(n_cells, 0);
+        inc.slice.resize((n_cells + 31) / 32);
         for (int f = 0; f < n_faces; ++f) {
-            st->csr_start[fn[f] + 1]++;
-            st->csr_start[fp[f] + 1]++;
+            ++inc.deg[fn[f]];
+            ++inc.deg[fp[f]];
         }
-        for (int i = 1; i <= n_cells; ++i) st->csr_start[i] += st->csr_start[i - 1];
-        st->csr_face.resize(st->csr_start[n_cells]);
-        st->csr_w.resize(st->csr_start[n_cells]);
-        {
-            std::vector<int> fill(n_cells, 0);
-            for (int f = 0; f < n_faces; ++f) {
-                const int ka = st->csr_start[fn[f]] + fill[fn[f]]++;
-                st->csr_face[ka] = f;
-                st->csr_w[ka] = +flux[f];
-                const int kb = st->csr_start[fp[f]] + fill[fp[f]]++;
-                st->csr_face[kb] = f;
-                st->csr_w[kb] = -flux[f];
-            }
-        }
-        // the same lists slot by slot per slice of 32 cells (k_amr_pressure)
-        std::vector<int> meta(n_cells), slice((n_cells + 31) / 32);
         size_t n_inc = 0;
-        for (size_t q = 0; q < slice.size(); ++q) {
-            int deg = 0;
-            for (int c = (int)(32 * q); c < std::min((int)(32 * q) + 32, n_cells); ++c) {
-                meta[c] = zero[c] ? -1 : st->csr_start[c + 1] - st->csr_start[c];
-                deg = std::max(deg, meta[c]);
-            }
-            slice[q] = (int)n_inc;
-            n_inc += 32 * (size_t)deg;
+        for (size_t q = 0; q < inc.slice.size(); ++q) {
+            const int *first = inc.deg.data() + 32 * q, *last = inc.deg.data() + std::min<size_t>(32 * q + 32, n_cells);
+            inc.slice[q] = (int)n_inc;
+            n_inc += 32 * (size_t)*std::max_element(first, last);
+            if (n_inc > INT_MAX) throw std::bad_alloc();
         }
-        if (n_inc > INT_MAX) throw std::bad_alloc();
-        std::vector<int2> inc(n_inc, make_int2(0, 0));
-        for (int c = 0; c < n_cells; ++c) {
-            int2* const e = inc.data() + slice[c >> 5] + (c & 31);
-            for (int k = 0; k < meta[c]; ++k) {
-                e[32 * k].x = st->csr_face[st->csr_start[c] + k];
-                memcpy(&e[32 * k].y, &st->csr_w[st->csr_start[c] + k], 4);
+        inc.e.reset(new int2[n_inc]);
+        std::vector<int> meta(n_cells, 0);   // faces placed so far, then what the kernel reads
+        for (int f = 0; f < n_faces; ++f) {
+            int2 v = make_int2(f, 0);
+            const float side[2] = {+flux[f], -flux[f]};
+            const int cell[2] = {fn[f], fp[f]};
+            for (int b = 0; b < 2; ++b) {
+                memcpy(&v.y, &side[b], 4);
+                inc.of(cell[b])[32 * meta[cell[b]]++] = v;
             }
         }
-        std::vector<int> scell, soff;
-        std::vector<float> scoef, swgt;
-        std::vector<unsigned> srow;
+        for (int i = 0; i < 32 * (int)inc.slice.size(); ++i) {   // unused slots
+            const int q = i >> 5, end = q + 1 < (int)inc.slice.size() ? inc.slice[q + 1] : (int)n_inc;
+            for (int k = i < n_cells ? meta[i] : 0; inc.slice[q] + 32 * k < end; ++k) inc.of(i)[32 * k] = make_int2(0, 0);
+        }
+        for (int i = 0; i < n_cells; ++i)
+            if (zero[i]) meta[i] = -1;
+        std::unique_ptr<StencilRows> rows;
         if (gradient_order == 8) {
             g_stage = "stencil.build";
-            build_stencil(st, scell, scoef);
-            if (number_stencils(st->face_neg, scell, scoef, srow, soff, swgt)) {
-                scell.clear();
-                scoef.clear();
-            } else {   // slot by slot
-                std::vector<int> tc(scell.size());
-                std::vector<float> tw(scoef.size());
-                for (size_t f = 0; f < (size_t)n_faces; ++f)
-                    for (int k = 0; k < kSW2; ++k) {
-                        tc[(size_t)k * n_faces + f] = scell[f * kSW2 + k];
-                        tw[(size_t)k * n_faces + f] = scoef[f * kSW2 + k];
-                    }
-                scell.swap(tc);
-                scoef.swap(tw);
-            }
+            rows.reset(new StencilRows(st->face_neg));
+            build_stencil(st, inc, *rows);
         }
         g_stage = "device";
         cudaError_t e = cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking);
@@ -1079,13 +1084,16 @@ AcousticAMRState* amr_create(int n_cells, const double* cc, const double* cv, co
         if (e == cudaSuccess) e = upload(&st->d_neg, st->face_neg.data(), nf, nf4);
         if (e == cudaSuccess) e = upload(&st->d_pos, st->face_pos.data(), nf, nf4);
         if (e == cudaSuccess) e = upload(&st->d_meta, meta);
-        if (e == cudaSuccess) e = upload(&st->d_slice, slice);
-        if (e == cudaSuccess) e = upload(&st->d_inc, inc);
-        if (e == cudaSuccess) e = upload(&st->d_scell, scell);
-        if (e == cudaSuccess) e = upload(&st->d_scoef, scoef);
-        if (e == cudaSuccess) e = upload(&st->d_srow, srow);
-        if (e == cudaSuccess) e = upload(&st->d_soff, soff);
-        if (e == cudaSuccess) e = upload(&st->d_swgt, swgt);
+        if (e == cudaSuccess) e = upload(&st->d_slice, inc.slice);
+        if (e == cudaSuccess) e = upload(&st->d_inc, inc.e.get(), n_inc, std::max<size_t>(n_inc, 1));
+        if (rows && rows->cell.empty()) {
+            if (e == cudaSuccess) e = upload(&st->d_srow, rows->row);
+            if (e == cudaSuccess) e = upload(&st->d_soff, rows->off.words);
+            if (e == cudaSuccess) e = upload(&st->d_swgt, rows->wgt.words);
+        } else if (rows) {
+            if (e == cudaSuccess) e = upload(&st->d_scell, rows->cell);
+            if (e == cudaSuccess) e = upload(&st->d_scoef, rows->coef);
+        }
         if (e == cudaSuccess) e = upload(&st->d_centers, st->centers.data(), st->centers.size(), st->centers.size());
         if (e == cudaSuccess) e = upload(&st->d_open, open);
         if (e == cudaSuccess) e = cudaMalloc(&st->d_best, kNearestBlocks * sizeof(double2));
