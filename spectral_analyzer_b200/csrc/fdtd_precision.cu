@@ -237,14 +237,15 @@ __global__ void k_src_rec(Field p, long long src, const double* sig, int step, i
     }
 }
 
-// A stored field decoded into the reference's compact layout (T: float holds every
-// mode's values but FP64's).
+// Cells q0 .. q0 + m - 1 of a stored field decoded into the reference's compact
+// layout (T: float holds every mode's values but FP64's).
 template <int M, class T>
-__global__ void __launch_bounds__(256) k_flat(Grid g, Field f, T* __restrict__ out)
+__global__ void __launch_bounds__(256) k_flat(Grid g, Field f, long long q0, int m, T* __restrict__ out)
 {
-    const long long q = blockIdx.x * 256LL + threadIdx.x, row = q / g.nz;   // one dimension: any extent of a room
-    if (row >= (long long)g.nx * g.ny) return;
-    out[q] = (T)ld<M>(f, row * g.sz + (q - row * g.nz));
+    const int t = blockIdx.x * 256 + threadIdx.x;   // one dimension: any extent of a room
+    if (t >= m) return;
+    const long long q = q0 + t, row = q / g.nz;
+    out[t] = (T)ld<M>(f, row * g.sz + (q - row * g.nz));
 }
 
 }  // namespace prec
@@ -286,7 +287,8 @@ struct FdtdB200Prec {
     double* d_rw = nullptr;
     double* d_trace = nullptr;
     int cap = 0, n_rec_steps = 0;
-    void* d_flat = nullptr;     // compact pressure for get_pressure
+    void* d_flat = nullptr;     // compact pressure for get_pressure: n_flat values at a time
+    size_t n_flat = 0;
     double* d_audit = nullptr;  // [cap_audit][2]
     std::vector<int> audit_steps;
     int cap_audit = 0;
@@ -721,23 +723,35 @@ int fdtd_b200_prec_get_pressure(FdtdB200Prec* p, double* out, int out_len)
     const Field& f = p->f[p->cur];
     const bool dbl = p->mode == kFP64;
     const size_t n = (size_t)p->N, vb = dbl ? 8 : 4;
-    if (!p->d_flat) {
-        PCK(cudaMalloc(&p->d_flat, n * vb));
+    if (!p->d_flat) {   // the whole field at once, or what the device has room for
+        cudaError_t e = cudaErrorMemoryAllocation;
+        for (size_t m = n; e == cudaErrorMemoryAllocation; m = (m + 1) / 2) {
+            e = cudaMalloc(&p->d_flat, m * vb);
+            p->n_flat = m;
+            if (m <= 1 << 16) break;
+        }
+        if (e != cudaSuccess) p->d_flat = nullptr;
+        PCK(e);
+        cudaGetLastError();   // of the larger tries
         p->allocs.push_back(p->d_flat);
     }
-    const unsigned block = 256, grid = (unsigned)((n + block - 1) / block);
-    switch (p->mode) {
-        case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
-        case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, (double*)p->d_flat); break;
-        case kBF16: k_flat<kBF16><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
-        case kFP16: k_flat<kFP16><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
-        case kBF16C: k_flat<kBF16C><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat); break;
-        default: k_flat<kFP16C><<<grid, block, 0, p->stream>>>(p->g, f, (float*)p->d_flat);
-    }
-    PCK(cudaGetLastError());
     unsigned char* const bytes = reinterpret_cast<unsigned char*>(out);
     unsigned char* const at = bytes + (dbl ? 0 : 4 * n);
-    PCK(cudaMemcpyAsync(at, p->d_flat, n * vb, cudaMemcpyDeviceToHost, p->stream));
+    for (size_t q = 0; q < n; q += p->n_flat) {
+        const int m = (int)std::min(p->n_flat, n - q);
+        const unsigned block = 256, grid = (m + block - 1) / block;
+        float* const x = (float*)p->d_flat;
+        switch (p->mode) {
+            case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
+            case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, q, m, (double*)p->d_flat); break;
+            case kBF16: k_flat<kBF16><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
+            case kFP16: k_flat<kFP16><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
+            case kBF16C: k_flat<kBF16C><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
+            default: k_flat<kFP16C><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x);
+        }
+        PCK(cudaGetLastError());
+        PCK(cudaMemcpyAsync(at + q * vb, p->d_flat, m * vb, cudaMemcpyDeviceToHost, p->stream));
+    }
     PCK(cudaStreamSynchronize(p->stream));
     if (!dbl) {
         constexpr size_t B = 2048;

@@ -64,3 +64,24 @@ def test_second_velocity_set_without_room(cuda, kernel):
     assert np.abs(y).max() > 0 and bits_equal(x, y), first_mismatch(x, y)
     for h in (a, b, warm):
         lib.fdtd_destroy(h)
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp16c", "fp64"])
+def test_pressure_is_read_in_parts_when_memory_is_short(cuda, mode):
+    from spectral_analyzer_b200.precision import PrecisionRoom
+    from spectral_analyzer_b200.rooms import seeded_room
+    room = seeded_room(250, 251, 253, 6, seed=2, n_rec=1, n_pml=4, source_kind="gaussian")
+    room.sigma_steps = 1.0
+    whole, parts = PrecisionRoom(room, mode), PrecisionRoom(room, mode)
+    for r in (whole, parts):
+        r.step(6)
+    ref = whole.pressure()                              # 15.9M values at once
+    whole.close()
+    cuda.cuda.empty_cache()
+    free = cuda.cuda.mem_get_info()[0]
+    rest = cuda.empty((free - (40 << 20) >> 21 << 21,), dtype=cuda.uint8, device="cuda")
+    got = parts.pressure()                              # in 40 MB
+    del rest
+    cuda.cuda.empty_cache()
+    parts.close()
+    assert np.abs(ref).max() > 0 and np.array_equal(got.view(np.uint64), ref.view(np.uint64))
