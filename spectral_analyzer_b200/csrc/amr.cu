@@ -8,16 +8,21 @@
  * face lists; graded absorbing borders; inverse-distance microphones.
  *
  * Device layout (HBM, structure of arrays, float32/int32):
- *   cells  p, P_damp, P_src_coeff, cell_inv_denom, zero flag (wall/plate),
- *          CSR of incident faces (starts, face index, signed flux weight);
- *   faces  v, V_damp, 1/distance, neg/pos cell, plate boundary code, and for
- *          gradient order 8 the 8-slot Fornberg stencil (cell, coefficient);
+ *   cells  p, P_damp, P_src_coeff, cell_inv_denom, the number of incident faces
+ *          (-1: wall or plate), and the faces with their signed flux weights, slot
+ *          by slot per slice of 32 cells (Incidence); for the nearest-cell search
+ *          the centres and an open flag;
+ *   faces  v, V_damp, 1/distance, neg/pos cell, plate boundary code, padded to a
+ *          multiple of four, and for gradient order 8 the numbers of the face's
+ *          rows of cell offsets and Fornberg weights (Stencils);
  *   plate  three displacement buffers rotated per step, external force,
  *          per-node CSR of the cells above and below.
- * One step = three kernels: k_amr_velocity (face gather; the plate's face
- * velocities are written in the same pass), k_amr_pressure (CSR divergence
- * and pressure update, wall/plate cells zeroed, divergence check fused),
- * k_amr_plate (Kirchhoff plate, force buffer cleared).  A diverged step
+ * One step = two kernels, and a third with a plate, each started while the one
+ * before drains (launch.h): k_amr_velocity (face gather, four faces a thread in
+ * order 2 and one in order 8; the plate's face velocities are written in the same
+ * pass), k_amr_pressure (divergence over the sliced lists and pressure update,
+ * wall/plate cells zeroed, divergence check fused), k_amr_plate (Kirchhoff plate,
+ * force buffer cleared).  A diverged step
  * latches its index in a status word; the later kernels of the window skip.
  *
  * Arithmetic is the reference's, operation for operation, with separately
@@ -343,9 +348,9 @@ __global__ void k_amr_plate(int n_nodes, const int* __restrict__ node_entry, con
 }
 
 // Adds `value` to the pressure of the acoustic cell nearest to (x, y, z): the
-// least squared distance, the lowest index among equals (cells that are not
-// Each block leaves its best; the
-// last one to finish picks among them and reports the cell (-1: none).
+// least squared distance, the lowest index among equals.  Cells whose open flag
+// is 0 are no candidates.  Each block leaves its best; the last one to finish picks
+// among them and reports the cell (-1: none).
 __global__ void __launch_bounds__(256) k_amr_add_nearest(int n_cells, const double* __restrict__ centers,
                                                          const unsigned char* __restrict__ open, double x, double y, double z, double2* __restrict__ best,
                                                          unsigned* __restrict__ done, float* __restrict__ p, float value,

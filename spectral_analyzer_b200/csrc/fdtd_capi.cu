@@ -1988,7 +1988,6 @@ void batch_drop_graph(FdtdB200Batch* b)
     b->graph_steps = 0;
 }
 
-// Pull the device step counters back into the member handles.
 // Planes of a member's work items when at most `most` are asked for: equal parts.
 int batch_item_planes(int nx, int most)
 {
@@ -2025,6 +2024,7 @@ double batch_makespan(AcousticFDTDState* const* members, int n, int shape, int m
     return load.rbegin()->first;
 }
 
+// Pull the device step counters back into the member handles.
 int batch_pull(FdtdB200Batch* b, int* steps_out, int* status_out)
 {
     const int n = (int)b->members.size();
