@@ -708,13 +708,14 @@ def amr_arm(args):
     nc, nf = s.n_cells, s.n_faces
     entries = 2 * nf
     # algorithmic bytes per step, every array element touched once per kernel:
-    # velocity: v in/out, V_damp, the gradient's operands (neg, pos, 1/d; or the
-    #           8-slot stencil's cells and weights) per face, p once per cell;
-    # pressure: p in/out, P_damp, P_src, 1/(V open), wall flag, CSR start per
-    #           cell, CSR face and weight per entry, v once per face
-    grad = (4 + 4 + 4) if args.amr_order == 2 else 8 * (4 + 4)
+    # velocity: v in/out, V_damp, the gradient's operands (neg, pos, 1/d; or neg and
+    #           the numbers of the stencil's rows, which stay in cache) per face, p
+    #           once per cell;
+    # pressure: p in/out, P_damp, P_src, 1/(V open), number of faces per cell, list
+    #           start per 32 cells, face and weight per entry, v once per face
+    grad = (4 + 4 + 4) if args.amr_order == 2 else 4 + 4
     face_b = nf * (4 + 4 + 4 + grad) + nf * 4
-    cell_b = nc * 4 + nc * (4 + 4 + 4 + 4 + 4 + 1 + 4) + entries * (4 + 4)
+    cell_b = nc * 4 + nc * (4 + 4 + 4 + 4 + 4 + 4) + nc // 8 + entries * (4 + 4)
     step_ms = ms / n
     peak, peak_kind = measured_peak()
     gbs = (face_b + cell_b) / (step_ms / 1e3) / 1e9

@@ -387,8 +387,9 @@ __device__ __forceinline__ void gradT4(const R* w, long long id, long long s, in
 // and the faces' E); C1: those that begin the step before it (U from Lp, z from
 // that step's states).  Both touch only a cell's own Lp, U and gradient, so
 // between two steps of a segment one pass does both: Lp stays in registers and
-// the gradient, 16 of a step's 152 bytes a cell, is read and written once
-// (128^3, a reverse step with its recompute: 73.6 us as three kernels, 60.5 now).
+// the gradient is read and written once, so that a step moves 128 bytes a cell
+// (cells 68, faces 60) in place of 152 (128^3, a reverse step with its recompute:
+// 73.6 us as three kernels, 60.5 now).
 template <class R, bool C2, bool C1>
 __global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? (C1 && C2 ? 6 : 5) : 2)
 k_adj_cells(Grid g, ACoef<R> cf, R* __restrict__ u, const R* __restrict__ w0, const R* __restrict__ w1,

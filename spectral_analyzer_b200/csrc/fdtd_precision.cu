@@ -240,12 +240,12 @@ __global__ void k_src_rec(Field p, long long src, const double* sig, int step, i
 // Cells q0 .. q0 + m - 1 of a stored field decoded into the reference's compact
 // layout (T: float holds every mode's values but FP64's).
 template <int M, class T>
-__global__ void __launch_bounds__(256) k_flat(Grid g, Field f, long long q0, int m, T* __restrict__ out)
+__global__ void __launch_bounds__(256) k_flat(Grid g, Field f, unsigned q0, int m, T* __restrict__ out)
 {
     const int t = blockIdx.x * 256 + threadIdx.x;   // one dimension: any extent of a room
     if (t >= m) return;
-    const long long q = q0 + t, row = q / g.nz;
-    out[t] = (T)ld<M>(f, row * g.sz + (q - row * g.nz));
+    const unsigned q = q0 + t, row = q / (unsigned)g.nz;
+    out[t] = (T)ld<M>(f, (long long)row * g.sz + (q - row * (unsigned)g.nz));
 }
 
 }  // namespace prec
@@ -742,12 +742,12 @@ int fdtd_b200_prec_get_pressure(FdtdB200Prec* p, double* out, int out_len)
         const unsigned block = 256, grid = (m + block - 1) / block;
         float* const x = (float*)p->d_flat;
         switch (p->mode) {
-            case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
-            case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, q, m, (double*)p->d_flat); break;
-            case kBF16: k_flat<kBF16><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
-            case kFP16: k_flat<kFP16><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
-            case kBF16C: k_flat<kBF16C><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x); break;
-            default: k_flat<kFP16C><<<grid, block, 0, p->stream>>>(p->g, f, q, m, x);
+            case kFP32: k_flat<kFP32><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, x); break;
+            case kFP64: k_flat<kFP64><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, (double*)p->d_flat); break;
+            case kBF16: k_flat<kBF16><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, x); break;
+            case kFP16: k_flat<kFP16><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, x); break;
+            case kBF16C: k_flat<kBF16C><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, x); break;
+            default: k_flat<kFP16C><<<grid, block, 0, p->stream>>>(p->g, f, (unsigned)q, m, x);
         }
         PCK(cudaGetLastError());
         PCK(cudaMemcpyAsync(at + q * vb, p->d_flat, m * vb, cudaMemcpyDeviceToHost, p->stream));
