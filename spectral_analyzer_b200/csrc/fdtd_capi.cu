@@ -688,6 +688,8 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
     if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0 && st->ps_done_step != st->step_count) {
         fuse_deposit = (fused || open2) && st->ps.n == 1 && st->ps.divisor == 0;
         if (!fuse_deposit) {
+            // the receivers hear the step before without this sample
+            if (int rc0 = flush_record(st)) return rc0;
             CK(launch_deposit(st->ps, st->d_ps_sig, st->step_count, 0.0f, st->P(), s));
             ++st->launches;
         }
