@@ -683,6 +683,9 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
     const bool open2 = open_two_pass(st), fused = !open2 && use_fused(st);
     if (!fused && !open2)
         if (int rc0 = flush_record(st)) return rc0;
+    // before the sample counts as deposited: a step without memory is taken again
+    if (fused && !st->v[st->cv ^ 1][0])
+        if (int rc0 = alloc_second_velocity_set(st)) return rc0;
     // point source: deposit s[n] before step n
     bool fuse_deposit = false;
     if (st->ps_n > 0 && st->step_count < st->ps_n && st->ps.n > 0 && st->ps_done_step != st->step_count) {
@@ -703,10 +706,6 @@ int one_step(AcousticFDTDState* st, bool sync_check, bool defer_record = false)
     int rc = prof_begin(st, &e1);
     if (rc) return rc;
     if (fused) {
-        if (!st->v[st->cv ^ 1][0]) {
-            int rc2 = alloc_second_velocity_set(st);
-            if (rc2) return rc2;
-        }
         if (!st->fcache) st->fcache = fused_cache_create();
         FusedArgs a{st->g, st->cf, st->tb, st->P(), st->Pn(),
                     {st->V(0), st->V(1), st->V(2)},

@@ -66,6 +66,34 @@ def test_second_velocity_set_without_room(cuda, kernel):
         lib.fdtd_destroy(h)
 
 
+def test_scheduled_source_without_room(cuda):
+    """The sample of a step that found no memory is deposited when the step is taken."""
+    from spectral_analyzer_b200 import _native
+    lib = _native.load()
+    dims = (256, 256, 256)
+    field = 4 * int(np.prod(dims))
+    a, b, warm = create(lib, dims), create(lib, dims), create(lib, (160, 128, 96))
+    signal = np.float32([1.0, 0.5, -0.25])
+    for h in (a, b):
+        assert lib.fdtd_b200_set_point_source(h, (dims[0] // 4) * 256 * 256 + 9000, ptr(signal, C.c_float), 3) == 0
+    lib.fdtd_b200_set_kernel(b, 1)
+    lib.fdtd_b200_set_kernel(warm, 3)
+    assert lib.fdtd_step(warm, 2) == 0
+    cuda.cuda.empty_cache()
+    free = cuda.cuda.mem_get_info()[0]
+    rest = cuda.empty((free - field - field // 2 >> 21 << 21,), dtype=cuda.uint8, device="cuda")
+    for _ in range(2):
+        assert lib.fdtd_step(a, 1) == _native.FDTD_ERR_CUDA
+    del rest
+    cuda.cuda.empty_cache()
+    for h in (a, b):
+        assert lib.fdtd_step(h, 5) == 0
+    x, y = pressure(lib, a, dims), pressure(lib, b, dims)
+    assert np.abs(y).max() > 0 and bits_equal(x, y), first_mismatch(x, y)
+    for h in (a, b, warm):
+        lib.fdtd_destroy(h)
+
+
 @pytest.mark.parametrize("mode", ["bf16", "fp16c", "fp64"])
 def test_pressure_is_read_in_parts_when_memory_is_short(cuda, mode):
     from spectral_analyzer_b200.precision import PrecisionRoom
