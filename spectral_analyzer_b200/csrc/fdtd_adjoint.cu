@@ -583,9 +583,16 @@ namespace {
 
 #define ACK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { record_cuda_error(e_, #x); return FDTD_ERR_CUDA; } } while (0)
 
+// Zeroed memory that the handle frees; *p stays null when there is none.
 int dalloc(FdtdB200Adj* h, void** p, size_t bytes)
 {
-    ACK(cudaMalloc(p, bytes));
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        record_cuda_error(e, "device memory of an adjoint handle");
+        cudaGetLastError();   // or the next launch would report it
+        return FDTD_ERR_CUDA;
+    }
     h->allocs.push_back(*p);
     ACK(cudaMemsetAsync(*p, 0, bytes, h->stream));
     return FDTD_OK;
@@ -634,22 +641,25 @@ int fwd_step(FdtdB200Adj* h, int n, void* p, void* const* vin, void* const* vout
     return FDTD_OK;
 }
 
+// Four fields in one allocation: P, then the three velocities.  All or, when
+// memory runs out, none.
+int alloc_state(FdtdB200Adj* h, int count, std::vector<void*>& P, std::vector<void*>& V)
+{
+    const size_t step = (field_bytes(h) + 255) & ~(size_t)255;
+    void* slab = nullptr;
+    if (int rc = dalloc(h, &slab, 4 * step * count)) return rc;
+    for (char* at = (char*)slab; count > 0; --count, at += 4 * step) {
+        P.push_back(at);
+        for (int c = 1; c <= 3; ++c) V.push_back(at + c * step);
+    }
+    return FDTD_OK;
+}
+
 int ensure_checkpoints(FdtdB200Adj* h, int n_steps)
 {
-    const size_t fb = field_bytes(h);
     const int n_ck = (n_steps + h->K - 1) / h->K;
-    while ((int)h->ckP.size() < n_ck) {
-        void* p = nullptr;
-        int rc = dalloc(h, &p, fb);
-        if (rc) return rc;
-        h->ckP.push_back(p);
-        for (int c = 0; c < 3; ++c) {
-            void* v = nullptr;
-            rc = dalloc(h, &v, fb);
-            if (rc) return rc;
-            h->ckV.push_back(v);
-        }
-    }
+    while ((int)h->ckP.size() < n_ck)
+        if (int rc = alloc_state(h, 1, h->ckP, h->ckV)) return rc;
     return FDTD_OK;
 }
 
@@ -741,34 +751,17 @@ int ensure_slots(FdtdB200Adj* h)
     // the states of a longest segment, in one allocation (128^3, 200 steps: the first
     // backward pass takes 25 ms, 300 to 380 with an allocation for each field)
     const int need = std::min(h->K, h->fwd_steps) + 1, have = (int)h->sP.size();
-    if (have < need) {
-        const size_t step = (fb + 255) & ~(size_t)255;
-        void* slab = nullptr;
-        if (int rc = dalloc(h, &slab, 4 * step * (need - have))) return rc;
-        char* at = (char*)slab;
-        for (int t = have; t < need; ++t) {
-            h->sP.push_back(at);
-            for (int c = 1; c <= 3; ++c) h->sV.push_back(at + c * step);
-            at += 4 * step;
-        }
-    }
-    if (!h->Lp) {
-        int rc = dalloc(h, &h->Lp, fb);
-        if (!rc) rc = dalloc(h, &h->U, fb);
-        for (int c = 0; c < 3 && !rc; ++c) rc = dalloc(h, &h->Lv[c], fb);
-        for (int c = 0; c < 3 && !rc; ++c) rc = dalloc(h, &h->E[c], fb);
-        if (!rc) {
-            void* gp = nullptr;
-            rc = dalloc(h, &gp, (size_t)h->g.cells * sizeof(double));
-            h->grad = (double*)gp;
-        }
-        if (!rc) {
-            void* gr = nullptr;
-            rc = dalloc(h, &gr, (size_t)h->N * sizeof(double));
-            h->grad_ref = (double*)gr;
-        }
-        if (rc) return rc;
-    }
+    if (have < need)
+        if (int rc = alloc_state(h, need - have, h->sP, h->sV)) return rc;
+    // each of the sweep's own fields that an earlier try found no memory for, too
+    void** const field[] = {&h->Lp, &h->U, &h->Lv[0], &h->Lv[1], &h->Lv[2], &h->E[0], &h->E[1], &h->E[2]};
+    for (void** p : field)
+        if (!*p)
+            if (int rc = dalloc(h, p, fb)) return rc;
+    if (!h->grad)
+        if (int rc = dalloc(h, (void**)&h->grad, (size_t)h->g.cells * sizeof(double))) return rc;
+    if (!h->grad_ref)
+        if (int rc = dalloc(h, (void**)&h->grad_ref, (size_t)h->N * sizeof(double))) return rc;
     return FDTD_OK;
 }
 
@@ -948,7 +941,8 @@ int fdtd_b200_adj_set_source(FdtdB200Adj* h, int cell, const double* signal, int
     drop_sweeps(h);
     dfree(h, h->sig);
     h->src = pad_index(h->g, cell);
-    h->n_sig = n;
+    h->n_sig = 0;
+    h->fwd_steps = -1;
     if (n > 0) {
         int rc = dalloc(h, &h->sig, (size_t)n * h->eb);
         if (rc) return rc;
@@ -960,7 +954,7 @@ int fdtd_b200_adj_set_source(FdtdB200Adj* h, int cell, const double* signal, int
         ACK(cudaMemcpyAsync(h->sig, buf.data(), buf.size(), cudaMemcpyHostToDevice, h->stream));
         ACK(cudaStreamSynchronize(h->stream));
     }
-    h->fwd_steps = -1;
+    h->n_sig = n;
     return FDTD_OK;
 }
 
@@ -997,8 +991,8 @@ int fdtd_b200_adj_set_receivers(FdtdB200Adj* h, int n_rec, const int* idx8, cons
     h->tap_start = nullptr;
     h->tap_ord = nullptr;
     h->n_tap_cells = 0;
-    h->n_rec = n_rec;
-    h->trace_cap = max_steps;
+    h->n_rec = h->trace_cap = 0;   // no forward runs until the new ones are complete
+    h->fwd_steps = -1;
     if (n_rec > 0) {
         void* p = nullptr;
         int rc = dalloc(h, &p, pi.size() * sizeof(long long));
@@ -1053,7 +1047,8 @@ int fdtd_b200_adj_set_receivers(FdtdB200Adj* h, int n_rec, const int* idx8, cons
         ACK(cudaMemcpyAsync(h->tap_ord, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         ACK(cudaStreamSynchronize(h->stream));
     }
-    h->fwd_steps = -1;
+    h->n_rec = n_rec;
+    h->trace_cap = max_steps;
     return FDTD_OK;
 }
 
