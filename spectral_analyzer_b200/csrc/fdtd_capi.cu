@@ -189,7 +189,8 @@ struct AcousticFDTDState {
     ResPlan res;
     void* res_x = nullptr;           // exchange buffer between bricks
     unsigned res_epoch = 0;          // steps taken through it
-    float* res_taps = nullptr;       // the receivers' taps of up to kCheckPeriod steps (behind it)
+    std::vector<float*> res_taps;    // the receivers' taps of up to kCheckPeriod steps: the last one is in use
+    size_t res_taps_n = 0;           // taps it holds
 
     long long launches = 0;          // kernels launched by this handle
 
@@ -821,9 +822,8 @@ int resident_window(AcousticFDTDState* st, int left)
     // bricks costs about what the march does (64^3: 15.5 against 15.3 us per call)
     const int m = std::min(left, kCheckPeriod - (st->step_count & (kCheckPeriod - 1)));
     if (m < 2) return 0;
-    if (!st->res_x) {   // both buffers once, in one allocation (at most 21 MB on 148 SMs), the taps' for the most receivers
-        const size_t xb = (st->res.xbytes + 255) & ~(size_t)255, tb = sizeof(float) * resident_max_taps() * kCheckPeriod;
-        if (cudaMalloc(&st->res_x, xb + tb) != cudaSuccess ||
+    if (!st->res_x) {
+        if (cudaMalloc(&st->res_x, st->res.xbytes) != cudaSuccess ||
             cudaMemsetAsync(st->res_x, 0, st->res.xbytes, st->stream) != cudaSuccess) {
             cudaGetLastError();
             cudaFree(st->res_x);
@@ -831,7 +831,21 @@ int resident_window(AcousticFDTDState* st, int left)
             st->res.ok = false;
             return 0;
         }
-        st->res_taps = reinterpret_cast<float*>(static_cast<char*>(st->res_x) + xb);
+    }
+    if (taps > st->res_taps_n) {
+        // At least twice the last one.  That one lives as long as the handle: queued
+        // launches may still write it, and to free it would wait for them.  All of a
+        // handle's are below 2 MB together.  (Room for the most receivers from the
+        // start, in the exchange buffer's allocation: the first call of a 109x87x61
+        // room took 2.4 ms in some runs and 4 to 8 in others, this way 2.4.)
+        const size_t n = std::max(taps, std::min(2 * st->res_taps_n, (size_t)resident_max_taps()));
+        float* buf = nullptr;
+        if (cudaMalloc(&buf, n * kCheckPeriod * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        st->res_taps.push_back(buf);
+        st->res_taps_n = n;
     }
     return m;
 }
@@ -870,8 +884,9 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check, int* taken)
         a.dep_k = (int)(c % st->g.sz);
     }
     const int rows = st->n_rec > 0 ? std::min(m, st->trace_cap - st->trace_len) : 0;
+    float* const taps = st->res_taps.empty() ? nullptr : st->res_taps.back();
     if (launch_resident(a, st->res, m, st->res_x, st->res_epoch, dep_from, dep_to, st->d_rec_idx,
-                        rows > 0 ? 8 * st->n_rec : 0, rows, st->res_taps, s) != cudaSuccess) {
+                        rows > 0 ? 8 * st->n_rec : 0, rows, taps, s) != cudaSuccess) {
         cudaGetLastError();   // an error of an earlier launch comes back from the next one
         st->res.ok = false;
         *taken = 0;
@@ -879,7 +894,7 @@ int resident_steps(AcousticFDTDState* st, int m, bool sync_check, int* taken)
     }
     ++st->launches;
     if (rows > 0) {
-        CK(launch_tap_rows(st->res_taps, st->d_rec_w, rows, st->n_rec, st->d_trace + (size_t)st->trace_len * st->n_rec, s));
+        CK(launch_tap_rows(taps, st->d_rec_w, rows, st->n_rec, st->d_trace + (size_t)st->trace_len * st->n_rec, s));
         ++st->launches;
         st->trace_len += rows;
     }
@@ -1074,6 +1089,7 @@ void free_state(AcousticFDTDState* st)
     for (cudaEvent_t e : st->prof.ev) cudaEventDestroy(e);
     fused_cache_destroy(st->fcache);
     cudaFree(st->res_x);
+    for (float* p : st->res_taps) cudaFree(p);
     if (st->own_stream) cudaStreamDestroy(st->own_stream);
     if (d >= 0 && d != st->device) cudaSetDevice(d);
     delete st;
