@@ -31,6 +31,7 @@ void set_err(cudaError_t e, const char* what)
 {
     std::lock_guard<std::mutex> lk(g_err_mu);
     snprintf(g_err, sizeof(g_err), "%s: %s (%d)", what, cudaGetErrorString(e), (int)e);
+    cudaGetLastError();   // or the next launch, of this handle or another, would report it again
 }
 
 }  // namespace

@@ -378,22 +378,27 @@ void record_now(FdtdB200Prec* p)
 
 // the second velocity set of the single-pass step, zeroed (faces it never
 // writes — the last face of each axis and the row padding — stay zero)
+// all of its arrays or, when memory runs out, none
 int ensure_v2(FdtdB200Prec* p)
 {
     if (p->v2[0].hi) return FDTD_OK;
     const size_t fb = (size_t)p->g.cells * elem_bytes(p->mode);
+    void* m[6] = {};
+    const int n = compensated(p->mode) ? 6 : 3;
+    cudaError_t e = cudaSuccess;
+    for (int q = 0; q < n && e == cudaSuccess; ++q) {
+        e = cudaMalloc(&m[q], fb);
+        if (e == cudaSuccess) e = cudaMemset(m[q], 0, fb);
+    }
+    if (e != cudaSuccess) {
+        for (void* q : m) cudaFree(q);
+        return fail(e, "second velocity set");
+    }
+    p->allocs.insert(p->allocs.end(), m, m + n);
     for (int q = 0; q < 3; ++q) {
-        Field& f = p->v2[q];
-        f = p->f[2 + q];
-        f.hi = f.lo = nullptr;
-        PCK(cudaMalloc(&f.hi, fb));
-        p->allocs.push_back(f.hi);
-        PCK(cudaMemset(f.hi, 0, fb));
-        if (compensated(p->mode)) {
-            PCK(cudaMalloc(&f.lo, fb));
-            p->allocs.push_back(f.lo);
-            PCK(cudaMemset(f.lo, 0, fb));
-        }
+        p->v2[q] = p->f[2 + q];
+        p->v2[q].hi = m[q];
+        p->v2[q].lo = m[3 + q];
     }
     return FDTD_OK;
 }
@@ -621,6 +626,7 @@ int fdtd_b200_prec_set_receivers(FdtdB200Prec* p, int n_rec, const int* idx8, co
                                  int capacity, int audit_capacity)
 {
     if (!p || (n_rec > 0 && (!idx8 || !wgt8))) return FDTD_ERR_NULL;
+    if (n_rec < 0) return FDTD_ERR_ARG;
     cudaSetDevice(p->device);
     std::vector<long long> pi((size_t)n_rec * 8);
     for (size_t q = 0; q < pi.size(); ++q) {
@@ -631,11 +637,9 @@ int fdtd_b200_prec_set_receivers(FdtdB200Prec* p, int n_rec, const int* idx8, co
     }
     cudaFree(p->d_ridx); cudaFree(p->d_rw); cudaFree(p->d_trace); cudaFree(p->d_audit);
     p->d_ridx = nullptr; p->d_rw = nullptr; p->d_trace = nullptr; p->d_audit = nullptr;
-    p->n_rec = n_rec;
-    p->cap = capacity;
+    p->n_rec = p->cap = p->cap_audit = 0;   // until their arrays are complete
     p->n_rec_steps = 0;
     p->audit_steps.clear();
-    p->cap_audit = audit_capacity;
     if (n_rec > 0) {
         PCK(cudaMalloc(&p->d_ridx, sizeof(long long) * pi.size()));
         PCK(cudaMalloc(&p->d_rw, sizeof(double) * pi.size()));
@@ -644,6 +648,9 @@ int fdtd_b200_prec_set_receivers(FdtdB200Prec* p, int n_rec, const int* idx8, co
         PCK(cudaMemcpy(p->d_rw, wgt8, sizeof(double) * pi.size(), cudaMemcpyHostToDevice));
     }
     if (audit_capacity > 0) PCK(cudaMalloc(&p->d_audit, sizeof(double) * 2 * audit_capacity));
+    p->n_rec = n_rec;
+    p->cap = capacity;
+    p->cap_audit = audit_capacity;
     return FDTD_OK;
 }
 

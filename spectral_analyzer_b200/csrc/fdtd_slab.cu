@@ -363,9 +363,7 @@ int fdtd_b200_slab_set_receivers(FdtdB200Slab* h, int n_rec, const int* idx8, co
     SCK(cudaSetDevice(h->device));
     cudaFree(h->d_ridx); cudaFree(h->d_rw); cudaFree(h->d_trace);
     h->d_ridx = nullptr; h->d_rw = nullptr; h->d_trace = nullptr;
-    h->n_rec = n_rec;
-    h->cap = capacity;
-    h->rows = 0;
+    h->n_rec = h->cap = h->rows = 0;   // until their arrays are complete
     if (n_rec > 0) {
         SCK(cudaMalloc(&h->d_ridx, sizeof(long long) * li.size()));
         SCK(cudaMalloc(&h->d_rw, sizeof(float) * li.size()));
@@ -373,6 +371,8 @@ int fdtd_b200_slab_set_receivers(FdtdB200Slab* h, int n_rec, const int* idx8, co
         SCK(cudaMemcpy(h->d_ridx, li.data(), sizeof(long long) * li.size(), cudaMemcpyHostToDevice));
         SCK(cudaMemcpy(h->d_rw, wgt8, sizeof(float) * li.size(), cudaMemcpyHostToDevice));
     }
+    h->n_rec = n_rec;
+    h->cap = capacity;
     return FDTD_OK;
 }
 
