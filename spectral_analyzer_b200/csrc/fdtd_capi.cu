@@ -2185,6 +2185,22 @@ int fdtd_b200_batch_set(FdtdB200Batch* b, AcousticFDTDState* const* members, con
         planes = seg[shape];
     }
     if (shape != b->set_shape) batch_drop_graph(b);   // it launches the other shape's kernel
+    // A set that fails part of the way leaves the batch without members: the device
+    // still describes the set before, whose rooms may be gone, and steps of an empty
+    // batch launch nothing.  The samples already deposited are in place.
+    struct Undo {
+        FdtdB200Batch* b;
+        ~Undo()
+        {
+            if (!b) return;
+            cudaStreamSynchronize(b->stream);
+            b->members.clear();
+            b->h.clear();
+            b->cur0.clear();
+            b->cv0.clear();
+            b->total_items = 0;
+        }
+    } undo{b};
     int tj, tk;
     b->set_shape = shape;
     b->grid_ctas = b->grid_ctas_shape[b->set_shape];
@@ -2274,6 +2290,7 @@ int fdtd_b200_batch_set(FdtdB200Batch* b, AcousticFDTDState* const* members, con
                        cudaMemcpyHostToDevice, b->stream));
     CK(cudaMemcpyAsync(b->d_hdr, &hh, sizeof(hh), cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));
+    undo.b = nullptr;
     return FDTD_OK;
 }
 

@@ -168,9 +168,10 @@ class EngineBatch:
         n = len(solvers)
         arr = (C.c_void_p * max(n, 1))(*[s._h.value for s in solvers])
         lim = np.ascontiguousarray(limits, dtype=np.int32)
-        self._check(self._lib.fdtd_b200_batch_set(self._h, C.cast(arr, C.POINTER(C.c_void_p)),
-                                                  lim.ctypes.data_as(C.POINTER(C.c_int)), n), "batch_set")
-        self.members = list(solvers)
+        rc = self._lib.fdtd_b200_batch_set(self._h, C.cast(arr, C.POINTER(C.c_void_p)),
+                                           lim.ctypes.data_as(C.POINTER(C.c_int)), n)
+        self.members = list(solvers) if rc == 0 else []   # a set that failed leaves the batch without members
+        self._check(rc, "batch_set")
 
     def step(self, n_steps: int, use_graph: bool = True):
         self._check(self._lib.fdtd_b200_batch_step(self._h, int(n_steps), 1 if use_graph else 0), "batch_step")

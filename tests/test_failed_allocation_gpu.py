@@ -100,3 +100,58 @@ def test_other_handles_step_after_a_room_that_did_not_fit(cuda):
     del rest
     cuda.cuda.empty_cache()
     assert np.abs(outs[0]).max() > 0 and bits_equal(*outs), first_mismatch(*outs)
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_batch_set_that_does_not_fit_leaves_no_members(cuda, graph):
+    """The set's first room is in order, its second finds no memory for its second
+    velocity set: the batch then steps nothing, and the first room goes on alone."""
+    from spectral_analyzer_b200 import _native
+    lib = _native.load()
+
+    def create(dims, kernel):
+        ct, pa = np.zeros(int(np.prod(dims)), np.uint8), np.zeros(dims[0] * dims[1], np.uint8)
+        u8 = C.POINTER(C.c_uint8)
+        h = C.c_void_p(lib.fdtd_create(*dims, 0.01, 343.0, 1.21, ct.ctypes.data_as(u8), -1, pa.ctypes.data_as(u8), 7.0,
+                                       0.45, 2.0, 1e-5, 4))
+        sig = np.float32([1.0, 0.5, 0.25, -1.0, 2.0, 0.125, 1.5, -0.5] * 5)
+        cell = dims[2] // 2 + dims[2] * (dims[1] // 2 + dims[1] * (dims[0] // 2))
+        assert h.value and lib.fdtd_b200_set_point_source(h, cell, sig.ctypes.data_as(_native.P_f32), sig.size) == 0
+        assert lib.fdtd_b200_set_kernel(h, kernel) == 0
+        return h
+
+    def pressure(h, dims):
+        out = np.empty(int(np.prod(dims)), np.float32)
+        assert lib.fdtd_get_pressure_field(h, out.ctypes.data_as(_native.P_f32), out.size) == 0
+        return out
+
+    small, large = (40, 36, 44), (256, 256, 256)
+    a, big, ref, ref_big = create(small, 3), create(large, 0), create(small, 1), create(large, 1)
+    b = C.c_void_p(lib.fdtd_b200_batch_create(0))
+    members = (C.c_void_p * 2)(a, big)
+    limits = np.int32([40, 8])
+    lim = limits.ctypes.data_as(C.POINTER(C.c_int))
+    assert lib.fdtd_step(a, 1) == 0                     # its second set is there
+    assert lib.fdtd_b200_batch_set(b, members, lim, 1) == 0 and lib.fdtd_b200_batch_step(b, 4, graph) == 0
+    rest = only(cuda, 4 * 256 ** 3 * 3 // 2)            # one field of three and a half
+    for _ in range(2):
+        assert lib.fdtd_b200_batch_set(b, members, lim, 2) == _native.FDTD_ERR_CUDA
+        assert "memory" in _native.last_error()
+        assert lib.fdtd_get_step_count(a) == 5
+        l0 = lib.fdtd_b200_batch_launch_count(b)
+        assert lib.fdtd_b200_batch_step(b, 4, graph) == 0 and lib.fdtd_b200_batch_launch_count(b) == l0
+        assert lib.fdtd_b200_batch_sync(b, None, None) == 0 and lib.fdtd_get_step_count(a) == 5
+    assert lib.fdtd_step(a, 4) == 0                     # alone, its next sample deposited once
+    del rest
+    cuda.cuda.empty_cache()
+    assert lib.fdtd_b200_batch_set(b, members, lim, 2) == 0
+    assert lib.fdtd_b200_batch_step(b, 40, graph) == 0 and lib.fdtd_b200_batch_sync(b, None, None) == 0
+    assert lib.fdtd_get_step_count(a) == 40 and lib.fdtd_get_step_count(big) == 8
+    assert lib.fdtd_b200_batch_set(b, None, None, 0) == 0
+    for h, g, dims, n in ((a, ref, small, 40), (big, ref_big, large, 8)):
+        assert lib.fdtd_step(g, n) == 0
+        x, y = pressure(h, dims), pressure(g, dims)
+        assert np.abs(y).max() > 0 and bits_equal(x, y), first_mismatch(x, y)
+    lib.fdtd_b200_batch_destroy(b)
+    for h in (a, big, ref, ref_big):
+        lib.fdtd_destroy(h)
