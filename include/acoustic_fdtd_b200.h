@@ -220,7 +220,8 @@ FDTD_B200_API void* fdtd_b200_get_stream(const AcousticFDTDState* st);
  * check; the first failure is latched and reported by fdtd_b200_synchronize.
  * A handle allocates the device buffers its steps work with on the first call
  * that needs them: the second velocity set, and for calls of several steps of a
- * small open room the exchange and tap buffers (at most 21 MB). */
+ * small open room the exchange and tap buffers (at most 21 MB), and a larger
+ * tap buffer when receivers grow (which does not wait for queued steps). */
 FDTD_B200_API int fdtd_b200_step_async(AcousticFDTDState* st, int n_steps);
 
 /* Waits for the handle's stream; returns FDTD_OK, FDTD_ERR_UNSTABLE (latched
@@ -320,7 +321,8 @@ FDTD_B200_API int fdtd_b200_sample_pressure_noalloc(const AcousticFDTDState* st,
 typedef struct FdtdB200Batch FdtdB200Batch;
 FDTD_B200_API FdtdB200Batch* fdtd_b200_batch_create(int device);
 FDTD_B200_API void fdtd_b200_batch_destroy(FdtdB200Batch* b);
-/* Replace the members; member q advances until its step count reaches limits[q]. */
+/* Replace the members; member q advances until its step count reaches limits[q].
+ * A set that fails leaves the batch without members. */
 FDTD_B200_API int fdtd_b200_batch_set(FdtdB200Batch* b, AcousticFDTDState* const* members,
                                       const int* limits, int n);
 /* Work-item tile: tile_k = 128 (8 rows x 128 columns) or 64 (16 rows x 64
